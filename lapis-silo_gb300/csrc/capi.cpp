@@ -565,7 +565,7 @@ struct ProgramCall {
    std::vector<const uint32_t*> sets;
 };
 
-ProgramCall plan_program(const RhyTable& table, const RhyOpProgram* prog, std::string* tree = nullptr) {
+ProgramCall plan_program(const RhyTable& table, const RhyOpProgram* prog, bool device, std::string* tree = nullptr) {
    need(prog, "program");
    if (prog->n_nodes) need(prog->nodes, "program nodes");
    if (prog->n_row_sets) need(prog->row_sets, "program row sets");
@@ -594,6 +594,7 @@ ProgramCall plan_program(const RhyTable& table, const RhyOpProgram* prog, std::s
    if (tree) *tree = op->to_string();
    rhygpu::LowerOptions o;
    o.rows = t.n_rows;
+   o.device = device;
    call.prog = rhygpu::lower(*op, rhygpu::rule_estimator(t), o);
    return call;
 }
@@ -618,7 +619,7 @@ int rhy_program_plan(const RhyTable* t, const RhyOpProgram* prog, char* tree_buf
    return guarded([&] {
       need(t, "table");
       std::string tree;
-      const ProgramCall c = plan_program(*t, prog, &tree);
+      const ProgramCall c = plan_program(*t, prog, false, &tree);
       if (tree_buf) {
          if (cap < tree.size() + 1) throw std::invalid_argument("buffer too small");
          std::memcpy(tree_buf, tree.c_str(), tree.size() + 1);
@@ -631,7 +632,7 @@ int rhy_program_plan(const RhyTable* t, const RhyOpProgram* prog, char* tree_buf
 int rhy_program_eval(RhyDevice* d, const RhyOpProgram* prog, void* stream, uint32_t* out_bits, uint64_t* out_count) {
    return guarded([&] {
       need(d, "device");
-      const ProgramCall c = plan_program(*d->table, prog);
+      const ProgramCall c = plan_program(*d->table, prog, true);
       d->engine->eval(c.prog, out_bits, out_count, static_cast<cudaStream_t>(stream), c.sets.data());
    });
 }
@@ -640,7 +641,7 @@ int rhy_program_count(RhyDevice* d, const RhyOpProgram* prog, void* stream, uint
    return guarded([&] {
       need(d, "device");
       need(out, "out");
-      const ProgramCall c = plan_program(*d->table, prog);
+      const ProgramCall c = plan_program(*d->table, prog, true);
       *out = d->engine->count(c.prog, static_cast<cudaStream_t>(stream), c.sets.data());
    });
 }
@@ -651,7 +652,7 @@ int rhy_program_mutations(RhyDevice* d, const RhyOpProgram* prog, uint32_t colum
       need(d, "device");
       need(counts, "counts");
       if (column >= d->table->image.seq.size()) throw std::invalid_argument("no such sequence column");
-      const ProgramCall c = plan_program(*d->table, prog);
+      const ProgramCall c = plan_program(*d->table, prog, true);
       d->engine->mutations(c.prog, static_cast<int>(column), counts, filter_count, static_cast<cudaStream_t>(stream),
                            c.sets.data());
    });

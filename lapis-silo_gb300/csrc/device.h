@@ -54,19 +54,40 @@ struct StreamRange {
 // CTAs of the container pass per SM (its shared-memory ring sets this); one range per CTA.
 constexpr uint32_t RING_CTAS_PER_SM = 3;
 
+// Filters read arrays of at least DENSE_MIN rows as bitsets: stored a second time as 8 KiB behind the
+// payload arena, under a second descriptor list (fctrs: the same containers, these as CT_BITSET). At
+// 1,024 rows a bitset costs four times the array's bytes and saves 1,024 shared-memory atomics and
+// two barriers per leaf; on the 2M-row table that is 150 extra bitsets per chunk of the nucleotide
+// column (37 MB). The Mutations passes read the arrays.
+constexpr uint32_t DENSE_MIN = 1024;
+struct DenseJob {
+   uint32_t src, dst, card;  // u16 offsets of the array and of its bitset in the arena
+};
+
+struct CovBound {
+   uint32_t row;   // row within chunk
+   uint32_t bound;
+};
+
 struct DevSeqCol {
    const CtrDesc* ctrs;
+   const CtrDesc* fctrs;       // the containers as filters read them (see DENSE_MIN)
    const uint16_t* payload;
    const uint32_t* off;        // nchunks * L + 1
-   const CovExc* exc;
-   const uint32_t* exc_off;    // nchunks + 1
-   const NRunEntry* nblk;
-   const uint32_t* nblk_off;   // nblocks * nchunks + 1
+   // Rows whose covered region starts late (bound = its start, descending) or ends early (bound = its
+   // end, ascending; rows without coverage: 0), per chunk; cov_rng[block * nchunks + chunk] = first
+   // late entry and their number with start > the block's first position, first early entry and their
+   // number with end <= its last one. A coverage leaf so reads only rows that miss its block.
+   const CovBound* cov_late;
+   const CovBound* cov_early;
+   const uint4* cov_rng;
+   // Missing intervals by (128-position block, chunk), sorted by row: row within the chunk | first
+   // position in the block << 16 | end << 24, each bucket from a multiple of 4 entries on (0 = none).
+   const uint32_t* nblk;
    const ArrUnit* au;          // array units of the Mutations container pass, chunk-major
    const OtherUnit* ou;        // its bitset and run units, chunk-major
    const StreamRange* ranges;  // its CTAs
-   const uint32_t* exc_toff;   // nchunks * TOFF_N: tile row-range offsets into exc
-   const uint32_t* nblk_toff;  // nblocks * nchunks * TOFF_N: the same into each nblk bucket
+   const uint32_t* nblk_toff;  // nblocks * nchunks * TOFF_N: tile row-range offsets into each nblk bucket
    const uint32_t* null_tiles; // nchunks * CHUNK_WORDS
    const uint8_t* local_ref;   // L
    const uint32_t* mstart;     // missing-interval start events (row << 8 | position in block)
@@ -96,23 +117,26 @@ struct EvItem {
 };
 
 struct DevDictCol {
-   const CtrDesc* ctrs;
+   const CtrDesc* fctrs;       // as filters read them (see DENSE_MIN)
    const uint16_t* payload;
    const uint32_t* off;        // nchunks * nkeys + 1
    uint32_t nkeys;
    uint32_t pad;
 };
 
-// Date column as a bit-sliced index: plane i holds bit i of (date - base) for every row (dense,
-// nchunks * CHUNK_WORDS words per plane), `nulls` the rows without a date. A range predicate then
-// reads nbits + 1 bits per row instead of a 32-bit value.
-constexpr uint32_t MAX_DATE_BITS = 32;
+// Date column as a range-encoded index: date - base is written in ndig digits of `width` bits, and
+// plane (i << width) + j holds the rows whose digit i is at most j (dense, nchunks * CHUNK_WORDS words
+// per plane; null dates in none). "date <= v" is then R[top][v_top - 1] | R[top][v_top] & (the same
+// over the lower digits): 2 ndig - 1 planes, so a DateBetween over three years (two digits, 82 planes)
+// reads 6 bits per row, where bit planes of the date took 12 and 20 operations per plane. Digits are at
+// most 7 bits wide: at most 128 planes each. The last plane holds every row with a date; `nulls` the others.
 struct DevDateCol {
-   const uint32_t* planes;     // nbits * nchunks * CHUNK_WORDS
+   const uint32_t* planes;
    const uint32_t* nulls;      // nchunks * CHUNK_WORDS
    int64_t base;               // smallest date
-   uint32_t nbits;             // 1..32
-   uint32_t pad;
+   uint32_t span;              // largest date - base
+   uint32_t ndig, width;       // digits (1..5) and their bits
+   uint32_t last;              // number of planes - 1
 };
 
 struct DevTable {
@@ -143,7 +167,7 @@ struct QueryDesc {
    uint32_t code_len;
    uint32_t out_tiles;    // 1 = write the row set to the query's output tiles
    uint32_t n_leaves;     // container leaves | coverage leaves << 16 (numbered 1.. in their c field)
-   uint32_t depth;        // stack tiles the program uses; the rest of the CTA's stack stages payloads
+   uint32_t depth;        // Program::tiles; the stack tiles it leaves free stage payloads
    uint32_t aux_base;     // its PUSH_AUX row sets are aux tiles aux_base + a
    uint32_t tile_bits;    // rows per work item of this query (its class's tile width)
 };
@@ -161,7 +185,7 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
                      uint32_t max_L, uint32_t* d_aux, void* stream);
 
 // ---- launchers (kernels.cu) ----
-// tile_bits: 4096, 8192, 16384, 32768 or 65536. stack_tiles: program depth. n_leaves: container
+// tile_bits: 4096, 8192, 16384, 32768 or 65536. stack_tiles: Program::tiles. n_leaves: container
 // leaves | coverage leaves << 16. d_trace (trace mode, optional): nchunks * (CHUNK_ROWS / tile_bits)
 // tiles x ncode x 2 u32 (cycles, result popcount per executed instruction), zeroed by the caller.
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
@@ -170,12 +194,19 @@ cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr
                           const uint32_t* d_aux = nullptr);
 
 // Batched: n_items work items over the programs in d_code; CTAs pull items from *d_next. Every
-// item uses its query's tile width (QueryDesc.tile_bits); stack_bytes of shared memory per CTA hold
-// the program stack of any of them (depth x tile bytes) and staged payloads in the rest.
-cudaError_t launch_filter_batch(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, const QueryDesc* d_queries,
-                         const WorkItem* d_items, uint32_t n_items, uint32_t stack_bytes,
+// item uses its query's tile width (QueryDesc.tile_bits); scratch_bytes of shared memory per CTA hold
+// the scratch tile of the widest, stack_bytes the program stack of any of them ((depth - 1) x tile
+// bytes) and staged payloads in the rest.
+cudaError_t launch_filter_batch(const DevTable* d_table, const Instr* d_code, const QueryDesc* d_queries,
+                         const WorkItem* d_items, uint32_t n_items, uint32_t scratch_bytes, uint32_t stack_bytes,
                          uint32_t* d_out_tiles /* per query nchunks*CHUNK_WORDS */, unsigned long long* d_counts,
                          uint32_t* d_next, uint32_t grid, int* d_err, void* stream, const uint32_t* d_aux = nullptr);
+
+// Builds the planes and nulls of a date column (days: INT32_MIN = null, n of them) with the digits given
+// in `col` (Engine's upload).
+cudaError_t launch_date_index(const int32_t* d_days, uint32_t n, uint32_t words, const DevDateCol& col, void* stream);
+// Writes the bitsets of the listed arrays (Engine's upload).
+cudaError_t launch_dense_forms(uint16_t* d_arena, const DenseJob* d_jobs, uint32_t n, void* stream);
 
 // Device error codes the kernels set in their error word: a bounded wait for bulk copies gave up
 // in a filter kernel (6) or in the Mutations container pass (7).

@@ -217,32 +217,109 @@ T* Engine::upload(const std::vector<T>& v, size_t min_elems) {
    return p;
 }
 
-// Bit-sliced date index: base = smallest date, nbits = bits of (largest - smallest), at least 1.
+// The payload arena with the dense forms behind it, and the descriptors that filters read.
+void Engine::upload_containers(const ContainerSet& cs, uint16_t*& payload, CtrDesc*& fctrs) {
+   std::vector<CtrDesc> f = cs.ctrs;
+   std::vector<DenseJob> jobs;
+   constexpr uint64_t BITSET = CHUNK_ROWS / 16;  // u16 per bitset
+   uint64_t end = (cs.payload.size() + 8 + 7) & ~7ull;
+   for (CtrDesc& d : f) {
+      if (d.type != CT_ARRAY || d.card_m1 + 1u < DENSE_MIN || end + BITSET > 0xFFFFFFFFull) continue;
+      jobs.push_back({d.payload, static_cast<uint32_t>(end), d.card_m1 + 1u});
+      d.type = CT_BITSET;
+      d.payload = static_cast<uint32_t>(end);
+      end += BITSET;
+   }
+   payload = static_cast<uint16_t*>(alloc(end * sizeof(uint16_t)));
+   if (!cs.payload.empty())
+      cuda_check(cudaMemcpy(payload, cs.payload.data(), cs.payload.size() * sizeof(uint16_t), cudaMemcpyHostToDevice), "upload");
+   fctrs = upload(f);
+   if (jobs.empty()) return;
+   DenseJob* d_jobs = nullptr;
+   cuda_check(cudaMalloc(&d_jobs, jobs.size() * sizeof(DenseJob)), "cudaMalloc");
+   cudaError_t e = cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(DenseJob), cudaMemcpyHostToDevice);
+   if (e == cudaSuccess) e = launch_dense_forms(payload, d_jobs, static_cast<uint32_t>(jobs.size()), stream_);
+   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+   cudaFree(d_jobs);
+   cuda_check(e, "dense forms");
+}
+
+// The lists of rows that a coverage leaf removes (see DevSeqCol).
+void Engine::upload_coverage(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d) {
+   std::vector<CovBound> late, early;
+   std::vector<uint4> rng(static_cast<size_t>(s.nblocks) * nchunks);
+   for (uint32_t v = 0; v < nchunks; ++v) {
+      const size_t l0 = late.size(), e0 = early.size();
+      for (uint32_t i = s.cov_exc_off[v]; i < s.cov_exc_off[v + 1]; ++i) {
+         const CovExc& x = s.cov_exc[i];
+         if (x.start >= x.end) {
+            early.push_back({x.row, 0});
+            continue;
+         }
+         if (x.start > 0) late.push_back({x.row, x.start});
+         if (x.end < s.L) early.push_back({x.row, x.end});
+      }
+      std::stable_sort(late.begin() + l0, late.end(), [](const CovBound& a, const CovBound& b) { return a.bound > b.bound; });
+      std::stable_sort(early.begin() + e0, early.end(), [](const CovBound& a, const CovBound& b) { return a.bound < b.bound; });
+      for (uint32_t b = 0; b < s.nblocks; ++b) {
+         const uint32_t first = b * NBLOCK, last = first + NBLOCK - 1;
+         const auto l = std::partition_point(late.begin() + l0, late.end(), [&](const CovBound& x) { return x.bound > first; });
+         const auto e = std::partition_point(early.begin() + e0, early.end(), [&](const CovBound& x) { return x.bound <= last; });
+         rng[static_cast<size_t>(b) * nchunks + v] =
+            make_uint4(static_cast<uint32_t>(l0), static_cast<uint32_t>(l - late.begin() - l0), static_cast<uint32_t>(e0),
+                       static_cast<uint32_t>(e - early.begin() - e0));
+      }
+   }
+   d.cov_late = upload(late, late.size() + 1);  // prefetches round the end up to 16 bytes
+   d.cov_early = upload(early, early.size() + 1);
+   d.cov_rng = upload(rng);
+}
+
+// The missing intervals as coverage leaves read them: 4 bytes each, buckets on 16-byte boundaries, and
+// the row-range offsets of the tiles in them.
+void Engine::upload_missing(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d) {
+   const size_t buckets = static_cast<size_t>(s.nblocks) * nchunks;
+   std::vector<uint32_t> ent, toff(buckets * TOFF_N);
+   ent.reserve(s.nblk.size() + 4 * buckets);
+   for (size_t b = 0; b < buckets; ++b) {
+      while (ent.size() % 4) ent.push_back(0);
+      const uint32_t first = static_cast<uint32_t>(ent.size());
+      for (uint32_t i = s.nblk_off[b]; i < s.nblk_off[b + 1]; ++i) {
+         const NRunEntry& x = s.nblk[i];
+         ent.push_back((x.row & 0xFFFFu) | static_cast<uint32_t>(x.lo) << 16 | static_cast<uint32_t>(x.hi) << 24);
+      }
+      for (uint32_t k = 0; k < TOFF_N; ++k) toff[b * TOFF_N + k] = first + (s.nblk_toff[b * TOFF_N + k] - s.nblk_off[b]);
+   }
+   d.nblk = upload(ent, ent.size() + 4);
+   d.nblk_toff = upload(toff);
+}
+
 void Engine::upload_dates(const DateColumnImage& dc, uint32_t nchunks, DevDateCol& out) {
    const size_t words = static_cast<size_t>(nchunks) * CHUNK_WORDS;
    int64_t lo = INT64_MAX, hi = INT64_MIN;
    for (int32_t d : dc.days)
       if (d != INT32_MIN) lo = std::min<int64_t>(lo, d), hi = std::max<int64_t>(hi, d);
    if (lo > hi) lo = hi = 0;
-   const uint64_t span = static_cast<uint64_t>(hi - lo);
-   uint32_t nbits = 1;
-   while (nbits < MAX_DATE_BITS && (span >> nbits) != 0) ++nbits;
-   std::vector<uint32_t> planes(static_cast<size_t>(nbits) * words, 0), nulls(words, 0);
-   for (size_t g = 0; g < dc.days.size() && g < words * 32; ++g) {
-      const int32_t d = dc.days[g];
-      if (d == INT32_MIN) {
-         nulls[g >> 5] |= 1u << (g & 31);
-         continue;
-      }
-      const uint64_t x = static_cast<uint64_t>(d - lo);
-      for (uint32_t i = 0; i < nbits; ++i)
-         if ((x >> i) & 1u) planes[i * words + (g >> 5)] |= 1u << (g & 31);
-   }
-   out.planes = upload(planes);
-   out.nulls = upload(nulls);
    out.base = lo;
-   out.nbits = nbits;
-   out.pad = 0;
+   out.span = static_cast<uint32_t>(hi - lo);
+   uint32_t nbits = 1;
+   while (nbits < 32 && (out.span >> nbits) != 0) ++nbits;
+   out.ndig = (nbits + 6) / 7;
+   out.width = (nbits + out.ndig - 1) / out.ndig;
+   const uint32_t top = out.width * (out.ndig - 1);
+   out.last = ((out.ndig - 1) << out.width) + (out.span >> top);
+   uint32_t* planes = static_cast<uint32_t*>(alloc((static_cast<size_t>(out.last) + 1) * words * 4));
+   uint32_t* nulls = static_cast<uint32_t*>(alloc(words * 4));
+   out.planes = planes;
+   out.nulls = nulls;
+   const uint32_t n = static_cast<uint32_t>(std::min(dc.days.size(), words * 32));
+   int32_t* days = nullptr;
+   cuda_check(cudaMalloc(&days, std::max<size_t>(n, 1) * sizeof(int32_t)), "cudaMalloc");
+   cudaError_t e = cudaMemcpy(days, dc.days.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice);
+   if (e == cudaSuccess) e = launch_date_index(days, n, static_cast<uint32_t>(words), out, stream_);
+   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+   cudaFree(days);
+   cuda_check(e, "date index");
 }
 
 Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), planner_(device) {
@@ -263,12 +340,14 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          const SeqColumnImage& s = t.seq[c];
          DevSeqCol& d = view_.seq[c];
          d.ctrs = upload(s.vertical.ctrs);
-         d.payload = upload(s.vertical.payload, 8);
+         uint16_t* payload = nullptr;
+         CtrDesc* fctrs = nullptr;
+         upload_containers(s.vertical, payload, fctrs);
+         d.payload = payload;
+         d.fctrs = fctrs;
          d.off = upload(s.vertical.off);
-         d.exc = upload(s.cov_exc);
-         d.exc_off = upload(s.cov_exc_off);
-         d.nblk = upload(s.nblk);
-         d.nblk_off = upload(s.nblk_off);
+         upload_coverage(s, nchunks, d);
+         upload_missing(s, nchunks, d);
          {
             const PassUnits P = pass_units(s, nchunks);
             d.au = upload(P.au);
@@ -282,8 +361,6 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
             d.ranges = upload(ranges);
             d.nranges = static_cast<uint32_t>(ranges.size());
          }
-         d.exc_toff = upload(s.exc_toff);
-         d.nblk_toff = upload(s.nblk_toff);
          std::vector<uint32_t> nulls(static_cast<size_t>(nchunks) * CHUNK_WORDS, 0);
          for (uint32_t g : s.null_rows) nulls[g >> 5] |= 1u << (g & 31);
          d.null_tiles = upload(nulls);
@@ -326,8 +403,11 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
       for (size_t c = 0; c < t.dict.size(); ++c) {
          const DictColumnImage& s = t.dict[c];
          DevDictCol& d = view_.dict[c];
-         d.ctrs = upload(s.inverted.ctrs);
-         d.payload = upload(s.inverted.payload, 8);
+         uint16_t* payload = nullptr;
+         CtrDesc* fctrs = nullptr;
+         upload_containers(s.inverted, payload, fctrs);
+         d.payload = payload;
+         d.fctrs = fctrs;
          d.off = upload(s.inverted.off);
          d.nkeys = s.inverted.nkeys;
          // for aggregation: every row's value id (from the inverted index) and the string order
@@ -461,10 +541,17 @@ uint64_t Engine::instr_bytes(const Instr& in) const {
       case OP_PUSH_COVERED: {
          const SeqColumnImage& c = table_.seq[in.col];
          const size_t blk = in.a / NBLOCK;
-         return c.cov_exc.size() * sizeof(CovExc) +
+         uint64_t bounds = 0;  // rows whose covered region misses the position
+         for (const CovExc& x : c.cov_exc) bounds += x.start > in.a || x.end <= in.a;
+         return bounds * sizeof(CovBound) +
                 static_cast<uint64_t>(c.nblk_off[(blk + 1) * nv] - c.nblk_off[blk * nv]) * sizeof(NRunEntry);
       }
-      case OP_PUSH_DATE: return static_cast<uint64_t>(view_.date[in.col].nbits + 1) * set_bytes;
+      case OP_PUSH_DATE: {  // the planes of its two comparisons (see DevDateCol), and the null dates where they match
+         const DevDateCol& c = view_.date[in.col];
+         const int64_t lo = static_cast<int32_t>(in.a) - c.base, hi = static_cast<int32_t>(in.b) - c.base;
+         const uint64_t per = 2 * c.ndig - 1;
+         return ((hi < static_cast<int64_t>(c.span) ? per : 1) + (lo > 0 ? per : 0) + (in.flags & 3)) * set_bytes;
+      }
       default: return 0;
    }
 }
@@ -484,6 +571,7 @@ uint64_t Engine::batch_filter_bytes(const BatchState& b) const {
 
 Program Engine::plan(const std::string& expr, const LowerOptions& opt, std::string* tree) const {
    LowerOptions o = opt;
+   o.device = true;
    if (o.rows <= 0) o.rows = table_.n_rows;  // early-exit tests where the estimates say they can fire
    return plan_filter(expr, table_, nullptr, o, tree);
 }
@@ -496,10 +584,7 @@ void Engine::upload_program(const Program& p, Instr* dst, cudaStream_t stream) {
 
 void Engine::launch_count(const Instr* code, const Program& p, unsigned long long* count, uint32_t* tiles,
                           cudaStream_t stream, const uint32_t* const* literals) {
-   uint32_t W = tile_bits;
-   // shared memory: keep the stack under 200 KiB
-   while (W > 4096 && static_cast<size_t>(p.max_depth) * (W / 8) > 200 * 1024) W >>= 1;
-   if (static_cast<size_t>(p.max_depth) * (W / 8) > 200 * 1024) throw IllegalQuery("filter expression nests too deeply");
+   const uint32_t W = fit_tile_bits(0, p);
    cudaGetLastError();  // an error left by an unrelated earlier call must not be reported here
    const uint32_t* aux = nullptr;
    if (p.n_literals > 0 && literals == nullptr) throw std::invalid_argument("the program reads caller row sets");
@@ -526,9 +611,9 @@ void Engine::launch_count(const Instr* code, const Program& p, unsigned long lon
    if (!p.aux.empty() || p.n_literals > 0) aux = d_aux_;
    const cudaError_t e = rhygpu::launch_filter(d_table_, nchunks(), code, static_cast<uint32_t>(p.code.size()),
                                                p.n_ctr_leaves | (p.n_cov_leaves << 16), W,
-                                               p.max_depth, tiles, count, d_err, stream, nullptr, aux);
+                                               p.tiles, tiles, count, d_err, stream, nullptr, aux);
    if (e != cudaSuccess)
-      throw CudaError("filter kernel launch (tile " + std::to_string(W) + " rows, stack " + std::to_string(p.max_depth) +
+      throw CudaError("filter kernel launch (tile " + std::to_string(W) + " rows, stack " + std::to_string(p.tiles) +
                       " tiles): " + cudaGetErrorString(e));
 }
 
@@ -617,10 +702,12 @@ void Engine::mutations(const Program& p, int column, uint32_t* host_counts, uint
 
 namespace rhygpu {
 
-uint32_t Engine::fit_tile_bits(uint32_t requested, uint32_t depth, bool batch) const {
+uint32_t Engine::fit_tile_bits(uint32_t requested, const Program& p, bool batch) const {
    uint32_t W = requested ? requested : batch ? batch_tile_bits : tile_bits;
-   while (W > 4096 && static_cast<size_t>(depth) * (W / 8) > 200 * 1024) W >>= 1;
-   if (static_cast<size_t>(depth) * (W / 8) > 200 * 1024) throw IllegalQuery("filter expression nests too deeply");
+   // shared memory: the program's tiles under 200 KiB; the depth limit of the narrowest tile is that
+   // of the whole stack
+   if (static_cast<size_t>(p.max_depth) * (4096 / 8) > 200 * 1024) throw IllegalQuery("filter expression nests too deeply");
+   while (W > 2048 && static_cast<size_t>(p.tiles) * (W / 8) > 200 * 1024) W >>= 1;
    return W;
 }
 
@@ -676,9 +763,11 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    const uint32_t n = static_cast<uint32_t>(qs.size());
    uint32_t depth = 1;
    size_t ncode = 0;
+   const Program* deepest = nullptr;
    for (const auto& q : qs) {
       if (q.prog.n_literals) throw std::invalid_argument("batched programs cannot read caller row sets");
       depth = std::max(depth, q.prog.max_depth);
+      if (!deepest || q.prog.tiles > deepest->tiles) deepest = &q.prog;
       ncode += q.prog.code.size();
       if (q.action == 1 && (q.column < 0 || static_cast<size_t>(q.column) >= table_.seq.size()))
          throw std::invalid_argument("no such sequence column");
@@ -686,19 +775,22 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    }
    // Filter classes: the stack of the deepest program sizes every CTA's shared memory, so programs
    // are grouped by tile width, chosen per program to keep the stack within the schedule's budget
-   // (40 KiB by default: with the leaf cache, four CTAs per SM) while the tile stays as wide as the
+   // (48 KiB by default: with the leaf cache and the scratch tile, three CTAs per SM) while the tile stays as wide as the
    // schedule allows; one persistent launch per class.
    const BatchSchedule& sch = batch_schedule;
-   auto class_w = [&](uint32_t d) {
-      if (requested_tile_bits) return fit_tile_bits(requested_tile_bits, depth, true);
+   auto class_w = [&](const Program& p) {
+      if (requested_tile_bits) {
+         fit_tile_bits(0, p, true);  // the program's own depth limit
+         return fit_tile_bits(requested_tile_bits, *deepest, true);
+      }
       uint32_t w = std::min(batch_tile_bits, std::max(sch.max_tile_bits, 4096u));
-      while (w > 16384 && static_cast<size_t>(d) * (w / 8) > static_cast<size_t>(sch.stack_kb) * 1024) w >>= 1;
-      return fit_tile_bits(w, d, true);
+      while (w > 16384 && static_cast<size_t>(p.tiles - 1) * (w / 8) > static_cast<size_t>(sch.stack_kb) * 1024) w >>= 1;
+      return fit_tile_bits(w, p, true);
    };
    std::map<uint32_t, std::vector<uint32_t>, std::greater<uint32_t>> by_w;
    std::vector<uint32_t> width(n);
    for (uint32_t i = 0; i < n; ++i) {
-      width[i] = class_w(qs[i].prog.max_depth);
+      width[i] = class_w(qs[i].prog);
       by_w[width[i]].push_back(i);
    }
    size_t nitems = 0;
@@ -809,7 +901,7 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
       std::memcpy(b.h_code + off, p.code.data(), p.code.size() * sizeof(Instr));
       b.h_q[i] = QueryDesc{static_cast<uint32_t>(off), static_cast<uint32_t>(p.code.size()),
                            b.slot_of_query[i] == UINT32_MAX ? 0u : b.slot_of_query[i] + 1,
-                           p.n_ctr_leaves | (p.n_cov_leaves << 16), std::max(p.max_depth, 1u),
+                           p.n_ctr_leaves | (p.n_cov_leaves << 16), p.tiles,
                            static_cast<uint32_t>(aux_off), width[i]};
       off += p.code.size();
       if (!p.aux.empty()) {
@@ -831,7 +923,7 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
       uint32_t gdepth = 1;
       for (uint32_t qi : qv) {
          costed |= qs[qi].cost > 0;
-         gdepth = std::max(gdepth, qs[qi].prog.max_depth);
+         gdepth = std::max(gdepth, qs[qi].prog.tiles);
       }
       if (costed)
          std::stable_sort(qv.begin(), qv.end(), [&](uint32_t x, uint32_t y) { return qs[x].cost > qs[y].cost; });
@@ -846,11 +938,15 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
       }
       b.fgroups.push_back(BatchState::FilterGroup{static_cast<uint32_t>(off), static_cast<uint32_t>(k - off), w, gdepth});
    }
-   size_t stack = 0;
-   for (const auto& g : b.fgroups) stack = std::max(stack, static_cast<size_t>(g.max_depth) * (g.tile_bits / 8));
-   uint32_t per_sm = static_cast<uint32_t>(filter_batch_blocks_per_sm(stack));
+   size_t stack = 0, scratch = 0;
+   for (const auto& g : b.fgroups) {
+      stack = std::max(stack, static_cast<size_t>(g.tiles - 1) * (g.tile_bits / 8));
+      scratch = std::max(scratch, static_cast<size_t>(g.tile_bits / 8));
+   }
+   uint32_t per_sm = static_cast<uint32_t>(filter_batch_blocks_per_sm(scratch, stack));
    if (sch.ctas_per_sm) per_sm = std::min(per_sm, sch.ctas_per_sm);
    b.stack_bytes = static_cast<uint32_t>(stack);
+   b.scratch_bytes = static_cast<uint32_t>(scratch);
    b.grid = static_cast<uint32_t>(props) * per_sm;
    std::memcpy(b.h_slot_query, slot_query.data(), slot_query.size() * sizeof(uint32_t));
    b.n_queries = n;
@@ -901,8 +997,8 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
       if (b.counts_words) cuda_check(cudaMemsetAsync(b.d_mcounts, 0, b.counts_words * 4, s), "memset");
       if (b.scratch_words) cuda_check(cudaMemsetAsync(b.d_mscratch, 0, b.scratch_words * 4, s), "memset");
       if (b.n_items)
-         cuda_check(launch_filter_batch(d_table_, nchunks(), b.d_code, b.d_q, b.d_items, b.n_items, b.stack_bytes, b.d_tiles,
-                                        b.d_counts, b.d_next, b.grid, b.d_err, s, b.n_aux ? b.d_aux : nullptr),
+         cuda_check(launch_filter_batch(d_table_, b.d_code, b.d_q, b.d_items, b.n_items, b.scratch_bytes, b.stack_bytes,
+                                        b.d_tiles, b.d_counts, b.d_next, b.grid, b.d_err, s, b.n_aux ? b.d_aux : nullptr),
                     "filter batch launch");
    }
    const size_t words = static_cast<size_t>(nchunks()) * CHUNK_WORDS;
@@ -1160,7 +1256,7 @@ std::vector<std::pair<BatchSchedule, double>> Engine::autotune_batch(const std::
    reps = std::max(1u, reps);
    std::vector<BatchSchedule> cands;
    for (uint32_t w : {16384u, 32768u, 65536u})
-      for (uint32_t kb : {24u, 40u, 64u})
+      for (uint32_t kb : {24u, 48u, 80u})
          for (uint32_t cps : {0u, 2u})
             for (uint32_t qm : {0u, 1u}) cands.push_back(BatchSchedule{w, kb, cps, qm});
    const BatchSchedule saved = batch_schedule;
@@ -1296,6 +1392,7 @@ size_t Engine::collect_traces(const std::vector<std::string>& exprs, std::vector
          LowerOptions o;
          o.early_exit = false;
          o.record_spans = true;
+         o.device = true;
          const Program p = lower(*op, ctx.rule, o);
          if (!p.aux.empty()) continue;  // MutationProfile row sets are not traced
          const uint32_t nc = static_cast<uint32_t>(p.code.size());
@@ -1309,10 +1406,10 @@ size_t Engine::collect_traces(const std::vector<std::string>& exprs, std::vector
          upload_program(p, d_code, s);
          cuda_check(cudaMemsetAsync(d_trace, 0, words * sizeof(uint32_t), s), "memset");
          cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s), "memset");
-         const uint32_t Wf = fit_tile_bits(W, p.max_depth);
+         const uint32_t Wf = fit_tile_bits(W, p);
          if (Wf != W) continue;  // too deep for the trace tile width: skip
          cudaGetLastError();
-         cuda_check(launch_filter(d_table_, nchunks(), d_code, nc, p.n_ctr_leaves | (p.n_cov_leaves << 16), W, p.max_depth,
+         cuda_check(launch_filter(d_table_, nchunks(), d_code, nc, p.n_ctr_leaves | (p.n_cov_leaves << 16), W, p.tiles,
                                   nullptr, d_count, d_err, s, d_trace),
                     "trace launch");
          trace.resize(words);
@@ -1377,6 +1474,7 @@ std::vector<BatchQuery> Engine::plan_batch(const std::vector<std::string>& exprs
       const Estimator est = rule_estimator(table_);
       LowerOptions lo;
       lo.rows = table_.n_rows;
+      lo.device = true;
       each([&](uint32_t i) { qs[i].prog = plan_filter(exprs[i], table_, &est, lo, nullptr); });
       batch_times.compile_ms += since(t0);
       return qs;
@@ -1478,6 +1576,7 @@ std::vector<BatchQuery> Engine::learned_lower(LearnedPlans& lp, const std::vecto
       };
       LowerOptions lo;
       lo.rows = table_.n_rows;
+      lo.device = true;
       qs[j].prog = lower(*lp.ops[i], learned, lo);
       qs[j].cost = lp.cost[i];
       lp.ops[i].reset();

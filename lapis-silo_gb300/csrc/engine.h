@@ -54,7 +54,7 @@ struct BatchQuery {
 // every tile of one query in turn). Results never depend on it.
 struct BatchSchedule {
    uint32_t max_tile_bits = 65536;
-   uint32_t stack_kb = 40;
+   uint32_t stack_kb = 48;
    uint32_t ctas_per_sm = 0;
    uint32_t query_major = 0;
 };
@@ -64,10 +64,10 @@ struct BatchState {
    // Classes of programs sharing a tile width (their work items are consecutive); one persistent
    // filter launch of `grid` CTAs with `stack_bytes` of stack takes the items of every class.
    struct FilterGroup {
-      uint32_t item_off, n_items, tile_bits, max_depth;
+      uint32_t item_off, n_items, tile_bits, tiles;
    };
    std::vector<FilterGroup> fgroups;
-   uint32_t stack_bytes = 0;
+   uint32_t stack_bytes = 0, scratch_bytes = 0;
    struct ColGroup {
       int column;
       uint32_t slot_begin, n;
@@ -162,7 +162,7 @@ class Engine {
    uint64_t sparse_rows_plain = 0, sparse_rows_batch = 0;
    BatchSchedule batch_schedule;  // used by batch_prepare unless a tile width is requested
    // Autotuner: prepares the batch under every candidate schedule (tile widths 16, 32 and 64 Kbit,
-   // stack budgets 24, 40 and 64 KiB, all or two CTAs per SM, both item orders), times its filter
+   // stack budgets 24, 48 and 80 KiB, all or two CTAs per SM, both item orders), times its filter
    // launches `reps` times with CUDA events on `stream` and keeps the fastest as batch_schedule.
    // Returns every candidate with its median milliseconds, the chosen one first. The caller holds mu.
    std::vector<std::pair<BatchSchedule, double>> autotune_batch(const std::vector<BatchQuery>& qs, cudaStream_t stream,
@@ -258,8 +258,8 @@ class Engine {
       double plan_ms = 0, prepare_ms = 0, device_ms = 0, output_ms = 0;
       double compile_ms = 0, predict_ms = 0, lower_ms = 0;
    } batch_times;
-   // Tile width that fits the batch's deepest program in the shared-memory budget.
-   uint32_t fit_tile_bits(uint32_t requested, uint32_t depth, bool batch = false) const;
+   // Tile width that fits the program's tiles in the shared-memory budget.
+   uint32_t fit_tile_bits(uint32_t requested, const Program& p, bool batch = false) const;
 
    // ---- learned planner ----
    // Runs every expression through the single-query path in trace mode (program lowered without
@@ -317,6 +317,9 @@ class Engine {
    template <typename T>
    T* upload(const std::vector<T>& v, size_t min_elems = 1);
    void* alloc(size_t bytes);
+   void upload_containers(const ContainerSet& cs, uint16_t*& payload, CtrDesc*& fctrs);
+   void upload_missing(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d);
+   void upload_coverage(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d);
    void upload_dates(const DateColumnImage& dc, uint32_t nchunks, DevDateCol& out);
 
    const TableImage& table_;
@@ -360,7 +363,7 @@ class Engine {
 
 };
 
-// Occupancy of the persistent filter kernel for a given shared-memory stack size.
-int filter_batch_blocks_per_sm(size_t smem_bytes);
+// Occupancy of the persistent filter kernel for given shared-memory scratch and stack sizes.
+int filter_batch_blocks_per_sm(size_t scratch_bytes, size_t stack_bytes);
 
 }  // namespace rhygpu

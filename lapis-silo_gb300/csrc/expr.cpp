@@ -1041,6 +1041,26 @@ struct Lowerer {
       return out;
    }
 
+   // An operator whose result the device has as a list of rows.
+   static bool row_list(const Op& o) {
+      if (o.t == OpT::INDEX_SCAN) return o.leaf.kind != Leaf::NULLS;
+      return o.t == OpT::SELECTION && o.children.empty() && o.preds.size() == 1 && o.preds[0].kind == Pred::COVERED &&
+             !o.preds[0].covered;
+   }
+   // Move the row lists to the front (returns their number, 0 when the code is not for the device) or
+   // to the end (returns the first one's index, the size when it is not): their order is free.
+   // Unions take them last, so that an operand that needs a stack of its own runs on an empty one.
+   size_t lists_first(std::vector<const Op*>& v) const {
+      if (!opt.device || opt.record_spans) return 0;
+      return static_cast<size_t>(
+         std::stable_partition(v.begin(), v.end(), [](const Op* o) { return row_list(*o); }) - v.begin());
+   }
+   size_t lists_last(std::vector<const Op*>& v) const {
+      if (!opt.device || opt.record_spans) return v.size();
+      return static_cast<size_t>(
+         std::stable_partition(v.begin(), v.end(), [](const Op* o) { return !row_list(*o); }) - v.begin());
+   }
+
    // A date comparison as "inside [lo, hi]" (or outside it) plus whether null dates match.
    struct DateLeaf {
       int col;
@@ -1129,6 +1149,7 @@ struct Lowerer {
          case OpT::INTERSECTION: {
             auto pos = order(op.children, true);
             auto neg = order(op.negated, false);
+            const size_t lists = lists_first(neg);  // one early-exit test for all of them
             std::vector<size_t> jumps;
             node(*pos[0]);
             double part = sel(*pos[0]);  // estimated selectivity of the partial result
@@ -1139,12 +1160,13 @@ struct Lowerer {
                pop();
                part *= sel(*pos[i]);
             }
-            for (const Op* c : neg) {
-               if (opt.early_exit && (opt.rows <= 0 || part <= opt.exit_sel)) jumps.push_back(jump(OP_JZ));
-               node(*c);
+            for (size_t i = 0; i < neg.size(); ++i) {
+               if (opt.early_exit && (opt.rows <= 0 || part <= opt.exit_sel) && (i == 0 || i >= lists))
+                  jumps.push_back(jump(OP_JZ));
+               node(*neg[i]);
                emit(OP_ANDNOT);
                pop();
-               part *= 1.0 - sel(*c);
+               part *= 1.0 - sel(*neg[i]);
             }
             patch(jumps);
             return;
@@ -1156,11 +1178,13 @@ struct Lowerer {
                return;
             }
             auto ch = order(op.children, false);
+            const size_t lists = lists_last(ch);  // one early-exit test for all of them
             std::vector<size_t> jumps;
             node(*ch[0]);
             double miss = 1.0 - sel(*ch[0]);  // estimated fraction of rows the partial union misses
             for (size_t i = 1; i < ch.size(); ++i) {
-               if (opt.early_exit && (opt.rows <= 0 || miss <= opt.exit_sel)) jumps.push_back(jump(OP_JFULL));
+               if (opt.early_exit && (opt.rows <= 0 || miss <= opt.exit_sel) && i <= lists)
+                  jumps.push_back(jump(OP_JFULL));
                node(*ch[i]);
                emit(OP_OR);
                pop();
@@ -1213,19 +1237,25 @@ struct Lowerer {
             uint32_t planes = 1;
             while ((1u << planes) - 1 < static_cast<uint32_t>(op.n) + 1) ++planes;
             if (planes > MAX_THR_PLANES) throw IllegalQuery("NOf threshold too large");
-            emit(OP_THR_BEGIN, 0, 0, planes);
+            const uint32_t P = opt.device ? threshold_planes(static_cast<uint32_t>(op.n), static_cast<uint32_t>(
+                                                                                             op.children.size() + op.negated.size()))
+                                          : planes;
+            emit(OP_THR_BEGIN, 0, 0, P);
             for (uint32_t i = 0; i < planes; ++i) push();
-            for (const auto& c : op.children) {
+            std::vector<const Op*> ch;
+            for (const auto& c : op.children) ch.push_back(c.get());
+            lists_first(ch);
+            for (const Op* c : ch) {
                node(*c);
-               emit(OP_THR_ADD, 0, 0, planes);
+               emit(OP_THR_ADD, 0, 0, P);
                pop();
             }
             for (const auto& c : op.negated) {
                node(*c);
-               emit(OP_THR_ADD, 0, 1, planes);
+               emit(OP_THR_ADD, 0, 1, P);
                pop();
             }
-            emit(OP_THR_END, 0, op.exact ? 1 : 0, planes, static_cast<uint32_t>(op.n));
+            emit(OP_THR_END, 0, op.exact ? 1 : 0, P, static_cast<uint32_t>(op.n));
             pop(planes);
             push();
             return;
@@ -1249,6 +1279,10 @@ struct Lowerer {
 
 }  // namespace
 
+namespace {
+constexpr size_t DEPTH_EXACT = 256;  // below this many pushed values no depth limit is in reach
+}
+
 Program lower(const Op& op, const Estimator& est, const LowerOptions& opt) {
    Lowerer l{est, opt, {}, 0};
    l.node(op);
@@ -1256,7 +1290,136 @@ Program lower(const Op& op, const Estimator& est, const LowerOptions& opt) {
    // caller row sets follow the MutationProfile row sets in the aux area
    for (Instr& in : l.prog.code)
       if (in.op == OP_PUSH_AUX && (in.flags & AUX_LITERAL)) in.a += static_cast<uint32_t>(l.prog.aux.size());
+   if (opt.device && !opt.record_spans) {
+      // the depth limit is that of the plain lowering, which pushes no more values than this
+      size_t pushes = 0;
+      for (const Instr& in : l.prog.code) pushes += in.op == OP_THR_BEGIN ? in.a + 1 : is_leaf(in.op) ? 1 : 0;
+      if (pushes > DEPTH_EXACT) {
+         LowerOptions plain = opt;
+         plain.device = false;
+         Lowerer d{est, plain, {}, 0};
+         d.node(op);
+         l.prog.max_depth = d.prog.max_depth;
+      }
+      fuse_leaves(l.prog.code);
+      group_leaves(l.prog.code);
+   }
+   l.prog.tiles = stack_tiles(l.prog.code);
    return std::move(l.prog);
+}
+
+void fuse_leaves(std::vector<Instr>& code) {
+   std::vector<uint32_t> at(code.size() + 1);  // new index of every instruction
+   std::vector<Instr> out;
+   out.reserve(code.size());
+   for (size_t i = 0; i < code.size(); ++i) {
+      at[i] = static_cast<uint32_t>(out.size());
+      Instr in = code[i];
+      if (is_leaf(in.op) && i + 1 < code.size()) {
+         const Instr& op = code[i + 1];
+         uint16_t f = 0;
+         if (op.op == OP_AND) f = fuse_flags(FUSE_AND, 0);
+         else if (op.op == OP_ANDNOT) f = fuse_flags(FUSE_ANDNOT, 0);
+         else if (op.op == OP_OR) f = fuse_flags(FUSE_OR, 0);
+         else if (op.op == OP_THR_ADD) f = fuse_flags(op.flags & 1 ? FUSE_THR_ADD_NOT : FUSE_THR_ADD, op.a);
+         if (f) {
+            in.flags = static_cast<uint16_t>(in.flags | f);
+            at[++i] = static_cast<uint32_t>(out.size());
+         }
+      }
+      out.push_back(in);
+   }
+   at[code.size()] = static_cast<uint32_t>(out.size());
+   for (Instr& in : out)
+      if (in.op == OP_JZ || in.op == OP_JFULL) in.a = at[in.a];
+   code.swap(out);
+}
+
+uint32_t threshold_planes(uint32_t n, uint32_t children) {
+   auto bits = [](uint32_t x) {
+      uint32_t b = 1;
+      while (b < 32 && (x >> b) != 0) ++b;
+      return b;
+   };
+   if (n > children) return bits(std::max(n, children));  // never reached: counts stay below n
+   return std::min(bits(children), bits(n) + 1);
+}
+
+void group_leaves(std::vector<Instr>& code) {
+   const size_t n = code.size();
+   std::vector<char> target(n + 1, 0);
+   for (const Instr& in : code)
+      if (in.op == OP_JZ || in.op == OP_JFULL) target[in.a] = 1;
+   auto list = [](const Instr& in) { return in.op == OP_PUSH_SCAN || in.op == OP_PUSH_DICT || in.op == OP_PUSH_COVERED; };
+   auto comp = [](const Instr& in) { return in.op == OP_PUSH_COVERED && !(in.flags & 1); };
+   // the row operation (and planes) of a fused row-list leaf, -1 if it has none
+   auto kind = [&](const Instr& in) -> int {
+      if (!list(in)) return -1;
+      const uint32_t f = leaf_fused(in.flags), P = leaf_planes(in.flags);
+      if (comp(in)) {
+         if (f == FUSE_AND) return A_ANDNOT;
+         return f == FUSE_THR_ADD_NOT ? static_cast<int>(A_ADD | (P << 4)) : -1;
+      }
+      if (f == FUSE_OR) return A_OR;
+      if (f == FUSE_ANDNOT) return A_ANDNOT;
+      return f == FUSE_THR_ADD ? static_cast<int>(A_ADD | (P << 4)) : -1;
+   };
+   std::vector<uint32_t> at(n + 1);
+   std::vector<Instr> out;
+   for (size_t i = 0; i < n;) {
+      at[i] = static_cast<uint32_t>(out.size());
+      int k = kind(code[i]);
+      bool push = false;
+      if (list(code[i]) && leaf_fused(code[i].flags) == FUSE_NONE) {  // a new tile that a run may extend
+         push = true;
+         k = comp(code[i]) ? A_ANDNOT : A_OR;
+      }
+      size_t e = i + 1;
+      if (k >= 0)
+         while (e < n && !target[e] && kind(code[e]) == k) ++e;
+      if (k < 0 || e - i < 2) {
+         out.push_back(code[i++]);
+         continue;
+      }
+      Instr g{OP_GROUP, 0, static_cast<uint16_t>((k & 15) | (push ? GROUP_PUSH : 0) | ((k >> 4) << 11)),
+              static_cast<uint32_t>(e - i), 0, 0};
+      std::vector<Instr> members(code.begin() + i, code.begin() + e);
+      std::stable_partition(members.begin(), members.end(), [](const Instr& in) { return in.op != OP_PUSH_COVERED; });
+      uint32_t mc = 0, mv = 0;
+      for (const Instr& in : members) {
+         uint32_t& f = in.op == OP_PUSH_COVERED ? g.c : g.b;
+         uint32_t& m = in.op == OP_PUSH_COVERED ? mv : mc;
+         if (m++ == 0) f = in.c;
+      }
+      g.b |= mc << 16;
+      g.c |= mv << 16;
+      out.push_back(g);
+      out.insert(out.end(), members.begin(), members.end());
+      i = e;  // no jump lands inside the run
+   }
+   at[n] = static_cast<uint32_t>(out.size());
+   for (Instr& in : out)
+      if (in.op == OP_JZ || in.op == OP_JFULL) in.a = at[in.a];
+   code.swap(out);
+}
+
+uint32_t stack_tiles(const std::vector<Instr>& code) {
+   uint32_t depth = 0, most = 0;  // a jump leaves the stack as the operands it skips do
+   for (size_t i = 0; i < code.size(); ++i) {
+      const Instr& in = code[i];
+      if (in.op == OP_GROUP) {
+         depth += in.flags & GROUP_PUSH ? 1 : 0;
+         i += in.a;
+         most = std::max(most, depth);
+         continue;
+      }
+      if (is_leaf(in.op)) depth += leaf_fused(in.flags) == FUSE_NONE ? 1 : 0;
+      else if (in.op == OP_AND || in.op == OP_ANDNOT || in.op == OP_OR || in.op == OP_THR_ADD) depth -= 1;
+      else if (in.op == OP_THR_BEGIN) depth += in.a;
+      else if (in.op == OP_THR_END) depth -= in.a - 1;
+      most = std::max(most, depth);
+   }
+   return most + 1;
 }
 
 OpPtr compile_filter(const std::string& text, const TableImage& t) {

@@ -147,7 +147,8 @@ struct NodeSpan {
 struct Program {
    std::vector<Instr> code;
    std::vector<NodeSpan> spans;  // with LowerOptions::record_spans; the ops belong to the caller's tree
-   uint32_t max_depth = 0;   // tiles of stack needed
+   uint32_t max_depth = 0;   // values on the stack at most (before leaves are fused)
+   uint32_t tiles = 2;       // tiles the device keeps: the deepest stack of the code as it is, and a scratch tile
    uint32_t n_leaves = 0;
    uint32_t n_ctr_leaves = 0;  // PUSH_SCAN / PUSH_DICT leaves, numbered 1.. in their c field
    uint32_t n_cov_leaves = 0;  // PUSH_COVERED leaves, numbered 1.. in their c field
@@ -167,12 +168,29 @@ struct LowerOptions {
    // elsewhere a tile practically never exits there and the test would cost a barrier for nothing.
    double rows = 0;
    double exit_sel = 0.01;
+   // For the device: counters with a sticky top plane (see threshold_planes) and, without spans, row
+   // lists next to each other, leaves fused with the operator that consumes them (fuse_leaves) and
+   // runs of row lists grouped (group_leaves). Program::max_depth does not depend on it.
+   bool device = false;
 };
 
 // parse -> rewrite(NONE) -> compile, without lowering.
 OpPtr compile_filter(const std::string& text, const TableImage& t);
 
 Program lower(const Op& op, const Estimator& est, const LowerOptions& opt);
+// Merges every leaf with the AND / ANDNOT / OR / THR_ADD that follows it and consumes its value
+// (program.h, FuseOp), and moves the jump targets along. A jump never lands between the two: it
+// lands after a whole operand.
+void fuse_leaves(std::vector<Instr>& code);
+// Puts an OP_GROUP before every run of at least two row-list leaves (containers, coverage) that are
+// applied to one target in the same way, and before the leaf whose new tile a run extends. Their order
+// does not matter, so the device applies them concurrently. No run contains a jump target.
+void group_leaves(std::vector<Instr>& code);
+// Planes of a device counter that compares the number of `children` holding a row with n: enough for
+// every possible count, or bits(n) and a sticky plane for counts of 2^bits(n) and more.
+uint32_t threshold_planes(uint32_t n, uint32_t children);
+// Program::tiles of a code.
+uint32_t stack_tiles(const std::vector<Instr>& code);
 
 // rewrite(NONE) -> compile -> lower (reference: src/rhydb/query_engine/operators/compute_filter.cpp:14-21).
 Program plan_filter(const std::string& text, const TableImage& t, const Estimator* est, const LowerOptions& opt,

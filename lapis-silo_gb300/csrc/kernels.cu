@@ -2,15 +2,24 @@
 // batch.cu, the output rows in rows.cu, Details in details.cu).
 //
 //  filter_kernel        one CTA per (chunk, tile of W rows): runs the postorder filter program over a
-//                       stack of W-bit tiles in shared memory; leaves expand array / bitset / run
-//                       containers straight into shared memory; writes the row-set tile and/or adds
+//                       stack of W-bit tiles in shared memory; writes the row-set tile and/or adds
 //                       its popcount (Count action, reference: copy_on_write_bitmap.cpp:108-118).
 //                       With a trace buffer it records every instruction's cycles and result size
 //                       (planner training).
 //  filter_batch_kernel  persistent variant: CTAs pull (query, tile) work items from a counter.
+//
+// What bounds them: issue slots and latency, not bytes (a container holds 36 rows on average, a tile is
+// 8 KiB). Hence a leaf followed by the operator that consumes it is one instruction (fuse_leaves),
+// whose rows go straight into the top tile or the counter planes; leaves whose order does not
+// matter are applied together, a warp each (group_leaves); arrays of DENSE_MIN rows and more are
+// stored a second time as bitsets, combined word by word by the threads that own the words.
+// Measured (2M rows, 4,096 trees of 1-64 leaves, one launch): 34.5 ms with a tile per leaf, 20.9 ms
+// this way; the benchmark's 2,048 queries 3.28 -> 3.05 ms. 128 threads per CTA instead of 256: 25.6
+// and 2.9 ms (the trees wait on latency, and more warps hide it).
 // All arithmetic is integer; results are bit-exact with the CPU operators.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -20,54 +29,13 @@ namespace rhygpu {
 
 namespace {
 
-constexpr uint32_t FT = 256;  // threads per filter CTA
+constexpr uint32_t FT = 256;  // threads per filter CTA (the single-query kernel takes fewer for narrow tiles)
 
 __device__ __forceinline__ uint32_t valid_word(uint32_t w, uint32_t nvalid) {
    const uint32_t b = w * 32;
    if (b + 32 <= nvalid) return 0xFFFFFFFFu;
    if (b >= nvalid) return 0u;
    return (1u << (nvalid - b)) - 1u;
-}
-
-// Sets bits [a, b) of a shared-memory tile.
-__device__ __forceinline__ void set_range(uint32_t* t, uint32_t a, uint32_t b) {
-   if (a >= b) return;
-   const uint32_t wa = a >> 5, wb = (b - 1) >> 5;
-   for (uint32_t w = wa; w <= wb; ++w) {
-      uint32_t m = 0xFFFFFFFFu;
-      if (w == wa) m &= 0xFFFFFFFFu << (a & 31);
-      if (w == wb) m &= 0xFFFFFFFFu >> (31 - ((b - 1) & 31));
-      atomicOr(&t[w], m);
-   }
-}
-
-// ORs the rows of one container that fall in [row0, row0 + W) into tile t.
-__device__ __forceinline__ void or_container(uint32_t* t, const CtrDesc& d, const uint16_t* __restrict__ payload,
-                                             uint32_t row0, uint32_t W) {
-   const uint16_t* p = payload + d.payload;
-   if (d.type == CT_ARRAY) {
-      const uint32_t card = d.card_m1 + 1u;
-      for (uint32_t i = threadIdx.x; i < card; i += blockDim.x) {
-         const uint32_t r = static_cast<uint32_t>(__ldg(p + i)) - row0;
-         if (r < W) atomicOr(&t[r >> 5], 1u << (r & 31));
-      }
-   } else if (d.type == CT_BITSET) {
-      const uint4* b = reinterpret_cast<const uint4*>(p) + (row0 >> 7);
-      for (uint32_t i = threadIdx.x; i < (W >> 7); i += blockDim.x) {
-         const uint4 x = __ldg(b + i);
-         if (x.x) atomicOr(&t[4 * i + 0], x.x);
-         if (x.y) atomicOr(&t[4 * i + 1], x.y);
-         if (x.z) atomicOr(&t[4 * i + 2], x.z);
-         if (x.w) atomicOr(&t[4 * i + 3], x.w);
-      }
-   } else {
-      for (uint32_t i = threadIdx.x; i < d.nruns; i += blockDim.x) {
-         const uint32_t s = __ldg(p + 2 * i);
-         const uint32_t e = s + __ldg(p + 2 * i + 1) + 1u;  // run covers [s, e)
-         const uint32_t a = max(s, row0), b = min(e, row0 + W);
-         if (a < b) set_range(t, a - row0, b - row0);
-      }
-   }
 }
 
 struct TileCtx {
@@ -79,49 +47,48 @@ struct TileCtx {
    const uint32_t* aux;  // the query's precomputed row sets (PUSH_AUX), nchunks * CHUNK_WORDS words each
 };
 
-// Per-item staging of the program's leaves for the chunk and row range of the current tile:
+// Per-item staging for the chunk and row range of the current tile:
+//  - the program's first LC_CODE instructions;
 //  - container leaves (PUSH_SCAN / PUSH_DICT, c = ordinal + 1): the slot offsets of all leaves are
-//    read in one round of loads and their descriptors in a second, so a leaf then costs one round
-//    trip (its payload) instead of three;
-//  - coverage leaves (PUSH_COVERED, c = ordinal + 1): the tile's ranges of coverage exceptions and
-//    missing intervals.
-// Array payloads of at most LC_SMALL rows are copied into shared memory by TMA bulk copies; every
-// other staged payload and range is handed to the TMA engine as a bulk L2 prefetch, so the leaves
-// find their data in L2 when the program reaches them.
+//    read in one round of loads and their descriptors in a second; every container whose symbol the
+//    leaf ORs becomes an entry, so a leaf costs no dependent loads when the program reaches it;
+//  - coverage leaves (PUSH_COVERED, c = ordinal + 1): the tile's ranges of uncovered rows and missing
+//    intervals.
+// Array payloads are copied into shared memory by TMA bulk copies while they fit; every other staged
+// payload and range is handed to the TMA engine as a bulk L2 prefetch.
 constexpr uint32_t LC_LEAVES = 128;
-constexpr uint32_t LC_DESCS = 256;
+constexpr uint32_t LC_ENTS = 256;
 constexpr uint32_t LC_COV = 64;
-constexpr uint32_t LC_NONE = 0xFFFFFFFFu;
-constexpr uint32_t LC_PAY = 2048;   // u16 of small-array payloads copied into shared memory per item
-constexpr uint32_t LC_SMALL = 64;   // arrays up to this cardinality are copied
-constexpr uint16_t LC_NOPAY = 0xFFFF;
+constexpr uint32_t LC_CODE = 128;
+constexpr uint16_t LC_NONE = 0xFFFF;
+constexpr uint32_t LC_PAY = 3072;      // u16 of array payloads copied into shared memory per item
 constexpr uint32_t LC_BIG = 0x80000000u;
-constexpr uint32_t LC_OWNER_MAX = 256;  // leaves of at most this many copied rows are set by their words' owners
+constexpr uint32_t LC_OWNER_MAX = 64;  // leaves of at most this many copied rows are set by their words' owners
+
+// A container of a staged leaf: y = kind << 28 | rows (runs for E_RUN), x = where its payload is.
+enum : uint32_t { E_COPIED = 0, E_ARRAY = 1, E_BITSET = 2, E_RUN = 3 };  // E_COPIED: x = byte offset in shared memory, else u16 offset in the arena
 
 struct LeafCache {
-   uint4 desc[LC_DESCS];
-   uint4 pay4[LC_PAY / 8];   // small-array payloads (TMA bulk copies, 16-byte aligned runs)
-   uint16_t poff[LC_DESCS];  // descriptor i's first element: u16 offset into pay4 (below LC_PAY), or
-                             // LC_PAY + offset into ext; LC_NOPAY when not copied
-   uint8_t dleaf[LC_DESCS];  // leaf (0-based) of staged descriptor i
-   uint32_t nstaged;         // staged descriptors: the staged leaves are a prefix of the leaves
-   uint32_t pay_used;        // u16 of pay4 reserved by this item's copies
-   uint16_t* ext;            // the stack tiles the item's program leaves free (16-byte aligned)
-   uint32_t ext_cap;         // their size in u16
-   uint32_t ext_used;        // u16 of ext reserved by this item's copies
-   uint64_t bar;             // completes the item's payload copies
-   const uint4* src[LC_LEAVES];
+   uint4 code[LC_CODE];
+   uint4 pay4[LC_PAY / 8];        // array payloads (TMA bulk copies, 16-byte aligned runs)
+   uint4 cov[LC_COV];             // a coverage leaf's late and early rows
+   uint2 covm[LC_COV];            // and its missing intervals
+   uint2 ent[LC_ENTS];            // leaf k's entries: arrays and runs from beg[k] up, bitsets from beg[k] + n[k] down
+   const uint4* src[LC_LEAVES];   // the leaf's descriptors
    const uint16_t* pay[LC_LEAVES];
-   uint32_t n[LC_LEAVES];
-   uint32_t symmask[LC_LEAVES];  // symbols the leaf ORs (every container for dictionary leaves)
-   uint32_t match[LC_LEAVES];    // staged leaves of at most 32 descriptors: bit i = descriptor i matches
-   uint32_t tot[LC_LEAVES];      // rows of the leaf's matching containers copied into shared memory;
-                                 // LC_BIG set when a matching container was not copied
-   uint32_t beg[LC_LEAVES];  // LC_NONE: not staged (the leaf reads its descriptors from global memory)
-   uint4 cov[LC_COV];        // exception range (x, y) and missing-interval range (z, w) of the tile
-   uint32_t nl;              // container leaves 1..nl are described by the table
-   uint32_t ncov;            // coverage leaves 1..ncov
+   uint32_t symmask[LC_LEAVES];   // symbols the leaf ORs (every container for dictionary leaves)
+   uint32_t cnt[LC_LEAVES];       // its array and run entries, bitset entries << 16
+   uint32_t tot[LC_LEAVES];       // rows of the leaf's copied arrays; LC_BIG: it has other arrays or runs
+   uint16_t n[LC_LEAVES];         // descriptors of the leaf's slot
+   uint16_t beg[LC_LEAVES];       // LC_NONE: not staged (the leaf reads its descriptors from global memory)
+   uint8_t dleaf[LC_ENTS];        // leaf (0-based) of staged descriptor i
+   uint64_t bar;                  // completes the item's payload copies
+   uint32_t nstaged;              // staged descriptors: the staged leaves are a prefix of the leaves
+   uint32_t pay_used;             // u16 of pay4 reserved by this item's copies
+   uint32_t ext_used;             // u16 of the program's free stack tiles reserved by this item's copies
+   uint32_t next_item;
 };
+static_assert(sizeof(LeafCache) % 16 == 0, "tiles follow the leaf cache");
 
 // Bulk prefetch of global bytes [a, b) into L2; a is rounded down and b up to 16 bytes, so the
 // caller guarantees the rounded range stays inside the allocation.
@@ -142,34 +109,19 @@ __device__ __forceinline__ void init_leaves(LeafCache& lc) {
    }
 }
 
-// Clears the leaf tables for nl container and ncov coverage leaves; a barrier must follow.
-__device__ __forceinline__ void clear_leaves(LeafCache& lc, uint32_t nl, uint32_t ncov, uint16_t* ext = nullptr,
-                                             uint32_t ext_cap = 0) {
-   if (threadIdx.x == 0) {
-      lc.nl = nl;
-      lc.ncov = ncov;
-      lc.pay_used = 0;
-      lc.ext = ext;
-      lc.ext_cap = ext ? ext_cap : 0u;
-      lc.ext_used = 0;
-   }
-   for (uint32_t k = threadIdx.x; k < nl; k += blockDim.x) {
-      lc.n[k] = 0;
-      lc.src[k] = nullptr;
-      lc.match[k] = 0;
-      lc.tot[k] = 0;
-   }
-   for (uint32_t k = threadIdx.x; k < ncov; k += blockDim.x) lc.cov[k] = make_uint4(0, 0, 0, 0);
-}
-
-// The tile's ranges in the coverage exceptions of chunk v and in the missing-interval bucket of
-// position pos (both lists are sorted by row; TOFF_ROWS divides every tile boundary).
-__device__ __forceinline__ uint4 cover_ranges(const DevTable* __restrict__ tab, const DevSeqCol* __restrict__ col,
-                                              uint32_t v, uint32_t row0, uint32_t W, uint32_t pos) {
-   const uint32_t k0 = row0 / TOFF_ROWS, k1 = (row0 + W) / TOFF_ROWS;
-   const uint32_t* xo = col->exc_toff + static_cast<size_t>(v) * TOFF_N;
-   const uint32_t* no = col->nblk_toff + (static_cast<size_t>(pos / NBLOCK) * tab->nchunks + v) * TOFF_N;
-   return make_uint4(__ldg(xo + k0), __ldg(xo + k1), __ldg(no + k0), __ldg(no + k1));
+// What a coverage leaf at pos reads for the tile: rng = its late and early rows of the chunk
+// (DevSeqCol::cov_rng), miss = its range in the missing-interval bucket of pos (sorted by row;
+// TOFF_ROWS divides every tile boundary or is divided by it).
+struct CoverRange {
+   uint4 rng;
+   uint2 miss;
+};
+__device__ __forceinline__ CoverRange cover_ranges(const DevTable* __restrict__ tab, const DevSeqCol* __restrict__ col,
+                                                   uint32_t v, uint32_t row0, uint32_t W, uint32_t pos) {
+   const uint32_t k0 = row0 / TOFF_ROWS, k1 = (row0 + W + TOFF_ROWS - 1) / TOFF_ROWS;
+   const size_t b = static_cast<size_t>(pos / NBLOCK) * tab->nchunks + v;
+   const uint32_t* no = col->nblk_toff + b * TOFF_N;
+   return CoverRange{__ldg(col->cov_rng + b), make_uint2(__ldg(no + k0), __ldg(no + k1))};
 }
 
 // Testing the failure path of the bounded waits: while set (on the current device), the threads that
@@ -185,6 +137,7 @@ __device__ uint32_t g_withhold_leaf_copies = 0;
 __device__ __forceinline__ bool wait_copies(LeafCache& lc, uint32_t parity, uint64_t limit_ns) {
    const uint32_t b = static_cast<uint32_t>(__cvta_generic_to_shared(&lc.bar));
    uint64_t t0 = 0;
+#pragma unroll 1
    for (uint32_t i = 0; i < (1u << 26); ++i) {
       uint32_t done;
       asm volatile(
@@ -201,29 +154,35 @@ __device__ __forceinline__ bool wait_copies(LeafCache& lc, uint32_t parity, uint
    return false;
 }
 
-// Stages the item's leaves (see LeafCache). Array containers of at most LC_SMALL rows are also
-// copied into shared memory by TMA bulk copies: each issuing thread announces its bytes on the
-// barrier (expect_tx) before starting its copy, and one thread arrives after every announcement,
-// so the phase completes when the last copy lands. `phase` is the parity of this item's wait,
-// flipped when copies were made. Returns false (error flag set) if the copies did not land.
+// Stages the item's instructions and leaves (see LeafCache). Array containers are also copied into
+// shared memory by TMA bulk copies, into pay4 or into the ext_cap u16 at ext (the stack tiles the
+// item's program leaves free): each issuing thread announces its bytes on the barrier (expect_tx)
+// before starting its copy, and one thread arrives after every announcement, so the phase completes
+// when the last copy lands. `phase` is the parity of this item's wait, flipped when copies were
+// made. With next_item, thread 0 claims the CTA's next work item into lc.next_item while the copies
+// are in flight. Returns false (error flag set) if the copies did not land. The caller has reset
+// pay_used and ext_used and passed a barrier since the previous item.
 __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __restrict__ code, uint32_t ncode,
-                             uint32_t& phase, int* err) {
+                             uint32_t nl, uint32_t ncov, uint16_t* ext, uint32_t ext_cap, uint32_t& phase,
+                             uint32_t* next_item, int* err) {
    const DevTable* __restrict__ tab = c.tab;
-   const uint32_t nl = lc.nl, ncov = lc.ncov;
    const bool withhold = *static_cast<volatile uint32_t*>(&g_withhold_leaf_copies) != 0;
-   // this thread's earlier shared-memory accesses (stack tiles, staged payloads of the previous
-   // item) are ordered before the bulk copies into the same memory issued after the next barrier
-   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < LC_ENTS; i += blockDim.x) lc.ent[i] = make_uint2(0, 0);  // E_COPIED, no rows
+#pragma unroll 1
    for (uint32_t i = threadIdx.x; i < ncode; i += blockDim.x) {
       const uint4 raw = __ldg(reinterpret_cast<const uint4*>(code) + i);
+      if (i < LC_CODE) lc.code[i] = raw;
       const Instr in = *reinterpret_cast<const Instr*>(&raw);
       if (in.op == OP_PUSH_COVERED) {
          if (in.c == 0 || in.c > ncov) continue;
          const DevSeqCol* col = &tab->seq[in.col];
-         const uint4 r = cover_ranges(tab, col, c.v, c.row0, c.W, in.a);
-         lc.cov[in.c - 1] = r;
-         prefetch_l2(col->exc + r.x, col->exc + r.y);
-         prefetch_l2(col->nblk + r.z, col->nblk + (r.w & ~1u));  // stays inside the 8-byte-entry array
+         const CoverRange r = cover_ranges(tab, col, c.v, c.row0, c.W, in.a);
+         lc.cov[in.c - 1] = r.rng;
+         lc.covm[in.c - 1] = r.miss;
+         prefetch_l2(col->cov_late + r.rng.x, col->cov_late + r.rng.x + r.rng.y);
+         prefetch_l2(col->cov_early + r.rng.z, col->cov_early + r.rng.z + r.rng.w);
+         prefetch_l2(col->nblk + r.miss.x, col->nblk + r.miss.y);
          continue;
       }
       if ((in.op != OP_PUSH_SCAN && in.op != OP_PUSH_DICT) || in.c == 0 || in.c > nl) continue;
@@ -233,27 +192,30 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
       size_t slot;
       if (in.op == OP_PUSH_SCAN) {
          const DevSeqCol* col = &tab->seq[in.col];
-         ctrs = col->ctrs;
+         ctrs = col->fctrs;
          off = col->off;
          payload = col->payload;
          slot = static_cast<size_t>(c.v) * col->L + in.a;
       } else {
          const DevDictCol* col = &tab->dict[in.col];
-         ctrs = col->ctrs;
+         ctrs = col->fctrs;
          off = col->off;
          payload = col->payload;
          slot = static_cast<size_t>(c.v) * col->nkeys + in.a;
       }
-      const uint32_t b = __ldg(off + slot), e = __ldg(off + slot + 1);
-      lc.src[in.c - 1] = reinterpret_cast<const uint4*>(ctrs) + b;
-      lc.pay[in.c - 1] = payload;
-      lc.n[in.c - 1] = e - b;
-      lc.symmask[in.c - 1] = in.op == OP_PUSH_SCAN ? in.b : 0xFFFFFFFFu;
+      const uint32_t b = __ldg(off + slot), e = __ldg(off + slot + 1), k = in.c - 1;
+      lc.src[k] = reinterpret_cast<const uint4*>(ctrs) + b;
+      lc.pay[k] = payload;
+      lc.n[k] = static_cast<uint16_t>(e - b);
+      lc.symmask[k] = in.op == OP_PUSH_SCAN ? in.b : 0xFFFFFFFFu;
+      lc.cnt[k] = 0;
+      lc.tot[k] = 0;
    }
    __syncthreads();
    if (threadIdx.x < 32) {  // exclusive scan of the counts; leaves that do not fit stay unstaged
       const uint32_t lane = threadIdx.x;
       uint32_t carry = 0, staged = 0;
+#pragma unroll 1
       for (uint32_t k0 = 0; k0 < nl; k0 += 32) {
          const uint32_t k = k0 + lane;
          const uint32_t x = k < nl ? lc.n[k] : 0u;
@@ -264,9 +226,10 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
             if (lane >= o) incl += y;
          }
          const uint32_t ex = carry + incl - x;
-         const bool fits = x > 0 && ex + x <= LC_DESCS;  // the leaves that fit are a prefix of them
-         if (k < nl) lc.beg[k] = fits ? ex : LC_NONE;
+         const bool fits = ex + x <= LC_ENTS;  // the leaves that fit are a prefix of them
+         if (k < nl) lc.beg[k] = fits ? static_cast<uint16_t>(ex) : LC_NONE;
          if (fits) {
+#pragma unroll 1
             for (uint32_t i = 0; i < x; ++i) lc.dleaf[ex + i] = static_cast<uint8_t>(k);
          }
          staged = max(staged, __reduce_max_sync(0xFFFFFFFFu, fits ? ex + x : 0u));
@@ -277,38 +240,35 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
    __syncthreads();
    // one staged descriptor per thread: its load, and the copy or prefetch of its payload
    const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(&lc.bar));
+   const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(&lc));
+#pragma unroll 1
    for (uint32_t j = threadIdx.x; j < lc.nstaged; j += blockDim.x) {
       const uint32_t k = lc.dleaf[j];
       const uint4 raw = __ldg(lc.src[k] + (j - lc.beg[k]));
-      lc.desc[j] = raw;
-      lc.poff[j] = LC_NOPAY;
       const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
-      if (!((lc.symmask[k] >> d.sym) & 1u)) continue;  // a symbol the leaf does not OR: no payload
-      if (lc.n[k] <= 32) atomicOr(&lc.match[k], 1u << (j - lc.beg[k]));
+      if (!((lc.symmask[k] >> d.sym) & 1u)) continue;  // a symbol the leaf does not OR
+      const uint32_t card = d.card_m1 + 1u;
+      uint32_t at_ent;
+      if (d.type == CT_BITSET) at_ent = lc.beg[k] + lc.n[k] - 1 - (atomicAdd(&lc.cnt[k], 0x10000u) >> 16);
+      else at_ent = lc.beg[k] + (atomicAdd(&lc.cnt[k], 1u) & 0xFFFFu);
       // the arena ends with 16 spare bytes, so rounding the end up stays inside it
       const uint16_t* p = lc.pay[k] + d.payload;
-      if (d.type == CT_ARRAY) {  // small arrays into pay4, any array into the free stack tiles
+      if (d.type == CT_ARRAY) {
          const uintptr_t a = reinterpret_cast<uintptr_t>(p);
          const uintptr_t a0 = a & ~static_cast<uintptr_t>(15);
-         const uint32_t bytes = static_cast<uint32_t>(((a + 2u * (d.card_m1 + 1u) + 15) & ~static_cast<uintptr_t>(15)) - a0);
-         uint32_t dst = 0, po = LC_NOPAY;
-         if (d.card_m1 < LC_SMALL) {
+         const uint32_t bytes = static_cast<uint32_t>(((a + 2u * card + 15) & ~static_cast<uintptr_t>(15)) - a0);
+         uint32_t dst = 0;
+         if (bytes <= 2 * LC_PAY) {
             const uint32_t at = atomicAdd(&lc.pay_used, bytes / 2);
-            if (at + bytes / 2 <= LC_PAY) {
-               po = at + static_cast<uint32_t>(a - a0) / 2;
-               dst = static_cast<uint32_t>(__cvta_generic_to_shared(lc.pay4)) + 2 * at;
-            }
+            if (at + bytes / 2 <= LC_PAY) dst = static_cast<uint32_t>(__cvta_generic_to_shared(lc.pay4)) + 2 * at;
          }
-         if (po == LC_NOPAY && lc.ext_cap) {
+         if (dst == 0 && ext_cap) {
             const uint32_t at = atomicAdd(&lc.ext_used, bytes / 2);
-            if (at + bytes / 2 <= lc.ext_cap) {
-               po = LC_PAY + at + static_cast<uint32_t>(a - a0) / 2;
-               dst = static_cast<uint32_t>(__cvta_generic_to_shared(lc.ext)) + 2 * at;
-            }
+            if (at + bytes / 2 <= ext_cap) dst = static_cast<uint32_t>(__cvta_generic_to_shared(ext)) + 2 * at;
          }
-         if (po != LC_NOPAY) {
-            lc.poff[j] = static_cast<uint16_t>(po);
-            atomicAdd(&lc.tot[k], d.card_m1 + 1u);
+         if (dst != 0) {
+            lc.ent[at_ent] = make_uint2(dst - base + static_cast<uint32_t>(a - a0), (E_COPIED << 28) | card);
+            atomicAdd(&lc.tot[k], card);
             asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
             if (!withhold)
                asm volatile(
@@ -317,103 +277,39 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
                   : "memory");
             continue;
          }
+         lc.ent[at_ent] = make_uint2(d.payload, (E_ARRAY << 28) | card);
+         atomicOr(&lc.tot[k], LC_BIG);
+         prefetch_l2(p, p + card);
+      } else if (d.type == CT_BITSET) {
+         lc.ent[at_ent] = make_uint2(d.payload, static_cast<uint32_t>(E_BITSET) << 28);
+         prefetch_l2(p + (c.row0 >> 4), p + ((c.row0 + c.W) >> 4));
+      } else {
+         lc.ent[at_ent] = make_uint2(d.payload, (E_RUN << 28) | d.nruns);
+         atomicOr(&lc.tot[k], LC_BIG);
+         prefetch_l2(p, p + 2u * d.nruns);
       }
-      atomicOr(&lc.tot[k], LC_BIG);
-      if (d.type == CT_ARRAY) prefetch_l2(p, p + d.card_m1 + 1u);
-      else if (d.type == CT_BITSET) prefetch_l2(p + (c.row0 >> 4), p + ((c.row0 + c.W) >> 4));
-      else prefetch_l2(p, p + 2u * d.nruns);
    }
    __syncthreads();
-   if (lc.pay_used == 0 && lc.ext_used == 0) return true;  // no copies this item
-   if (threadIdx.x == 0)
-      asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
-   const uint64_t limit = withhold ? 1000000ull : 2000000000ull;
-   bool ok = wait_copies(lc, phase, limit);
-   if (!ok) ok = wait_copies(lc, phase, limit);  // once more before giving up with copies possibly in flight
-   phase ^= 1u;
-   if (!__syncthreads_and(ok)) {
-      if (threadIdx.x == 0) atomicExch(err, 6);
-      return false;
+   uint32_t claimed = 0;
+   if (next_item && threadIdx.x == 0) claimed = atomicAdd(next_item, 1u);
+   bool ok = true;
+   if (lc.pay_used != 0 || lc.ext_used != 0) {  // otherwise no copies this item
+      if (threadIdx.x == 0)
+         asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
+      const uint64_t limit = withhold ? 1000000ull : 2000000000ull;
+      ok = wait_copies(lc, phase, limit);
+      if (!ok) ok = wait_copies(lc, phase, limit);  // once more before giving up with copies possibly in flight
+      phase ^= 1u;
+      ok = __syncthreads_and(ok);
+      if (!ok && threadIdx.x == 0) atomicExch(err, DEVERR_WAIT_FILTER);
    }
-   return true;
+   if (next_item && threadIdx.x == 0) lc.next_item = claimed;  // read after the caller's next barrier
+   return ok;
 }
 
-// OR of the containers of one slot whose symbol is in `mask` (all of them when !use_mask), from
-// the staged descriptors when the leaf was staged.
-__device__ void push_containers(uint32_t* t, const TileCtx& c, const CtrDesc* __restrict__ ctrs,
-                                const uint16_t* __restrict__ payload, const uint32_t* __restrict__ off, size_t slot,
-                                uint32_t mask, bool use_mask, const LeafCache& lc, uint32_t leaf) {
-   const uint4* src;
-   uint32_t n;
-   if (leaf >= 1 && leaf <= lc.nl && lc.beg[leaf - 1] != LC_NONE) {
-      src = lc.desc + lc.beg[leaf - 1];
-      n = lc.n[leaf - 1];
-   } else {
-      const uint32_t b = __ldg(off + slot), e = __ldg(off + slot + 1);
-      src = reinterpret_cast<const uint4*>(ctrs) + b;
-      n = e - b;
-   }
-   const bool staged = leaf >= 1 && leaf <= lc.nl && lc.beg[leaf - 1] != LC_NONE;
-   // staged leaves of at most 32 descriptors visit only the matching ones
-   uint32_t todo = staged && n <= 32 ? lc.match[leaf - 1] : 0u;
-   const bool listed = staged && n <= 32;
-   for (uint32_t i = 0; listed ? todo != 0u : i < n; ++i) {
-      if (listed) {
-         i = __ffs(todo) - 1;
-         todo &= todo - 1;
-      }
-      const uint4 raw = src[i];
-      const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
-      if (use_mask && !((mask >> d.sym) & 1u)) continue;
-      const uint16_t po = staged ? lc.poff[lc.beg[leaf - 1] + i] : LC_NOPAY;
-      if (po != LC_NOPAY) {  // array copied into shared memory with the item's leaves
-         const uint16_t* sp = po < LC_PAY ? reinterpret_cast<const uint16_t*>(lc.pay4) + po : lc.ext + (po - LC_PAY);
-         const uint32_t card = d.card_m1 + 1u;
-         for (uint32_t k = threadIdx.x; k < card; k += blockDim.x) {
-            const uint32_t r = static_cast<uint32_t>(sp[k]) - c.row0;
-            if (r < c.W) atomicOr(&t[r >> 5], 1u << (r & 31));
-         }
-      } else {
-         or_container(t, d, payload, c.row0, c.W);
-      }
-   }
-}
-
-// A staged leaf of at most 32 descriptors whose matching containers are arrays copied into shared
-// memory, LC_OWNER_MAX rows at most: set by the owners of its words (see below), with no CTA
-// barrier. Each thread clears the words it owns; each warp then reads every row of the leaf and sets
-// those in the words its lanes own (shared-memory atomics: two lanes may hit one word), fenced by
-// __syncwarp on both sides. Returns false (nothing done) for any other leaf.
-__device__ __forceinline__ bool push_owned(uint4* t4, uint32_t* t, const TileCtx& c, const LeafCache& lc, uint32_t leaf) {
-   if (leaf < 1 || leaf > lc.nl) return false;
-   const uint32_t k = leaf - 1;
-   if (lc.beg[k] == LC_NONE || lc.n[k] > 32 || lc.tot[k] > LC_OWNER_MAX) return false;
-   const uint32_t W4 = c.W >> 7, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = make_uint4(0, 0, 0, 0);
-   __syncwarp();
-   uint32_t todo = lc.match[k];
-   while (todo) {
-      const uint32_t i = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t j = lc.beg[k] + i;
-      const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&lc.desc[j]);
-      const uint16_t po = lc.poff[j];
-      const uint16_t* sp = po < LC_PAY ? reinterpret_cast<const uint16_t*>(lc.pay4) + po : lc.ext + (po - LC_PAY);
-      const uint32_t card = d.card_m1 + 1u;
-      for (uint32_t e = lane; e < card; e += 32) {
-         const uint32_t r = static_cast<uint32_t>(sp[e]) - c.row0;
-         if (r < c.W && (((r >> 7) % FT) >> 5) == warp) atomicOr(&t[r >> 5], 1u << (r & 31));
-      }
-   }
-   __syncwarp();
-   return true;
-}
-
-// Word-parallel tile operations use one fixed mapping: thread i owns the uint4 words i, i +
-// blockDim.x, ... of every tile. Consecutive word-parallel operations therefore need no barrier
-// between them; leaves that scatter with shared-memory atomics (or write per warp) are fenced by
-// barriers on both sides, except the small staged leaves that only their words' owning warps write
-// (push_owned, fenced per warp).
+// Every tile has one fixed mapping: thread t owns the uint4 words t, t + blockDim.x, ... of every tile.
+// Operators on whole tiles therefore need no barrier; only row lists write words that a thread does
+// not own.
 __device__ __forceinline__ uint4 valid4(uint32_t w4, const TileCtx& c) {
    if (c.nvalid == c.W) return make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
    return make_uint4(valid_word(4 * w4, c.nvalid), valid_word(4 * w4 + 1, c.nvalid), valid_word(4 * w4 + 2, c.nvalid),
@@ -423,390 +319,614 @@ __device__ __forceinline__ uint4 and4(uint4 a, uint4 b) { return make_uint4(a.x 
 __device__ __forceinline__ uint4 andnot4(uint4 a, uint4 b) {
    return make_uint4(a.x & ~b.x, a.y & ~b.y, a.z & ~b.z, a.w & ~b.w);
 }
+__device__ __forceinline__ uint4 xor4(uint4 a, uint4 b) { return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w); }
 __device__ __forceinline__ uint4 or4(uint4 a, uint4 b) { return make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w); }
 __device__ __forceinline__ bool any4(uint4 a) { return (a.x | a.y | a.z | a.w) != 0u; }
 __device__ __forceinline__ bool ne4(uint4 a, uint4 b) {
    return ((a.x ^ b.x) | (a.y ^ b.y) | (a.z ^ b.z) | (a.w ^ b.w)) != 0u;
 }
-__device__ __forceinline__ uint32_t get4(const uint4& a, uint32_t i) { return i == 0 ? a.x : i == 1 ? a.y : i == 2 ? a.z : a.w; }
 
-// Rows covered at pos (or not covered when `negate`): all valid rows minus the exceptions whose
-// covered region misses pos and the rows with a missing interval over pos, within the tile's
-// ranges r of both lists.
-__device__ void push_covered(uint32_t* t, const TileCtx& c, const DevSeqCol* __restrict__ col, uint32_t pos, bool negate,
-                             uint4 r) {
-   const uint32_t W4 = c.W >> 7;
-   uint4* t4 = reinterpret_cast<uint4*>(t);
-   for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = valid4(w4, c);
-   __syncthreads();
-   constexpr uint32_t U = 4;  // entries per thread in flight
-   const uint4* exc = reinterpret_cast<const uint4*>(col->exc);
-   for (uint32_t i0 = r.x + threadIdx.x; i0 < r.y; i0 += U * blockDim.x) {
-      uint4 e[U];
-#pragma unroll
-      for (uint32_t u = 0; u < U; ++u) {
-         const uint32_t i = i0 + u * blockDim.x;
-         e[u] = i < r.y ? __ldg(exc + i) : make_uint4(c.row0, 0, 0xFFFFFFFFu, 0);
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < U; ++u) {
-         const uint32_t row = e[u].x - c.row0;
-         if (row < c.W && !(e[u].y <= pos && pos < e[u].z)) atomicAnd(&t[row >> 5], ~(1u << (row & 31)));
-      }
-   }
-   const uint32_t q = pos % NBLOCK;
-   const uint2* nb = reinterpret_cast<const uint2*>(col->nblk);
-   for (uint32_t i0 = r.z + threadIdx.x; i0 < r.w; i0 += U * blockDim.x) {
-      uint2 e[U];
-#pragma unroll
-      for (uint32_t u = 0; u < U; ++u) {
-         const uint32_t i = i0 + u * blockDim.x;
-         e[u] = i < r.w ? __ldg(nb + i) : make_uint2(0, 0);
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < U; ++u) {
-         const uint32_t row = (e[u].x & 0xFFFFu) - c.row0;
-         const uint32_t lo = e[u].y & 0xFFFFu, hi = e[u].y >> 16;
-         if (row < c.W && lo <= q && q < hi) atomicAnd(&t[row >> 5], ~(1u << (row & 31)));
+
+// ---- applying a leaf ----
+//
+// A leaf's rows are applied one by one where its value is consumed: set in or removed from the top
+// tile, or added to the counter planes, with shared-memory atomics. Leaves are sparse (36 rows per
+// container on average), so this takes a fraction of the instructions of building the leaf's tile
+// and combining it word by word.
+
+// Rows r0 and, with `two`, r1 of the tile at T (A_ADD: of the P counter planes at T, WW words apart), their
+// atomics in flight together. Additions commute, also when threads add to one row at a time: each
+// plane's exchange returns the old bit as the carry, so a plane receives half as many carries as the
+// one below it received bits, in any order; the top plane only ever gets set.
+__device__ __forceinline__ void apply_rows(uint32_t* T, uint32_t WW, uint32_t P, uint32_t A, uint32_t r0, bool one,
+                                           uint32_t r1, bool two) {
+   uint32_t b0 = one ? 1u << (r0 & 31) : 0u, b1 = two ? 1u << (r1 & 31) : 0u;
+   uint32_t* q0 = T + (r0 >> 5);
+   uint32_t* q1 = T + (r1 >> 5);
+   if (A == A_ADD) {
+#pragma unroll 1
+      for (uint32_t i = 0; i + 1 < P && (b0 | b1); ++i, q0 += WW, q1 += WW) {
+         uint32_t o0 = 0, o1 = 0;
+         if (b0) o0 = atomicXor(q0, b0);
+         if (b1) o1 = atomicXor(q1, b1);
+         b0 &= o0;
+         b1 &= o1;
       }
    }
-   __syncthreads();
-   if (negate) {
-      for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = andnot4(valid4(w4, c), t4[w4]);
+   if (A == A_ANDNOT) {
+      if (b0) atomicAnd(q0, ~b0);
+      if (b1) atomicAnd(q1, ~b1);
+   } else {
+      if (b0) atomicOr(q0, b0);
+      if (b1) atomicOr(q1, b1);
+   }
+}
+__device__ __forceinline__ void apply_row(uint32_t* T, uint32_t WW, uint32_t P, uint32_t A, uint32_t r) {
+   apply_rows(T, WW, P, A, r, true, 0, false);
+}
+
+// The value v of uint4 word w4 meets the target: stored, combined with the tile at T4, or (FUSE_THR_ADD)
+// added to the P counter planes at T4.
+__device__ __forceinline__ void put_word(uint4* T4, uint32_t W4, uint32_t P, uint32_t f, uint32_t w4, uint4 v) {
+   uint4* q = T4 + w4;
+   if (f == FUSE_THR_ADD) {
+#pragma unroll 1
+      for (uint32_t i = 0; i + 1 < P && any4(v); ++i, q += W4) {  // ripple carry
+         const uint4 p = *q;
+         *q = make_uint4(p.x ^ v.x, p.y ^ v.y, p.z ^ v.z, p.w ^ v.w);
+         v = and4(v, p);
+      }
+      if (any4(v)) *q = or4(*q, v);
+   } else if (f == FUSE_NONE) {
+      *q = v;
+   } else {
+      const uint4 x = *q;
+      *q = f == FUSE_AND ? and4(x, v) : f == FUSE_OR ? or4(x, v) : andnot4(x, v);
    }
 }
 
-// Rows whose date lies in [lo, hi] (outside it when `invert`); null dates match when `with_nulls`.
-// Every comparison of the date predicates and the two-sided DateBetween reduce to this form. The
-// bit-sliced index is compared against the clamped bounds from the top bit down (lo <= x keeps
-// "greater" and "equal" masks, x <= hi "less" and "equal"); word-parallel in the fixed mapping.
-__device__ void push_date(uint4* t4, const TileCtx& c, const DevDateCol* __restrict__ col, int32_t lo, int32_t hi,
-                          bool invert, bool with_nulls) {
-   const uint32_t W4 = c.W >> 7, nbits = col->nbits;
-   const int64_t maxv = (int64_t{1} << nbits) - 1;
-   const int64_t l = static_cast<int64_t>(lo) - col->base, h = static_cast<int64_t>(hi) - col->base;
-   const bool empty = lo > hi || h < 0 || l > maxv;
-   const uint32_t L = static_cast<uint32_t>(l < 0 ? 0 : l), H = static_cast<uint32_t>(h > maxv ? maxv : h);
-   const size_t stride4 = static_cast<size_t>(c.tab->nchunks) * (CHUNK_WORDS / 4);
-   const size_t base4 = (static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5)) / 4;
-   const uint4* planes = reinterpret_cast<const uint4*>(col->planes) + base4;
-   const uint4* nulls = reinterpret_cast<const uint4*>(col->nulls) + base4;
-   const uint4 ones = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-   for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
-      uint4 inside = make_uint4(0, 0, 0, 0);
-      if (!empty) {
-         uint4 eqL = ones, gtL = inside, eqH = ones, ltH = inside;
-#pragma unroll 4
-         for (int i = static_cast<int>(nbits) - 1; i >= 0; --i) {
-            const uint4 x = __ldg(planes + static_cast<size_t>(i) * stride4 + w4);
-            if ((L >> i) & 1u) {
-               eqL = and4(eqL, x);
-            } else {
-               gtL = or4(gtL, and4(eqL, x));
-               eqL = andnot4(eqL, x);
+// Thread t of nt: its share of the rows of an array in global memory, read 8 at a time (the arena ends
+// with 16 spare bytes).
+__device__ __forceinline__ void apply_array(uint32_t* T, uint32_t P, uint32_t A, const TileCtx& c,
+                                            const uint16_t* __restrict__ p, uint32_t n, uint32_t t, uint32_t nt) {
+   const uint32_t lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p) & 15u) / 2;
+   const uint4* a = reinterpret_cast<const uint4*>(p - lead);
+#pragma unroll 1
+   for (uint32_t i = 8 * t; i < lead + n; i += 8 * nt) {
+      uint4 v = __ldg(a + (i >> 3));
+#pragma unroll 1
+      for (uint32_t j = i; j < i + 8; j += 2) {
+         const uint32_t r0 = (v.x & 0xFFFFu) - c.row0, r1 = (v.x >> 16) - c.row0;
+         apply_rows(T, c.W >> 5, P, A, r0, j >= lead && j < lead + n && r0 < c.W, r1,
+                    j + 1 >= lead && j + 1 < lead + n && r1 < c.W);
+         v = make_uint4(v.y, v.z, v.w, 0);
+      }
+   }
+}
+__device__ __forceinline__ void apply_runs(uint32_t* T, uint32_t P, uint32_t A, const TileCtx& c,
+                                           const uint16_t* __restrict__ p, uint32_t n, uint32_t t, uint32_t nt) {
+#pragma unroll 1
+   for (uint32_t i = t; i < n; i += nt) {
+      const uint32_t s = __ldg(p + 2 * i);
+      const uint32_t e = s + __ldg(p + 2 * i + 1) + 1u;  // run covers [s, e)
+      const uint32_t a = max(s, c.row0), b = min(e, c.row0 + c.W);
+#pragma unroll 1
+      for (uint32_t r = a; r < b; ++r) apply_row(T, c.W >> 5, P, A, r - c.row0);
+   }
+}
+
+// A container leaf that was not staged, from its descriptors; every thread takes part, with barriers.
+__device__ __noinline__ void apply_unstaged(uint32_t* T, uint32_t P, uint32_t A, const Instr& in, const TileCtx& c) {
+   const CtrDesc* ctrs;
+   const uint16_t* payload;
+   const uint32_t* off;
+   size_t slot;
+   uint32_t mask = 0xFFFFFFFFu;
+   if (in.op == OP_PUSH_SCAN) {
+      const DevSeqCol* col = &c.tab->seq[in.col];
+      ctrs = col->fctrs, payload = col->payload, off = col->off, mask = in.b;
+      slot = static_cast<size_t>(c.v) * col->L + in.a;
+   } else {
+      const DevDictCol* col = &c.tab->dict[in.col];
+      ctrs = col->fctrs, payload = col->payload, off = col->off;
+      slot = static_cast<size_t>(c.v) * col->nkeys + in.a;
+   }
+   const uint32_t b = __ldg(off + slot), e = __ldg(off + slot + 1), W4 = c.W >> 7;
+   const uint32_t f = A == A_OR ? FUSE_OR : A == A_ANDNOT ? FUSE_ANDNOT : FUSE_THR_ADD;
+   __syncthreads();
+#pragma unroll 1
+   for (uint32_t i = b; i < e; ++i) {
+      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(ctrs) + i);
+      const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
+      if (!((mask >> d.sym) & 1u)) continue;
+      const uint16_t* p = payload + d.payload;
+      if (d.type == CT_BITSET) {
+         const uint4* src = reinterpret_cast<const uint4*>(p) + (c.row0 >> 7);
+#pragma unroll 1
+         for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x)
+            put_word(reinterpret_cast<uint4*>(T), W4, P, f, w4, __ldg(src + w4));
+      } else if (d.type == CT_ARRAY) {
+         apply_array(T, P, A, c, p, d.card_m1 + 1u, threadIdx.x, blockDim.x);
+      } else {
+         apply_runs(T, P, A, c, p, d.nruns, threadIdx.x, blockDim.x);
+      }
+      __syncthreads();
+   }
+}
+
+// Applies the rows not covered at pos: those whose covered region starts after pos or ends before it, and
+// those with a missing interval over pos (intervals lie inside the covered region, so no row comes
+// twice). All threads share the lists.
+__device__ __forceinline__ void apply_uncovered(uint32_t* T, uint32_t P, uint32_t A, const TileCtx& c,
+                                                const DevSeqCol* __restrict__ col, uint32_t pos, const CoverRange& r) {
+   const uint32_t WW = c.W >> 5, nb = r.rng.y + r.rng.w;
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) {
+      const bool late = i < r.rng.y;
+      const uint2 e = __ldg(reinterpret_cast<const uint2*>(late ? col->cov_late + r.rng.x + i : col->cov_early + r.rng.z + (i - r.rng.y)));
+      const uint32_t row = e.x - c.row0;
+      if (row < c.W && (e.y > pos) == late) apply_row(T, WW, P, A, row);
+   }
+   // four intervals per load: 256 threads read a chunk's bucket of a 128-position block (about 540) at once
+   const uint32_t q = pos % NBLOCK;
+   const uint4* nblk = reinterpret_cast<const uint4*>(col->nblk);
+#pragma unroll 1
+   for (uint32_t i = r.miss.x / 4 + threadIdx.x; i < (r.miss.y + 3) / 4; i += blockDim.x) {
+      uint4 e = __ldg(nblk + i);
+#pragma unroll 1
+      for (uint32_t k = 0; k < 2; ++k) {
+         const uint32_t r0 = (e.x & 0xFFFFu) - c.row0, r1 = (e.y & 0xFFFFu) - c.row0;
+         apply_rows(T, WW, P, A, r0, r0 < c.W && ((e.x >> 16) & 0xFFu) <= q && q < (e.x >> 24), r1,
+                    r1 < c.W && ((e.y >> 16) & 0xFFu) <= q && q < (e.y >> 24));
+         e = make_uint4(e.z, e.w, 0, 0);
+      }
+   }
+}
+
+__device__ __forceinline__ Instr fetch(const Instr* __restrict__ code, uint32_t pc, const LeafCache& lc) {
+   const uint4 raw = pc < LC_CODE ? lc.code[pc] : __ldg(reinterpret_cast<const uint4*>(code) + pc);
+   return *reinterpret_cast<const Instr*>(&raw);
+}
+
+// Applies row-list leaves to one target (the tile, scratch tile or counter planes at T): mc container
+// leaves with ordinals k0 + 1 .., their instructions from pc on, then mv coverage leaves. Bitsets
+// first, each owner its own words; then, between two barriers, the staged entries and the coverage
+// lists. A group's entries are shared out over the warps, so that a leaf costs one warp a few
+// instructions per 32 rows instead of every warp its control work; a lone leaf's rows over all
+// threads; a lone leaf of at most LC_OWNER_MAX rows goes to the warps that own its words (every warp
+// reads every row), with no CTA barrier.
+__device__ __forceinline__ void apply_leaves(uint32_t* T, uint32_t P, uint32_t A, const Instr* __restrict__ code,
+                                             uint32_t pc, uint32_t k0, uint32_t mc, uint32_t mv, const TileCtx& c,
+                                             const LeafCache& lc, uint32_t nl, uint32_t ncov) {
+   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W4 = c.W >> 7;
+   bool owner = false;
+   if (mc > 0 && (k0 + mc > nl || lc.beg[k0 + mc - 1] == LC_NONE)) {
+#pragma unroll 1
+      for (uint32_t i = 0; i < mc; ++i) apply_unstaged(T, P, A, fetch(code, pc + i, lc), c);
+      if (mv == 0) return;
+   } else {
+      if (mc > 0) {
+         // bitsets, three at a time: their loads in flight together, and a full adder in front of the planes
+         const uint32_t f = A == A_OR ? FUSE_OR : A == A_ANDNOT ? FUSE_ANDNOT : FUSE_THR_ADD;
+         uint32_t l = k0, nb = lc.cnt[k0] >> 16;
+#pragma unroll 1
+         for (;;) {
+            const uint4 *p0 = nullptr, *p1 = nullptr, *p2 = nullptr;
+            uint32_t have = 0;
+#pragma unroll 1
+            while (have < 3) {
+               if (nb == 0) {
+                  if (++l >= k0 + mc) break;
+                  nb = lc.cnt[l] >> 16;
+                  continue;
+               }
+               const uint4* p = reinterpret_cast<const uint4*>(lc.pay[l] + lc.ent[lc.beg[l] + lc.n[l] - nb].x) + (c.row0 >> 7);
+               --nb;
+               if (have == 0) p0 = p;
+               else if (have == 1) p1 = p;
+               else p2 = p;
+               ++have;
             }
-            if ((H >> i) & 1u) {
-               ltH = or4(ltH, andnot4(eqH, x));
-               eqH = and4(eqH, x);
-            } else {
-               eqH = andnot4(eqH, x);
+            if (have == 0) break;
+#pragma unroll 2
+            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
+               uint4* T4 = reinterpret_cast<uint4*>(T);
+               const uint4 zero = make_uint4(0, 0, 0, 0);
+               const uint4 x = __ldg(p0 + w4), y = have > 1 ? __ldg(p1 + w4) : zero, z = have > 2 ? __ldg(p2 + w4) : zero;
+               if (f == FUSE_THR_ADD && P > 1) {
+                  const uint4 u = xor4(x, y), carry = or4(and4(x, y), and4(u, z));
+                  put_word(T4, W4, P, f, w4, xor4(u, z));
+                  if (any4(carry)) put_word(T4 + W4, W4, P - 1, f, w4, carry);
+               } else {
+                  put_word(T4, W4, P, f, w4, or4(or4(x, y), z));
+               }
+            }
+            if (l >= k0 + mc) break;
+         }
+         if (mc == 1 && mv == 0) {
+            const uint32_t tot = lc.tot[k0];
+            if (tot == 0) return;  // bitsets only, or nothing
+            owner = tot <= LC_OWNER_MAX;
+         }
+      }
+      if (owner) __syncwarp();
+      else __syncthreads();
+      if (mc > 0) {
+         const bool lone = mc == 1;
+         const uint32_t j0 = lone && !owner ? threadIdx.x : lane, js = lone && !owner ? blockDim.x : 32u;
+         const uint32_t wmask = owner ? (blockDim.x >> 5) - 1u : 0u, wsel = owner ? warp : 0u;
+         const uint32_t e = lc.beg[k0 + mc - 1] + lc.n[k0 + mc - 1];
+         uint32_t turn = lone ? 0u : warp;  // entries to pass over before this warp's next
+#pragma unroll 1
+         for (uint32_t i0 = lc.beg[k0]; i0 < e; i0 += 32) {
+            const uint2 mine = i0 + lane < e ? lc.ent[i0 + lane] : make_uint2(0, 0);
+            uint32_t todo = __ballot_sync(0xFFFFFFFFu, (mine.y & 0x0FFFFFFFu) != 0u);  // bitsets have no count
+#pragma unroll 1
+            for (; todo; todo &= todo - 1) {
+               if (turn) {
+                  --turn;
+                  continue;
+               }
+               turn = lone ? 0u : (blockDim.x >> 5) - 1u;
+               const uint32_t l = __ffs(todo) - 1;
+               const uint32_t x = __shfl_sync(0xFFFFFFFFu, mine.x, l), y = __shfl_sync(0xFFFFFFFFu, mine.y, l);
+               const uint32_t kind = y >> 28, n = y & 0x0FFFFFFFu;
+               if (kind == E_COPIED) {
+                  const uint16_t* sp = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(&lc) + x);
+#pragma unroll 1
+                  for (uint32_t j = j0; j < n; j += 2 * js) {
+                     const uint32_t r0 = static_cast<uint32_t>(sp[j]) - c.row0;
+                     const uint32_t r1 = j + js < n ? static_cast<uint32_t>(sp[j + js]) - c.row0 : 0xFFFFFFFFu;
+                     apply_rows(T, c.W >> 5, P, A, r0, r0 < c.W && ((r0 >> 12) & wmask) == wsel, r1,
+                                r1 < c.W && ((r1 >> 12) & wmask) == wsel);
+                  }
+               } else if (kind == E_ARRAY) {
+                  apply_array(T, P, A, c, lc.pay[lc.dleaf[i0 + l]] + x, n, j0, js);
+               } else {
+                  apply_runs(T, P, A, c, lc.pay[lc.dleaf[i0 + l]] + x, n, j0, js);
+               }
+               __syncwarp();
             }
          }
-         inside = and4(or4(gtL, eqL), or4(ltH, eqH));
       }
-      const uint4 nul = __ldg(nulls + w4);
-      const uint4 m = invert ? andnot4(ones, inside) : inside;
-      const uint4 res = with_nulls ? or4(andnot4(m, nul), nul) : andnot4(m, nul);
-      t4[w4] = and4(res, valid4(w4, c));
    }
+#pragma unroll 1
+   for (uint32_t i = 0; i < mv; ++i) {
+      const Instr in = fetch(code, pc + mc + i, lc);
+      const DevSeqCol* col = &c.tab->seq[in.col];
+      const CoverRange r = (in.c >= 1 && in.c <= ncov) ? CoverRange{lc.cov[in.c - 1], lc.covm[in.c - 1]}
+                                                       : cover_ranges(c.tab, col, c.v, c.row0, c.W, in.a);
+      apply_uncovered(T, P, A, c, col, in.a, r);
+   }
+   if (owner) __syncwarp();
+   else __syncthreads();
 }
 
-// Runs a filter program for one tile. The result is left in stack slot 0, complete for the thread
-// that owns each uint4 word (see valid4); a barrier is needed before other threads read it.
-// Returns false on a malformed program (the error flag is set).
-// With `trace` (trace mode of the single-query kernel, for planner training) every executed
-// instruction pc stores trace[2 pc] = its cycles (first thread, between barriers around the
-// instruction) and trace[2 pc + 1] = the population count of the top of the stack after it.
-__device__ bool run_program(const TileCtx& c, const Instr* __restrict__ code, uint32_t ncode, uint32_t* stk,
-                            uint32_t cap, const LeafCache& lc, int* err, uint32_t* trace = nullptr) {
-   __shared__ uint32_t tred[FT / 32];
-   const uint32_t WW = c.W >> 5, W4 = c.W >> 7;
-   uint4* stk4 = reinterpret_cast<uint4*>(stk);
+// Rows whose date lies in [lo, hi] (outside it: flags & 2); null dates match with flags & 1. Every
+// comparison of the date predicates and the two-sided DateBetween reduce to this form: dates up to
+// hi but not up to lo - 1, read from the range-encoded index (DevDateCol).
+struct DateLeaf {
+   const uint4* planes;
+   const uint4* nulls;
+   size_t stride4;
+   uint32_t ndig, width, last;
+   uint32_t hi, below;           // offsets from the index's base; below = lo - 1
+   bool none, all_up, no_below;  // no date in [lo, hi]; hi at or past the last date; lo at or before the first
+   uint32_t flags;
+};
+__device__ __forceinline__ DateLeaf date_leaf(const TileCtx& c, const DevDateCol* __restrict__ col, int32_t lo, int32_t hi,
+                                              uint32_t flags) {
+   DateLeaf d;
+   const int64_t l = static_cast<int64_t>(lo) - col->base, h = static_cast<int64_t>(hi) - col->base, span = col->span;
+   d.none = lo > hi || h < 0 || l > span;
+   d.all_up = h >= span;
+   d.no_below = l <= 0;
+   d.hi = static_cast<uint32_t>(h);
+   d.below = static_cast<uint32_t>(l - 1);
+   d.ndig = col->ndig;
+   d.width = col->width;
+   d.last = col->last;
+   d.stride4 = static_cast<size_t>(c.tab->nchunks) * (CHUNK_WORDS / 4);
+   const size_t base4 = (static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5)) / 4;
+   d.planes = reinterpret_cast<const uint4*>(col->planes) + base4;
+   d.nulls = reinterpret_cast<const uint4*>(col->nulls) + base4;
+   d.flags = flags;
+   return d;
+}
+// The rows whose date offset is at most v, from the lowest digit up.
+__device__ __forceinline__ uint4 date_upto(const DateLeaf& d, uint32_t v, uint32_t w4) {
+   const uint4* p = d.planes + w4;
+   const uint32_t m = (1u << d.width) - 1u;
+   uint4 acc = __ldg(p + (v & m) * d.stride4);
+#pragma unroll 1
+   for (uint32_t i = 1; i < d.ndig; ++i) {
+      const uint32_t g = (i << d.width) + ((v >> (d.width * i)) & m);
+      const uint4 x = __ldg(p + g * d.stride4);
+      const uint4 y = (g & m) ? __ldg(p + (g - 1) * d.stride4) : make_uint4(0, 0, 0, 0);
+      acc = or4(y, and4(x, acc));
+   }
+   return acc;
+}
+__device__ __forceinline__ uint4 date_word(const DateLeaf& d, uint32_t w4) {
+   uint4 in = make_uint4(0, 0, 0, 0);
+   if (!d.none) {
+      in = d.all_up ? __ldg(d.planes + d.last * d.stride4 + w4) : date_upto(d, d.hi, w4);
+      if (!d.no_below) in = andnot4(in, date_upto(d, d.below, w4));
+   }
+   if (d.flags & 2) in = andnot4(__ldg(d.planes + d.last * d.stride4 + w4), in);
+   if (d.flags & 1) in = or4(in, __ldg(d.nulls + w4));
+   return in;
+}
+
+// Runs a filter program for one tile over a stack of `cap` tiles at stk4; the result is left in tile 0,
+// complete for the thread that owns each word. X4 is the scratch tile: zero between leaves, it holds
+// the rows of the few leaves whose operator needs all of them at once (AND of a row list, and the
+// operators that take its complement). Returns false on a malformed program (the error flag is set).
+// With TRACE (the single-query kernel's trace mode, for planner training) every executed instruction pc
+// stores trace[2 pc] = its cycles (first thread, between barriers around the instruction) and
+// trace[2 pc + 1] = the population count of the top of the stack after it.
+// Every part of the interpreter exists once in the code, and its loops are not unrolled far: the
+// warps of an SM are in different instructions, and a first version specialised by tile width and
+// operator (575 KB of code) spent most of its time on instruction fetches.
+template <bool TRACE>
+__device__ __forceinline__ bool run_program(const TileCtx& c, const Instr* __restrict__ code, uint32_t ncode,
+                                            uint4* stk4, uint32_t cap, uint4* X4, const LeafCache& lc, uint32_t nl,
+                                            uint32_t ncov, int* err, uint32_t* trace) {
+   const uint32_t W4 = c.W >> 7;
    uint32_t sp = 0;
-   uint32_t pc = 0;
    uint32_t steps = 0;
-   bool synced = true;  // no word-parallel write since the last barrier
-   while (pc < ncode) {
+   int bad = 0;
+#pragma unroll 1
+   for (uint32_t pc = 0; pc < ncode;) {
       if (++steps > 4u * MAX_PROGRAM) {  // jumps only go forward; this bounds a corrupted program
-         if (threadIdx.x == 0) atomicExch(err, 3);
-         return false;
+         bad = 3;
+         break;
       }
       long long t_start = 0;
-      if (trace) {
+      if (TRACE) {
          __syncthreads();
          t_start = clock64();
       }
-      Instr in;
-      {
-         const uint4 raw = __ldg(reinterpret_cast<const uint4*>(code) + pc);
-         in = *reinterpret_cast<const Instr*>(&raw);
-      }
+      const Instr in = fetch(code, pc, lc);
       uint32_t next = pc + 1;
-      switch (in.op) {
-         case OP_PUSH_EMPTY:
-         case OP_PUSH_FULL:
-         case OP_PUSH_SCAN:
-         case OP_PUSH_NULLS:
-         case OP_PUSH_DICT:
-         case OP_PUSH_COVERED:
-         case OP_PUSH_DATE:
-         case OP_PUSH_AUX: {
-            if (sp >= cap) {
-               if (threadIdx.x == 0) atomicExch(err, 1);
-               return false;
-            }
-            uint32_t* t = stk + sp * WW;
-            uint4* t4 = stk4 + sp * W4;
+      // what combines with the target word by word, if anything does
+      enum : uint32_t { S_NONE, S_ZERO, S_FULL, S_SET, S_DATE, S_SCRATCH, S_TILE };
+      uint32_t src = S_NONE, f = FUSE_NONE, P = 0;
+      const uint4* from = nullptr;
+      bool negate = false;
+      uint4* T4 = stk4;
+      if (is_leaf(in.op) || in.op == OP_GROUP) {
+         const bool group = in.op == OP_GROUP;
+         const bool list = group || in.op == OP_PUSH_SCAN || in.op == OP_PUSH_DICT || in.op == OP_PUSH_COVERED;
+         P = leaf_planes(in.flags);
+         bool add, push;
+         uint32_t A = in.flags & 3u;
+         if (group) {
+            add = A == A_ADD;
+            push = in.flags & GROUP_PUSH;
+            next = pc + 1 + in.a;
+            if (next > ncode) bad = 4;
+         } else {
+            f = leaf_fused(in.flags);
+            add = f == FUSE_THR_ADD || f == FUSE_THR_ADD_NOT;
+            push = f == FUSE_NONE;
+         }
+         if (push) {
+            if (sp >= cap) bad = 1;
             ++sp;
-            if (in.op == OP_PUSH_FULL) {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = valid4(w4, c);
-               synced = false;
-            } else if (in.op == OP_PUSH_EMPTY) {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = make_uint4(0, 0, 0, 0);
-               synced = false;
-            } else if (in.op == OP_PUSH_NULLS) {
-               const uint4* src = reinterpret_cast<const uint4*>(c.tab->seq[in.col].null_tiles +
-                                                                 static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5));
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = __ldg(src + w4);
-               synced = false;
-            } else if (in.op == OP_PUSH_AUX) {
-               if (c.aux == nullptr) {
-                  if (threadIdx.x == 0) atomicExch(err, 5);
-                  return false;
-               }
-               const uint4* src = reinterpret_cast<const uint4*>(
-                  c.aux + static_cast<size_t>(in.a) * c.tab->nchunks * CHUNK_WORDS + static_cast<size_t>(c.v) * CHUNK_WORDS +
-                  (c.row0 >> 5));
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = __ldg(src + w4);
-               synced = false;
-            } else if (in.op == OP_PUSH_COVERED) {
-               const DevSeqCol* col = &c.tab->seq[in.col];
-               const uint4 r = (in.c >= 1 && in.c <= lc.ncov) ? lc.cov[in.c - 1]
-                                                              : cover_ranges(c.tab, col, c.v, c.row0, c.W, in.a);
-               push_covered(t, c, col, in.a, in.flags & 1, r);
-               synced = !(in.flags & 1);
-            } else if (in.op == OP_PUSH_DATE) {
-               push_date(t4, c, &c.tab->date[in.col], static_cast<int32_t>(in.a), static_cast<int32_t>(in.b), in.flags & 2,
-                         in.flags & 1);
-               synced = false;
-            } else if (push_owned(t4, t, c, lc, in.c)) {
-               synced = false;
-            } else {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) t4[w4] = make_uint4(0, 0, 0, 0);
-               __syncthreads();
-               if (in.op == OP_PUSH_SCAN) {
-                  const DevSeqCol* col = &c.tab->seq[in.col];
-                  push_containers(t, c, col->ctrs, col->payload, col->off, static_cast<size_t>(c.v) * col->L + in.a, in.b,
-                                  true, lc, in.c);
+         } else if (sp < (add ? P : 1u)) {
+            bad = 2;
+         }
+         if (bad) break;
+         T4 = stk4 + (sp - (add ? P : 1u)) * W4;  // the new tile, the top tile, or the counter's planes
+         if (list) {
+            bool scratch = false;
+            if (!group) {
+               // the leaf is a list of rows, or (comp) all valid rows but those listed
+               const bool comp = in.op == OP_PUSH_COVERED && !(in.flags & 1);
+               if (f == (comp ? FUSE_THR_ADD_NOT : FUSE_THR_ADD)) {
+                  A = A_ADD;
+               } else if (comp ? (push || f == FUSE_AND) : f == FUSE_ANDNOT) {
+                  A = A_ANDNOT;
                } else {
-                  const DevDictCol* col = &c.tab->dict[in.col];
-                  push_containers(t, c, col->ctrs, col->payload, col->off, static_cast<size_t>(c.v) * col->nkeys + in.a, 0,
-                                  false, lc, in.c);
+                  A = A_OR;
+                  scratch = comp || (!push && f != FUSE_OR);
                }
-               __syncthreads();
-               synced = true;
-            }
-            break;
-         }
-         case OP_AND:
-         case OP_ANDNOT:
-         case OP_OR: {
-            if (sp < 2) {
-               if (threadIdx.x == 0) atomicExch(err, 2);
-               return false;
-            }
-            uint4* x = stk4 + (sp - 2) * W4;
-            const uint4* y = stk4 + (sp - 1) * W4;
-            if (in.op == OP_AND) {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) x[w4] = and4(x[w4], y[w4]);
-            } else if (in.op == OP_ANDNOT) {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) x[w4] = andnot4(x[w4], y[w4]);
-            } else {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) x[w4] = or4(x[w4], y[w4]);
-            }
-            --sp;
-            synced = false;
-            break;
-         }
-         case OP_NOT: {
-            if (sp < 1) {
-               if (threadIdx.x == 0) atomicExch(err, 2);
-               return false;
-            }
-            uint4* x = stk4 + (sp - 1) * W4;
-            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) x[w4] = andnot4(valid4(w4, c), x[w4]);
-            synced = false;
-            break;
-         }
-         case OP_THR_BEGIN: {
-            if (sp + in.a > cap) {
-               if (threadIdx.x == 0) atomicExch(err, 1);
-               return false;
-            }
-            for (uint32_t i = 0; i < in.a; ++i)
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) stk4[(sp + i) * W4 + w4] = make_uint4(0, 0, 0, 0);
-            sp += in.a;
-            synced = false;
-            break;
-         }
-         case OP_THR_ADD: {
-            const uint32_t P = in.a;
-            if (sp < P + 1) {
-               if (threadIdx.x == 0) atomicExch(err, 2);
-               return false;
-            }
-            const uint4* x4 = stk4 + (sp - 1) * W4;
-            uint4* planes4 = stk4 + (sp - 1 - P) * W4;
-            const bool neg = in.flags & 1;
-            // ripple-carry add of one bit per row into the bit-sliced counter, four words at a time
-            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
-               uint4 carry = neg ? andnot4(valid4(w4, c), x4[w4]) : x4[w4];
-               for (uint32_t i = 0; i < P && (carry.x | carry.y | carry.z | carry.w); ++i) {
-                  const uint4 p = planes4[i * W4 + w4];
-                  planes4[i * W4 + w4] = make_uint4(p.x ^ carry.x, p.y ^ carry.y, p.z ^ carry.z, p.w ^ carry.w);
-                  carry = make_uint4(carry.x & p.x, carry.y & p.y, carry.z & p.z, carry.w & p.w);
-               }
-               if (carry.x | carry.y | carry.z | carry.w) {  // saturate at 2^P - 1
-                  for (uint32_t i = 0; i < P; ++i) {
-                     const uint4 p = planes4[i * W4 + w4];
-                     planes4[i * W4 + w4] = make_uint4(p.x | carry.x, p.y | carry.y, p.z | carry.z, p.w | carry.w);
-                  }
+               if (scratch) {  // then the scratch tile, or its complement, meets the target
+                  src = S_SCRATCH;
+                  negate = add || f == FUSE_OR;
+                  if (add) f = FUSE_THR_ADD;
+                  else if (f == FUSE_ANDNOT) f = FUSE_AND;  // not (valid but X): X
                }
             }
-            --sp;
-            synced = false;
-            break;
-         }
-         case OP_THR_END: {
-            const uint32_t P = in.a, n = in.b;
-            if (sp < P) {
-               if (threadIdx.x == 0) atomicExch(err, 2);
-               return false;
+            if (push) {
+#pragma unroll 1
+               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x)
+                  T4[w4] = A == A_ANDNOT ? valid4(w4, c) : make_uint4(0, 0, 0, 0);
             }
-            uint4* planes4 = stk4 + (sp - P) * W4;
-            const bool exact = in.flags & 1;
-            // compare the counter with n from the top plane down, four words at a time
-            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
-               uint4 gt = make_uint4(0, 0, 0, 0), eq = make_uint4(~0u, ~0u, ~0u, ~0u);
-               for (int i = static_cast<int>(P) - 1; i >= 0; --i) {
-                  const uint4 p = planes4[i * W4 + w4];
-                  const uint32_t nb = ((n >> i) & 1u) ? 0xFFFFFFFFu : 0u;
-                  gt = make_uint4(gt.x | (eq.x & p.x & ~nb), gt.y | (eq.y & p.y & ~nb), gt.z | (eq.z & p.z & ~nb),
-                                  gt.w | (eq.w & p.w & ~nb));
-                  eq = make_uint4(eq.x & ~(p.x ^ nb), eq.y & ~(p.y ^ nb), eq.z & ~(p.z ^ nb), eq.w & ~(p.w ^ nb));
+            const uint32_t mc = group ? in.b >> 16 : in.op != OP_PUSH_COVERED, mv = group ? in.c >> 16 : mc ^ 1u;
+            apply_leaves(reinterpret_cast<uint32_t*>(scratch ? X4 : T4), P, A, code, group ? pc + 1 : pc,
+                         (group ? in.b & 0xFFFFu : in.c) - 1, mc, mv, c, lc, nl, ncov);
+         } else {
+            if (f == FUSE_THR_ADD_NOT) {
+               negate = true;
+               f = FUSE_THR_ADD;
+            }
+            src = in.op == OP_PUSH_DATE ? S_DATE : in.op == OP_PUSH_FULL ? S_FULL : in.op == OP_PUSH_EMPTY ? S_ZERO : S_SET;
+            if (src == S_SET) {
+               const uint32_t* set = in.op == OP_PUSH_NULLS ? c.tab->seq[in.col].null_tiles : c.aux;
+               if (set == nullptr) {
+                  bad = 5;
+                  break;
                }
-               if (n >> P) eq = make_uint4(0, 0, 0, 0);  // n does not fit: the saturated count is below it
-               const uint4 vm = valid4(w4, c);
-               planes4[w4] = exact ? make_uint4(eq.x & vm.x, eq.y & vm.y, eq.z & vm.z, eq.w & vm.w)
-                                   : make_uint4((gt.x | eq.x) & vm.x, (gt.y | eq.y) & vm.y, (gt.z | eq.z) & vm.z,
-                                                (gt.w | eq.w) & vm.w);
+               if (in.op == OP_PUSH_AUX) set += static_cast<size_t>(in.a) * c.tab->nchunks * CHUNK_WORDS;
+               from = reinterpret_cast<const uint4*>(set + static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5));
             }
-            sp = sp - P + 1;
-            synced = false;
+         }
+      } else if (in.op == OP_AND || in.op == OP_ANDNOT || in.op == OP_OR || in.op == OP_THR_ADD) {
+         const bool add = in.op == OP_THR_ADD;
+         P = add ? in.a : 1u;
+         if (sp < P + 1) {
+            bad = 2;
             break;
          }
-         case OP_JZ:
-         case OP_JFULL: {
-            if (sp < 1) {
-               if (threadIdx.x == 0) atomicExch(err, 2);
-               return false;
-            }
-            const uint4* x = stk4 + (sp - 1) * W4;
-            int differs = 0;
-            if (in.op == OP_JZ) {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) differs |= any4(x[w4]);
-            } else {
-               for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) differs |= ne4(x[w4], valid4(w4, c));
-            }
-            differs = __syncthreads_or(differs);
-            synced = true;
-            if (!differs) {
-               if (in.a <= pc || in.a > ncode) {
-                  if (threadIdx.x == 0) atomicExch(err, 4);
-                  return false;
+         --sp;
+         src = S_TILE;
+         from = stk4 + sp * W4;
+         T4 = stk4 + (sp - P) * W4;
+         f = in.op == OP_AND ? FUSE_AND : in.op == OP_OR ? FUSE_OR : add ? FUSE_THR_ADD : FUSE_ANDNOT;
+         negate = add && (in.flags & 1);
+      } else if (in.op == OP_NOT) {
+         if (sp < 1) {
+            bad = 2;
+            break;
+         }
+         src = S_TILE;
+         from = T4 = stk4 + (sp - 1) * W4;
+         negate = true;
+      } else if (in.op == OP_THR_BEGIN) {
+         if (sp + in.a > cap) {
+            bad = 1;
+            break;
+         }
+#pragma unroll 1
+         for (uint32_t i = sp; i < sp + in.a; ++i)
+#pragma unroll 1
+            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) stk4[i * W4 + w4] = make_uint4(0, 0, 0, 0);
+         sp += in.a;
+      } else if (in.op == OP_THR_END) {
+         const uint32_t n = in.b;
+         P = in.a;
+         if (sp < P) {
+            bad = 2;
+            break;
+         }
+         sp -= P;
+#pragma unroll 1
+         for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {  // compare with n from the top plane down
+            uint4 gt = make_uint4(0, 0, 0, 0), eq = make_uint4(~0u, ~0u, ~0u, ~0u);
+#pragma unroll 2
+            for (int i = static_cast<int>(P) - 1; i >= 0; --i) {
+               const uint4 p = stk4[(sp + i) * W4 + w4];
+               if ((n >> i) & 1u) {
+                  eq = and4(eq, p);
+               } else {
+                  gt = or4(gt, and4(eq, p));
+                  eq = andnot4(eq, p);
                }
-               next = in.a;
             }
+            if (n >> P) eq = gt = make_uint4(0, 0, 0, 0);  // n does not fit: more than the children
+            stk4[sp * W4 + w4] = and4((in.flags & 1) ? eq : or4(gt, eq), valid4(w4, c));
+         }
+         ++sp;
+      } else if (in.op == OP_JZ || in.op == OP_JFULL) {
+         if (sp < 1) {
+            bad = 2;
             break;
          }
-         default:
-            if (threadIdx.x == 0) atomicExch(err, 5);
-            return false;
+         const uint4* x4 = stk4 + (sp - 1) * W4;
+         int differs = 0;
+#pragma unroll 1
+         for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x)
+            differs |= ne4(x4[w4], in.op == OP_JZ ? make_uint4(0, 0, 0, 0) : valid4(w4, c));
+         if (!__syncthreads_or(differs)) {
+            next = in.a;
+            if (in.a <= pc || in.a > ncode) {
+               bad = 4;
+               break;
+            }
+         }
+      } else {
+         bad = 5;
+         break;
       }
-      if (trace) {
+      if (src != S_NONE) {
+         DateLeaf d;
+         if (src == S_DATE)
+            d = date_leaf(c, &c.tab->date[in.col], static_cast<int32_t>(in.a), static_cast<int32_t>(in.b), in.flags);
+#pragma unroll 1
+         for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (src == S_TILE) {
+               v = from[w4];
+            } else if (src == S_SCRATCH) {
+               v = X4[w4];
+               X4[w4] = make_uint4(0, 0, 0, 0);
+            } else if (src == S_SET) {
+               v = __ldg(from + w4);
+            } else if (src == S_DATE) {
+               v = and4(date_word(d, w4), valid4(w4, c));
+            } else if (src == S_FULL) {
+               v = valid4(w4, c);
+            }
+            if (negate) v = andnot4(valid4(w4, c), v);
+            put_word(T4, W4, P, f, w4, v);
+         }
+         if (src == S_SCRATCH) __syncwarp();  // the cleared words before the next leaf's rows
+      }
+      if (TRACE) {
+         __shared__ uint32_t tred[FT / 32];
          __syncthreads();
          const long long t_end = clock64();
          uint32_t n = 0;
          if (sp >= 1) {
-            const uint4* x = stk4 + (sp - 1) * W4;
-            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x)
-               n += __popc(x[w4].x) + __popc(x[w4].y) + __popc(x[w4].z) + __popc(x[w4].w);
+#pragma unroll 1
+            for (uint32_t w4 = threadIdx.x; w4 < W4; w4 += blockDim.x) {
+               const uint4 x = stk4[(sp - 1) * W4 + w4];
+               n += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+            }
          }
          n = __reduce_add_sync(0xFFFFFFFFu, n);
          if ((threadIdx.x & 31) == 0) tred[threadIdx.x >> 5] = n;
          __syncthreads();
          if (threadIdx.x == 0) {
             uint32_t s = 0;
+#pragma unroll 1
             for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) s += tred[w];
             const long long dt = t_end - t_start;
             trace[2 * pc] = static_cast<uint32_t>(dt < 1 ? 1 : (dt > 0xFFFFFFFFll ? 0xFFFFFFFFll : dt));
             trace[2 * pc + 1] = s;
          }
          __syncthreads();
-         synced = true;
       }
       pc = next;
    }
-   if (sp != 1) {
-      if (threadIdx.x == 0) atomicExch(err, 2);
-      return false;
+   if (!bad && sp != 1) bad = 2;
+   if (bad && threadIdx.x == 0) atomicExch(err, bad);
+   return !bad;
+}
+
+// One tile: runs the program, adds the result's population count to *count and copies it to dst
+// (both optional). A tile without rows has an empty result.
+template <bool TRACE>
+__device__ __forceinline__ bool run_tile(const TileCtx& c, const Instr* __restrict__ code, uint32_t ncode, uint4* stk4,
+                                         uint32_t cap, uint4* X4, const LeafCache& lc, uint32_t nl, uint32_t ncov,
+                                         uint32_t* dst, unsigned long long* count, int* err, uint32_t* trace = nullptr) {
+   if (c.nvalid && !run_program<TRACE>(c, code, ncode, stk4, cap, X4, lc, nl, ncov, err, trace)) return false;
+   uint32_t pc = 0;
+#pragma unroll 1
+   for (uint32_t w4 = threadIdx.x; w4 < (c.W >> 7); w4 += blockDim.x) {
+      const uint4 x = c.nvalid ? stk4[w4] : make_uint4(0, 0, 0, 0);
+      pc += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+      if (dst) reinterpret_cast<uint4*>(dst)[w4] = x;
+   }
+   if (count) {
+      pc = __reduce_add_sync(0xFFFFFFFFu, pc);
+      if ((threadIdx.x & 31) == 0 && pc) atomicAdd(count, static_cast<unsigned long long>(pc));
    }
    return true;
 }
 
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
-   v = __reduce_add_sync(0xFFFFFFFFu, v);
-   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   __syncthreads();
-   if (lane == 0) red[warp] = v;
-   __syncthreads();
-   uint32_t s = 0;
-   if (threadIdx.x == 0) {
-      for (uint32_t i = 0; i < (blockDim.x >> 5); ++i) s += red[i];
-   }
-   return s;  // valid in thread 0
-}
+// Dynamic shared memory of both kernels: the leaf cache, the scratch tile (of the widest tile), the stack tiles.
+constexpr size_t LC_BYTES = sizeof(LeafCache);
 
-// Popcount of the result tile (slot 0) by the owners of its words, optionally copied to dst.
-__device__ __forceinline__ uint32_t result_popc(const uint32_t* smem, uint32_t W, uint32_t* dst) {
-   const uint4* r4 = reinterpret_cast<const uint4*>(smem);
-   uint4* d4 = reinterpret_cast<uint4*>(dst);
-   uint32_t pc = 0;
-   for (uint32_t w4 = threadIdx.x; w4 < (W >> 7); w4 += blockDim.x) {
-      const uint4 x = r4[w4];
-      pc += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
-      if (dst) d4[w4] = x;
-   }
-   return pc;
-}
-
+template <bool TRACE>
 __global__ void __launch_bounds__(FT) filter_kernel(const DevTable* __restrict__ tab, const Instr* __restrict__ code,
                                                     uint32_t ncode, uint32_t n_leaves, uint32_t tile_bits, uint32_t cap,
                                                     uint32_t* __restrict__ out_tiles, unsigned long long* count, int* err,
                                                     uint32_t* trace, const uint32_t* __restrict__ aux) {
-   extern __shared__ __align__(16) uint32_t smem[];
-   __shared__ uint32_t red[FT / 32];
-   __shared__ LeafCache lc;
+   extern __shared__ __align__(16) uint8_t smem[];
+   LeafCache& lc = *reinterpret_cast<LeafCache*>(smem);
    const uint32_t T = CHUNK_ROWS / tile_bits;
    TileCtx c;
    c.tab = tab;
@@ -816,55 +936,59 @@ __global__ void __launch_bounds__(FT) filter_kernel(const DevTable* __restrict__
    c.aux = aux;
    const uint32_t csize = __ldg(tab->chunk_sizes + c.v);
    c.nvalid = csize > c.row0 ? min(tile_bits, csize - c.row0) : 0u;
-   if (c.nvalid == 0) {
-      for (uint32_t w4 = threadIdx.x; w4 < (tile_bits >> 7); w4 += blockDim.x)
-         reinterpret_cast<uint4*>(smem)[w4] = make_uint4(0, 0, 0, 0);
-   } else {
+   const uint32_t nl = min(n_leaves & 0xFFFFu, LC_LEAVES), ncov = min(n_leaves >> 16, LC_COV);
+   uint4* X4 = reinterpret_cast<uint4*>(smem + LC_BYTES);
+   uint4* stk4 = X4 + (tile_bits >> 7);
+   if (c.nvalid) {
       init_leaves(lc);
-      clear_leaves(lc, min(n_leaves & 0xFFFFu, LC_LEAVES), min(n_leaves >> 16, LC_COV));
+      if (threadIdx.x == 0) lc.pay_used = lc.ext_used = 0;
+#pragma unroll 1
+      for (uint32_t w4 = threadIdx.x; w4 < (tile_bits >> 7); w4 += blockDim.x) X4[w4] = make_uint4(0, 0, 0, 0);
       __syncthreads();
       uint32_t phase = 0;
-      if (!stage_leaves(lc, c, code, ncode, phase, err)) return;
-      if (!run_program(c, code, ncode, smem, cap, lc, err,
-                       trace ? trace + static_cast<size_t>(blockIdx.x) * ncode * 2 : nullptr))
-         return;
+      if (!stage_leaves(lc, c, code, ncode, nl, ncov, nullptr, 0, phase, nullptr, err)) return;
    }
-   const uint32_t pc =
-      result_popc(smem, tile_bits, out_tiles ? out_tiles + static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5) : nullptr);
-   if (count) {
-      const uint32_t s = block_sum(pc, red);
-      if (threadIdx.x == 0 && s) atomicAdd(count, static_cast<unsigned long long>(s));
-   }
+   uint32_t* dst = out_tiles ? out_tiles + static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5) : nullptr;
+   run_tile<TRACE>(c, code, ncode, stk4, cap, X4, lc, nl, ncov, dst, count, err,
+                   TRACE ? trace + static_cast<size_t>(blockIdx.x) * ncode * 2 : nullptr);
 }
 
-__global__ void __launch_bounds__(FT) filter_batch_kernel(const DevTable* __restrict__ tab, const Instr* __restrict__ code,
+// launch bounds: three CTAs per SM (at most 85 registers a thread; 64 for four cost 17%).
+__global__ void __launch_bounds__(FT, 3) filter_batch_kernel(const DevTable* __restrict__ tab, const Instr* __restrict__ code,
                                                           const QueryDesc* __restrict__ queries,
                                                           const WorkItem* __restrict__ items, uint32_t n_items,
-                                                          uint32_t stack_words, uint32_t* __restrict__ out_tiles,
-                                                          unsigned long long* counts, uint32_t* next_item, int* err,
+                                                          uint32_t scratch_bytes, uint32_t stack_bytes,
+                                                          uint32_t* __restrict__ out_tiles, unsigned long long* counts,
+                                                          uint32_t* next_item, int* err,
                                                           const uint32_t* __restrict__ aux) {
-   extern __shared__ __align__(16) uint32_t smem[];
-   __shared__ uint32_t red[FT / 32];
-   __shared__ uint32_t item_idx;
-   __shared__ LeafCache lc;
+   extern __shared__ __align__(16) uint8_t smem[];
+   LeafCache& lc = *reinterpret_cast<LeafCache*>(smem);
    const size_t per_query = static_cast<size_t>(tab->nchunks) * CHUNK_WORDS;
+   uint4* X4 = reinterpret_cast<uint4*>(smem + LC_BYTES);
+   uint8_t* stack = smem + LC_BYTES + scratch_bytes;
    init_leaves(lc);
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < scratch_bytes / 16; i += FT) X4[i] = make_uint4(0, 0, 0, 0);
    uint32_t phase = 0;
+   if (threadIdx.x == 0) lc.next_item = atomicAdd(next_item, 1u);
+#pragma unroll 1
    for (;;) {
-      if (threadIdx.x == 0) item_idx = atomicAdd(next_item, 1u);
+      // this thread's earlier shared-memory accesses (stack tiles, staged payloads of the previous
+      // item) are ordered before the bulk copies into the same memory issued after the barrier
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      if (threadIdx.x == 0) lc.pay_used = lc.ext_used = 0;
       __syncthreads();
-      const uint32_t it = item_idx;
+      const uint32_t it = lc.next_item;
       if (it >= n_items) return;
       const WorkItem wi = items[it];
       const QueryDesc q = queries[wi.query];
       const uint32_t tile_bits = q.tile_bits, T = CHUNK_ROWS / tile_bits;
-      const uint32_t cap = stack_words / (tile_bits >> 5);  // stack tiles of this width
-      // the program uses q.depth stack tiles; the CTA's other tiles take this item's payloads
-      const uint32_t depth = min(max(q.depth, 1u), cap);
-      const uint32_t ext_cap = min((cap - depth) * (tile_bits / 16), 65535u - LC_PAY - 16u) & ~7u;
-      clear_leaves(lc, min(q.n_leaves & 0xFFFFu, LC_LEAVES), min(q.n_leaves >> 16, LC_COV),
-                   reinterpret_cast<uint16_t*>(smem + static_cast<size_t>(depth) * (tile_bits >> 5)), ext_cap);
-      __syncthreads();
+      // the program uses q.depth - 1 stack tiles; the CTA's other tiles take this item's payloads
+      const uint32_t cap = stack_bytes / (tile_bits >> 3);
+      const uint32_t tiles = min(max(q.depth, 2u) - 1u, cap);
+      uint16_t* ext = reinterpret_cast<uint16_t*>(stack + static_cast<size_t>(tiles) * (tile_bits >> 3));
+      const uint32_t ext_cap = (cap - tiles) * (tile_bits / 16);
+      const uint32_t nl = min(q.n_leaves & 0xFFFFu, LC_LEAVES), ncov = min(q.n_leaves >> 16, LC_COV);
       TileCtx c;
       c.tab = tab;
       c.v = wi.tile / T;
@@ -873,22 +997,60 @@ __global__ void __launch_bounds__(FT) filter_batch_kernel(const DevTable* __rest
       c.aux = aux ? aux + static_cast<size_t>(q.aux_base) * per_query : nullptr;
       const uint32_t csize = __ldg(tab->chunk_sizes + c.v);
       c.nvalid = csize > c.row0 ? min(tile_bits, csize - c.row0) : 0u;
-      if (c.nvalid == 0) {
-         for (uint32_t w4 = threadIdx.x; w4 < (tile_bits >> 7); w4 += blockDim.x)
-            reinterpret_cast<uint4*>(smem)[w4] = make_uint4(0, 0, 0, 0);
+      const Instr* prog = code + q.code_off;
+      if (c.nvalid) {
+         if (!stage_leaves(lc, c, prog, q.code_len, nl, ncov, ext, ext_cap, phase, next_item, err)) return;
       } else {
-         if (!stage_leaves(lc, c, code + q.code_off, q.code_len, phase, err)) return;
-         // the stack may not grow past the program's depth into the staged payloads
-         if (!run_program(c, code + q.code_off, q.code_len, smem, depth, lc, err)) return;
+         __syncthreads();  // every thread has read lc.next_item
+         if (threadIdx.x == 0) lc.next_item = atomicAdd(next_item, 1u);
       }
       uint32_t* dst = q.out_tiles ? out_tiles + static_cast<size_t>(q.out_tiles - 1) * per_query +
                                        static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5)
                                   : nullptr;
-      const uint32_t pc = result_popc(smem, tile_bits, dst);
-      const uint32_t s = block_sum(pc, red);
-      if (threadIdx.x == 0 && s) atomicAdd(counts + wi.query, static_cast<unsigned long long>(s));
-      __syncthreads();
+      unsigned long long* count = counts + wi.query;
+      uint4* stk4 = reinterpret_cast<uint4*>(stack);
+      // the stack may not grow past the program's tiles into the staged payloads
+      const bool ok = run_tile<false>(c, prog, q.code_len, stk4, tiles, X4, lc, nl, ncov, dst, count, err);
+      if (!ok) return;
    }
+}
+
+// Planes of a date column: one warp per word of 32 rows, a ballot per plane.
+__global__ void __launch_bounds__(256) date_index_kernel(const int32_t* __restrict__ days, uint32_t n, uint32_t words,
+                                                         const DevDateCol col, uint32_t* planes, uint32_t* nulls) {
+   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+   if (w >= words) return;  // the whole warp leaves
+   const uint32_t g = 32 * w + lane;
+   const int32_t day = g < n ? days[g] : INT32_MIN;
+   const bool has = day != INT32_MIN;
+   const uint32_t x = has ? static_cast<uint32_t>(day - col.base) : 0u, m = (1u << col.width) - 1u;
+#pragma unroll 1
+   for (uint32_t k = 0; k <= col.last; ++k) {
+      const uint32_t digit = (x >> (col.width * (k >> col.width))) & m;
+      const uint32_t b = __ballot_sync(0xFFFFFFFFu, has && digit <= (k & m));
+      if (lane == 0) planes[static_cast<size_t>(k) * words + w] = b;
+   }
+   const uint32_t b = __ballot_sync(0xFFFFFFFFu, g < n && !has);
+   if (lane == 0) nulls[w] = b;
+}
+
+// Dense forms of the filter path: one CTA per array of at least DENSE_MIN rows writes its bitset.
+__global__ void __launch_bounds__(256) dense_forms_kernel(uint16_t* arena, const DenseJob* __restrict__ jobs) {
+   __shared__ uint4 tile[CHUNK_WORDS / 4];
+   const DenseJob j = jobs[blockIdx.x];
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < CHUNK_WORDS / 4; i += blockDim.x) tile[i] = make_uint4(0, 0, 0, 0);
+   __syncthreads();
+   uint32_t* t = reinterpret_cast<uint32_t*>(tile);
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < j.card; i += blockDim.x) {
+      const uint32_t r = arena[j.src + i];
+      atomicOr(&t[r >> 5], 1u << (r & 31));
+   }
+   __syncthreads();
+   uint4* dst = reinterpret_cast<uint4*>(arena + j.dst);
+#pragma unroll 1
+   for (uint32_t i = threadIdx.x; i < CHUNK_WORDS / 4; i += blockDim.x) dst[i] = tile[i];
 }
 }  // namespace
 
@@ -898,41 +1060,55 @@ __global__ void __launch_bounds__(FT) filter_batch_kernel(const DevTable* __rest
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
                           uint32_t n_leaves, uint32_t tile_bits, uint32_t stack_tiles, uint32_t* d_out_tiles, unsigned long long* d_count,
                           int* d_err, void* stream, uint32_t* d_trace, const uint32_t* d_aux) {
-   const uint32_t T = CHUNK_ROWS / tile_bits;
-   const size_t smem = static_cast<size_t>(stack_tiles) * (tile_bits / 8);
-   cudaError_t e = cudaFuncSetAttribute(filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem > 48 * 1024 ? smem : 48 * 1024));
+   const uint32_t grid = nchunks * (CHUNK_ROWS / tile_bits);
+   const uint32_t threads = std::max(32u, std::min(FT, tile_bits / 128));
+   const size_t smem = LC_BYTES + static_cast<size_t>(std::max(stack_tiles, 1u)) * (tile_bits / 8);
+   const auto kernel = d_trace ? filter_kernel<true> : filter_kernel<false>;
+   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
    if (e != cudaSuccess) return e;
-   filter_kernel<<<nchunks * T, FT, smem, static_cast<cudaStream_t>(stream)>>>(
-      d_table, d_code, ncode, n_leaves, tile_bits, stack_tiles, d_out_tiles, d_count, d_err, d_trace, d_aux);
+   kernel<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(d_table, d_code, ncode, n_leaves, tile_bits,
+                                                                      stack_tiles - 1, d_out_tiles, d_count, d_err, d_trace,
+                                                                      d_aux);
    return cudaGetLastError();
 }
 
-int filter_batch_blocks_per_sm(size_t smem_bytes) {
-   if (cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            static_cast<int>(smem_bytes > 48 * 1024 ? smem_bytes : 48 * 1024)) != cudaSuccess) {
+int filter_batch_blocks_per_sm(size_t scratch_bytes, size_t stack_bytes) {
+   const size_t smem = LC_BYTES + scratch_bytes + stack_bytes;
+   if (cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+       cudaSuccess) {
       cudaGetLastError();
       return 1;
    }
    int n = 0;
-   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, filter_batch_kernel, FT, smem_bytes) != cudaSuccess) {
+   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, filter_batch_kernel, FT, smem) != cudaSuccess) {
       cudaGetLastError();
       return 1;
    }
    return n > 0 ? n : 1;
 }
 
-cudaError_t launch_filter_batch(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, const QueryDesc* d_queries,
-                         const WorkItem* d_items, uint32_t n_items, uint32_t stack_bytes, uint32_t* d_out_tiles,
-                         unsigned long long* d_counts, uint32_t* d_next, uint32_t grid, int* d_err, void* stream,
-                         const uint32_t* d_aux) {
-   (void)nchunks;
-   const size_t smem = stack_bytes;
-   cudaError_t e = cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem > 48 * 1024 ? smem : 48 * 1024));
+cudaError_t launch_filter_batch(const DevTable* d_table, const Instr* d_code, const QueryDesc* d_queries,
+                         const WorkItem* d_items, uint32_t n_items, uint32_t scratch_bytes, uint32_t stack_bytes,
+                         uint32_t* d_out_tiles, unsigned long long* d_counts, uint32_t* d_next, uint32_t grid, int* d_err,
+                         void* stream, const uint32_t* d_aux) {
+   const size_t smem = LC_BYTES + scratch_bytes + stack_bytes;
+   cudaError_t e =
+      cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
    if (e != cudaSuccess) return e;
    filter_batch_kernel<<<grid, FT, smem, static_cast<cudaStream_t>(stream)>>>(
-      d_table, d_code, d_queries, d_items, n_items, stack_bytes / 4, d_out_tiles, d_counts, d_next, d_err, d_aux);
+      d_table, d_code, d_queries, d_items, n_items, scratch_bytes, stack_bytes, d_out_tiles, d_counts, d_next, d_err, d_aux);
+   return cudaGetLastError();
+}
+
+cudaError_t launch_date_index(const int32_t* d_days, uint32_t n, uint32_t words, const DevDateCol& col, void* stream) {
+   date_index_kernel<<<(words + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      d_days, n, words, col, const_cast<uint32_t*>(col.planes), const_cast<uint32_t*>(col.nulls));
+   return cudaGetLastError();
+}
+
+cudaError_t launch_dense_forms(uint16_t* d_arena, const DenseJob* d_jobs, uint32_t n, void* stream) {
+   if (n == 0) return cudaSuccess;
+   dense_forms_kernel<<<n, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_arena, d_jobs);
    return cudaGetLastError();
 }
 

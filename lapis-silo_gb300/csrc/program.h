@@ -27,15 +27,37 @@ enum OpCode : uint8_t {
    OP_OR = 9,            // pop y, pop x, push x | y
    OP_NOT = 10,          // pop x, push valid & ~x
    OP_THR_BEGIN = 11,    // a = planes: push `a` zero counter planes
-   OP_THR_ADD = 12,      // a = planes, flags&1 = negated child: pop x, saturating count += x (or ~x)
+   OP_THR_ADD = 12,      // a = planes, flags&1 = negated child: pop x, count += x (or ~x). The top plane is
+                         // sticky: once a count reaches 2^(a-1) it stays above n, whatever is added
    OP_THR_END = 13,      // a = planes, b = n, flags&1 = exactly: pop planes, push count >= n (== n)
    OP_JZ = 14,           // a = target: jump if the top tile is all zero
    OP_JFULL = 15,        // a = target: jump if the top tile holds every valid row
+   OP_GROUP = 17,        // the next a instructions are row-list leaves applied together (see group_leaves):
+                         // b = first container leaf | their number << 16, c = first coverage leaf |
+                         // their number << 16 (the container leaves come first); flags: GroupFlags
    OP_PUSH_AUX = 16,     // a = index of a row set computed (a MutationProfile) or uploaded (a caller's row
                          // set, flags & AUX_LITERAL) before the program runs
 };
 
 constexpr uint16_t AUX_LITERAL = 1;  // PUSH_AUX of a caller's row set
+
+constexpr bool is_leaf(uint8_t op) { return op <= OP_PUSH_DATE || op == OP_PUSH_AUX; }
+
+// A leaf whose value the next instruction consumes at once is one instruction: bits 8..10 of the
+// leaf's flags name the operator applied to the top of the stack (AND, ANDNOT, OR) or to the counter
+// planes on top of it (THR_ADD, with the leaf's complement for FUSE_THR_ADD_NOT), bits 11..15 the
+// number of planes. See fuse_leaves.
+enum FuseOp : uint32_t {
+   FUSE_NONE = 0,
+   FUSE_AND = 1,
+   FUSE_ANDNOT = 2,
+   FUSE_OR = 3,
+   FUSE_THR_ADD = 4,
+   FUSE_THR_ADD_NOT = 5,
+};
+constexpr uint32_t leaf_fused(uint16_t flags) { return (flags >> 8) & 7u; }
+constexpr uint32_t leaf_planes(uint16_t flags) { return (flags >> 11) & 31u; }
+constexpr uint16_t fuse_flags(FuseOp op, uint32_t planes) { return static_cast<uint16_t>((op << 8) | (planes << 11)); }
 
 // Comparators of the date predicate (reference: src/rhydb/query_engine/filter/operators/selection.h:40-72).
 enum CmpCode : uint32_t { CMP_EQ = 0, CMP_NE = 1, CMP_LT = 2, CMP_LE = 3, CMP_GT = 4, CMP_GE = 5 };
@@ -49,6 +71,12 @@ struct Instr {
    uint32_t c;
 };
 static_assert(sizeof(Instr) == 16, "instruction layout");
+
+// How a leaf's rows reach their target: set in the top tile, removed from it, or counted in the planes.
+enum RowOp : int { A_OR = 0, A_ANDNOT = 1, A_ADD = 2 };
+// OP_GROUP flags: bits 0..1 the RowOp, bit 2: a new tile first (empty for A_OR, every valid row for
+// A_ANDNOT), bits 11..15 the planes of A_ADD (as in a leaf's flags).
+constexpr uint16_t GROUP_PUSH = 4;
 
 constexpr uint32_t MAX_PROGRAM = 4096;   // instructions per program
 constexpr uint32_t MAX_THR_PLANES = 16;  // counter planes (NOf up to 65,534 children)

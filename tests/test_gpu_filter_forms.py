@@ -1,0 +1,95 @@
+"""The forms a filter leaf takes on the device, at the sizes where they can go wrong, against the oracle:
+grouped row lists and their counters at every tile width, thresholds around the counters' sticky plane,
+arrays stored as bitsets, the digits of the date index, and the row lists of coverage leaves at the
+edges of position blocks. Row sets and counts are equal bit for bit."""
+import numpy as np
+import pytest
+
+import rhydb_gpu as R
+from rawtable import RawBuilder, accession_table, oracle_for
+
+pytestmark = pytest.mark.gpu
+
+
+def check(dev, orc, queries):
+    want = []
+    for q in queries:
+        bits, n = dev.compute_filter(q)
+        obits, on = orc.compute_filter(q)
+        assert n == on and np.array_equal(bits, obits), q
+        want.append(on)
+    counts, _ = dev.batch(queries)
+    assert counts.tolist() == want
+    return want
+
+
+@pytest.fixture(scope="module")
+def dense():
+    """140,000 rows over few sites: bitsets, arrays on both sides of the dense limit, null rows, a
+    ragged last chunk."""
+    t = R.Table.generate(140000, seed=21, genome_len=600, pool_sites=120, n_aa_genes=2, null_fraction=0.01)
+    dev = R.Device(t, 0)
+    yield t, dev, oracle_for(t)
+    dev.close()
+
+
+@pytest.mark.parametrize("width", [4096, 8192, 16384, 32768, 65536])
+def test_trees_at_every_tile_width(dense, width):
+    t, dev, orc = dense
+    qs = t.queries(40, seed=width, max_nof_children=24, max_leaves=48, use_aa=True, use_metadata=True)
+    want = check(dev, orc, qs)
+    own = R.Device(t, 0)  # set_tile_bits sets the widths of both paths
+    own.set_tile_bits(width)
+    assert check(own, orc, qs) == want
+    own.close()
+    counts, _ = dev.batch(qs, tile_bits=width)
+    assert counts.tolist() == want
+
+
+@pytest.mark.parametrize("children", [2, 3, 7, 8, 15, 16])
+def test_thresholds_around_the_sticky_plane(dense, children):
+    t, dev, orc = dense
+    pos, chunk, sym, card, _ = t.containers(0)
+    rows = {p: int(card[pos == p].sum()) for p in np.unique(pos)}
+    common = sorted(rows, key=lambda p: -rows[p])[:children]  # the densest sites: counts pass every n
+    qs = []
+    for n in range(1, children):
+        leaves = [f"HasMut(main,{p + 1})" for p in common]
+        leaves[0] = f"Not({leaves[0]})"
+        for kind in ("atleast", "exactly"):
+            qs.append(f"NOf({n},{kind},{','.join(leaves)})")
+            qs.append(f"NOf({n},{kind},{','.join(leaves[1:])},SymEq(main,{common[0] + 1},N))")
+    check(dev, orc, qs)
+
+
+@pytest.mark.parametrize("span", [0, 1, 127, 128, 16383, 16384, 2097151, 2097152])
+def test_date_index_digits(span):
+    n, base = 3000, 1000
+    rng = np.random.default_rng(span)
+    days = [None if i % 11 == 3 else base + int(rng.integers(0, span + 1)) for i in range(n)]
+    days[0], days[1] = base, base + span
+    b = RawBuilder(n).add_sequences("main", 0, "ACGT", ["ACGT"] * n).add_dates("date", days)  # owns raw's buffers
+    raw = b.raw()
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    ends = sorted({base - 1, base, base + 1, base + span // 2, base + span - 1, base + span, base + span + 1,
+                   base + (span & 127), base + (span | 127), base + (span & ~127) - 1, base + 127, base + 128})
+    qs = [f"DateBetween(date,{a},{b})" for a in ends for b in ends if a <= b]
+    qs += [f"DateBetween(date,*,{b})" for b in ends] + [f"DateBetween(date,{a},*)" for a in ends]
+    qs += [f"Not({q})" for q in qs[:20]] + [f"NOf(2,exactly,{qs[0]},{qs[-1]},{qs[len(qs) // 2]})"]
+    check(dev, orc, qs)
+    dev.close()
+
+
+def test_coverage_lists_at_block_edges():
+    b, raw, _ = accession_table(n_rows=3000, L=300, seed=9)
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    qs = []
+    for p in (1, 2, 19, 20, 126, 127, 128, 129, 130, 255, 256, 257, 281, 299, 300):
+        c = t.local_reference(0)[p - 1]
+        qs += [f"SymEq(main,{p},N)", f"SymEq(main,{p},{c})", f"Not(SymEq(main,{p},{c}))", f"Maybe(SymEq(main,{p},A))",
+               f"Or(SymEq(main,{p},N),SymEq(main,{301 - p},{t.local_reference(0)[300 - p]}))",
+               f"NOf(2,atleast,SymEq(main,{p},N),SymEq(main,{p},{c}),Not(SymEq(main,{301 - p},N)),HasMut(main,{p}))"]
+    check(dev, orc, qs)
+    dev.close()
