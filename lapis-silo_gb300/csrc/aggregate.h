@@ -29,11 +29,12 @@ struct AggCount {
 };
 
 constexpr uint32_t AGG_BLOCK = 4096;     // keys per block of the compaction
+constexpr uint64_t AGG_DENSE = 8192;     // up to this many keys the counters go to the host as they are
 constexpr uint64_t AGG_MAX_KEYS = 1ull << 26;  // dense key space at most (256 MiB of counters)
 
 // counters[key] += 1 for every row of the filter (dense, nchunks * CHUNK_WORDS words).
-void launch_agg_keys(const DevTable* d_table, uint32_t nchunks, const uint32_t* d_filter, const AggDim* d_dims,
-                     uint32_t nd, uint32_t* d_counters, void* stream);
+cudaError_t launch_agg_keys(const DevTable* d_table, uint32_t nchunks, const uint32_t* d_filter, const AggDim* d_dims,
+                            uint32_t nd, uint64_t keys, uint32_t* d_counters, void* stream);
 // Nonzero counters per block of AGG_BLOCK keys, then their (key, count) at the blocks' offsets.
 void launch_agg_nonzero(const uint32_t* d_counters, uint64_t keys, uint32_t* d_block_nonzero, void* stream);
 void launch_agg_write(const uint32_t* d_counters, uint64_t keys, const uint32_t* d_block_off, AggCount* d_out,

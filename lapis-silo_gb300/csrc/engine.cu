@@ -475,6 +475,7 @@ Engine::~Engine() {
    if (h_code_) cudaFreeHost(h_code_);
    if (h_count_) cudaFreeHost(h_count_);
    if (h_err_) cudaFreeHost(h_err_);
+   if (h_agg_) cudaFreeHost(h_agg_);
    if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -1629,25 +1630,37 @@ void Engine::aggregate(const Program& p, const std::vector<AggSpec>& spec, std::
    cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream), "memset");
    cuda_check(cudaMemsetAsync(d_agg_counters_, 0, keys * sizeof(uint32_t), stream), "memset");
    launch_count(d_code, p, d_count, d_filter, stream);
-   launch_agg_keys(d_table_, nchunks(), d_filter, d_agg_dims_, static_cast<uint32_t>(dims.size()), d_agg_counters_,
-                   stream);
-   launch_agg_nonzero(d_agg_counters_, keys, d_agg_blocks_, stream);
-   cuda_check(cudaGetLastError(), "aggregation launch");
-   std::vector<uint32_t> block(nblocks);
-   cuda_check(cudaMemcpyAsync(block.data(), d_agg_blocks_, nblocks * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
-              "D2H");
+   cuda_check(launch_agg_keys(d_table_, nchunks(), d_filter, d_agg_dims_, static_cast<uint32_t>(dims.size()), keys,
+                              d_agg_counters_, stream),
+              "aggregation launch");
+   const bool dense = keys <= AGG_DENSE;  // the counters as they are: no compaction, no second round trip
+   if (dense) {
+      if (!h_agg_) cuda_check(cudaMallocHost(&h_agg_, AGG_DENSE * sizeof(uint32_t)), "cudaMallocHost");
+      cuda_check(cudaMemcpyAsync(h_agg_, d_agg_counters_, keys * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "D2H");
+   } else {
+      launch_agg_nonzero(d_agg_counters_, keys, d_agg_blocks_, stream);
+      cuda_check(cudaGetLastError(), "aggregation launch");
+   }
+   std::vector<uint32_t> block(dense ? 0 : nblocks);
+   if (!dense)
+      cuda_check(cudaMemcpyAsync(block.data(), d_agg_blocks_, nblocks * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
+                 "D2H");
    cuda_check(cudaMemcpyAsync(h_count_, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream), "D2H");
    cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "D2H");
    cuda_check(cudaStreamSynchronize(stream), "aggregation");
    check_error_flag();
    uint64_t total = 0;
-   for (uint64_t b = 0; b < nblocks; ++b) {
-      const uint32_t n = block[b];
-      block[b] = static_cast<uint32_t>(total);
-      total += n;
+   for (uint32_t& n : block) {
+      const uint32_t x = n;
+      n = static_cast<uint32_t>(total);
+      total += x;
    }
    std::vector<AggCount> out(total);
-   if (total) {
+   if (dense) {
+      for (uint64_t k = 0; k < keys; ++k)
+         if (h_agg_[k]) out.push_back({k, h_agg_[k], 0});
+      total = out.size();
+   } else if (total) {
       grow_device(d_agg_out_, agg_out_cap_, total);
       cuda_check(cudaMemcpyAsync(d_agg_blocks_, block.data(), nblocks * sizeof(uint32_t), cudaMemcpyHostToDevice, stream),
                  "H2D");

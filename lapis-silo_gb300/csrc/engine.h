@@ -352,6 +352,7 @@ class Engine {
    uint32_t* d_agg_counters_ = nullptr;
    uint32_t* d_agg_blocks_ = nullptr;
    AggCount* d_agg_out_ = nullptr;
+   uint32_t* h_agg_ = nullptr;             // pinned, AGG_DENSE counters
    size_t agg_dims_cap_ = 0, agg_counters_cap_ = 0, agg_blocks_cap_ = 0, agg_out_cap_ = 0;
    // MutationProfile row sets of the single-query path
    DevProfile* d_prof_ = nullptr;
