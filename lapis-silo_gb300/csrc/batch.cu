@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(MUT_SEG) mut_final_batch_kernel(const DevTable
       return;
    }
    uint32_t* c = counts + static_cast<size_t>(q) * cs->nsym * L;
-   final_position_counts(cs, total, c, scratch + static_cast<size_t>(q) * mut_scratch_words(L), red);
+   final_position_counts(cs, total, c, scratch + static_cast<size_t>(q) * mut_scratch_words(L));
    if (rowblk == nullptr) return;
    // each thread reads back its own position's counts (plain loads: it has just written one)
    const uint32_t p = blockIdx.x * MUT_SEG + threadIdx.x;

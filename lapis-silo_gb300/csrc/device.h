@@ -94,6 +94,7 @@ struct DevSeqCol {
    const uint32_t* mend;       // missing-interval end events
    const CovEvent* cstart;     // coverage starts > 0
    const CovEvent* cend;       // coverage ends < L
+   uint32_t n_cstart, n_cend;
    const uint32_t* hrow_off;   // row index: nchunks * CHUNK_ROWS + 1 offsets into hent
    const uint32_t* hent;       // row index entries (position << 5 | code)
    uint32_t L;
@@ -227,8 +228,7 @@ enum : uint32_t { BMUT_PART_TRANSPOSE = 1, BMUT_PART_CTR = 2, BMUT_PART_COV = 4,
 // of the container and coverage passes: their rows read their row-index entries.
 enum : uint32_t { MUT_PART_SPARSE = 8 };
 void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
-                      const EvItem* d_ev, uint32_t n_ev, const uint32_t* d_filter,
-                      const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
+                      const uint32_t* d_filter, const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
                       void* stream, uint32_t parts = MUT_PART_ALL | MUT_PART_SPARSE, uint64_t sparse_max = 0);
 // Testing the failure path of the filter kernels' bounded waits on the current device: while on,
 // the leaf payload copies they announce are never issued, so their waits give up and the kernels

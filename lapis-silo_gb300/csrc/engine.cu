@@ -381,6 +381,8 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          d.mend = upload(s.mend);
          d.cstart = upload(s.cstart);
          d.cend = upload(s.cend);
+         d.n_cstart = static_cast<uint32_t>(s.cstart.size());
+         d.n_cend = static_cast<uint32_t>(s.cend.size());
          d.hrow_off = upload(s.hrow_off);
          d.hent = upload(s.hent, s.hent.size() + 8);  // 8 entries of tail: the profile pass reads whole uint4 pairs
          // coverage-pass work items: event ranges of at most EV_PER_CTA, never spanning two blocks
@@ -621,8 +623,7 @@ void Engine::launch_count(const Instr* code, const Program& p, unsigned long lon
 void Engine::launch_mutations(int column, const uint32_t* filter, const unsigned long long* count, uint32_t* counts,
                               uint32_t* scratch, cudaStream_t stream, uint32_t parts) {
    const DevSeqCol& c = view_.seq[column];
-   rhygpu::launch_mutations(d_table_, c, static_cast<uint32_t>(column), nchunks(), d_ev_[column], n_ev_[column],
-                            filter, count, counts, scratch, d_err, stream, parts, sparse_rows_plain);
+   rhygpu::launch_mutations(d_table_, c, static_cast<uint32_t>(column), nchunks(), filter, count, counts, scratch, d_err, stream, parts, sparse_rows_plain);
    cuda_check(cudaGetLastError(), "mutations kernel launch");
 }
 

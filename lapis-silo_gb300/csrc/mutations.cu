@@ -4,9 +4,8 @@
 //                    chunk staged in shared memory; integer counts per (symbol, position)
 //                    (reference: mutations_node.cpp:139-189). A producer warp bulk-copies units of
 //                    at most WU array elements into a shared-memory ring that consumer warps count.
-//  mut_cov_kernel    rows of F outside their covered region and inside missing intervals, from
-//                    position-sorted start / end events aggregated per position with warp ballots
-//                    (reference: mutations_node.cpp:51-136).
+//  mut_cov_kernel    rows of F outside their covered region and inside missing intervals, as
+//                    differences over positions (reference: mutations_node.cpp:51-136).
 //  mut_final_kernel  prefix sums and the local-reference count per position
 //                    (reference: mutations_node.cpp:192-203).
 //  mut_sparse_kernel filters of few rows: each row of F adds its row-index entries, the same counts
@@ -415,81 +414,107 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
    }
 }
 
-// One CTA per event item. Missing events add +1 (start) / -1 (end) at their position; coverage
-// events count rows whose covered region starts (ends) there.
+// Coverage of the filter per position, as differences over positions (reference:
+// mutations_node.cpp:51-136). The first CTAs take COV_BLOCKS x COV_CHUNKS buckets of missing intervals
+// each (the lists of the coverage leaves: row, first position and end in one word per interval and
+// 128-position block): the chunks' filter tiles are staged in shared memory, a warp reads a bucket
+// and adds +1 / -1 at the block-local boundaries of the intervals whose row is in F to a shared
+// histogram; boundaries on the block's edges are counted in registers. The others count the rows of F
+// whose covered region starts (ends) at each position, one event per thread.
+// Bound: 4 bytes per interval (15.6 MB at 2M rows) and 8 KiB of filter per CTA and chunk. It replaced a
+// pass over position-sorted start and end events (31 MB), each testing a filter bit in L2: 58.8 us at
+// 2M rows and 400,000 filtered rows, one 32-byte sector per event.
+constexpr uint32_t COV_BLOCKS = 4, COV_CHUNKS = 4;
+constexpr uint32_t COV_EVENTS = 8 * MT;  // boundary events per CTA
 __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict__ tab, uint32_t col,
-                                                     const EvItem* __restrict__ items,
                                                      const uint32_t* __restrict__ filter,
                                                      const unsigned long long* __restrict__ fcount,
                                                      unsigned long long sparse_max, uint32_t* scratch) {
-   __shared__ int cnt[NBLOCK + 1];
+   __shared__ __align__(16) uint32_t F[COV_CHUNKS][CHUNK_WORDS];
+   __shared__ int hist[COV_BLOCKS][NBLOCK + 1];
    const unsigned long long fc = *fcount;
    if (fc == 0 || fc <= sparse_max) return;  // empty, or counted by the row-index pass
-   const bool full = fc == tab->n_rows;
    const DevSeqCol* cs = &tab->seq[col];
-   const uint32_t L = cs->L, nseg = mut_nseg(L);
+   const uint32_t L = cs->L, nseg = mut_nseg(L), nchunks = tab->nchunks, nblocks = cs->nblocks;
    uint32_t* start_hist = scratch;
    uint32_t* end_hist = scratch + (L + 1);
    uint32_t* ndiff = scratch + 2 * (L + 1);
    uint32_t* seg_s = scratch + 3 * (L + 1);
    uint32_t* seg_e = seg_s + nseg;
    uint32_t* seg_n = seg_e + nseg;
-   const EvItem it = items[blockIdx.x];
    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   if (it.list <= EV_MEND) {
-      for (uint32_t i = threadIdx.x; i <= NBLOCK; i += blockDim.x) cnt[i] = 0;
+   const uint32_t gv = (nchunks + COV_CHUNKS - 1) / COV_CHUNKS, gb = (nblocks + COV_BLOCKS - 1) / COV_BLOCKS;
+   if (blockIdx.x < gb * gv) {
+      const uint32_t b0 = blockIdx.x / gv * COV_BLOCKS, v0 = blockIdx.x % gv * COV_CHUNKS;
+      const uint32_t nv = min(COV_CHUNKS, nchunks - v0), nb = min(COV_BLOCKS, nblocks - b0);
+      const uint4* src = reinterpret_cast<const uint4*>(filter + static_cast<size_t>(v0) * CHUNK_WORDS);
+      for (uint32_t i = threadIdx.x; i < nv * (CHUNK_WORDS / 4); i += MT) reinterpret_cast<uint4*>(F[0])[i] = __ldg(src + i);
+      for (uint32_t i = threadIdx.x; i < COV_BLOCKS * (NBLOCK + 1); i += MT) hist[0][i] = 0;
       __syncthreads();
-      const uint32_t* ev = it.list == EV_MSTART ? cs->mstart : cs->mend;
-      constexpr uint32_t U = 4;  // events per lane in flight
-      for (uint32_t base = it.begin + warp * 32 * U; base < it.end; base += blockDim.x * U) {
-         uint32_t e[U], bit[U];
+      for (uint32_t j = warp; j < nb * nv; j += NW) {
+         const uint32_t bl = j / nv, v = j % nv;
+         const uint32_t* toff = cs->nblk_toff + (static_cast<size_t>(b0 + bl) * nchunks + v0 + v) * TOFF_N;
+         const uint32_t e0 = __ldg(toff) / 4, e1 = (__ldg(toff + TOFF_N - 1) + 3) / 4;  // buckets start on 16 bytes, zeros after
+         uint32_t at0 = 0, at_end = 0;
+         constexpr uint32_t U = 4;  // loads in flight per lane
+         for (uint32_t i0 = e0 + lane; i0 < e1; i0 += 32 * U) {
+            uint4 x[U];
 #pragma unroll
-         for (uint32_t k = 0; k < U; ++k) {
-            const uint32_t i = base + 32 * k + lane;
-            e[k] = i < it.end ? __ldg(ev + i) : 0xFFFFFFFFu;
-         }
+            for (uint32_t u = 0; u < U; ++u)
+               x[u] = i0 + 32 * u < e1 ? __ldg(reinterpret_cast<const uint4*>(cs->nblk) + i0 + 32 * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-         for (uint32_t k = 0; k < U; ++k) {
-            const uint32_t row = e[k] >> 8;
-            bit[k] = (e[k] != 0xFFFFFFFFu && (full || ((__ldg(filter + (row >> 5)) >> (row & 31)) & 1u))) ? 1u : 0u;
-         }
+            for (uint32_t u = 0; u < U; ++u) {
+               const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
 #pragma unroll
-         for (uint32_t k = 0; k < U; ++k) {
-            const bool active = e[k] != 0xFFFFFFFFu;
-            const uint32_t pos = e[k] & 0xFFu;
-            const uint32_t amask = __ballot_sync(0xFFFFFFFFu, active);
-            const uint32_t bits = __ballot_sync(0xFFFFFFFFu, bit[k]);
-            // lanes with equal positions form one group (events are sorted by position)
-            const uint32_t grp = __match_any_sync(0xFFFFFFFFu, active ? pos : 0xFFFFu) & amask;
-            if (active && lane == static_cast<uint32_t>(__ffs(grp) - 1)) {
-               const uint32_t n = __popc(bits & grp);
-               if (n) atomicAdd(&cnt[pos], static_cast<int>(n));
+               for (uint32_t k = 0; k < 4; ++k) {
+                  const uint32_t lo = (w[k] >> 16) & 0xFFu, hi = w[k] >> 24;
+                  const bool in = hi != 0 && ((F[v][(w[k] & 0xFFFFu) >> 5] >> (w[k] & 31u)) & 1u);
+                  if (!in) continue;
+                  if (lo == 0) ++at0;
+                  else atomicAdd(&hist[bl][lo], 1);
+                  if (hi == NBLOCK) ++at_end;
+                  else atomicSub(&hist[bl][hi], 1);
+               }
             }
          }
+         at0 = __reduce_add_sync(0xFFFFFFFFu, at0);
+         at_end = __reduce_add_sync(0xFFFFFFFFu, at_end);
+         if (lane == 0) {
+            atomicAdd(&hist[bl][0], static_cast<int>(at0));
+            atomicSub(&hist[bl][NBLOCK], static_cast<int>(at_end));
+         }
       }
       __syncthreads();
-      const int sign = it.list == EV_MSTART ? 1 : -1;
-      for (uint32_t q = threadIdx.x; q <= NBLOCK; q += blockDim.x) {
-         const int x = cnt[q];
-         const uint32_t p = it.block * NBLOCK + q;
-         if (x != 0 && p <= L) {
-            atomicAdd(&ndiff[p], static_cast<uint32_t>(sign * x));
-            atomicAdd(&seg_n[p / MUT_SEG], static_cast<uint32_t>(sign * x));
+      const uint32_t seg = b0 * NBLOCK / MUT_SEG;  // COV_BLOCKS * NBLOCK divides MUT_SEG: only the last edge may lie past it
+      for (uint32_t i0 = 0; i0 < nb * (NBLOCK + 1); i0 += MT) {
+         const uint32_t i = i0 + threadIdx.x;
+         const int x = i < nb * (NBLOCK + 1) ? hist[0][i] : 0;
+         const uint32_t p = (b0 + i / (NBLOCK + 1)) * NBLOCK + i % (NBLOCK + 1);
+         const bool add = x != 0 && p <= L;
+         if (add) {
+            atomicAdd(&ndiff[p], static_cast<uint32_t>(x));
+            if (p / MUT_SEG != seg) atomicAdd(&seg_n[p / MUT_SEG], static_cast<uint32_t>(x));
          }
+         const int s = __reduce_add_sync(0xFFFFFFFFu, add && p / MUT_SEG == seg ? x : 0);
+         if (lane == 0 && s) atomicAdd(&seg_n[seg], static_cast<uint32_t>(s));
       }
    } else {
-      const CovEvent* ev = it.list == EV_CSTART ? cs->cstart : cs->cend;
-      uint32_t* hist = it.list == EV_CSTART ? start_hist : end_hist;
-      uint32_t* seg = it.list == EV_CSTART ? seg_s : seg_e;
-      for (uint32_t i = it.begin + threadIdx.x; i < it.end; i += blockDim.x) {
-         const uint2 e = __ldg(reinterpret_cast<const uint2*>(ev) + i);
-         if (full || ((__ldg(filter + (e.x >> 5)) >> (e.x & 31)) & 1u)) {
-            atomicAdd(&hist[e.y], 1u);
-            atomicAdd(&seg[e.y / MUT_SEG], 1u);
-         }
+      const uint32_t ns = cs->n_cstart, n = ns + cs->n_cend;
+      const uint32_t base = (blockIdx.x - gb * gv) * COV_EVENTS;
+      for (uint32_t i0 = base; i0 < min(n, base + COV_EVENTS); i0 += MT) {
+         const uint32_t i = i0 + threadIdx.x;
+         const bool start = i < ns;
+         const uint2 e = i < n ? __ldg(reinterpret_cast<const uint2*>(start ? cs->cstart + i : cs->cend + (i - ns))) : make_uint2(0, 0);
+         const bool in = i < n && ((__ldg(filter + (e.x >> 5)) >> (e.x & 31)) & 1u);
+         if (in) atomicAdd((start ? start_hist : end_hist) + e.y, 1u);
+         // events are sorted by position: the lanes of a segment add once
+         const uint32_t key = in ? (start ? 0u : nseg) + e.y / MUT_SEG : 0xFFFFFFFFu;
+         const uint32_t same = __match_any_sync(0xFFFFFFFFu, key);
+         if (in && lane == static_cast<uint32_t>(__ffs(same) - 1)) atomicAdd(seg_s + key, static_cast<uint32_t>(__popc(same)));
       }
    }
 }
+static_assert(MUT_SEG % (COV_BLOCKS * NBLOCK) == 0, "a CTA's positions lie in one segment");
 
 // Filters of 1..sparse_max rows: one warp per 32 filter words at a time.
 __global__ void __launch_bounds__(MT) mut_sparse_kernel(const DevTable* __restrict__ tab, uint32_t col,
@@ -510,9 +535,7 @@ __global__ void __launch_bounds__(MT) mut_sparse_kernel(const DevTable* __restri
 __global__ void __launch_bounds__(MUT_SEG) mut_final_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                             const unsigned long long* __restrict__ fcount,
                                                             uint32_t* counts, const uint32_t* __restrict__ scratch) {
-   __shared__ uint32_t red[MUT_SEG / 32];
-   const DevSeqCol* cs = &tab->seq[col];
-   final_position_counts(cs, static_cast<uint32_t>(*fcount), counts, scratch, red);
+   final_position_counts(&tab->seq[col], static_cast<uint32_t>(*fcount), counts, scratch);
 }
 
 }  // namespace
@@ -531,7 +554,7 @@ void mutations_setup() {
 }
 
 void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
-                      const EvItem* d_ev, uint32_t n_ev, const uint32_t* d_filter,
+                      const uint32_t* d_filter,
                       const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
                       void* stream, uint32_t parts, uint64_t sparse_max) {
    cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -544,9 +567,13 @@ void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32
    if ((parts & MUT_PART_CTR) && col_host.nranges > 0)
       mut_ring_kernel<<<col_host.nranges, RING_T, RING_SMEM, s>>>(
          d_table, col, d_filter, d_filter_count, static_cast<unsigned long long>(sparse_max), d_counts, d_err);
-   if ((parts & MUT_PART_COV) && n_ev > 0)
-      mut_cov_kernel<<<n_ev, MT, 0, s>>>(d_table, col, d_ev, d_filter, d_filter_count,
-                                         static_cast<unsigned long long>(sparse_max), d_scratch);
+   if (parts & MUT_PART_COV) {
+      const uint32_t buckets =
+         ((nchunks + COV_CHUNKS - 1) / COV_CHUNKS) * ((col_host.nblocks + COV_BLOCKS - 1) / COV_BLOCKS);
+      const uint32_t events = (col_host.n_cstart + col_host.n_cend + COV_EVENTS - 1) / COV_EVENTS;
+      mut_cov_kernel<<<buckets + events, MT, 0, s>>>(d_table, col, d_filter, d_filter_count,
+                                                     static_cast<unsigned long long>(sparse_max), d_scratch);
+   }
    if (parts & MUT_PART_FINAL)
       mut_final_kernel<<<(col_host.L + MUT_SEG - 1) / MUT_SEG, MUT_SEG, 0, s>>>(d_table, col, d_filter_count, d_counts,
                                                                                d_scratch);
