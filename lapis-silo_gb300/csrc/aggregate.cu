@@ -49,21 +49,22 @@ __device__ __forceinline__ void tile_symbols(uint8_t* sym, const DevTable* __res
       if (r < AGG_TILE && ((e >> 16) & 0xFFu) <= q && q < (e >> 24)) sym[r] = missing;
    }
    const size_t slot = static_cast<size_t>(v) * cs->L + pos;
-   for (uint32_t c = __ldg(cs->off + slot); c < __ldg(cs->off + slot + 1); ++c) {
+   const uint32_t lane = threadIdx.x & 31;
+   for (uint32_t c = __ldg(cs->off + slot) + (threadIdx.x >> 5); c < __ldg(cs->off + slot + 1); c += AT / 32) {  // a warp each
       const uint4 raw = __ldg(reinterpret_cast<const uint4*>(cs->fctrs) + c);
       const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
       const uint16_t* p = cs->payload + d.payload;
       if (d.type == CT_BITSET) {
          const uint32_t* words = reinterpret_cast<const uint32_t*>(p) + (row0 >> 5);
-         for (uint32_t w = threadIdx.x; w < AGG_TILE / 32; w += AT)
+         for (uint32_t w = lane; w < AGG_TILE / 32; w += 32)
             for (uint32_t x = __ldg(words + w); x; x &= x - 1) sym[32 * w + (__ffs(x) - 1)] = d.sym;
       } else if (d.type == CT_ARRAY) {
-         for (uint32_t i = threadIdx.x; i <= d.card_m1; i += AT) {
+         for (uint32_t i = lane; i <= d.card_m1; i += 32) {
             const uint32_t r = static_cast<uint32_t>(__ldg(p + i)) - row0;
             if (r < AGG_TILE) sym[r] = d.sym;
          }
       } else {
-         for (uint32_t i = threadIdx.x; i < d.nruns; i += AT) {
+         for (uint32_t i = lane; i < d.nruns; i += 32) {
             const uint32_t s = __ldg(p + 2 * i), e = s + __ldg(p + 2 * i + 1) + 1u;
             for (uint32_t r = max(s, row0); r < min(e, row0 + AGG_TILE); ++r) sym[r - row0] = d.sym;
          }

@@ -238,12 +238,16 @@ void set_copy_withholding(bool on);
 // but withheld, so its consumers' waits give up and it sets DEVERR_WAIT_MUTATIONS.
 void set_ring_withholding(bool on);
 
-// One unit of the batched container pass: the containers of position `pos` in chunks [v0, v1),
-// at most CTR_UNIT_CHUNKS chunks and, unless a single chunk exceeds it, CTR_UNIT_ELEMENTS elements.
+// One unit of the batched container pass: the containers of position `pos` in chunks [v0, v1), at most
+// CTR_UNIT_CHUNKS chunks and CTR_UNIT_ELEMENTS elements. A chunk with more is cut into parts of its own:
+// each takes the bitset words [32 w0, 32 w1), the first one the arrays and runs too (a bitset of 30,000
+// rows is a thousand dependent steps for one warp: whole, such units set the kernel's time).
 struct CtrUnit {
    uint32_t pos;
    uint16_t v0, v1;
+   uint16_t w0, w1;
 };
+constexpr uint32_t CTR_WORD_GROUPS = CHUNK_WORDS / 32;
 constexpr uint32_t CTR_UNIT_CHUNKS = 32;
 constexpr uint32_t CTR_UNIT_ELEMENTS = 4096;
 

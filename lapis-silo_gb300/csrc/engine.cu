@@ -79,12 +79,20 @@ void* Engine::alloc(size_t bytes) {
 }
 
 // Work units of the batched container pass: per position, runs of consecutive chunks holding at
-// most CTR_UNIT_ELEMENTS container elements (a heavier chunk forms a unit of its own) and at most
+// most CTR_UNIT_ELEMENTS container elements (a heavier chunk forms units of its own) and at most
 // CTR_UNIT_CHUNKS chunks; positions without containers have none. Sorted by element count,
 // heaviest first, so the long units start in the first wave.
 std::vector<CtrUnit> container_units(const SeqColumnImage& s, uint32_t nchunks) {
    const ContainerSet& cs = s.vertical;
    std::vector<std::pair<uint32_t, CtrUnit>> units;
+   auto push = [&](uint32_t p, uint32_t v0, uint32_t v1, uint32_t acc) {
+      const uint32_t parts = v1 - v0 == 1 ? (acc + CTR_UNIT_ELEMENTS - 1) / CTR_UNIT_ELEMENTS : 1;
+      for (uint32_t k = 0; k < parts; ++k)
+         units.push_back({(acc + parts - 1) / parts,
+                          CtrUnit{p, static_cast<uint16_t>(v0), static_cast<uint16_t>(v1),
+                                  static_cast<uint16_t>(CTR_WORD_GROUPS * k / parts),
+                                  static_cast<uint16_t>(CTR_WORD_GROUPS * (k + 1) / parts)}});
+   };
    for (uint32_t p = 0; p < s.L; ++p) {
       uint32_t v0 = 0, acc = 0;
       for (uint32_t v = 0; v < nchunks; ++v) {
@@ -92,13 +100,13 @@ std::vector<CtrUnit> container_units(const SeqColumnImage& s, uint32_t nchunks) 
          for (uint32_t i = cs.off[static_cast<size_t>(v) * s.L + p]; i < cs.off[static_cast<size_t>(v) * s.L + p + 1]; ++i)
             w += cs.ctrs[i].card_m1 + 1u;
          if (v > v0 && (acc + w > CTR_UNIT_ELEMENTS || v - v0 == CTR_UNIT_CHUNKS)) {
-            if (acc) units.push_back({acc, CtrUnit{p, static_cast<uint16_t>(v0), static_cast<uint16_t>(v)}});
+            if (acc) push(p, v0, v, acc);
             v0 = v;
             acc = 0;
          }
          acc += w;
       }
-      if (acc) units.push_back({acc, CtrUnit{p, static_cast<uint16_t>(v0), static_cast<uint16_t>(nchunks)}});
+      if (acc) push(p, v0, nchunks, acc);
    }
    std::stable_sort(units.begin(), units.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
    std::vector<CtrUnit> out(units.size());

@@ -425,7 +425,6 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
 // pass over position-sorted start and end events (31 MB), each testing a filter bit in L2: 58.8 us at
 // 2M rows and 400,000 filtered rows, one 32-byte sector per event.
 constexpr uint32_t COV_BLOCKS = 4, COV_CHUNKS = 4;
-constexpr uint32_t COV_EVENTS = 8 * MT;  // boundary events per CTA
 __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                      const uint32_t* __restrict__ filter,
                                                      const unsigned long long* __restrict__ fcount,
@@ -437,11 +436,9 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
    const DevSeqCol* cs = &tab->seq[col];
    const uint32_t L = cs->L, nseg = mut_nseg(L), nchunks = tab->nchunks, nblocks = cs->nblocks;
    uint32_t* start_hist = scratch;
-   uint32_t* end_hist = scratch + (L + 1);
-   uint32_t* ndiff = scratch + 2 * (L + 1);
+   uint32_t* ndiff = scratch + 2 * (L + 1);  // (the ends' histogram lies between)
    uint32_t* seg_s = scratch + 3 * (L + 1);
-   uint32_t* seg_e = seg_s + nseg;
-   uint32_t* seg_n = seg_e + nseg;
+   uint32_t* seg_n = seg_s + 2 * nseg;
    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const uint32_t gv = (nchunks + COV_CHUNKS - 1) / COV_CHUNKS, gb = (nblocks + COV_BLOCKS - 1) / COV_BLOCKS;
    if (blockIdx.x < gb * gv) {
@@ -500,18 +497,17 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
       }
    } else {
       const uint32_t ns = cs->n_cstart, n = ns + cs->n_cend;
-      const uint32_t base = (blockIdx.x - gb * gv) * COV_EVENTS;
-      for (uint32_t i0 = base; i0 < min(n, base + COV_EVENTS); i0 += MT) {
-         const uint32_t i = i0 + threadIdx.x;
-         const bool start = i < ns;
-         const uint2 e = i < n ? __ldg(reinterpret_cast<const uint2*>(start ? cs->cstart + i : cs->cend + (i - ns))) : make_uint2(0, 0);
-         const bool in = i < n && ((__ldg(filter + (e.x >> 5)) >> (e.x & 31)) & 1u);
-         if (in) atomicAdd((start ? start_hist : end_hist) + e.y, 1u);
-         // events are sorted by position: the lanes of a segment add once
-         const uint32_t key = in ? (start ? 0u : nseg) + e.y / MUT_SEG : 0xFFFFFFFFu;
-         const uint32_t same = __match_any_sync(0xFFFFFFFFu, key);
-         if (in && lane == static_cast<uint32_t>(__ffs(same) - 1)) atomicAdd(seg_s + key, static_cast<uint32_t>(__popc(same)));
-      }
+      const uint32_t i = (blockIdx.x - gb * gv) * MT + threadIdx.x;  // one event per thread
+      const bool start = i < ns;
+      const uint2 e = i < n ? __ldg(reinterpret_cast<const uint2*>(start ? cs->cstart + i : cs->cend + (i - ns))) : make_uint2(0, 0);
+      const bool in = i < n && ((__ldg(filter + (e.x >> 5)) >> (e.x & 31)) & 1u);
+      // events are sorted by position: the lanes of a position, and those of a segment, add once
+      const uint32_t at = in ? (start ? 0u : L + 1) + e.y : 0xFFFFFFFFu;
+      const uint32_t same = __match_any_sync(0xFFFFFFFFu, at);
+      if (in && lane == static_cast<uint32_t>(__ffs(same) - 1)) atomicAdd(start_hist + at, static_cast<uint32_t>(__popc(same)));
+      const uint32_t key = in ? (start ? 0u : nseg) + e.y / MUT_SEG : 0xFFFFFFFFu;
+      const uint32_t segm = __match_any_sync(0xFFFFFFFFu, key);
+      if (in && lane == static_cast<uint32_t>(__ffs(segm) - 1)) atomicAdd(seg_s + key, static_cast<uint32_t>(__popc(segm)));
    }
 }
 static_assert(MUT_SEG % (COV_BLOCKS * NBLOCK) == 0, "a CTA's positions lie in one segment");
@@ -570,7 +566,7 @@ void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32
    if (parts & MUT_PART_COV) {
       const uint32_t buckets =
          ((nchunks + COV_CHUNKS - 1) / COV_CHUNKS) * ((col_host.nblocks + COV_BLOCKS - 1) / COV_BLOCKS);
-      const uint32_t events = (col_host.n_cstart + col_host.n_cend + COV_EVENTS - 1) / COV_EVENTS;
+      const uint32_t events = (col_host.n_cstart + col_host.n_cend + MT - 1) / MT;
       mut_cov_kernel<<<buckets + events, MT, 0, s>>>(d_table, col, d_filter, d_filter_count,
                                                      static_cast<unsigned long long>(sparse_max), d_scratch);
    }
