@@ -298,7 +298,8 @@ void Engine::upload_missing(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol
       }
       for (uint32_t k = 0; k < TOFF_N; ++k) toff[b * TOFF_N + k] = first + (s.nblk_toff[b * TOFF_N + k] - s.nblk_off[b]);
    }
-   d.nblk = upload(ent, ent.size() + 4);
+   while (ent.size() % 4) ent.push_back(0);  // the last bucket's tail is read too
+   d.nblk = upload(ent);
    d.nblk_toff = upload(toff);
 }
 
