@@ -88,35 +88,48 @@ __global__ void __launch_bounds__(AT) agg_keys_kernel(const DevTable* __restrict
    constexpr uint32_t T = CHUNK_ROWS / AGG_TILE, TW = AGG_TILE / 32;
    const uint32_t v = blockIdx.x / T, row0 = blockIdx.x % T * AGG_TILE;
    const uint32_t* Ft = F + static_cast<size_t>(v) * CHUNK_WORDS + (row0 >> 5);
-   uint32_t any = 0;
-   for (uint32_t w = threadIdx.x; w < TW; w += AT) any |= __ldg(Ft + w);
-   if (!__syncthreads_or(any != 0)) return;
+   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   // warp w owns the 32 row words from 32 w on, lane l holds the l-th; a step takes four of them, so that
+   // their loads are in flight together
+   static_assert(TW == AT, "one row word per thread");
+   const uint32_t Fw = __ldg(Ft + threadIdx.x);
+   const uint32_t busy = __ballot_sync(0xFFFFFFFFu, Fw != 0);
+   if (!__syncthreads_or(busy != 0)) return;
    if (hist)
       for (uint32_t k = threadIdx.x; k < keys; k += AT) local[k] = 0;
-   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    for (uint32_t d = 0; d < nd; ++d) {
       const AggDim dim = dims[d];
       const uint32_t stride = static_cast<uint32_t>(dim.stride);
       const DevSeqCol* cs = &tab->seq[dim.col];  // of a sequence dimension
       if (dim.kind == AGG_SEQUENCE) tile_symbols(sym, tab, cs, v, row0, dim.pos);
-      for (uint32_t w = warp; w < TW; w += AT / 32) {
-         if (!((__ldg(Ft + w) >> lane) & 1u)) continue;
-         const uint32_t r = 32 * w + lane, g0 = v * CHUNK_ROWS + row0 + r;
-         uint32_t g;
-         if (dim.kind == AGG_SEQUENCE) {
-            g = ((__ldg(cs->null_tiles + (g0 >> 5)) >> lane) & 1u) ? cs->nsym : sym[r];
-         } else {
-            const uint32_t id = __ldg(dim.ids + g0);
-            g = id == 0xFFFFFFFFu ? dim.ngroups - 1 : __ldg(dim.rank + id);
+      const uint32_t r0 = 1024 * warp + lane, g0 = v * CHUNK_ROWS + row0 + r0;
+      const uint32_t nulls = dim.kind == AGG_SEQUENCE ? __ldg(cs->null_tiles + (v * CHUNK_ROWS + row0) / 32 + threadIdx.x) : 0u;
+      for (uint32_t j0 = 0; j0 < 32; j0 += 4) {
+         if (!((busy >> j0) & 15u)) continue;  // four words without rows
+         uint32_t g[4];
+         bool in[4];
+#pragma unroll
+         for (uint32_t j = 0; j < 4; ++j) {
+            in[j] = (__shfl_sync(0xFFFFFFFFu, Fw, j0 + j) >> lane) & 1u;
+            const uint32_t null_word = __shfl_sync(0xFFFFFFFFu, nulls, j0 + j);
+            if (dim.kind == AGG_SEQUENCE) g[j] = ((null_word >> lane) & 1u) ? cs->nsym : sym[r0 + 32 * (j0 + j)];
+            else g[j] = in[j] ? __ldg(dim.ids + g0 + 32 * (j0 + j)) : 0xFFFFFFFFu;
          }
-         key[r] = (d ? key[r] : 0u) + g * stride;
+         if (dim.kind != AGG_SEQUENCE) {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) g[j] = g[j] == 0xFFFFFFFFu ? dim.ngroups - 1 : __ldg(dim.rank + g[j]);
+         }
+#pragma unroll
+         for (uint32_t j = 0; j < 4; ++j) {
+            uint32_t& k = key[r0 + 32 * (j0 + j)];
+            if (in[j]) k = (d ? k : 0u) + g[j] * stride;
+         }
       }
       __syncthreads();  // sym is rewritten by the next dimension
    }
-   for (uint32_t w = warp; w < TW; w += AT / 32) {
-      if (!((__ldg(Ft + w) >> lane) & 1u)) continue;
-      atomicAdd((hist ? local : counters) + key[32 * w + lane], 1u);
-   }
+   for (uint32_t j = 0; j < 32; ++j)
+      if ((__shfl_sync(0xFFFFFFFFu, Fw, j) >> lane) & 1u)
+         atomicAdd((hist ? local : counters) + key[1024 * warp + 32 * j + lane], 1u);
    if (!hist) return;
    __syncthreads();
    for (uint32_t k = threadIdx.x; k < keys; k += AT)
