@@ -64,6 +64,8 @@ struct DenseJob {
    uint32_t src, dst, card;  // u16 offsets of the array and of its bitset in the arena
 };
 
+constexpr uint32_t MEV_NONE = 0x00FF0000u;
+
 struct CovBound {
    uint32_t row;   // row within chunk
    uint32_t bound;
@@ -90,6 +92,13 @@ struct DevSeqCol {
    const uint32_t* nblk_toff;  // nblocks * nchunks * TOFF_N: tile row-range offsets into each nblk bucket
    const uint32_t* null_tiles; // nchunks * CHUNK_WORDS
    const uint8_t* local_ref;   // L
+   // Boundaries of the missing intervals by (128-position block, chunk), sorted by row, for the single-query
+   // coverage pass: row within the chunk | position in the block << 16 | 1 << 31 for an interval's first
+   // position, 0 for the one after its last; each bucket from a multiple of 4 entries on, padded with
+   // MEV_NONE; offsets per bucket.
+   const uint32_t* mev;
+   const uint32_t* mev_off;    // nblocks_ev * nchunks + 1
+   uint32_t nblocks_ev;        // blocks of the positions 0 .. L
    const uint32_t* mstart;     // missing-interval start events (row << 8 | position in block)
    const uint32_t* mend;       // missing-interval end events
    const CovEvent* cstart;     // coverage starts > 0

@@ -301,6 +301,48 @@ void Engine::upload_missing(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol
    while (ent.size() % 4) ent.push_back(0);  // the last bucket's tail is read too
    d.nblk = upload(ent);
    d.nblk_toff = upload(toff);
+   // the whole intervals' boundaries: counted, then placed in row order
+   d.nblocks_ev = s.L / NBLOCK + 1;
+   const size_t nb = static_cast<size_t>(d.nblocks_ev) * nchunks;
+   std::vector<uint32_t> off(nb + 1, 0);
+   auto each = [&](auto&& fn) {
+      for (uint32_t v = 0; v < nchunks; ++v)
+         for (uint32_t r = 0; r < CHUNK_ROWS; ++r) {
+            const size_t g = static_cast<size_t>(v) * CHUNK_ROWS + r;
+            for (uint32_t i = s.nrow_off[g]; i < s.nrow_off[g + 1]; ++i) {
+               const uint32_t a = s.nrow_start[i], z = s.nrow_end[i];
+               fn(static_cast<size_t>(a / NBLOCK) * nchunks + v, r | (a % NBLOCK) << 16 | 1u << 31);
+               fn(static_cast<size_t>(z / NBLOCK) * nchunks + v, r | (z % NBLOCK) << 16);
+            }
+         }
+   };
+   each([&](size_t b, uint32_t) { ++off[b + 1]; });
+   for (size_t b = 0; b < nb; ++b) off[b + 1] = off[b] + ((off[b + 1] + 3) & ~3u);
+   std::vector<uint32_t> at(off.begin(), off.end() - 1), mev(off[nb], MEV_NONE);
+   each([&](size_t b, uint32_t e) { mev[at[b]++] = e; });
+   d.mev = upload(mev);
+   d.mev_off = upload(off);
+}
+
+// Every row's distance to the local reference as a profile (DevSeqCol::home).
+void Engine::profile_home(const SeqColumnImage& s, uint32_t col) {
+   const Alphabet& A = alphabet(s.kind);
+   std::vector<uint2> terms(s.L + 1, make_uint2(0, 0));
+   uint32_t base = 0;
+   for (uint32_t p = 0; p < s.L; ++p) {
+      const uint32_t m = profile_mask(A, s.local_ref[p]), lbit = (m >> s.local_ref[p]) & 1u;
+      terms[p].x = m | lbit << 31;
+      terms[p + 1].y = terms[p].y + ((m >> A.missing) & 1u) - lbit;
+      base += lbit;
+   }
+   uint2* d_terms = nullptr;
+   cuda_check(cudaMalloc(&d_terms, terms.size() * sizeof(uint2)), "cudaMalloc");
+   cudaError_t e = cudaMemcpy(d_terms, terms.data(), terms.size() * sizeof(uint2), cudaMemcpyHostToDevice);
+   if (e == cudaSuccess)
+      e = launch_profile_home(d_table_, col, nchunks(), d_terms, base, const_cast<int32_t*>(view_.seq[col].home), stream_);
+   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+   cudaFree(d_terms);
+   cuda_check(e, "profile distances");
 }
 
 void Engine::upload_dates(const DateColumnImage& dc, uint32_t nchunks, DevDateCol& out) {

@@ -415,26 +415,25 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
 }
 
 // Coverage of the filter per position, as differences over positions (reference:
-// mutations_node.cpp:51-136). The first CTAs take COV_BLOCKS x COV_CHUNKS buckets of missing intervals
-// each (the lists of the coverage leaves: row, first position and end in one word per interval and
-// 128-position block): the chunks' filter tiles are staged in shared memory, a warp reads a bucket
-// and adds +1 / -1 at the block-local boundaries of the intervals whose row is in F to a shared
-// histogram; boundaries on the block's edges are counted in registers. The others count the rows of F
-// whose covered region starts (ends) at each position, one event per thread.
-// Bound: 4 bytes per interval (15.6 MB at 2M rows) and 8 KiB of filter per CTA and chunk. It replaced a
-// pass over position-sorted start and end events (31 MB), each testing a filter bit in L2: 58.8 us at
-// 2M rows and 400,000 filtered rows, one 32-byte sector per event.
+// mutations_node.cpp:51-136). The first CTAs take COV_BLOCKS x COV_CHUNKS buckets of missing-interval
+// boundaries each: the chunks' filter tiles are staged in shared memory, a warp reads a bucket and adds
+// +1 (first positions) or -1 (positions after the last) of the intervals whose row is in F to a shared
+// histogram. The others count the rows of F whose covered region starts (ends) at each position, one
+// event per thread.
+// Bound: 4 bytes and about 14 instructions per boundary (31 MB at 2M rows) and 8 KiB of filter per CTA and
+// chunk. Before, the same boundaries sorted by position over all chunks each tested a filter bit in L2:
+// 58.8 us at 2M rows and 400,000 filtered rows, one 32-byte sector per boundary.
 constexpr uint32_t COV_BLOCKS = 4, COV_CHUNKS = 4;
 __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                      const uint32_t* __restrict__ filter,
                                                      const unsigned long long* __restrict__ fcount,
                                                      unsigned long long sparse_max, uint32_t* scratch) {
    __shared__ __align__(16) uint32_t F[COV_CHUNKS][CHUNK_WORDS];
-   __shared__ int hist[COV_BLOCKS][NBLOCK + 1];
+   __shared__ int hist[COV_BLOCKS][NBLOCK];
    const unsigned long long fc = *fcount;
    if (fc == 0 || fc <= sparse_max) return;  // empty, or counted by the row-index pass
    const DevSeqCol* cs = &tab->seq[col];
-   const uint32_t L = cs->L, nseg = mut_nseg(L), nchunks = tab->nchunks, nblocks = cs->nblocks;
+   const uint32_t L = cs->L, nseg = mut_nseg(L), nchunks = tab->nchunks, nblocks = cs->nblocks_ev;
    uint32_t* start_hist = scratch;
    uint32_t* ndiff = scratch + 2 * (L + 1);  // (the ends' histogram lies between)
    uint32_t* seg_s = scratch + 3 * (L + 1);
@@ -446,53 +445,41 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
       const uint32_t nv = min(COV_CHUNKS, nchunks - v0), nb = min(COV_BLOCKS, nblocks - b0);
       const uint4* src = reinterpret_cast<const uint4*>(filter + static_cast<size_t>(v0) * CHUNK_WORDS);
       for (uint32_t i = threadIdx.x; i < nv * (CHUNK_WORDS / 4); i += MT) reinterpret_cast<uint4*>(F[0])[i] = __ldg(src + i);
-      for (uint32_t i = threadIdx.x; i < COV_BLOCKS * (NBLOCK + 1); i += MT) hist[0][i] = 0;
+      for (uint32_t i = threadIdx.x; i < COV_BLOCKS * NBLOCK; i += MT) hist[0][i] = 0;
       __syncthreads();
       for (uint32_t j = warp; j < nb * nv; j += NW) {
          const uint32_t bl = j / nv, v = j % nv;
-         const uint32_t* toff = cs->nblk_toff + (static_cast<size_t>(b0 + bl) * nchunks + v0 + v) * TOFF_N;
-         const uint32_t e0 = __ldg(toff) / 4, e1 = (__ldg(toff + TOFF_N - 1) + 3) / 4;  // buckets start on 16 bytes, zeros after
-         uint32_t at0 = 0, at_end = 0;
-         constexpr uint32_t U = 4;  // loads in flight per lane
-         for (uint32_t i0 = e0 + lane; i0 < e1; i0 += 32 * U) {
+         const uint32_t* off = cs->mev_off + static_cast<size_t>(b0 + bl) * nchunks + v0 + v;
+         const uint32_t e0 = __ldg(off) / 4, e1 = __ldg(off + 1) / 4;
+         const uint4* ev = reinterpret_cast<const uint4*>(cs->mev);
+         constexpr uint32_t U = 4;  // loads in flight per lane: about 270 boundaries per bucket
+         for (uint32_t i0 = e0; i0 < e1; i0 += 32 * U) {
             uint4 x[U];
 #pragma unroll
-            for (uint32_t u = 0; u < U; ++u)
-               x[u] = i0 + 32 * u < e1 ? __ldg(reinterpret_cast<const uint4*>(cs->nblk) + i0 + 32 * u) : make_uint4(0, 0, 0, 0);
+            for (uint32_t u = 0; u < U; ++u) {
+               const uint32_t i = i0 + 32 * u + lane;
+               x[u] = i < e1 ? __ldg(ev + i) : make_uint4(MEV_NONE, MEV_NONE, MEV_NONE, MEV_NONE);
+            }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
+               if (i0 + 32 * u >= e1) break;
                const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
 #pragma unroll
                for (uint32_t k = 0; k < 4; ++k) {
-                  const uint32_t lo = (w[k] >> 16) & 0xFFu, hi = w[k] >> 24;
-                  const bool in = hi != 0 && ((F[v][(w[k] & 0xFFFFu) >> 5] >> (w[k] & 31u)) & 1u);
-                  if (!in) continue;
-                  if (lo == 0) ++at0;
-                  else atomicAdd(&hist[bl][lo], 1);
-                  if (hi == NBLOCK) ++at_end;
-                  else atomicSub(&hist[bl][hi], 1);
+                  const uint32_t in = F[v][(w[k] & 0xFFFFu) >> 5] >> (w[k] & 31u);
+                  const uint32_t p = (w[k] >> 16) & 0xFFu;
+                  if ((in & 1u) && p < NBLOCK) atomicAdd(&hist[bl][p], (w[k] >> 31) ? 1 : -1);
                }
             }
          }
-         at0 = __reduce_add_sync(0xFFFFFFFFu, at0);
-         at_end = __reduce_add_sync(0xFFFFFFFFu, at_end);
-         if (lane == 0) {
-            atomicAdd(&hist[bl][0], static_cast<int>(at0));
-            atomicSub(&hist[bl][NBLOCK], static_cast<int>(at_end));
-         }
       }
       __syncthreads();
-      const uint32_t seg = b0 * NBLOCK / MUT_SEG;  // COV_BLOCKS * NBLOCK divides MUT_SEG: only the last edge may lie past it
-      for (uint32_t i0 = 0; i0 < nb * (NBLOCK + 1); i0 += MT) {
-         const uint32_t i = i0 + threadIdx.x;
-         const int x = i < nb * (NBLOCK + 1) ? hist[0][i] : 0;
-         const uint32_t p = (b0 + i / (NBLOCK + 1)) * NBLOCK + i % (NBLOCK + 1);
-         const bool add = x != 0 && p <= L;
-         if (add) {
-            atomicAdd(&ndiff[p], static_cast<uint32_t>(x));
-            if (p / MUT_SEG != seg) atomicAdd(&seg_n[p / MUT_SEG], static_cast<uint32_t>(x));
-         }
-         const int s = __reduce_add_sync(0xFFFFFFFFu, add && p / MUT_SEG == seg ? x : 0);
+      const uint32_t seg = b0 * NBLOCK / MUT_SEG;  // COV_BLOCKS * NBLOCK divides MUT_SEG
+      for (uint32_t i = threadIdx.x; i < COV_BLOCKS * NBLOCK; i += MT) {
+         const int x = hist[0][i];
+         const uint32_t p = b0 * NBLOCK + i;  // at most L where x is not 0
+         if (x != 0) atomicAdd(&ndiff[p], static_cast<uint32_t>(x));
+         const int s = __reduce_add_sync(0xFFFFFFFFu, x);
          if (lane == 0 && s) atomicAdd(&seg_n[seg], static_cast<uint32_t>(s));
       }
    } else {
@@ -565,7 +552,7 @@ void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32
          d_table, col, d_filter, d_filter_count, static_cast<unsigned long long>(sparse_max), d_counts, d_err);
    if (parts & MUT_PART_COV) {
       const uint32_t buckets =
-         ((nchunks + COV_CHUNKS - 1) / COV_CHUNKS) * ((col_host.nblocks + COV_BLOCKS - 1) / COV_BLOCKS);
+         ((nchunks + COV_CHUNKS - 1) / COV_CHUNKS) * ((col_host.nblocks_ev + COV_BLOCKS - 1) / COV_BLOCKS);
       const uint32_t events = (col_host.n_cstart + col_host.n_cend + MT - 1) / MT;
       mut_cov_kernel<<<buckets + events, MT, 0, s>>>(d_table, col, d_filter, d_filter_count,
                                                      static_cast<unsigned long long>(sparse_max), d_scratch);
