@@ -104,6 +104,7 @@ struct DevSeqCol {
    const CovEvent* cstart;     // coverage starts > 0
    const CovEvent* cend;       // coverage ends < L
    uint32_t n_cstart, n_cend;
+   const int32_t* home;        // nchunks * CHUNK_ROWS: differences from the local reference (MutationProfile)
    const uint32_t* hrow_off;   // row index: nchunks * CHUNK_ROWS + 1 offsets into hent
    const uint32_t* hent;       // row index entries (position << 5 | code)
    uint32_t L;
@@ -182,17 +183,24 @@ struct QueryDesc {
    uint32_t tile_bits;    // rows per work item of this query (its class's tile width)
 };
 
-// A MutationProfile row set to compute before the filter programs (see ProfileSpec): the column,
-// the distance and the counting terms in device memory, terms[p] = (mask[p], diff[p]) for
-// p <= L (mask[L] = 0), so that any row-index entry needs one 8-byte load.
+// A MutationProfile row set to compute before the filter programs (see ProfileSpec): the column, the
+// distance and, in device memory, its differences from the local reference (n_delta of them, 16 bytes
+// each; terms null) or the counting terms, terms[p] = (mask[p], diff[p]) for p <= L (mask[L] = 0), so
+// that any row-index entry needs one 8-byte load.
 struct DevProfile {
-   uint32_t col, distance, base, pad;
+   uint32_t col, distance, base, n_delta;
    const uint2* terms;
+   const uint4* delta;  // ProfileDelta
 };
-// aux[k] (nchunks * CHUNK_WORDS words each) = the rows of profiles[k] within its distance.
-// max_L: the longest genome among the profiles' columns.
+// aux[k] (nchunks * CHUNK_WORDS words each) = the rows of profiles[k] within its distance. any_delta:
+// some profile is counted from its differences; max_L: the longest genome among the columns of the
+// others (0: none).
 void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile* d_profiles, uint32_t n,
-                     uint32_t max_L, uint32_t* d_aux, void* stream);
+                     bool any_delta, uint32_t max_L, uint32_t* d_aux, void* stream);
+// home[row] = the row's number of differences from the local reference (null rows: unused): base plus
+// its row-index entries' terms (as DevProfile's; Engine's upload).
+cudaError_t launch_profile_home(const DevTable* d_table, uint32_t col, uint32_t nchunks, const uint2* d_terms, uint32_t base,
+                                int32_t* d_home, void* stream);
 
 // ---- launchers (kernels.cu) ----
 // tile_bits: 4096, 8192, 16384, 32768 or 65536. stack_tiles: Program::tiles. n_leaves: container

@@ -34,30 +34,45 @@ void grow_host(T*& p, size_t n, size_t& cap) {
    cap = want;
 }
 // The profiles of a program as DevProfile entries whose arrays start at `base` (device memory of
-// profile_words(aux) words, 8-byte aligned) and the words to copy there: per profile the
-// interleaved (mask, diff) pairs of positions 0 .. L.
-uint32_t profile_max_L(const std::vector<std::shared_ptr<const ProfileSpec>>& aux) {
+// profile_words(aux) words, 16-byte aligned) and the words to copy there: per profile its differences, or
+// the interleaved (mask, diff) pairs of positions 0 .. L.
+using Profiles = std::vector<std::shared_ptr<const ProfileSpec>>;
+uint32_t profile_max_L(const Profiles& aux) {  // of the profiles counted from the row index
    uint32_t L = 0;
-   for (const auto& x : aux) L = std::max(L, static_cast<uint32_t>(x->mask.size()));
+   for (const auto& x : aux)
+      if (!x->use_delta) L = std::max(L, static_cast<uint32_t>(x->mask.size()));
    return L;
 }
-size_t profile_words(const std::vector<std::shared_ptr<const ProfileSpec>>& aux) {
+bool profile_any_delta(const Profiles& aux) {
+   return std::any_of(aux.begin(), aux.end(), [](const auto& x) { return x->use_delta; });
+}
+size_t profile_words(const ProfileSpec& x) {
+   return x.use_delta ? 4 * x.delta.size() : (2 * x.diff.size() + 3) & ~static_cast<size_t>(3);
+}
+size_t profile_words(const Profiles& aux) {
    size_t n = 0;
-   for (const auto& x : aux) n += 2 * x->diff.size();
+   for (const auto& x : aux) n += profile_words(*x);
    return n;
 }
-void pack_profiles(const std::vector<std::shared_ptr<const ProfileSpec>>& aux, const uint32_t* base,
-                   DevProfile* profs, uint32_t* data) {
+static_assert(sizeof(ProfileDelta) == 16, "a difference is one 16-byte load");
+void pack_profiles(const Profiles& aux, const uint32_t* base, DevProfile* profs, uint32_t* data) {
    size_t off = 0;
    for (size_t k = 0; k < aux.size(); ++k) {
       const ProfileSpec& x = *aux[k];
-      profs[k] = DevProfile{static_cast<uint32_t>(x.col), x.distance, x.base, 0,
-                            reinterpret_cast<const uint2*>(base + off)};
-      for (size_t p = 0; p < x.diff.size(); ++p) {
-         data[off + 2 * p] = p < x.mask.size() ? x.mask[p] : 0u;
-         data[off + 2 * p + 1] = x.diff[p];
+      const uint32_t* at = base + off;
+      const uint32_t col = static_cast<uint32_t>(x.col);
+      if (x.use_delta) {
+         profs[k] = DevProfile{col, x.distance, static_cast<uint32_t>(x.base_delta), static_cast<uint32_t>(x.delta.size()),
+                               nullptr, reinterpret_cast<const uint4*>(at)};
+         if (!x.delta.empty()) std::memcpy(data + off, x.delta.data(), x.delta.size() * sizeof(ProfileDelta));
+      } else {
+         profs[k] = DevProfile{col, x.distance, x.base, 0, reinterpret_cast<const uint2*>(at), nullptr};
+         for (size_t p = 0; p < x.diff.size(); ++p) {
+            data[off + 2 * p] = p < x.mask.size() ? x.mask[p] : 0u;
+            data[off + 2 * p + 1] = x.diff[p];
+         }
       }
-      off += 2 * x.diff.size();
+      off += profile_words(x);
    }
 }
 }  // namespace
@@ -488,8 +503,11 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          dict_by_rank_.push_back(std::move(by_rank));
       }
       for (size_t c = 0; c < t.date.size(); ++c) upload_dates(t.date[c], nchunks, view_.date[c]);
+      for (size_t c = 0; c < t.seq.size(); ++c)
+         view_.seq[c].home = static_cast<int32_t*>(alloc(static_cast<size_t>(nchunks) * CHUNK_ROWS * sizeof(int32_t)));
       d_table_ = static_cast<DevTable*>(alloc(sizeof(DevTable)));
       cuda_check(cudaMemcpy(d_table_, &view_, sizeof(DevTable), cudaMemcpyHostToDevice), "upload table view");
+      for (size_t c = 0; c < t.seq.size(); ++c) profile_home(t.seq[c], static_cast<uint32_t>(c));
 
       d_filter = static_cast<uint32_t*>(alloc(static_cast<size_t>(nchunks) * CHUNK_WORDS * 4));
       d_count = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long)));
@@ -529,6 +547,9 @@ Engine::~Engine() {
    if (h_count_) cudaFreeHost(h_count_);
    if (h_err_) cudaFreeHost(h_err_);
    if (h_agg_) cudaFreeHost(h_agg_);
+   if (h_prof_) cudaFreeHost(h_prof_);
+   if (h_prof_data_) cudaFreeHost(h_prof_data_);
+   if (prof_ev_) cudaEventDestroy(prof_ev_);
    if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -650,13 +671,17 @@ void Engine::launch_count(const Instr* code, const Program& p, unsigned long lon
       const size_t nw = profile_words(p.aux);
       grow_device(d_prof_, prof_cap_, n);
       grow_device(d_prof_data_, prof_data_cap_, nw);
-      std::vector<DevProfile> profs(n);
-      std::vector<uint32_t> data(nw);
-      pack_profiles(p.aux, d_prof_data_, profs.data(), data.data());
-      cuda_check(cudaMemcpyAsync(d_prof_, profs.data(), n * sizeof(DevProfile), cudaMemcpyHostToDevice, stream), "H2D");
-      cuda_check(cudaMemcpyAsync(d_prof_data_, data.data(), nw * 4, cudaMemcpyHostToDevice, stream), "H2D");
-      cuda_check(cudaStreamSynchronize(stream), "profile upload");  // the host arrays go out of scope
-      launch_profiles(d_table_, nchunks(), d_prof_, n, profile_max_L(p.aux), d_aux_, stream);
+      // pinned staging, free again once the copies of the call before have passed
+      if (!prof_ev_) cuda_check(cudaEventCreateWithFlags(&prof_ev_, cudaEventDisableTiming), "event");
+      cuda_check(cudaEventSynchronize(prof_ev_), "profile staging");
+      grow_host(h_prof_, n, h_prof_cap_);
+      grow_host(h_prof_data_, nw, h_prof_data_cap_);
+      pack_profiles(p.aux, d_prof_data_, h_prof_, h_prof_data_);
+      cuda_check(cudaMemcpyAsync(d_prof_, h_prof_, n * sizeof(DevProfile), cudaMemcpyHostToDevice, stream), "H2D");
+      if (nw) cuda_check(cudaMemcpyAsync(d_prof_data_, h_prof_data_, nw * 4, cudaMemcpyHostToDevice, stream), "H2D");
+      cuda_check(cudaEventRecord(prof_ev_, stream), "event");
+      launch_profiles(d_table_, nchunks(), d_prof_, n, profile_any_delta(p.aux), profile_max_L(p.aux), d_aux_, stream);
+      cuda_check(cudaGetLastError(), "profile launch");
    }
    for (uint32_t k = 0; k < p.n_literals; ++k)  // the caller's row sets after the profiles' (the caller owns them)
       cuda_check(cudaMemcpyAsync(d_aux_ + (p.aux.size() + k) * set_words, literals[k], set_words * 4,
@@ -889,10 +914,12 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    if (n_ids > 0xFFFFFFFFull) throw std::invalid_argument("details: too many row ids requested");
    size_t n_aux = 0, n_prof_data = 0;
    b.profile_max_L = 0;
+   b.profile_any_delta = false;
    for (const auto& q : qs) {
       n_aux += q.prog.aux.size();
       n_prof_data += profile_words(q.prog.aux);
       b.profile_max_L = std::max(b.profile_max_L, profile_max_L(q.prog.aux));
+      b.profile_any_delta |= profile_any_delta(q.prog.aux);
    }
    grow_host(b.h_prof, n_aux, b.hc_prof);
    grow_device(b.d_prof, b.dc_prof, n_aux);
@@ -1041,7 +1068,7 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
       cuda_check(cudaMemsetAsync(b.d_err, 0, sizeof(int), s), "memset");
    }
    if ((parts & 1) && b.n_aux) {
-      launch_profiles(d_table_, nchunks(), b.d_prof, b.n_aux, b.profile_max_L, b.d_aux, s);
+      launch_profiles(d_table_, nchunks(), b.d_prof, b.n_aux, b.profile_any_delta, b.profile_max_L, b.d_aux, s);
       cuda_check(cudaGetLastError(), "profile launch");
    }
    if (parts & 1) {

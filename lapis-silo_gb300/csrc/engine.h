@@ -122,6 +122,7 @@ struct BatchState {
    uint32_t* d_prof_data = nullptr;
    uint32_t* d_aux = nullptr;         // n_aux row sets of nchunks * CHUNK_WORDS words
    uint32_t n_aux = 0, profile_max_L = 0;
+   bool profile_any_delta = false;
    size_t n_prof_data = 0;
    size_t hc_prof = 0, hc_prof_data = 0, dc_prof = 0, dc_prof_data = 0, dc_aux = 0;
    // capacities (elements), one per buffer
@@ -320,6 +321,7 @@ class Engine {
    void upload_containers(const ContainerSet& cs, uint16_t*& payload, CtrDesc*& fctrs);
    void upload_missing(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d);
    void upload_coverage(const SeqColumnImage& s, uint32_t nchunks, DevSeqCol& d);
+   void profile_home(const SeqColumnImage& s, uint32_t col);
    void upload_dates(const DateColumnImage& dc, uint32_t nchunks, DevDateCol& out);
 
    const TableImage& table_;
@@ -359,6 +361,10 @@ class Engine {
    uint32_t* d_prof_data_ = nullptr;
    uint32_t* d_aux_ = nullptr;
    size_t prof_cap_ = 0, prof_data_cap_ = 0, aux_cap_ = 0;
+   DevProfile* h_prof_ = nullptr;          // pinned staging of the two arrays, reused once prof_ev_ has passed
+   uint32_t* h_prof_data_ = nullptr;
+   size_t h_prof_cap_ = 0, h_prof_data_cap_ = 0;
+   cudaEvent_t prof_ev_ = nullptr;
    // Runs the expressions through the single-query path in trace mode; one sample per node.
    size_t collect_traces(const std::vector<std::string>& exprs, std::vector<PlannerSample>& out);
 

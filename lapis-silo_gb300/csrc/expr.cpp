@@ -726,23 +726,39 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
    auto spec = std::make_shared<ProfileSpec>();
    spec->col = ci;
    spec->distance = static_cast<uint32_t>(e.n);
-   spec->mask.resize(L);
-   spec->diff.assign(L + 1, 0);
-   uint32_t loc = 0;
-   for (uint32_t p = 0; p < L; ++p) {
-      const uint32_t m = profile[p] == A.missing ? 0u : A.all_mask & ~A.ambiguity[profile[p]];
-      const uint32_t lbit = (m >> col.local_ref[p]) & 1u;
-      spec->mask[p] = m | lbit << 31;
-      spec->diff[p + 1] = spec->diff[p] + ((m >> A.missing) & 1u) - lbit;
-      loc += lbit;
+   for (uint32_t p = 0; p < L && spec->delta.size() <= PROFILE_DELTA_MAX; ++p) {
+      if (profile[p] == col.local_ref[p]) continue;
+      const uint32_t m = profile_mask(A, profile[p]), h = profile_mask(A, col.local_ref[p]);
+      if (m == h) continue;
+      const int32_t d = static_cast<int32_t>((m >> col.local_ref[p]) & 1u) - static_cast<int32_t>((h >> col.local_ref[p]) & 1u);
+      spec->delta.push_back({p, m, h, d});
+      spec->base_delta += d;
    }
-   spec->base = loc;
+   spec->use_delta = spec->delta.size() <= PROFILE_DELTA_MAX;
+   if (!spec->use_delta) {
+      spec->delta.clear();
+      spec->mask.resize(L);
+      spec->diff.assign(L + 1, 0);
+      uint32_t loc = 0;
+      for (uint32_t p = 0; p < L; ++p) {
+         const uint32_t m = profile_mask(A, profile[p]);
+         const uint32_t lbit = (m >> col.local_ref[p]) & 1u;
+         spec->mask[p] = m | lbit << 31;
+         spec->diff[p + 1] = spec->diff[p] + ((m >> A.missing) & 1u) - lbit;
+         loc += lbit;
+      }
+      spec->base = loc;
+   }
    auto o = mk(OpT::PROFILE);
    o->profile = std::move(spec);
    return o;
 }
 
 }  // namespace
+
+uint32_t profile_mask(const Alphabet& A, uint8_t symbol) {
+   return symbol == A.missing ? 0u : A.all_mask & ~A.ambiguity[symbol];
+}
 
 OpPtr compile(const Expr& e, const TableImage& t) {
    switch (e.kind) {

@@ -78,10 +78,25 @@ enum class OpT : uint8_t { EMPTY, FULL, INDEX_SCAN, INTERSECTION, UNION, COMPLEM
 // (reference: src/rhydb/query_engine/scalar_expressions/mutation_profile.cpp:198-257). Counted per
 // row from the row index: `base` differences for a covered row holding the local reference
 // everywhere, corrected by the row's own symbols and by the positions it does not cover.
+struct ProfileDelta {
+   uint32_t pos;
+   uint32_t mask;   // symbols that count as a difference from the profile here
+   uint32_t home;   // symbols that count as a difference from the local reference here
+   int32_t d_ref;   // the local reference's bit in mask minus its bit in home
+};
+// The symbols that differ from `symbol` as a profile's symbol (none for the missing symbol).
+uint32_t profile_mask(const Alphabet& a, uint8_t symbol);
+
 struct ProfileSpec {
    int col = 0;
    uint32_t distance = 0;
    uint32_t base = 0;
+   // Where the profile differs from the local reference at no more than PROFILE_DELTA_MAX positions, the
+   // differences only: the device starts from every row's distance to the local reference (a stored
+   // index), adds base_delta and corrects the rows listed at these positions. Else (delta unused):
+   bool use_delta = false;
+   int32_t base_delta = 0;  // sum of d_ref over the positions
+   std::vector<ProfileDelta> delta;
    // L: bit s = symbol s counts as a difference at the position; bit 31 = the local reference
    // symbol does (alphabets have at most 28 symbols)
    std::vector<uint32_t> mask;

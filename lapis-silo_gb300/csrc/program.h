@@ -78,6 +78,11 @@ enum RowOp : int { A_OR = 0, A_ANDNOT = 1, A_ADD = 2 };
 // A_ANDNOT), bits 11..15 the planes of A_ADD (as in a leaf's flags).
 constexpr uint16_t GROUP_PUSH = 4;
 
+// A MutationProfile that differs from the local reference at up to this many positions is counted from
+// the differences (profile_delta_kernel), any other from the whole row index (see profile.cu): 72 us for
+// 1,344 positions at 2M rows and about 50 us per further thousand, against 133 us for the row index.
+constexpr uint32_t PROFILE_DELTA_MAX = 2048;
+
 constexpr uint32_t MAX_PROGRAM = 4096;   // instructions per program
 constexpr uint32_t MAX_THR_PLANES = 16;  // counter planes (NOf up to 65,534 children)
 

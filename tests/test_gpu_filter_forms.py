@@ -1,7 +1,7 @@
 """The forms a filter leaf takes on the device, at the sizes where they can go wrong, against the oracle:
 grouped row lists and their counters at every tile width, thresholds around the counters' sticky plane,
-arrays stored as bitsets, the digits of the date index, and the row lists of coverage leaves at the
-edges of position blocks. Row sets and counts are equal bit for bit."""
+arrays stored as bitsets, the digits of the date index, the row lists of coverage leaves at the edges of
+position blocks, and MutationProfiles on both sides of the limit between their two passes. Row sets and counts are equal bit for bit."""
 import numpy as np
 import pytest
 
@@ -91,5 +91,25 @@ def test_coverage_lists_at_block_edges():
         qs += [f"SymEq(main,{p},N)", f"SymEq(main,{p},{c})", f"Not(SymEq(main,{p},{c}))", f"Maybe(SymEq(main,{p},A))",
                f"Or(SymEq(main,{p},N),SymEq(main,{301 - p},{t.local_reference(0)[300 - p]}))",
                f"NOf(2,atleast,SymEq(main,{p},N),SymEq(main,{p},{c}),Not(SymEq(main,{301 - p},N)),HasMut(main,{p}))"]
+    check(dev, orc, qs)
+    dev.close()
+
+
+@pytest.mark.parametrize("genome,rows,differences", [(600, 70000, 0), (600, 70000, 1), (600, 70000, 33), (600, 70000, 600),
+                                                     (3000, 900, 2048), (3000, 900, 2049), (40000, 300, 2049)])
+def test_profile_passes(genome, rows, differences):
+    """Up to 2,048 positions off the local reference a profile is counted from its differences, above
+    from the row index (terms in shared memory up to 32,767 positions, through the caches beyond)."""
+    t = R.Table.generate(rows, seed=3, genome_len=genome, pool_sites=min(200, genome // 3), null_fraction=0.01)
+    dev, orc = R.Device(t, 0), oracle_for(t)
+    rng = np.random.default_rng(differences)
+    ref = t.local_reference(0)
+    seq = list(ref)
+    for p in rng.choice(genome, differences, replace=False):
+        seq[p] = "ACGT"["ACGT".index(seq[p]) - 1] if rng.random() < 0.8 else "N"
+    seq = "".join(seq)
+    off = sum(c != "N" and c != r for c, r in zip(seq, ref))
+    short = f"MutProfileMutations(main,9,{1 + genome // 2}:A,{genome}:C)"
+    qs = [f"MutProfile(main,{off + d},{seq})" for d in (0, 25)] + [short, f"And({short},HasMut(main,{genome // 2}))"]
     check(dev, orc, qs)
     dev.close()
