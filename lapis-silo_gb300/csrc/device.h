@@ -255,6 +255,29 @@ void set_copy_withholding(bool on);
 // but withheld, so its consumers' waits give up and it sets DEVERR_WAIT_MUTATIONS.
 void set_ring_withholding(bool on);
 
+// Output rows of the Mutations action (same layout as RhyMutationRow in the C-ABI header).
+struct DevMutationRow {
+   uint32_t position;  // 1-based
+   char from, to;
+   uint16_t pad;
+   uint32_t count;
+   uint32_t coverage;
+   double proportion;
+};
+static_assert(sizeof(DevMutationRow) == 24, "row layout");
+// Where the batched final pass puts the Mutations rows of a group of slots: their number per (slot, block
+// of ROWS_BLOCK positions) in blk (nullptr: no rows wanted) and the place of the block's rows in the
+// staging buffer in base; cursor counts the rows staged so far, cap the buffer's (blocks past it are
+// made by the write pass).
+struct RowsOut {
+   const double* min_prop;  // per slot
+   uint32_t* blk;
+   uint32_t* base;
+   DevMutationRow* stage;
+   uint32_t* cursor;
+   uint32_t cap;
+};
+
 // One unit of the batched container pass: the containers of position `pos` in chunks [v0, v1), at most
 // CTR_UNIT_CHUNKS chunks and CTR_UNIT_ELEMENTS elements. A chunk with more is cut into parts of its own:
 // each takes the bitset words [32 w0, 32 w1), the first one the arrays and runs too (a bitset of 30,000
@@ -275,9 +298,8 @@ constexpr uint32_t CTR_UNIT_ELEMENTS = 4096;
 // On the device, once the filters are known, the slots split by their filter's cardinality: empty
 // filters need no pass, filters of at most sparse_max rows (0: none) take the row-index pass (part
 // BMUT_PART_SPARSE), the others the dense passes over the slots listed in d_lists (2 * nq + 2 u32
-// of scratch: the dense and the sparse slot lists and their lengths). With d_rowblk, the final
-// pass also counts every slot's Mutations output rows (minimum proportion d_min_prop[slot]) per
-// block of ROWS_BLOCK positions into d_rowblk, as launch_rows_count would.
+// of scratch: the dense and the sparse slot lists and their lengths). With rows.blk, the final pass
+// also makes every slot's Mutations output rows (RowsOut).
 enum : uint32_t { BMUT_PART_SPARSE = 16 };
 size_t mutations_batch_mask_bytes(uint32_t nq, uint32_t nchunks);
 void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
@@ -285,31 +307,18 @@ void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, 
                             const uint32_t* d_slot_query, const EvItem* d_ev, uint32_t n_ev, const CtrUnit* d_units,
                             uint32_t n_units, uint16_t* d_masks, uint32_t* d_counts, uint32_t* d_scratch,
                             uint32_t* d_lists, uint64_t sparse_max, void* stream,
-                            uint32_t parts = BMUT_PART_ALL | BMUT_PART_SPARSE, const double* d_min_prop = nullptr,
-                            uint32_t* d_rowblk = nullptr);
+                            uint32_t parts, const RowsOut& rows);
 
-// Output rows of the Mutations action (same layout as RhyMutationRow in the C-ABI header).
-struct DevMutationRow {
-   uint32_t position;  // 1-based
-   char from, to;
-   uint16_t pad;
-   uint32_t count;
-   uint32_t coverage;
-   double proportion;
-};
-static_assert(sizeof(DevMutationRow) == 24, "row layout");
 
-// Rows of nq query slots whose dense counts lie at d_counts + slot * nsym * L, with per-slot minimum
-// proportions. The batched final pass counts them (launch_mutations_batch with d_rowblk):
-// d_blk[slot * rows_blocks(L) + b] = rows of position block b; the scan turns n entries into
-// exclusive offsets with the total at d_blk[n]; the write pass emits the rows at their offsets in
-// (slot, position, symbol) order, skipping the blocks without rows.
+// Rows of nq query slots whose dense counts lie at d_counts + slot * nsym * L. The batched final pass
+// makes them (RowsOut): blk[slot * rows_blocks(L) + b] = rows of position block b; the scan turns n
+// entries into exclusive offsets with the total at d_blk[n]; the write pass puts the rows at their
+// offsets in (slot, position, symbol) order, skipping the blocks without rows.
 constexpr uint32_t ROWS_BLOCK = 1024;
 uint32_t rows_blocks(uint32_t L);
 void launch_rows_scan(uint32_t* d_blk, uint32_t n, void* stream);
 void launch_rows_write(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, const uint32_t* d_counts,
-                       uint32_t nq, const double* d_min_prop, const uint32_t* d_blk, DevMutationRow* d_rows,
-                       void* stream);
+                       uint32_t nq, const RowsOut& out, DevMutationRow* d_rows, void* stream);
 
 // Details: the first k_of[q] row ids (ascending) of each of nq dense row sets (nchunks * CHUNK_WORDS
 // words apart) to d_ids + out_off[q]; d_n[q] receives min(k, |row set|).

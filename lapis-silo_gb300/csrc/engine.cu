@@ -802,7 +802,8 @@ void Engine::batch_free(BatchState& b) {
                    static_cast<void*>(b.d_slot_query), static_cast<void*>(b.d_counts), static_cast<void*>(b.d_next),
                    static_cast<void*>(b.d_tiles), static_cast<void*>(b.d_mcounts), static_cast<void*>(b.d_mscratch),
                    static_cast<void*>(b.d_masks), static_cast<void*>(b.d_minprop), static_cast<void*>(b.d_rowblk),
-                   static_cast<void*>(b.d_rows), static_cast<void*>(b.d_err), static_cast<void*>(b.d_k),
+                   static_cast<void*>(b.d_rows), static_cast<void*>(b.d_rowbase), static_cast<void*>(b.d_stage),
+                   static_cast<void*>(b.d_err), static_cast<void*>(b.d_k),
                    static_cast<void*>(b.d_ids), static_cast<void*>(b.d_nids), static_cast<void*>(b.d_lists),
                    static_cast<void*>(b.d_prof), static_cast<void*>(b.d_prof_data), static_cast<void*>(b.d_aux)})
       if (p) cudaFree(p);
@@ -821,7 +822,8 @@ size_t Engine::batch_device_bytes(const std::vector<BatchQuery>& qs, uint32_t ti
       if (q.action == 1 && q.column >= 0 && static_cast<size_t>(q.column) < per_col.size()) {
          const DevSeqCol& dc = view_.seq[q.column];
          bytes += tile_bytes + static_cast<size_t>(dc.nsym) * dc.L * 4 + mut_scratch_words(dc.L) * 4 + 16 + 8 +
-                  (rows_blocks(dc.L) + 1) * 4 + static_cast<size_t>(dc.L) * 2 * sizeof(DevMutationRow);
+                  (rows_blocks(dc.L) + 1) * 8 + static_cast<size_t>(dc.L) * 2 * sizeof(DevMutationRow) +
+                  ROWS_STAGED * sizeof(DevMutationRow);
          ++per_col[q.column];
       } else if (q.action == 2) {
          bytes += tile_bytes + static_cast<size_t>(q.k) * 4 + 16;
@@ -949,6 +951,8 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    grow_device(b.d_minprop, b.dc_minprop, nslots);
    grow_host(b.h_rowblk, static_cast<size_t>(n_blk) + 1, b.hc_rowblk);
    grow_device(b.d_rowblk, b.dc_rowblk, static_cast<size_t>(n_blk) + 1);
+   grow_device(b.d_rowbase, b.dc_rowbase, static_cast<size_t>(n_blk) + 1);  // and the staging cursor
+   grow_device(b.d_stage, b.dc_stage, ROWS_STAGED * static_cast<size_t>(n_mut));
    grow_host(b.h_err, 1, b.hc_err);
    grow_device(b.d_err, b.dc_err, 1);
    grow_host(b.h_k, 2 * static_cast<size_t>(n_det), b.hc_k);
@@ -1089,8 +1093,7 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
                              n_cu_[g.column], b.d_masks, b.d_mcounts + g.counts_off, b.d_mscratch + g.scratch_off,
                              b.d_lists + g.lists_off, sparse_rows_batch, s,
                              (parts >> 1) & (BMUT_PART_ALL | BMUT_PART_SPARSE),
-                             b.rows_in_final ? b.d_minprop + g.slot_begin : nullptr,
-                             b.rows_in_final ? b.d_rowblk + g.blk_off : nullptr);
+                             b.rows_in_final ? rows_out(b, g) : RowsOut{});
       cuda_check(cudaGetLastError(), "mutations batch launch");
    }
    if (b.n_details && (parts & 1)) {
@@ -1106,6 +1109,11 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
       copy_details(b, s);
       cuda_check(cudaMemcpyAsync(b.h_err, b.d_err, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
    }
+}
+
+RowsOut Engine::rows_out(const BatchState& b, const BatchState::ColGroup& g) const {
+   return RowsOut{b.d_minprop + g.slot_begin, b.d_rowblk + g.blk_off, b.d_rowbase + g.blk_off, b.d_stage, b.d_rowbase + b.n_blk,
+                  ROWS_STAGED * b.n_mut_slots};
 }
 
 void Engine::copy_details(BatchState& b, cudaStream_t s) {
@@ -1125,8 +1133,9 @@ void Engine::check_batch_error(BatchState& b) {
 void Engine::rows_phase1(BatchState& b, cudaStream_t s) {
    s = stream_for(s);
    if (b.n_queries == 0) return;
-   b.rows_in_final = true;  // the final pass counts the rows per block (no separate counting pass)
+   b.rows_in_final = true;  // the final pass makes the rows
    try {
+      if (b.n_mut_slots) cuda_check(cudaMemsetAsync(b.d_rowbase + b.n_blk, 0, sizeof(uint32_t), s), "memset");
       batch_enqueue(b, s, true, false);
    } catch (...) {
       b.rows_in_final = false;
@@ -1155,7 +1164,7 @@ size_t Engine::rows_phase2(BatchState& b, cudaStream_t s, DevMutationRow* rows, 
       grow_device(b.d_rows, b.dc_rows, total);
       for (const auto& g : b.groups)
          launch_rows_write(d_table_, view_.seq[g.column], static_cast<uint32_t>(g.column), b.d_mcounts + g.counts_off, g.n,
-                           b.d_minprop + g.slot_begin, b.d_rowblk + g.blk_off, b.d_rows, s);
+                           rows_out(b, g), b.d_rows, s);
       cuda_check(cudaGetLastError(), "rows launch");
       if (rows && total <= cap)
          cuda_check(cudaMemcpyAsync(rows, b.d_rows, total * sizeof(DevMutationRow), cudaMemcpyDeviceToHost, s), "D2H");

@@ -103,6 +103,8 @@ struct BatchState {
    double* d_minprop = nullptr;
    uint32_t* d_rowblk = nullptr;
    DevMutationRow* d_rows = nullptr;
+   uint32_t* d_rowbase = nullptr;     // n_blk places in d_stage, then its cursor
+   DevMutationRow* d_stage = nullptr; // rows as the final pass makes them, ROWS_STAGED per Mutations slot
    int* d_err = nullptr;              // error flag of this batch's kernels
    int* h_err = nullptr;              // pinned
    uint32_t* d_k = nullptr;           // Details: k per slot, then offsets into the ids
@@ -112,7 +114,7 @@ struct BatchState {
    uint32_t* d_nids = nullptr;        // Details: ids per slot
    uint32_t* h_nids = nullptr;
    uint32_t n_blk = 0;                // row-block table entries (Mutations slots)
-   bool rows_in_final = false;        // the final Mutations pass also counts the rows per block
+   bool rows_in_final = false;        // the final Mutations pass also makes the rows
    size_t n_rows = 0;                 // rows of the last row pass
    uint32_t n_mut_slots = 0, n_details = 0, n_ids = 0;
    // MutationProfile row sets of the batch's programs (QueryDesc.aux_base numbers them)
@@ -130,7 +132,7 @@ struct BatchState {
           hc_rowblk = 0, hc_err = 0, hc_k = 0, hc_ids = 0, hc_nids = 0;
    size_t dc_code = 0, dc_q = 0, dc_items = 0, dc_slot_query = 0, dc_counts = 0, dc_next = 0, dc_tiles = 0,
           dc_mcounts = 0, dc_mscratch = 0, dc_masks = 0, dc_minprop = 0, dc_rowblk = 0, dc_rows = 0, dc_err = 0, dc_k = 0,
-          dc_ids = 0, dc_nids = 0, dc_lists = 0;
+          dc_ids = 0, dc_nids = 0, dc_lists = 0, dc_rowbase = 0, dc_stage = 0;
    cudaGraphExec_t graph = nullptr;
 };
 
@@ -242,6 +244,9 @@ class Engine {
    // the Aggregated counts in parts of about PIPELINE_COUNTS. Results equal batch_rows of the whole
    // batch; the rows come in part order. Counts fewer than PIPELINE_PART join the part before them.
    // The caller holds mu.
+   // Rows the staging buffer holds per Mutations slot, over all of them (the benchmark's batch makes 54
+   // per slot; a filter of few rows some hundred). Blocks past it are made by the write pass.
+   static constexpr uint32_t ROWS_STAGED = 256;
    static constexpr uint32_t PIPELINE_PART = 256;
    static constexpr uint32_t PIPELINE_HEAVY = 1024;
    static constexpr uint32_t PIPELINE_COUNTS = 768;
@@ -342,6 +347,7 @@ class Engine {
    std::vector<std::unique_ptr<BatchState>> parts_;      // parts 1.. of batch_rows_pipelined
    std::vector<BatchState*> rows_parts_{&batch_};        // states holding the last rows, in row order
    void copy_details(BatchState& b, cudaStream_t s);
+   RowsOut rows_out(const BatchState& b, const BatchState::ColGroup& g) const;
    Planner planner_;
    bool use_learned_ = false;
    std::unique_ptr<FeatureContext> fctx_;  // built on first use

@@ -8,11 +8,11 @@
 // a quotient), so the values equal the host's bit for bit.
 //
 // Three steps keep the output packed and in (slot, position, symbol) order:
-//   the batched final pass (mut_final_batch_kernel) counts the rows per block of ROWS_BLOCK
-//                      positions of every slot, from the counts it has just completed
+//   the batched final pass (mut_final_batch_kernel) makes the rows per block of ROWS_BLOCK positions of
+//                      every slot from the counts it has just completed, and stages them
 //   rows_scan_kernel   exclusive prefix over all (slot, block) counts; the total follows them
-//   rows_write_kernel  recomputes the rows of each block that has any and writes them at their
-//                      offsets (blocks without rows, most of them, read no counts)
+//   rows_write_kernel  copies each block's staged rows to their offsets; a block whose rows did not fit
+//                      the staging buffer is made again from its counts
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -71,18 +71,24 @@ __global__ void __launch_bounds__(RT) rows_scan_kernel(uint32_t* blk, uint32_t n
 
 __global__ void __launch_bounds__(RT) rows_write_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                         const uint32_t* __restrict__ counts,
-                                                        const double* __restrict__ min_prop,
-                                                        const uint32_t* __restrict__ blk, DevMutationRow* rows) {
+                                                        RowsOut out, DevMutationRow* rows) {
    __shared__ uint32_t wsum[RT / 32];
    const size_t bi = static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x;
-   const uint32_t at0 = blk[bi];
-   if (blk[bi + 1] == at0) return;  // a block without rows (the scan's next entry, or its total, is equal)
+   const uint32_t at0 = out.blk[bi], n = out.blk[bi + 1] - at0;
+   if (n == 0) return;  // a block without rows (the scan's next entry, or its total, is equal)
+   const uint32_t base = out.base[bi];
+   if (base + n <= out.cap) {
+      const uint2* src = reinterpret_cast<const uint2*>(out.stage + base);
+      uint2* dst = reinterpret_cast<uint2*>(rows + at0);
+      for (uint32_t i = threadIdx.x; i < n * (sizeof(DevMutationRow) / 8); i += RT) dst[i] = src[i];
+      return;
+   }
    const DevSeqCol* cs = &tab->seq[col];
    const uint32_t q = blockIdx.y, p = blockIdx.x * RT + threadIdx.x;
    const uint32_t L = cs->L;
    const uint32_t* c = counts + static_cast<size_t>(q) * cs->nsym * L;
    PosRows r{0, 0, 0, 0};
-   if (p < L) r = position_rows(cs, c, p, min_prop[q]);
+   if (p < L) r = position_rows(cs, c, p, out.min_prop[q]);
    uint32_t total;
    uint32_t at = at0 + block_scan_excl(r.n, wsum, &total);
    if (r.n == 0) return;
@@ -91,15 +97,7 @@ __global__ void __launch_bounds__(RT) rows_write_kernel(const DevTable* __restri
       if (!((valid >> s) & 1u) || s == r.ref) continue;
       const uint32_t k = __ldg(c + static_cast<size_t>(s) * L + p);
       if (k <= r.thr) continue;
-      DevMutationRow o;
-      o.position = p + 1;
-      o.from = cs->chars[r.ref];
-      o.to = cs->chars[s];
-      o.pad = 0;
-      o.count = k;
-      o.coverage = r.total;
-      o.proportion = static_cast<double>(k) / static_cast<double>(r.total);
-      rows[at++] = o;
+      rows[at++] = mutation_row(cs, p, r, s, k);
    }
 }
 
@@ -112,11 +110,10 @@ void launch_rows_scan(uint32_t* d_blk, uint32_t n, void* stream) {
 }
 
 void launch_rows_write(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, const uint32_t* d_counts,
-                       uint32_t nq, const double* d_min_prop, const uint32_t* d_blk, DevMutationRow* d_rows,
-                       void* stream) {
+                       uint32_t nq, const RowsOut& out, DevMutationRow* d_rows, void* stream) {
    if (nq == 0) return;
-   rows_write_kernel<<<dim3(rows_blocks(col_host.L), nq), RT, 0, static_cast<cudaStream_t>(stream)>>>(
-      d_table, col, d_counts, d_min_prop, d_blk, d_rows);
+   rows_write_kernel<<<dim3(rows_blocks(col_host.L), nq), RT, 0, static_cast<cudaStream_t>(stream)>>>(d_table, col, d_counts,
+                                                                                                    out, d_rows);
 }
 
 }  // namespace rhygpu

@@ -36,4 +36,34 @@ __device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ c
    return r;
 }
 
+// The same with the position's counts in registers (`valid`: the column's valid symbols, 0 for no rows).
+template <uint32_t NS>
+__device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ cs, uint32_t p, uint32_t valid,
+                                                 double min_prop, const uint32_t (&c)[NS]) {
+   PosRows r{0, 0, 0, 0};
+#pragma unroll
+   for (uint32_t s = 0; s < NS; ++s)
+      if ((valid >> s) & 1u) r.total += c[s];
+   if (r.total == 0) return r;
+   r.thr = min_prop == 0.0 ? 0u : static_cast<uint32_t>(ceil(static_cast<double>(r.total) * min_prop) - 1.0);
+   r.ref = __ldg(cs->global_ref + p);
+#pragma unroll
+   for (uint32_t s = 0; s < NS; ++s)
+      if (((valid >> s) & 1u) && s != r.ref && c[s] > r.thr) ++r.n;
+   return r;
+}
+
+__device__ __forceinline__ DevMutationRow mutation_row(const DevSeqCol* __restrict__ cs, uint32_t p, const PosRows& r,
+                                                       uint32_t symbol, uint32_t count) {
+   DevMutationRow o;
+   o.position = p + 1;
+   o.from = cs->chars[r.ref];
+   o.to = cs->chars[symbol];
+   o.pad = 0;
+   o.count = count;
+   o.coverage = r.total;
+   o.proportion = static_cast<double>(count) / static_cast<double>(r.total);
+   return o;
+}
+
 }  // namespace rhygpu

@@ -113,3 +113,22 @@ def test_profile_passes(genome, rows, differences):
     qs = [f"MutProfile(main,{off + d},{seq})" for d in (0, 25)] + [short, f"And({short},HasMut(main,{genome // 2}))"]
     check(dev, orc, qs)
     dev.close()
+
+
+@pytest.mark.parametrize("proportion,staged", [(0.0, False), (0.1, True), (1.0, True)])
+def test_rows_of_the_final_pass(proportion, staged):
+    """Mutations rows of a batch on both sides of its staging buffer (256 rows per slot over all slots), of
+    nucleotide and amino-acid columns, with filters of no rows between them, in three position blocks."""
+    t = R.Table.generate(3000, seed=12, genome_len=2500, pool_sites=1500, n_aa_genes=1, null_fraction=0.01)
+    dev, orc = R.Device(t, 0), oracle_for(t)
+    qs = t.queries(40, seed=13) + ["True", "And(True,Not(True))", "HasMut(main,1024)"]
+    col = [i % 2 for i in range(len(qs))]
+    want = [t.mutation_rows(c, orc.mutations(q, c)[0], proportion) for q, c in zip(qs, col)]
+    n_rows = sum(map(len, want))
+    assert (n_rows <= 256 * len(qs)) == staged
+    for _ in range(2):  # the buffers of the first batch are taken again
+        counts, rows, begin, cnt = dev.batch_rows(qs, [1] * len(qs), col, [proportion] * len(qs))
+        got = [[(int(r["position"]), r["from_"].decode(), r["to"].decode(), int(r["count"]), int(r["coverage"]),
+                 float(r["proportion"])) for r in rows[int(b):int(b) + int(n)]] for b, n in zip(begin, cnt)]
+        assert got == want
+    dev.close()
