@@ -498,16 +498,15 @@ __global__ void __launch_bounds__(BT) mut_sparse_batch_kernel(const DevTable* __
 
 // grid (ceil(L / MUT_SEG), nq): reference counts of slot blockIdx.y. With out.blk (the Mutations rows are
 // wanted), the CTA also makes the output rows of its MUT_SEG (= ROWS_BLOCK) positions under the slot's
-// minimum proportion from the counts it holds in registers: their number goes to out.blk[slot *
+// minimum proportion from the counts it has just read: their number goes to out.blk[slot *
 // gridDim.x + blockIdx.x] and the rows, where they fit, to the next free part of out.stage, which the
 // write pass copies into their final order (see rows.cu). A count is so read once; the write pass that
 // made the rows from the count tables took 0.46 ms for the 2,048-query batch, the copy takes 0.11.
-template <uint32_t NS>
-__global__ void __launch_bounds__(MUT_SEG) mut_final_batch_kernel(const DevTable* __restrict__ tab, uint32_t col,
-                                                                  const unsigned long long* __restrict__ fcounts,
-                                                                  const uint32_t* __restrict__ slot_query,
-                                                                  uint32_t* __restrict__ counts,
-                                                                  const uint32_t* __restrict__ scratch, RowsOut out) {
+__global__ void __launch_bounds__(MUT_SEG, 2) mut_final_batch_kernel(const DevTable* __restrict__ tab, uint32_t col,
+                                                                     const unsigned long long* __restrict__ fcounts,
+                                                                     const uint32_t* __restrict__ slot_query,
+                                                                     uint32_t* counts,
+                                                                     const uint32_t* __restrict__ scratch, RowsOut out) {
    static_assert(MUT_SEG == ROWS_BLOCK, "a final CTA covers one block of the row counts");
    __shared__ uint32_t wtot[MUT_SEG / 32], base_sh;
    const DevSeqCol* cs = &tab->seq[col];
@@ -518,13 +517,13 @@ __global__ void __launch_bounds__(MUT_SEG) mut_final_batch_kernel(const DevTable
       if (out.blk != nullptr && threadIdx.x == 0) out.blk[bi] = 0;
       return;
    }
-   uint32_t c[NS];
-   final_position_counts<NS>(cs, total, counts + static_cast<size_t>(q) * cs->nsym * L,
-                             scratch + static_cast<size_t>(q) * mut_scratch_words(L), c);
+   uint32_t* cnt = counts + static_cast<size_t>(q) * cs->nsym * L;
+   const FinalCount f = final_position_counts(cs, total, cnt, scratch + static_cast<size_t>(q) * mut_scratch_words(L));
    if (out.blk == nullptr) return;
    const uint32_t p = blockIdx.x * MUT_SEG + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   const uint32_t valid = p < L ? cs->valid_mask : 0u;
-   PosRows r = position_rows<NS>(cs, p, valid, out.min_prop[q], c);
+   const uint32_t syms = p < L ? cs->valid_mask & (cs->syms[p] | 1u << f.local) : 0u;
+   auto count = [&](uint32_t k) { return k == f.local ? f.count : cnt[static_cast<size_t>(k) * L + p]; };
+   const PosRows r = position_rows(cs, p, syms, out.min_prop[q], count);
    uint32_t incl = r.n;
 #pragma unroll
    for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -544,9 +543,10 @@ __global__ void __launch_bounds__(MUT_SEG) mut_final_batch_kernel(const DevTable
    __syncthreads();
    if (base_sh + sum > out.cap || r.n == 0) return;  // the write pass makes the rows of a block that did not fit
    DevMutationRow* o = out.stage + base_sh + before + incl - r.n;
-#pragma unroll
-   for (uint32_t k = 0; k < NS; ++k)
-      if (((valid >> k) & 1u) && k != r.ref && c[k] > r.thr) *o++ = mutation_row(cs, p, r, k, c[k]);
+   for (uint32_t m = syms & ~(1u << r.ref); m; m &= m - 1) {
+      const uint32_t k = __ffs(m) - 1, n = count(k);
+      if (n > r.thr) *o++ = mutation_row(cs, p, r, k, n);
+   }
 }
 static_assert(MUT_SEG / 32 == 32, "one lane per warp's total");
 
@@ -587,8 +587,7 @@ void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, 
    }
    if (parts & BMUT_PART_FINAL) {
       dim3 fin((col_host.L + MUT_SEG - 1) / MUT_SEG, nq);
-      (col_host.nsym <= 16 ? mut_final_batch_kernel<16> : mut_final_batch_kernel<32>)<<<fin, MUT_SEG, 0, s>>>(
-         d_table, col, d_fcounts, d_slot_query, d_counts, d_scratch, rows);
+      mut_final_batch_kernel<<<fin, MUT_SEG, 0, s>>>(d_table, col, d_fcounts, d_slot_query, d_counts, d_scratch, rows);
    }
 }
 

@@ -92,6 +92,7 @@ struct DevSeqCol {
    const uint32_t* nblk_toff;  // nblocks * nchunks * TOFF_N: tile row-range offsets into each nblk bucket
    const uint32_t* null_tiles; // nchunks * CHUNK_WORDS
    const uint8_t* local_ref;   // L
+   const uint32_t* syms;       // L: bit s: the position has containers of symbol s (all others count 0)
    // Boundaries of the missing intervals by (128-position block, chunk), sorted by row, for the single-query
    // coverage pass: row within the chunk | position in the block << 16 | 1 << 31 for an interval's first
    // position, 0 for the one after its last; each bucket from a multiple of 4 entries on, padded with

@@ -431,6 +431,11 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          for (uint32_t g : s.null_rows) nulls[g >> 5] |= 1u << (g & 31);
          d.null_tiles = upload(nulls);
          d.local_ref = upload(s.local_ref);
+         {
+            std::vector<uint32_t> syms(s.L, 0);
+            for (const CtrDesc& x : s.vertical.ctrs) syms[x.key] |= 1u << x.sym;
+            d.syms = upload(syms);
+         }
          d.global_ref = upload(s.global_ref);
          {
             const Alphabet& A = alphabet(s.kind);

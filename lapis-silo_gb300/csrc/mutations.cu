@@ -515,12 +515,10 @@ __global__ void __launch_bounds__(MT) mut_sparse_kernel(const DevTable* __restri
       row_index_pass32(cs, filter, w, words, counts, scratch, list[warp]);
 }
 
-template <uint32_t NS>
-__global__ void __launch_bounds__(MUT_SEG) mut_final_kernel(const DevTable* __restrict__ tab, uint32_t col,
+__global__ void __launch_bounds__(MUT_SEG, 2) mut_final_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                             const unsigned long long* __restrict__ fcount,
                                                             uint32_t* counts, const uint32_t* __restrict__ scratch) {
-   uint32_t c[NS];
-   final_position_counts<NS>(&tab->seq[col], static_cast<uint32_t>(*fcount), counts, scratch, c);
+   final_position_counts(&tab->seq[col], static_cast<uint32_t>(*fcount), counts, scratch);
 }
 
 }  // namespace
@@ -560,9 +558,8 @@ void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32
                                                      static_cast<unsigned long long>(sparse_max), d_scratch);
    }
    if (parts & MUT_PART_FINAL)
-      (col_host.nsym <= 16 ? mut_final_kernel<16> : mut_final_kernel<32>)<<<(col_host.L + MUT_SEG - 1) / MUT_SEG, MUT_SEG, 0,
-                                                                            s>>>(d_table, col, d_filter_count, d_counts,
-                                                                                 d_scratch);
+      mut_final_kernel<<<(col_host.L + MUT_SEG - 1) / MUT_SEG, MUT_SEG, 0, s>>>(d_table, col, d_filter_count, d_counts,
+                                                                               d_scratch);
 }
 
 }  // namespace rhygpu

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "device.h"
+#include "rows_rule.cuh"
 
 namespace rhygpu {
 
@@ -61,30 +62,34 @@ __device__ __forceinline__ uint32_t count_range(const uint32_t* F, uint32_t a, u
 // Final pass for positions [blockIdx.x * MUT_SEG, +MUT_SEG) of one query (blockDim.x == MUT_SEG):
 //   ref(p) = |F| - #(start > p) - #(end <= p) - missing(p) - sum_s counts[s][p]
 //   counts[local_ref[p]][p] += ref(p)
-// All arithmetic is modulo 2^32 like the reference's uint32 vectors; the result is exact. Returns ref(p)
-// (0 past the genome) and leaves the position's counts, as they are to be stored, in c (NS >= nsym of
-// them; the local reference's is the only one changed). The loads of a position (its histograms and its
-// symbols' counts) all start before the block scan of the three prefix sums, which takes two barriers.
-template <uint32_t NS>
-__device__ __forceinline__ void final_position_counts(const DevSeqCol* cs, uint32_t total, uint32_t* counts,
-                                                      const uint32_t* __restrict__ scratch, uint32_t (&c)[NS]) {
+// All arithmetic is modulo 2^32 like the reference's uint32 vectors; the result is exact. Returns the
+// position's local reference and its final count (0, 0 past the genome). Bound by latency: a load of the
+// symbols' mask, the counts of the symbols in it (a position has a few of the column's 16 or 28, and reading
+// the others' zeros took most of the pass's bytes) and a block scan of three prefix sums; 32 registers let
+// two CTAs share an SM.
+struct FinalCount {
+   uint32_t local;
+   uint32_t count;
+};
+__device__ __forceinline__ FinalCount final_position_counts(const DevSeqCol* cs, uint32_t total, uint32_t* counts,
+                                                            const uint32_t* __restrict__ scratch) {
    __shared__ uint32_t wtot[3][MUT_SEG / 32], pre[4];
-   const uint32_t L = cs->L, nsym = cs->nsym, nseg = mut_nseg(L);
+   const uint32_t L = cs->L, nseg = mut_nseg(L);
    const uint32_t* seg_s = scratch + 3 * (L + 1);
    const uint32_t* seg_e = seg_s + nseg;
    const uint32_t* seg_n = seg_e + nseg;
    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const uint32_t p = blockIdx.x * MUT_SEG + threadIdx.x;
    const bool in = p < L;
-   uint32_t s = 0, e = 0, n = 0, local = 0;
+   uint32_t s = 0, e = 0, n = 0, rest = 0;
+   FinalCount f{0, 0};
    if (in) {
       s = scratch[p];
       e = scratch[L + 1 + p];
       n = scratch[2 * (L + 1) + p];
-      local = cs->local_ref[p];
+      f.local = cs->local_ref[p];
+      rest = sum_counts(cs->syms[p], [&](uint32_t k) { return counts[static_cast<size_t>(k) * L + p]; });
    }
-#pragma unroll
-   for (uint32_t k = 0; k < NS; ++k) c[k] = in && k < nsym ? counts[static_cast<size_t>(k) * L + p] : 0u;
    if (warp == MUT_SEG / 32 - 1) {  // the segments before this one, and every start
       uint32_t ps = 0, pe = 0, pn = 0, ts = 0;
       for (uint32_t k = lane; k < nseg; k += 32) {
@@ -136,16 +141,12 @@ __device__ __forceinline__ void final_position_counts(const DevSeqCol* cs, uint3
    __syncthreads();
    if (in) {  // no early return: a caller may follow with barriers
       const uint32_t sl = s + wtot[0][warp] + pre[0], el = e + wtot[1][warp] + pre[1], nl = n + wtot[2][warp] + pre[2];
-      uint32_t ref = total - (pre[3] - sl) - el - nl;
-#pragma unroll
-      for (uint32_t k = 0; k < NS; ++k) ref -= c[k];
-#pragma unroll
-      for (uint32_t k = 0; k < NS; ++k) {
-         if (k != local) continue;
-         c[k] += ref;
-         counts[static_cast<size_t>(k) * L + p] = c[k];
-      }
+      f.count = total - (pre[3] - sl) - el - nl - rest;
+      uint32_t* at = counts + static_cast<size_t>(f.local) * L + p;
+      if ((cs->syms[p] >> f.local) & 1u) f.count += *at;
+      *at = f.count;
    }
+   return f;
 }
 static_assert(MUT_SEG / 32 == 32, "one warp scans the warps' totals");
 

@@ -26,12 +26,6 @@ namespace {
 
 constexpr uint32_t RT = ROWS_BLOCK;  // one thread per position
 
-__device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ cs, const uint32_t* __restrict__ c,
-                                                 uint32_t p, double min_prop) {
-   const uint32_t L = cs->L;
-   return position_rows(cs, p, min_prop, [&](uint32_t s) { return __ldg(c + static_cast<size_t>(s) * L + p); });
-}
-
 __device__ __forceinline__ uint32_t block_scan_excl(uint32_t x, uint32_t* wsum, uint32_t* total) {
    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
    uint32_t incl = x;
@@ -87,17 +81,15 @@ __global__ void __launch_bounds__(RT) rows_write_kernel(const DevTable* __restri
    const uint32_t q = blockIdx.y, p = blockIdx.x * RT + threadIdx.x;
    const uint32_t L = cs->L;
    const uint32_t* c = counts + static_cast<size_t>(q) * cs->nsym * L;
-   PosRows r{0, 0, 0, 0};
-   if (p < L) r = position_rows(cs, c, p, out.min_prop[q]);
+   const uint32_t syms = p < L ? cs->valid_mask & (cs->syms[p] | 1u << cs->local_ref[p]) : 0u;
+   auto count = [&](uint32_t k) { return __ldg(c + static_cast<size_t>(k) * L + p); };
+   const PosRows r = position_rows(cs, p, syms, out.min_prop[q], count);
    uint32_t total;
    uint32_t at = at0 + block_scan_excl(r.n, wsum, &total);
    if (r.n == 0) return;
-   const uint32_t valid = cs->valid_mask;
-   for (uint32_t s = 0; s < cs->nsym; ++s) {
-      if (!((valid >> s) & 1u) || s == r.ref) continue;
-      const uint32_t k = __ldg(c + static_cast<size_t>(s) * L + p);
-      if (k <= r.thr) continue;
-      rows[at++] = mutation_row(cs, p, r, s, k);
+   for (uint32_t m = syms & ~(1u << r.ref); m; m &= m - 1) {
+      const uint32_t k = __ffs(m) - 1, n = count(k);
+      if (n > r.thr) rows[at++] = mutation_row(cs, p, r, k, n);
    }
 }
 

@@ -18,38 +18,36 @@ struct PosRows {
    uint32_t ref;    // global reference symbol
 };
 
-// total = sum of the counts of the valid symbols (0: no rows); threshold = (min_prop == 0) ? 0 :
-// u32(ceil(total * min_prop) - 1); a row for every valid symbol other than the global reference
-// whose count exceeds the threshold. count(s) returns the count of symbol s at p.
+// Sum of count(s) over the symbols of the mask, four loads in flight.
 template <typename CountOf>
-__device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ cs, uint32_t p, double min_prop,
-                                                 CountOf&& count) {
-   PosRows r{0, 0, 0, 0};
-   const uint32_t nsym = cs->nsym, valid = cs->valid_mask;
-   for (uint32_t s = 0; s < nsym; ++s)
-      if ((valid >> s) & 1u) r.total += count(s);
-   if (r.total == 0) return r;
-   r.thr = min_prop == 0.0 ? 0u : static_cast<uint32_t>(ceil(static_cast<double>(r.total) * min_prop) - 1.0);
-   r.ref = __ldg(cs->global_ref + p);
-   for (uint32_t s = 0; s < nsym; ++s)
-      if (((valid >> s) & 1u) && s != r.ref && count(s) > r.thr) ++r.n;
-   return r;
+__device__ __forceinline__ uint32_t sum_counts(uint32_t m, CountOf&& count) {
+   uint32_t sum = 0;
+   while (m) {
+      uint32_t c[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+         c[k] = m ? count(__ffs(m) - 1) : 0u;
+         m &= m - 1;
+      }
+      sum += c[0] + c[1] + c[2] + c[3];
+   }
+   return sum;
 }
 
-// The same with the position's counts in registers (`valid`: the column's valid symbols, 0 for no rows).
-template <uint32_t NS>
-__device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ cs, uint32_t p, uint32_t valid,
-                                                 double min_prop, const uint32_t (&c)[NS]) {
+// total = sum of the counts of the valid symbols (0: no rows); threshold = (min_prop == 0) ? 0 :
+// u32(ceil(total * min_prop) - 1); a row for every valid symbol other than the global reference
+// whose count exceeds the threshold. count(s) returns the count of symbol s at p; syms: the valid
+// symbols whose counts can be other than zero.
+template <typename CountOf>
+__device__ __forceinline__ PosRows position_rows(const DevSeqCol* __restrict__ cs, uint32_t p, uint32_t syms,
+                                                 double min_prop, CountOf&& count) {
    PosRows r{0, 0, 0, 0};
-#pragma unroll
-   for (uint32_t s = 0; s < NS; ++s)
-      if ((valid >> s) & 1u) r.total += c[s];
+   r.total = sum_counts(syms, count);
    if (r.total == 0) return r;
    r.thr = min_prop == 0.0 ? 0u : static_cast<uint32_t>(ceil(static_cast<double>(r.total) * min_prop) - 1.0);
    r.ref = __ldg(cs->global_ref + p);
-#pragma unroll
-   for (uint32_t s = 0; s < NS; ++s)
-      if (((valid >> s) & 1u) && s != r.ref && c[s] > r.thr) ++r.n;
+   const uint32_t thr = r.thr;
+   r.n = sum_counts(syms & ~(1u << r.ref), [&](uint32_t s) { return count(s) > thr ? 1u : 0u; });
    return r;
 }
 
