@@ -203,14 +203,31 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
 cudaError_t launch_profile_home(const DevTable* d_table, uint32_t col, uint32_t nchunks, const uint2* d_terms, uint32_t base,
                                 int32_t* d_home, void* stream);
 
+// How a single call gets its result: the filter kernel's CTAs add to acc, and the last of them (ticket)
+// stores the count in d_count and, with the error flag, in pinned host memory, and resets acc and ticket
+// for the next call. The call so needs no clearing and no copies besides the kernel, each of which was an
+// operation on the stream that the next one waited for (a count over 100,000 rows: 39 -> 31 us with the
+// program in the launch's parameters, of which the kernel takes 11). One call of an engine is in flight at
+// a time.
+struct CallResult {
+   unsigned long long count;
+   int err;
+};
+struct CallEnd {
+   unsigned long long* acc;
+   uint32_t* ticket;
+   CallResult* host;  // nullptr: the count is added to d_count and nothing is delivered
+};
+
 // ---- launchers (kernels.cu) ----
+// With inline_code (host memory, at most INLINE_CODE instructions) the program travels with the launch.
 // tile_bits: 4096, 8192, 16384, 32768 or 65536. stack_tiles: Program::tiles. n_leaves: container
 // leaves | coverage leaves << 16. d_trace (trace mode, optional): nchunks * (CHUNK_ROWS / tile_bits)
 // tiles x ncode x 2 u32 (cycles, result popcount per executed instruction), zeroed by the caller.
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
                           uint32_t n_leaves, uint32_t tile_bits, uint32_t stack_tiles, uint32_t* d_out_tiles,
                           unsigned long long* d_count, int* d_err, void* stream, uint32_t* d_trace = nullptr,
-                          const uint32_t* d_aux = nullptr);
+                          const uint32_t* d_aux = nullptr, const CallEnd& end = {}, const Instr* inline_code = nullptr);
 
 // Batched: n_items work items over the programs in d_code; CTAs pull items from *d_next. Every
 // item uses its query's tile width (QueryDesc.tile_bits); scratch_bytes of shared memory per CTA hold

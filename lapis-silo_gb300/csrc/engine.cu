@@ -518,20 +518,24 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
       d_count = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long)));
       counts_words = max_words;
       scratch_words = mut_scratch_words(max_L);
-      d_counts = static_cast<uint32_t*>(alloc(counts_words * 4));
-      d_scratch = static_cast<uint32_t*>(alloc(scratch_words * 4));
+      d_counts = static_cast<uint32_t*>(alloc((counts_words + scratch_words) * 4));
+      d_scratch = d_counts + counts_words;
       d_code = static_cast<Instr*>(alloc(MAX_PROGRAM * sizeof(Instr)));
       d_err = static_cast<int*>(alloc(sizeof(int)));
       cuda_check(cudaMemset(d_err, 0, sizeof(int)), "memset");
       cuda_check(cudaMallocHost(&h_code_, MAX_PROGRAM * sizeof(Instr)), "cudaMallocHost");
-      cuda_check(cudaMallocHost(&h_count_, sizeof(unsigned long long)), "cudaMallocHost");
       cuda_check(cudaMallocHost(&h_err_, sizeof(int)), "cudaMallocHost");
+      *h_err_ = 0;
+      end_.acc = static_cast<unsigned long long*>(alloc(16));
+      cuda_check(cudaMemset(end_.acc, 0, 16), "memset");
+      end_.ticket = reinterpret_cast<uint32_t*>(end_.acc + 1);
+      cuda_check(cudaMallocHost(&end_.host, sizeof(CallResult)), "cudaMallocHost");
       cuda_check(cudaDeviceSynchronize(), "open");
    } catch (...) {
       for (void* p : allocs_) cudaFree(p);
       if (h_code_) cudaFreeHost(h_code_);
-      if (h_count_) cudaFreeHost(h_count_);
       if (h_err_) cudaFreeHost(h_err_);
+      if (end_.host) cudaFreeHost(end_.host);
       if (stream_) cudaStreamDestroy(stream_);
       throw;
    }
@@ -549,8 +553,9 @@ Engine::~Engine() {
       if (p) cudaFree(p);
    for (void* p : allocs_) cudaFree(p);
    if (h_code_) cudaFreeHost(h_code_);
-   if (h_count_) cudaFreeHost(h_count_);
    if (h_err_) cudaFreeHost(h_err_);
+   if (end_.host) cudaFreeHost(end_.host);
+   if (h_bits_) cudaFreeHost(h_bits_);
    if (h_agg_) cudaFreeHost(h_agg_);
    if (h_prof_) cudaFreeHost(h_prof_);
    if (h_prof_data_) cudaFreeHost(h_prof_data_);
@@ -664,6 +669,25 @@ void Engine::upload_program(const Program& p, Instr* dst, cudaStream_t stream) {
 
 void Engine::launch_count(const Instr* code, const Program& p, unsigned long long* count, uint32_t* tiles,
                           cudaStream_t stream, const uint32_t* const* literals) {
+   launch_program(code, nullptr, p, count, tiles, stream, literals, CallEnd{});
+}
+
+void Engine::launch_call(const Program& p, uint32_t* tiles, cudaStream_t stream, const uint32_t* const* literals) {
+   const bool inl = p.code.size() <= INLINE_CODE;
+   if (!inl) upload_program(p, d_code, stream);
+   launch_program(d_code, inl ? p.code.data() : nullptr, p, d_count, tiles, stream, literals, end_);
+}
+
+uint64_t Engine::call_result() {
+   if (end_.host->err != 0) {
+      *h_err_ = end_.host->err;
+      check_error_flag();
+   }
+   return end_.host->count;
+}
+
+void Engine::launch_program(const Instr* code, const Instr* inline_code, const Program& p, unsigned long long* count,
+                            uint32_t* tiles, cudaStream_t stream, const uint32_t* const* literals, const CallEnd& end) {
    const uint32_t W = fit_tile_bits(0, p);
    cudaGetLastError();  // an error left by an unrelated earlier call must not be reported here
    const uint32_t* aux = nullptr;
@@ -695,7 +719,8 @@ void Engine::launch_count(const Instr* code, const Program& p, unsigned long lon
    if (!p.aux.empty() || p.n_literals > 0) aux = d_aux_;
    const cudaError_t e = rhygpu::launch_filter(d_table_, nchunks(), code, static_cast<uint32_t>(p.code.size()),
                                                p.n_ctr_leaves | (p.n_cov_leaves << 16), W,
-                                               p.tiles, tiles, count, d_err, stream, nullptr, aux);
+                                               p.tiles, tiles, count, d_err, stream, nullptr, aux, end,
+                                               inline_code);
    if (e != cudaSuccess)
       throw CudaError("filter kernel launch (tile " + std::to_string(W) + " rows, stack " + std::to_string(p.tiles) +
                       " tiles): " + cudaGetErrorString(e));
@@ -727,14 +752,9 @@ uint64_t Engine::count(const Program& p, cudaStream_t stream, const uint32_t* co
    std::lock_guard<std::mutex> lock(mu);
    cuda_check(cudaSetDevice(device_), "cudaSetDevice");
    if (!stream) stream = stream_;
-   upload_program(p, d_code, stream);
-   cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream), "memset");
-   launch_count(d_code, p, d_count, nullptr, stream, literals);
-   cuda_check(cudaMemcpyAsync(h_count_, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream), "copy count");
-   cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "copy error flag");
+   launch_call(p, nullptr, stream, literals);
    cuda_check(cudaStreamSynchronize(stream), "count");
-   check_error_flag();
-   return *h_count_;
+   return call_result();
 }
 
 void Engine::eval(const Program& p, uint32_t* host_bits, uint64_t* host_count, cudaStream_t stream,
@@ -742,18 +762,15 @@ void Engine::eval(const Program& p, uint32_t* host_bits, uint64_t* host_count, c
    std::lock_guard<std::mutex> lock(mu);
    cuda_check(cudaSetDevice(device_), "cudaSetDevice");
    if (!stream) stream = stream_;
-   upload_program(p, d_code, stream);
-   cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream), "memset");
-   launch_count(d_code, p, d_count, d_filter, stream, literals);
-   if (host_bits)
-      cuda_check(cudaMemcpyAsync(host_bits, d_filter, static_cast<size_t>(nchunks()) * CHUNK_WORDS * 4, cudaMemcpyDeviceToHost,
-                                 stream),
-                 "copy row set");
-   cuda_check(cudaMemcpyAsync(h_count_, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream), "copy count");
-   cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "copy error flag");
+   const size_t words = static_cast<size_t>(nchunks()) * CHUNK_WORDS;
+   // the kernel writes the row set into pinned host memory, from where one copy takes it to the caller's
+   // (a copy from device to pageable memory goes through the driver's staging buffers, piece by piece)
+   if (host_bits) grow_host(h_bits_, words, h_bits_cap_);
+   launch_call(p, host_bits ? h_bits_ : d_filter, stream, literals);
    cuda_check(cudaStreamSynchronize(stream), "eval");
-   check_error_flag();
-   if (host_count) *host_count = *h_count_;
+   const uint64_t n = call_result();
+   if (host_bits) std::memcpy(host_bits, h_bits_, words * 4);
+   if (host_count) *host_count = n;
 }
 
 void Engine::mutations(const Program& p, int column, uint32_t* host_counts, uint64_t* filter_count, cudaStream_t stream,
@@ -764,18 +781,15 @@ void Engine::mutations(const Program& p, int column, uint32_t* host_counts, uint
    if (!stream) stream = stream_;
    const DevSeqCol& c = view_.seq[column];
    const size_t words = static_cast<size_t>(c.nsym) * c.L;
-   upload_program(p, d_code, stream);
-   cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream), "memset");
-   cuda_check(cudaMemsetAsync(d_counts, 0, words * 4, stream), "memset");
-   cuda_check(cudaMemsetAsync(d_scratch, 0, mut_scratch_words(c.L) * 4, stream), "memset");
-   launch_count(d_code, p, d_count, d_filter, stream, literals);
-   launch_mutations(column, d_filter, d_count, d_counts, d_scratch, stream);
-   cuda_check(cudaMemcpyAsync(h_count_, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream), "copy count");
+   uint32_t* scratch = d_counts + words;  // cleared together
+   cuda_check(cudaMemsetAsync(d_counts, 0, (words + mut_scratch_words(c.L)) * 4, stream), "memset");
+   launch_call(p, d_filter, stream, literals);
+   launch_mutations(column, d_filter, d_count, d_counts, scratch, stream);
    cuda_check(cudaMemcpyAsync(host_counts, d_counts, words * 4, cudaMemcpyDeviceToHost, stream), "copy counts");
    cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "copy error flag");
    cuda_check(cudaStreamSynchronize(stream), "mutations");
    check_error_flag();
-   if (filter_count) *filter_count = *h_count_;
+   if (filter_count) *filter_count = end_.host->count;
 }
 
 }  // namespace rhygpu
@@ -1719,10 +1733,8 @@ void Engine::aggregate(const Program& p, const std::vector<AggSpec>& spec, std::
    grow_device(d_agg_blocks_, agg_blocks_cap_, nblocks);
    cuda_check(cudaMemcpyAsync(d_agg_dims_, dims.data(), dims.size() * sizeof(AggDim), cudaMemcpyHostToDevice, stream),
               "H2D");
-   upload_program(p, d_code, stream);
-   cuda_check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream), "memset");
    cuda_check(cudaMemsetAsync(d_agg_counters_, 0, keys * sizeof(uint32_t), stream), "memset");
-   launch_count(d_code, p, d_count, d_filter, stream);
+   launch_call(p, d_filter, stream);
    cuda_check(launch_agg_keys(d_table_, nchunks(), d_filter, d_agg_dims_, static_cast<uint32_t>(dims.size()), keys,
                               d_agg_counters_, stream),
               "aggregation launch");
@@ -1738,10 +1750,8 @@ void Engine::aggregate(const Program& p, const std::vector<AggSpec>& spec, std::
    if (!dense)
       cuda_check(cudaMemcpyAsync(block.data(), d_agg_blocks_, nblocks * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
                  "D2H");
-   cuda_check(cudaMemcpyAsync(h_count_, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream), "D2H");
-   cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "D2H");
    cuda_check(cudaStreamSynchronize(stream), "aggregation");
-   check_error_flag();
+   const uint64_t filtered = call_result();
    uint64_t total = 0;
    for (uint32_t& n : block) {
       const uint32_t x = n;
@@ -1774,7 +1784,7 @@ void Engine::aggregate(const Program& p, const std::vector<AggSpec>& spec, std::
          groups[i * dims.size() + d] = v;
       }
    }
-   if (filter_count) *filter_count = *h_count_;
+   if (filter_count) *filter_count = filtered;
 }
 
 }  // namespace rhygpu

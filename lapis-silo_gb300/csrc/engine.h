@@ -196,6 +196,10 @@ class Engine {
                      cudaStream_t stream, const uint32_t* const* literals = nullptr);
    void launch_mutations(int column, const uint32_t* d_filter, const unsigned long long* d_count, uint32_t* d_counts,
                          uint32_t* d_scratch, cudaStream_t stream, uint32_t parts = MUT_PART_ALL);
+   // The same for a call that waits for its result: the program's upload, and the count and the error flag
+   // delivered to the host (call_result, after the stream was synchronised).
+   void launch_call(const Program& p, uint32_t* d_tiles, cudaStream_t stream, const uint32_t* const* literals = nullptr);
+   uint64_t call_result();
    void check_error_flag();
 
    // ---- batched path ----
@@ -313,7 +317,7 @@ class Engine {
    uint32_t* d_filter = nullptr;      // nchunks * CHUNK_WORDS
    unsigned long long* d_count = nullptr;
    uint32_t* d_counts = nullptr;      // max nsym * L
-   uint32_t* d_scratch = nullptr;     // 3 * (max L + 1)
+   uint32_t* d_scratch = nullptr;     // after the counts: mut_scratch_words(max L)
    Instr* d_code = nullptr;           // MAX_PROGRAM
    int* d_err = nullptr;
    size_t counts_words = 0, scratch_words = 0;
@@ -340,8 +344,12 @@ class Engine {
    std::vector<CtrUnit*> d_cu_;  // container units of the batched Mutations pass, heaviest first
    std::vector<uint32_t> n_cu_;
    Instr* h_code_ = nullptr;               // pinned staging
-   unsigned long long* h_count_ = nullptr; // pinned
    int* h_err_ = nullptr;                  // pinned
+   CallEnd end_{};                         // single calls: acc and ticket on the device, host pinned
+   uint32_t* h_bits_ = nullptr;            // pinned: a call's row set as the filter kernel writes it
+   size_t h_bits_cap_ = 0;
+   void launch_program(const Instr* d_code, const Instr* inline_code, const Program& p, unsigned long long* d_count,
+                       uint32_t* d_tiles, cudaStream_t stream, const uint32_t* const* literals, const CallEnd& end);
    uint64_t device_bytes_ = 0;
    BatchState batch_;
    std::vector<std::unique_ptr<BatchState>> parts_;      // parts 1.. of batch_rows_pipelined

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <stdexcept>
 #include <string>
 
@@ -59,7 +60,7 @@ struct TileCtx {
 constexpr uint32_t LC_LEAVES = 128;
 constexpr uint32_t LC_ENTS = 256;
 constexpr uint32_t LC_COV = 64;
-constexpr uint32_t LC_CODE = 128;
+constexpr uint32_t LC_CODE = INLINE_CODE;
 constexpr uint16_t LC_NONE = 0xFFFF;
 constexpr uint32_t LC_PAY = 3072;      // u16 of array payloads copied into shared memory per item
 constexpr uint32_t LC_BIG = 0x80000000u;
@@ -171,7 +172,7 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
    for (uint32_t i = threadIdx.x; i < LC_ENTS; i += blockDim.x) lc.ent[i] = make_uint2(0, 0);  // E_COPIED, no rows
 #pragma unroll 1
    for (uint32_t i = threadIdx.x; i < ncode; i += blockDim.x) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(code) + i);
+      const uint4 raw = reinterpret_cast<const uint4*>(code)[i];  // global memory or the kernel's parameters
       if (i < LC_CODE) lc.code[i] = raw;
       const Instr in = *reinterpret_cast<const Instr*>(&raw);
       if (in.op == OP_PUSH_COVERED) {
@@ -920,12 +921,30 @@ __device__ __forceinline__ bool run_tile(const TileCtx& c, const Instr* __restri
 // Dynamic shared memory of both kernels: the leaf cache, the scratch tile (of the widest tile), the stack tiles.
 constexpr size_t LC_BYTES = sizeof(LeafCache);
 
+// The CTA's part of a call's end (see CallEnd): the last CTA delivers the count and the error flag.
+__device__ __forceinline__ void end_call(const CallEnd& end, unsigned long long* count, int* err) {
+   __syncthreads();  // the count's additions of every warp
+   if (threadIdx.x != 0) return;
+   __threadfence();
+   if (atomicAdd(end.ticket, 1u) != gridDim.x - 1) return;
+   __threadfence();
+   const unsigned long long total = atomicExch(end.acc, 0ull);
+   *end.ticket = 0;  // for the next call
+   *count = total;
+   end.host->count = total;
+   end.host->err = atomicAdd(err, 0);
+}
+
+// The program comes in the kernel's parameters (ic, at most INLINE_CODE instructions) or, with code, from
+// global memory. With end.host the count goes through end.acc and the call's end is delivered.
 template <bool TRACE>
-__global__ void __launch_bounds__(FT) filter_kernel(const DevTable* __restrict__ tab, const Instr* __restrict__ code,
+__global__ void __launch_bounds__(FT) filter_kernel(const DevTable* __restrict__ tab, const Instr* gcode,
                                                     uint32_t ncode, uint32_t n_leaves, uint32_t tile_bits, uint32_t cap,
                                                     uint32_t* __restrict__ out_tiles, unsigned long long* count, int* err,
-                                                    uint32_t* trace, const uint32_t* __restrict__ aux) {
+                                                    uint32_t* trace, const uint32_t* __restrict__ aux, const CallEnd end,
+                                                    const __grid_constant__ InlineCode ic) {
    extern __shared__ __align__(16) uint8_t smem[];
+   const Instr* code = gcode ? gcode : ic.code;
    LeafCache& lc = *reinterpret_cast<LeafCache*>(smem);
    const uint32_t T = CHUNK_ROWS / tile_bits;
    TileCtx c;
@@ -946,11 +965,15 @@ __global__ void __launch_bounds__(FT) filter_kernel(const DevTable* __restrict__
       for (uint32_t w4 = threadIdx.x; w4 < (tile_bits >> 7); w4 += blockDim.x) X4[w4] = make_uint4(0, 0, 0, 0);
       __syncthreads();
       uint32_t phase = 0;
-      if (!stage_leaves(lc, c, code, ncode, nl, ncov, nullptr, 0, phase, nullptr, err)) return;
+      if (!stage_leaves(lc, c, code, ncode, nl, ncov, nullptr, 0, phase, nullptr, err)) {
+         if (end.host) end_call(end, count, err);
+         return;
+      }
    }
    uint32_t* dst = out_tiles ? out_tiles + static_cast<size_t>(c.v) * CHUNK_WORDS + (c.row0 >> 5) : nullptr;
-   run_tile<TRACE>(c, code, ncode, stk4, cap, X4, lc, nl, ncov, dst, count, err,
+   run_tile<TRACE>(c, code, ncode, stk4, cap, X4, lc, nl, ncov, dst, end.host ? end.acc : count, err,
                    TRACE ? trace + static_cast<size_t>(blockIdx.x) * ncode * 2 : nullptr);
+   if (end.host) end_call(end, count, err);
 }
 
 // launch bounds: three CTAs per SM (at most 85 registers a thread; 64 for four cost 17%).
@@ -1059,16 +1082,22 @@ __global__ void __launch_bounds__(256) dense_forms_kernel(uint16_t* arena, const
 
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
                           uint32_t n_leaves, uint32_t tile_bits, uint32_t stack_tiles, uint32_t* d_out_tiles, unsigned long long* d_count,
-                          int* d_err, void* stream, uint32_t* d_trace, const uint32_t* d_aux) {
+                          int* d_err, void* stream, uint32_t* d_trace, const uint32_t* d_aux, const CallEnd& end,
+                          const Instr* inline_code) {
+   InlineCode ic;
+   if (inline_code) {
+      if (ncode > INLINE_CODE) return cudaErrorInvalidValue;
+      std::memcpy(ic.code, inline_code, ncode * sizeof(Instr));
+   }
    const uint32_t grid = nchunks * (CHUNK_ROWS / tile_bits);
    const uint32_t threads = std::max(32u, std::min(FT, tile_bits / 128));
    const size_t smem = LC_BYTES + static_cast<size_t>(std::max(stack_tiles, 1u)) * (tile_bits / 8);
    const auto kernel = d_trace ? filter_kernel<true> : filter_kernel<false>;
    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
    if (e != cudaSuccess) return e;
-   kernel<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(d_table, d_code, ncode, n_leaves, tile_bits,
+   kernel<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(d_table, inline_code ? nullptr : d_code, ncode, n_leaves, tile_bits,
                                                                       stack_tiles - 1, d_out_tiles, d_count, d_err, d_trace,
-                                                                      d_aux);
+                                                                      d_aux, end, ic);
    return cudaGetLastError();
 }
 

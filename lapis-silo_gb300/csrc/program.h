@@ -84,6 +84,13 @@ constexpr uint16_t GROUP_PUSH = 4;
 constexpr uint32_t PROFILE_DELTA_MAX = 2048;
 
 constexpr uint32_t MAX_PROGRAM = 4096;   // instructions per program
+// A single query's program of up to this many instructions travels in the filter kernel's parameters (2 KiB
+// of their 4), a longer one is copied to device memory first: the copy is an operation of its own on the
+// stream, which the kernel waits for. Generated trees have 5 to 60 instructions.
+constexpr uint32_t INLINE_CODE = 128;
+struct InlineCode {
+   Instr code[INLINE_CODE];
+};
 constexpr uint32_t MAX_THR_PLANES = 16;  // counter planes (NOf up to 65,534 children)
 
 }  // namespace rhygpu

@@ -132,3 +132,21 @@ def test_rows_of_the_final_pass(proportion, staged):
                  float(r["proportion"])) for r in rows[int(b):int(b) + int(n)]] for b, n in zip(begin, cnt)]
         assert got == want
     dev.close()
+
+
+@pytest.mark.parametrize("children", [20, 60, 300])
+def test_programs_around_the_launch_parameters(children):
+    """Programs below and above 128 instructions (the launch's parameters, then device memory) alternate with
+    short ones: count, row set and Mutations of one engine share the state that a call's end resets."""
+    t = R.Table.generate(90000, seed=31, genome_len=900, pool_sites=400, null_fraction=0.01)
+    dev, orc = R.Device(t, 0), oracle_for(t)
+    long = "NOf(3,atleast," + ",".join(f"Or(HasMut(main,{2 * p + 1}),HasMut(main,{2 * p + 2}))" for p in range(children)) + ")"
+    for q in (long, "HasMut(main,9)", long, "Not(HasMut(main,10))", "True"):
+        obits, n = orc.compute_filter(q)
+        assert dev.count(q) == n
+        bits, m = dev.compute_filter(q)
+        assert m == n and np.array_equal(bits, obits)
+        counts, filtered = dev.mutations(q, 0)
+        want, wn = orc.mutations(q, 0)
+        assert filtered == wn == n and np.array_equal(counts, want)
+    dev.close()
