@@ -1153,20 +1153,9 @@ int rhy_planner_predict(RhyDevice* d, const float* x, uint32_t n, double* sel, d
    return guarded([&] {
       need(d, "device");
       if (n) need(x, "x");
-      std::vector<std::array<float, rhygpu::PLAN_FEATURES>> rows(n);
-      for (uint32_t i = 0; i < n; ++i) std::copy(x + static_cast<size_t>(i) * RHY_PLANNER_FEATURES,
-                                                 x + static_cast<size_t>(i + 1) * RHY_PLANNER_FEATURES, rows[i].begin());
-      std::vector<double> s, c;
-      {
-         std::lock_guard<std::mutex> lock(d->engine->mu);
-         rhygpu::cuda_check(cudaSetDevice(d->engine->device()), "cudaSetDevice");
-         if (!d->engine->planner().trained) throw std::invalid_argument("the planner network is not trained");
-         d->engine->planner().predict(rows, s, c);
-      }
-      for (uint32_t i = 0; i < n; ++i) {
-         if (sel) sel[i] = s[i];
-         if (cost) cost[i] = c[i];
-      }
+      std::lock_guard<std::mutex> lock(d->engine->mu);
+      rhygpu::cuda_check(cudaSetDevice(d->engine->device()), "cudaSetDevice");
+      d->engine->planner().predict(x, n, sel, cost);
    });
 }
 
@@ -1188,9 +1177,9 @@ int rhy_mlp_gradient(RhyDevice* d, const float* w, const float* x, const float* 
          need(t, "t");
       }
       rhygpu::cuda_check(cudaSetDevice(d->engine->device()), "cudaSetDevice");
-      rhygpu::PlannerNet net(d->engine->device());
-      net.set_master(w);
-      net.gradient(x, t, n, grad, loss, y);
+      std::unique_ptr<rhygpu::PlannerNet> net = d->engine->take_net();
+      net->gradient_at(w, x, t, n, grad, loss, y);
+      d->engine->give_net(std::move(net));
    });
 }
 

@@ -1554,6 +1554,16 @@ size_t Engine::collect_traces(const std::vector<std::string>& exprs, std::vector
    return added;
 }
 
+std::unique_ptr<PlannerNet> Engine::take_net() {
+   std::lock_guard<std::mutex> lock(net_mu_);
+   return net_ ? std::move(net_) : std::make_unique<PlannerNet>(device_);
+}
+
+void Engine::give_net(std::unique_ptr<PlannerNet> net) {
+   std::lock_guard<std::mutex> lock(net_mu_);
+   if (!net_ && net->capacity() <= NET_KEPT) net_ = std::move(net);
+}
+
 PlannerStats Engine::planner_train(uint32_t epochs, uint32_t batch, float lr, uint64_t seed) {
    std::lock_guard<std::mutex> lock(mu);
    cuda_check(cudaSetDevice(device_), "cudaSetDevice");

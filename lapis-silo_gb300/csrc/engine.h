@@ -285,6 +285,12 @@ class Engine {
    void set_planner_mode(int mode);
    int planner_mode() const { return use_learned_ ? 1 : 0; }
    Planner& planner() { return planner_; }
+   // A network of its own for a call that brings its weights: the one kept from the last such call if no
+   // other thread has it, else a new one. A call gives it back when it has succeeded; one is kept, if its
+   // buffers hold at most NET_KEPT samples (15 MB). Making and freeing one took 200 us of such a call.
+   std::unique_ptr<PlannerNet> take_net();
+   void give_net(std::unique_ptr<PlannerNet> net);
+   static constexpr uint32_t NET_KEPT = 1u << 17;
    // Plans a batch: rule-based, or with the learned planner's estimates (one GPU inference over
    // all operator nodes of all expressions) and a predicted cost per query. `rule_only` plans with
    // the rule even when the learned planner is on. The caller holds mu.
@@ -350,6 +356,8 @@ class Engine {
    size_t h_bits_cap_ = 0;
    void launch_program(const Instr* d_code, const Instr* inline_code, const Program& p, unsigned long long* d_count,
                        uint32_t* d_tiles, cudaStream_t stream, const uint32_t* const* literals, const CallEnd& end);
+   std::mutex net_mu_;
+   std::unique_ptr<PlannerNet> net_;       // see take_net
    uint64_t device_bytes_ = 0;
    BatchState batch_;
    std::vector<std::unique_ptr<BatchState>> parts_;      // parts 1.. of batch_rows_pipelined

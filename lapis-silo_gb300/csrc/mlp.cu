@@ -2,7 +2,11 @@
 //
 //   mlp_forward_kernel   one thread per sample; the BF16 weights are widened once per CTA into
 //                        shared memory; the second hidden layer is folded into the output as it
-//                        is produced, so only the first hidden layer lives in registers.
+//                        is produced, so only the first hidden layer lives in registers. Bound by
+//                        the chains of dependent additions (30,000 samples put two warps on an SM's
+//                        scheduler), so four units of the second layer go at a time, each in the
+//                        order of its inputs. The planner's form takes raw features and returns
+//                        selectivity and cost.
 //   mlp_grad_kernel      forward + backward of the mean squared error for 128 samples per CTA, the
 //                        hidden layers' products on the tensor cores (tcgen05.mma, accumulators in
 //                        tensor memory), FP32 operands entering as split BF16 parts.
@@ -27,9 +31,11 @@ __device__ __forceinline__ void load_weights(const __nv_bfloat16* __restrict__ w
    __syncthreads();
 }
 
+template <bool PLAN>
 __global__ void __launch_bounds__(FWD_T) mlp_forward_kernel(const __nv_bfloat16* __restrict__ w,
                                                             const float* __restrict__ X, uint32_t n,
-                                                            float* __restrict__ Y) {
+                                                            float* __restrict__ Y, const MlpScale scale,
+                                                            double* __restrict__ sel, double* __restrict__ cost) {
    extern __shared__ float sw[];
    load_weights(w, sw);
    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -43,6 +49,11 @@ __global__ void __launch_bounds__(FWD_T) mlp_forward_kernel(const __nv_bfloat16*
    float x[MLP_IN];
 #pragma unroll
    for (uint32_t i = 0; i < MLP_IN; ++i) x[i] = X[static_cast<size_t>(s) * MLP_IN + i];
+   const float x0 = x[0], x1 = x[1], x8 = x[8];
+   if (PLAN) {
+#pragma unroll
+      for (uint32_t i = 0; i < MLP_IN; ++i) x[i] = __fdiv_rn(__fsub_rn(x[i], scale.mean[i]), scale.std[i]);
+   }
    float h1[MLP_H];
 #pragma unroll
    for (uint32_t j = 0; j < MLP_H; ++j) {
@@ -52,16 +63,34 @@ __global__ void __launch_bounds__(FWD_T) mlp_forward_kernel(const __nv_bfloat16*
       h1[j] = fmaxf(a, 0.0f);
    }
    float y0 = B3[0], y1 = B3[1];
-   for (uint32_t j = 0; j < MLP_H; ++j) {
-      float a = B2[j];
+   constexpr uint32_t U = 4;
+#pragma unroll 1
+   for (uint32_t j = 0; j < MLP_H; j += U) {
+      float a[U];
 #pragma unroll
-      for (uint32_t i = 0; i < MLP_H; ++i) a = fmaf(W2[j * MLP_H + i], h1[i], a);
-      a = fmaxf(a, 0.0f);
-      y0 = fmaf(W3[j], a, y0);
-      y1 = fmaf(W3[MLP_H + j], a, y1);
+      for (uint32_t u = 0; u < U; ++u) a[u] = B2[j + u];
+#pragma unroll
+      for (uint32_t i = 0; i < MLP_H; ++i) {
+#pragma unroll
+         for (uint32_t u = 0; u < U; ++u) a[u] = fmaf(W2[(j + u) * MLP_H + i], h1[i], a[u]);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+         const float h = fmaxf(a[u], 0.0f);
+         y0 = fmaf(W3[j + u], h, y0);
+         y1 = fmaf(W3[MLP_H + j + u], h, y1);
+      }
    }
-   Y[2 * static_cast<size_t>(s)] = y0;
-   Y[2 * static_cast<size_t>(s) + 1] = y1;
+   if (PLAN) {
+      const double rule = static_cast<double>(x8) * -scale.min_log_sel;
+      const double ls = x0 > 0.5f || x1 > 0.5f ? rule : rule + static_cast<double>(y0) * scale.tstd[0] + scale.tmean[0];
+      const double m = ls < 0.0 ? ls : 0.0;  // also for a NaN
+      sel[s] = exp(scale.min_log_sel < m ? m : scale.min_log_sel);
+      cost[s] = exp(static_cast<double>(y1) * scale.tstd[1] + scale.tmean[1]);
+   } else {
+      Y[2 * static_cast<size_t>(s)] = y0;
+      Y[2 * static_cast<size_t>(s) + 1] = y1;
+   }
 }
 
 // ---- gradient on the tensor cores ----
@@ -107,7 +136,7 @@ constexpr uint32_t SO_END = SO_TMEM + 8;
 constexpr uint32_t TM_Z1 = 0, TM_Z2 = 64, TM_G1 = 128, TM_DW2 = 192, TM_DW1 = 272, TM_COLS = 512;
 
 // a device error of the gradient kernel (a bounded wait for its MMAs that gave up); read and cleared
-// by mlp_take_error
+// by mlp_read_error and mlp_clear_error
 __device__ int g_mlp_err = 0;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -442,7 +471,15 @@ cudaError_t mlp_cast(const float* d_master, __nv_bfloat16* d_w, cudaStream_t s) 
 cudaError_t mlp_forward(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, float* d_Y, cudaStream_t s) {
    if (n == 0) return cudaSuccess;
    const size_t smem = MLP_NPARAM * sizeof(float);
-   mlp_forward_kernel<<<(n + FWD_T - 1) / FWD_T, FWD_T, smem, s>>>(d_w, d_X, n, d_Y);
+   mlp_forward_kernel<false><<<(n + FWD_T - 1) / FWD_T, FWD_T, smem, s>>>(d_w, d_X, n, d_Y, MlpScale{}, nullptr, nullptr);
+   return cudaGetLastError();
+}
+
+cudaError_t mlp_predict(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, const MlpScale& scale, double* d_sel,
+                        double* d_cost, cudaStream_t s) {
+   if (n == 0) return cudaSuccess;
+   const size_t smem = MLP_NPARAM * sizeof(float);
+   mlp_forward_kernel<true><<<(n + FWD_T - 1) / FWD_T, FWD_T, smem, s>>>(d_w, d_X, n, nullptr, scale, d_sel, d_cost);
    return cudaGetLastError();
 }
 
@@ -455,12 +492,13 @@ cudaError_t mlp_gradient(const __nv_bfloat16* d_w, const float* d_X, const float
    return cudaGetLastError();
 }
 
-int mlp_take_error() {
-   int v = 0;
+cudaError_t mlp_read_error(int* v, cudaStream_t s) {
+   return cudaMemcpyFromSymbolAsync(v, g_mlp_err, sizeof(int), 0, cudaMemcpyDeviceToHost, s);
+}
+
+cudaError_t mlp_clear_error() {
    const int zero = 0;
-   if (cudaMemcpyFromSymbol(&v, g_mlp_err, sizeof(int)) != cudaSuccess) return -1;
-   if (v != 0 && cudaMemcpyToSymbol(g_mlp_err, &zero, sizeof(int)) != cudaSuccess) return -1;
-   return v;
+   return cudaMemcpyToSymbol(g_mlp_err, &zero, sizeof(int));
 }
 
 cudaError_t mlp_adam(float* d_master, __nv_bfloat16* d_w, float* d_grad, float* d_m, float* d_v, float lr, uint32_t step,

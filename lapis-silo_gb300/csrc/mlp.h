@@ -23,13 +23,24 @@ constexpr uint32_t MLP_NPARAM = MLP_B3 + MLP_OUT;
 cudaError_t mlp_cast(const float* d_master, __nv_bfloat16* d_w, cudaStream_t s);
 // Y[n][2] = net(X[n][24]).
 cudaError_t mlp_forward(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, float* d_Y, cudaStream_t s);
+// The planner's prediction around the network: the features' and targets' statistics, and the limits of the
+// selectivity's logarithm.
+struct MlpScale {
+   float mean[MLP_IN], std[MLP_IN];
+   double tmean[MLP_OUT], tstd[MLP_OUT];
+   double min_log_sel;  // ln of the smallest selectivity; feature 8 is a rule estimate's ln over -min_log_sel
+};
+// sel[n], cost[n] of n raw feature rows X[n][24] (see Planner::selectivity_of and cost_of).
+cudaError_t mlp_predict(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, const MlpScale& scale, double* d_sel,
+                        double* d_cost, cudaStream_t s);
 // Adds the gradient of mean_n sum_k (net(X)_k - T_k)^2 with respect to the BF16 weights to d_grad
 // and the loss to *d_loss.
 cudaError_t mlp_gradient(const __nv_bfloat16* d_w, const float* d_X, const float* d_T, uint32_t n, float* d_grad,
                          float* d_loss, cudaStream_t s);
-// A device error of the gradient kernel since the last call (1: a bounded wait for its tensor-core
-// products gave up; -1: the flag could not be read), cleared on reading; 0 if none.
-int mlp_take_error();
+// A device error of the gradient kernel since it was cleared last (1: a bounded wait for its tensor-core
+// products gave up): read on the stream into *v, which is valid once the stream has passed it.
+cudaError_t mlp_read_error(int* v, cudaStream_t s);
+cudaError_t mlp_clear_error();
 // One Adam step (beta 0.9 / 0.999, eps 1e-8, bias-corrected at `step` >= 1) on the master weights;
 // refreshes the BF16 copy and clears the gradient.
 cudaError_t mlp_adam(float* d_master, __nv_bfloat16* d_w, float* d_grad, float* d_m, float* d_v, float lr, uint32_t step,

@@ -188,7 +188,7 @@ PlannerNet::~PlannerNet() {
    cudaSetDevice(device_);
    for (void* p : {static_cast<void*>(d_master_), static_cast<void*>(d_m_), static_cast<void*>(d_v_),
                    static_cast<void*>(d_grad_), static_cast<void*>(d_loss_), static_cast<void*>(d_w_),
-                   static_cast<void*>(d_X_), static_cast<void*>(d_T_), static_cast<void*>(d_Y_)})
+                   static_cast<void*>(d_X_), static_cast<void*>(d_T_), static_cast<void*>(d_Y_), static_cast<void*>(d_P_)})
       if (p) cudaFree(p);
    if (h_X_) cudaFreeHost(h_X_);
    if (h_Y_) cudaFreeHost(h_Y_);
@@ -222,12 +222,16 @@ void PlannerNet::reserve(uint32_t n) {
       cuda_check(cudaMalloc(&d_w_, MLP_NPARAM * sizeof(__nv_bfloat16)), "cudaMalloc (planner)");
    }
    if (n > cap_) {
-      for (float* p : {d_X_, d_T_, d_Y_})
+      for (void* p : {static_cast<void*>(d_X_), static_cast<void*>(d_T_), static_cast<void*>(d_Y_), static_cast<void*>(d_P_)})
          if (p) cudaFree(p);
+      d_X_ = d_T_ = d_Y_ = nullptr;
+      d_P_ = nullptr;
+      cap_ = 0;
       const uint32_t c = std::max(n, 1024u);
       cuda_check(cudaMalloc(&d_X_, static_cast<size_t>(c) * MLP_IN * sizeof(float)), "cudaMalloc (planner)");
       cuda_check(cudaMalloc(&d_T_, static_cast<size_t>(c) * MLP_OUT * sizeof(float)), "cudaMalloc (planner)");
       cuda_check(cudaMalloc(&d_Y_, static_cast<size_t>(c) * MLP_OUT * sizeof(float)), "cudaMalloc (planner)");
+      cuda_check(cudaMalloc(&d_P_, static_cast<size_t>(c) * MLP_OUT * sizeof(double)), "cudaMalloc (planner)");
       cap_ = c;
    }
 }
@@ -261,10 +265,25 @@ void PlannerNet::gradient(const float* X, const float* T, uint32_t n, float* gra
    if (grad) cuda_check(cudaMemcpyAsync(grad, d_grad_, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
    if (loss) cuda_check(cudaMemcpyAsync(loss, d_loss_, sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
    if (Y) cuda_check(cudaMemcpyAsync(Y, d_Y_, static_cast<size_t>(n) * MLP_OUT * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
-   cuda_check(cudaStreamSynchronize(s), "mlp gradient");
-   if (mlp_take_error() != 0) throw std::runtime_error("planner network: a bounded wait of the gradient kernel gave up");
-   cuda_check(cudaMemsetAsync(d_grad_, 0, MLP_NPARAM * sizeof(float), s), "memset");
-   cuda_check(cudaStreamSynchronize(s), "mlp gradient");
+   cuda_check(cudaMemsetAsync(d_grad_, 0, MLP_NPARAM * sizeof(float), s), "memset");  // as training expects it
+   finish(s, "mlp gradient");
+}
+
+void PlannerNet::gradient_at(const float* w, const float* X, const float* T, uint32_t n, float* grad, float* loss,
+                             float* Y) {
+   reserve(n);
+   cuda_check(cudaMemcpyAsync(d_master_, w, MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice, stream_), "upload weights");
+   cuda_check(mlp_cast(d_master_, d_w_, stream_), "cast weights");
+   gradient(X, T, n, grad, loss, Y);
+}
+
+void PlannerNet::finish(cudaStream_t s, const char* what) {
+   int e = 0;
+   cuda_check(mlp_read_error(&e, s), "planner error flag");
+   cuda_check(cudaStreamSynchronize(s), what);
+   if (e == 0) return;
+   mlp_clear_error();
+   throw std::runtime_error("planner network: a bounded wait of the gradient kernel gave up");
 }
 
 float PlannerNet::train(const std::vector<float>& X, const std::vector<float>& T, uint32_t n, uint32_t epochs,
@@ -299,8 +318,7 @@ float PlannerNet::train(const std::vector<float>& X, const std::vector<float>& T
       }
       float loss = 0.0f;
       cuda_check(cudaMemcpyAsync(&loss, d_loss_, sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
-      cuda_check(cudaStreamSynchronize(s), "train epoch");
-      if (mlp_take_error() != 0) throw std::runtime_error("planner network: a bounded wait of the gradient kernel gave up");
+      finish(s, "train epoch");
       last = loss / static_cast<float>(std::max(1u, nb));
    }
    return last;
@@ -315,6 +333,18 @@ void PlannerNet::predict(const float* X, uint32_t n, float* Y) {
    cuda_check(mlp_forward(d_w_, d_X_, n, d_Y_, s), "mlp forward");
    cuda_check(cudaMemcpyAsync(Y, d_Y_, static_cast<size_t>(n) * MLP_OUT * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
    cuda_check(cudaStreamSynchronize(s), "mlp forward");
+}
+
+void PlannerNet::predict_rows(const float* X, uint32_t n, const MlpScale& scale, double* sel, double* cost) {
+   if (!d_master_) throw std::logic_error("planner network not initialised");
+   if (n == 0) return;
+   reserve(n);
+   cudaStream_t s = stream_;
+   cuda_check(cudaMemcpyAsync(d_X_, X, static_cast<size_t>(n) * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
+   cuda_check(mlp_predict(d_w_, d_X_, n, scale, d_P_, d_P_ + n, s), "mlp predict");
+   if (sel) cuda_check(cudaMemcpyAsync(sel, d_P_, n * sizeof(double), cudaMemcpyDeviceToHost, s), "D2H");
+   if (cost) cuda_check(cudaMemcpyAsync(cost, d_P_ + n, n * sizeof(double), cudaMemcpyDeviceToHost, s), "D2H");
+   cuda_check(cudaStreamSynchronize(s), "mlp predict");
 }
 
 float* PlannerNet::staged_input(uint32_t n) {
@@ -466,19 +496,15 @@ PlannerStats Planner::train(uint32_t epochs, uint32_t batch, float lr, uint64_t 
    return st;
 }
 
-void Planner::predict(const std::vector<std::array<float, PLAN_FEATURES>>& x, std::vector<double>& sel,
-                      std::vector<double>& cost) {
-   const uint32_t n = static_cast<uint32_t>(x.size());
-   sel.assign(n, std::nan(""));
-   cost.assign(n, std::nan(""));
-   if (!trained || n == 0) return;
-   std::vector<float> X(static_cast<size_t>(n) * PLAN_FEATURES), Y(static_cast<size_t>(n) * 2);
-   for (uint32_t i = 0; i < n; ++i) normalize(x[i].data(), X.data() + static_cast<size_t>(i) * PLAN_FEATURES);
-   net.predict(X.data(), n, Y.data());
-   for (uint32_t i = 0; i < n; ++i) {
-      sel[i] = selectivity_of(x[i].data(), Y.data() + 2 * i);
-      cost[i] = cost_of(Y.data() + 2 * i);
-   }
+void Planner::predict(const float* x, uint32_t n, double* sel, double* cost) {
+   if (!trained) throw std::invalid_argument("the planner network is not trained");
+   MlpScale scale;
+   std::copy(fmean.begin(), fmean.end(), scale.mean);
+   std::copy(fstd.begin(), fstd.end(), scale.std);
+   std::copy(tmean, tmean + 2, scale.tmean);
+   std::copy(tstd, tstd + 2, scale.tstd);
+   scale.min_log_sel = std::log(MIN_SEL);
+   net.predict_rows(x, n, scale, sel, cost);
 }
 
 void Planner::normalize(const float* x, float* out) const {

@@ -83,7 +83,12 @@ class PlannerNet {
    // Minibatch Adam over shuffled (X, T); returns the final epoch's mean loss.
    float train(const std::vector<float>& X, const std::vector<float>& T, uint32_t n, uint32_t epochs, uint32_t batch,
                float lr, uint64_t seed);
+   // The same under the weights w (MLP_NPARAM host floats), which become the network's.
+   void gradient_at(const float* w, const float* X, const float* T, uint32_t n, float* grad, float* loss, float* Y);
    void predict(const float* X, uint32_t n, float* Y);
+   // Selectivity and cost (either may be null) of n raw feature rows.
+   void predict_rows(const float* X, uint32_t n, const MlpScale& scale, double* sel, double* cost);
+   uint32_t capacity() const { return cap_; }  // samples its buffers hold
    // Pinned host rows (n x MLP_IN) to fill before predict_staged, which runs the network on them
    // and returns its outputs (n x MLP_OUT, pinned, valid until the next call).
    float* staged_input(uint32_t n);
@@ -91,6 +96,7 @@ class PlannerNet {
 
   private:
    void reserve(uint32_t n);
+   void finish(cudaStream_t s, const char* what);  // waits for the stream; throws if a bounded wait gave up
    float* h_X_ = nullptr;  // pinned staging
    float* h_Y_ = nullptr;
    uint32_t hcap_ = 0;
@@ -104,6 +110,7 @@ class PlannerNet {
    float* d_X_ = nullptr;
    float* d_T_ = nullptr;
    float* d_Y_ = nullptr;
+   double* d_P_ = nullptr;  // predict_rows: selectivities, then costs
    uint32_t cap_ = 0;
    uint32_t step_ = 0;
    cudaStream_t stream_ = nullptr;
@@ -125,9 +132,9 @@ class Planner {
    // another table) with the statistics and the acceptance rule of train's held-out split; the
    // verdict is returned, not applied.
    PlannerStats evaluate(const std::vector<PlannerSample>& set);
-   // Selectivity (fraction of rows) and cycles per tile for each feature row.
-   void predict(const std::vector<std::array<float, PLAN_FEATURES>>& x, std::vector<double>& sel,
-                std::vector<double>& cost);
+   // Selectivity (fraction of rows) and cycles per tile of n feature rows, on the device (30,000 rows:
+   // 1.0 ms with the rows normalised and the results' exponentials taken on the host, 93 us so).
+   void predict(const float* x, uint32_t n, double* sel, double* cost);
    // The same one row at a time around the network: its normalised input, then the selectivity
    // and cost from the raw features and the network's two outputs.
    void normalize(const float* x, float* out) const;

@@ -144,3 +144,47 @@ def test_model_trained_on_one_table_plans_another(setup):
     with pytest.raises(R.RhyError):
         dst.planner_import(bad)  # zero deviations
     dst.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 5000])
+def test_predictions_from_raw_rows(setup, n):
+    """Normalisation, network and the exponentials of the device's prediction against the same network's
+    outputs on rows normalised here (the same FP32 operations); index scans keep the rule estimate."""
+    t, _, _, _ = setup
+    dev = R.Device(t, 0)
+    rng = np.random.default_rng(n)
+    w, x, target = random_case(500 + n, n)
+    x[:, 0] = rng.random(n) < 0.3  # index scans
+    x[:, 8] = -rng.random(n)       # the rule estimate
+    model = R.PlannerModel()
+    mean, std = rng.normal(size=24).astype(np.float32), rng.uniform(0.5, 2, 24).astype(np.float32)
+    tmean, tstd = np.array([0.3, 7.0], np.float32).astype(float), np.array([1.5, 0.7], np.float32).astype(float)
+    model.weights[:] = w.tolist()
+    model.feature_mean[:] = mean.tolist()
+    model.feature_std[:] = std.tolist()
+    model.target_mean[:] = tmean.tolist()
+    model.target_std[:] = tstd.tolist()
+    model.accepted = 1
+    dev.planner_import(model)
+    sel, cost = dev.planner_predict(x)
+    y = dev.mlp_gradient(w, (x - mean) / std, target)[2].astype(np.float64)
+    low = np.log(1e-7)
+    rule = x[:, 8].astype(np.float64) * -low
+    log_sel = np.where((x[:, 0] > 0.5) | (x[:, 1] > 0.5), rule, rule + y[:, 0] * tstd[0] + tmean[0])
+    assert np.allclose(sel, np.exp(np.maximum(low, np.minimum(0, log_sel))), rtol=1e-12, atol=0)
+    assert np.allclose(cost, np.exp(y[:, 1] * tstd[1] + tmean[1]), rtol=1e-12, atol=0)
+    dev.close()
+
+
+def test_gradient_calls_of_several_threads(setup):
+    """Calls of several threads and sizes at once: one finds the kept network, the others make their own."""
+    from concurrent.futures import ThreadPoolExecutor
+    _, dev, _, _ = setup
+    cases = [random_case(900 + i, n) for i, n in enumerate([1, 130, 3000, 64, 1025, 200])]
+    with ThreadPoolExecutor(3) as pool:
+        got = list(pool.map(lambda c: dev.mlp_gradient(*c), cases * 3))
+    for (w, x, t), (g, loss, y) in zip(cases * 3, got):
+        oloss, og, oy = M.loss_and_grad(w, x, t)
+        assert np.allclose(y, oy, rtol=1e-4, atol=1e-4)
+        assert loss == pytest.approx(oloss, rel=1e-4)
+        assert np.allclose(g, og, rtol=2e-3, atol=2e-5 * np.abs(og).max())
