@@ -95,8 +95,13 @@ __global__ void __launch_bounds__(FWD_T) mlp_forward_kernel(const __nv_bfloat16*
 
 // ---- gradient on the tensor cores ----
 //
-// One CTA of 128 threads per 128 samples (the MMA's M); thread t owns sample t, which is row t of
-// every accumulator in tensor memory (TMEM lane t). The products run as tcgen05.mma (kind::f16,
+// One CTA of 512 threads per 128 samples (the MMA's M): sample r is row r of every accumulator in tensor
+// memory (TMEM lane r), and its four threads take 16 of the 64 units each (a warp reads the 32 TMEM lanes of
+// its index modulo 4). The kernel is bound by the latency of its phases, one CTA per SM: with one thread per
+// sample, 2-byte stores of every operand element and one atomic per gradient element and thread a CTA took
+// 60 us, so operand rows are stored 16 bytes at a time, the partial gradients are put in order in shared
+// memory and added 16 bytes at a time, and the sums over a warp's samples are taken for 32 values at once
+// (30,011 samples: 128 -> 25 us). The products run as tcgen05.mma (kind::f16,
 // BF16 operands, FP32 accumulation) issued by one thread, operands in shared memory in the
 // no-swizzle K-major layout (8 x 16-byte core matrices), accumulators in TMEM:
 //   phase 0  Z1 = X W1^T                     (M 128, N 64, K 32: the 24 features and zeros)
@@ -107,10 +112,10 @@ __global__ void __launch_bounds__(FWD_T) mlp_forward_kernel(const __nv_bfloat16*
 // The network keeps FP32 arithmetic: an FP32 operand v enters as two BF16 parts, hi = bf16(v) and
 // lo = bf16(v - hi), and the products add the parts' MMAs (the weights are BF16 already, so a
 // forward product takes two MMAs; a weight gradient takes all four combinations, the lo rows of
-// its A operand giving the second half of the accumulator rows, which the threads add when they
-// write the gradient out). That leaves a relative error near 2^-16 per product. The output layer,
+// its A operand giving the second half of the accumulator rows, which are added when the
+// gradient is written out). That leaves a relative error near 2^-16 per product. The output layer,
 // dW3 and db3 (two outputs) stay on the CUDA cores with warp reductions.
-constexpr uint32_t TC_S = 128;
+constexpr uint32_t TC_S = 128, TC_T = 512;
 // byte offset of element (r, k) in a K-major operand of kc 16-byte chunks along K
 __device__ __forceinline__ uint32_t cm_off(uint32_t r, uint32_t k, uint32_t kc) {
    return ((((r >> 3) * kc) + (k >> 3)) << 7) + ((r & 7) << 4) + ((k & 7) << 1);
@@ -129,9 +134,15 @@ constexpr uint32_t SO_H1B_HI = 86016;      // [H1^T; 1; 0] [80 x 128], hi / lo
 constexpr uint32_t SO_H1B_LO = 106496;
 constexpr uint32_t SO_D2T = 126976;        // [D2_hi^T; D2_lo^T] [128 x 128]
 constexpr uint32_t SO_F32 = 159744;        // W3 (128), b1 (64), b2 (64), b3 (2) as floats
-constexpr uint32_t SO_BAR = SO_F32 + 1040;
+constexpr uint32_t SO_Y = SO_F32 + 1040;       // the output layer's partial sums (4 quarters x 128 samples x 2 floats)
+constexpr uint32_t SO_BAR = SO_Y + 4096;
 constexpr uint32_t SO_TMEM = SO_BAR + 8;
 constexpr uint32_t SO_END = SO_TMEM + 8;
+// over dead operands: accumulator rows on their way to the gradient, in padded rows of floats
+constexpr uint32_t GR2 = 68;               // [dW2 | db2] (128 x 65) over H1B, read until phase 2
+constexpr uint32_t GR1 = 28;               // [dW1 | db1] (128 x 25) over XA and XB, read until phase 3
+static_assert(128 * GR2 * 4 <= SO_D2T - SO_H1B_HI && 128 * GR1 * 4 <= SO_W1, "gradient rows fit the operands they replace");
+static_assert(MLP_W1 % 8 == 0 && MLP_W2 % 8 == 0 && MLP_IN % 8 == 0, "weight rows load 16 bytes at a time");
 // TMEM columns of the accumulators
 constexpr uint32_t TM_Z1 = 0, TM_Z2 = 64, TM_G1 = 128, TM_DW2 = 192, TM_DW1 = 272, TM_COLS = 512;
 
@@ -215,14 +226,44 @@ __device__ __forceinline__ float warp_sum(float v) {
    for (uint32_t o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
    return v;
 }
+// The warp's sums of 32 values: lane l returns the sum of v[l] (31 shuffles; 160 one value at a time).
+__device__ __forceinline__ float warp_sums32(float (&v)[32], uint32_t lane) {
+#pragma unroll
+   for (uint32_t m = 16; m > 0; m >>= 1) {
+      const bool up = lane & m;
+#pragma unroll
+      for (uint32_t i = 0; i < m; ++i) {
+         const float keep = up ? v[i + m] : v[i], send = up ? v[i] : v[i + m];
+         v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, m);
+      }
+   }
+   return v[0];
+}
+// Eight values as BF16 parts: hi = bf16(v), lo = bf16(v - hi), each 16 bytes.
+struct Split8 {
+   __align__(16) __nv_bfloat16 hi[8], lo[8];
+};
+__device__ __forceinline__ Split8 split8(const float* v) {
+   Split8 p;
+#pragma unroll
+   for (uint32_t i = 0; i < 8; ++i) {
+      p.hi[i] = __float2bfloat16_rn(v[i]);
+      p.lo[i] = __float2bfloat16_rn(v[i] - __bfloat162float(p.hi[i]));
+   }
+   return p;
+}
+__device__ __forceinline__ void put8(uint8_t* base, uint32_t off, const __nv_bfloat16 (&v)[8]) {
+   *reinterpret_cast<uint4*>(base + off) = *reinterpret_cast<const uint4*>(v);
+}
 
-__global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* __restrict__ w,
+__global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* __restrict__ w,
                                                            const float* __restrict__ X, const float* __restrict__ T,
                                                            uint32_t n, float inv_total, float* __restrict__ grad,
                                                            float* __restrict__ loss) {
    extern __shared__ __align__(1024) uint8_t sm[];
    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
-   const uint32_t s = blockIdx.x * TC_S + t;
+   const uint32_t r = t & (TC_S - 1), q = t / TC_S, u0 = 16 * q;  // sample row, quarter, its first unit
+   const uint32_t s = blockIdx.x * TC_S + r;
    const bool live = s < n;
    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SO_BAR);
    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SO_TMEM);
@@ -230,6 +271,7 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
    float* b1f = W3f + 2 * MLP_H;
    float* b2f = b1f + MLP_H;
    float* b3f = b2f + MLP_H;
+   float2* ypart = reinterpret_cast<float2*>(sm + SO_Y);
    if (t == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -240,36 +282,52 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
                    : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
    }
+   const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f), one = __float2bfloat16_rn(1.0f);
    // weights: W1 [64 x 32] (zeros past the 24 inputs), W2 and W2^T [64 x 64]; the rest as floats
-   for (uint32_t i = t; i < MLP_H * 32; i += TC_S) {
-      const uint32_t j = i / 32, k = i % 32;
-      put_bf16(sm + SO_W1, cm_off(j, k, 4), k < MLP_IN ? w[MLP_W1 + j * MLP_IN + k] : __float2bfloat16_rn(0.0f));
+   if (t < MLP_H * 4) {
+      const uint32_t j = t / 4, k = 8 * (t % 4);
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (k < MLP_IN) v = *reinterpret_cast<const uint4*>(w + MLP_W1 + j * MLP_IN + k);
+      *reinterpret_cast<uint4*>(sm + SO_W1 + cm_off(j, k, 4)) = v;
    }
-   for (uint32_t i = t; i < MLP_H * MLP_H; i += TC_S) {
-      const uint32_t j = i / MLP_H, k = i % MLP_H;
-      const __nv_bfloat16 v = w[MLP_W2 + i];
-      put_bf16(sm + SO_W2, cm_off(j, k, 8), v);
-      put_bf16(sm + SO_W2T, cm_off(k, j, 8), v);
+   {
+      const uint32_t j = t / 8, k = 8 * (t % 8);
+      Split8 v;
+      *reinterpret_cast<uint4*>(v.hi) = *reinterpret_cast<const uint4*>(w + MLP_W2 + j * MLP_H + k);
+      put8(sm + SO_W2, cm_off(j, k, 8), v.hi);
+#pragma unroll
+      for (uint32_t i = 0; i < 8; ++i) put_bf16(sm + SO_W2T, cm_off(k + i, j, 8), v.hi[i]);
    }
-   for (uint32_t i = t; i < 2 * MLP_H; i += TC_S) W3f[i] = __bfloat162float(w[MLP_W3 + i]);
-   if (t < MLP_H) {
-      b1f[t] = __bfloat162float(w[MLP_B1 + t]);
-      b2f[t] = __bfloat162float(w[MLP_B2 + t]);
+   if (t < 2 * MLP_H) W3f[t] = __bfloat162float(w[MLP_W3 + t]);
+   else if (t < 3 * MLP_H) b1f[t - 2 * MLP_H] = __bfloat162float(w[MLP_B1 + t - 2 * MLP_H]);
+   else if (t < 4 * MLP_H) b2f[t - 3 * MLP_H] = __bfloat162float(w[MLP_B2 + t - 3 * MLP_H]);
+   else if (t < 4 * MLP_H + MLP_OUT) b3f[t - 4 * MLP_H] = __bfloat162float(w[MLP_B3 + t - 4 * MLP_H]);
+   float t0 = 0.0f, t1 = 0.0f;
+   if (live) {
+      t0 = T[static_cast<size_t>(s) * MLP_OUT];
+      t1 = T[static_cast<size_t>(s) * MLP_OUT + 1];
    }
-   if (t < MLP_OUT) b3f[t] = __bfloat162float(w[MLP_B3 + t]);
-   // this sample's features: row t of X (hi, lo) and column t of [X^T; 1; 0]
-   for (uint32_t k = 0; k < 32; ++k) {
-      const float v = (live && k < MLP_IN) ? X[static_cast<size_t>(s) * MLP_IN + k] : 0.0f;
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v), lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-      put_bf16(sm + SO_XA_HI, cm_off(t, k, 4), hi);
-      put_bf16(sm + SO_XA_LO, cm_off(t, k, 4), lo);
-      put_bf16(sm + SO_XB_HI, cm_off(k, t, 16), k == MLP_IN ? __float2bfloat16_rn(1.0f) : hi);
-      put_bf16(sm + SO_XB_LO, cm_off(k, t, 16), lo);
+   {  // eight of the sample's features: row r of X (hi, lo) and column r of [X^T; 1; 0]
+      const uint32_t k0 = 8 * q;
+      float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (live && k0 < MLP_IN) {
+         const float4* src = reinterpret_cast<const float4*>(X + static_cast<size_t>(s) * MLP_IN + k0);
+         const float4 a = src[0], b = src[1];
+         v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+      }
+      const Split8 p = split8(v);
+      put8(sm + SO_XA_HI, cm_off(r, k0, 4), p.hi);
+      put8(sm + SO_XA_LO, cm_off(r, k0, 4), p.lo);
+#pragma unroll
+      for (uint32_t i = 0; i < 8; ++i) {
+         put_bf16(sm + SO_XB_HI, cm_off(k0 + i, r, 16), k0 + i == MLP_IN ? one : p.hi[i]);
+         put_bf16(sm + SO_XB_LO, cm_off(k0 + i, r, 16), p.lo[i]);
+      }
    }
    operands_ready();
    const uint32_t tmem = *tmem_slot;
    const uint32_t base = smem_u32(sm);
-   const uint32_t lane_addr = tmem + ((32u * warp) << 16);
+   const uint32_t lane_addr = tmem + ((32u * (warp & 3)) << 16);
    bool ok = true;
    uint32_t committed = 0;  // MMA phases committed to the barrier (the same in every thread)
    // ---- phase 0: Z1 = X W1^T
@@ -280,27 +338,33 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
    }
    ++committed;
    ok = mma_wait(bar, 0);
-   uint32_t mask1[2] = {0, 0}, mask2[2] = {0, 0};
+   uint32_t mask1 = 0, mask2 = 0;  // the quarter's units with a positive input
    if (ok) {
-      // h1 = relu(z1 + b1): row t of H1 (hi, lo) and column t of [H1^T; 1; 0]
-      for (uint32_t c0 = 0; c0 < MLP_H; c0 += 16) {
-         float z[16];
-         tmem_ld16(lane_addr + TM_Z1 + c0, z);
+      // h1 = relu(z1 + b1): row r of H1 (hi, lo) and column r of [H1^T; 1; 0]
+      float z[16];
+      tmem_ld16(lane_addr + TM_Z1 + u0, z);
 #pragma unroll
-         for (uint32_t j = 0; j < 16; ++j) {
-            const float a = z[j] + b1f[c0 + j];
-            const float h = fmaxf(a, 0.0f);
-            if (a > 0.0f) mask1[(c0 + j) >> 5] |= 1u << ((c0 + j) & 31);
-            const __nv_bfloat16 hi = __float2bfloat16_rn(h), lo = __float2bfloat16_rn(h - __bfloat162float(hi));
-            put_bf16(sm + SO_A_HI, cm_off(t, c0 + j, 8), hi);
-            put_bf16(sm + SO_A_LO, cm_off(t, c0 + j, 8), lo);
-            put_bf16(sm + SO_H1B_HI, cm_off(c0 + j, t, 16), hi);
-            put_bf16(sm + SO_H1B_LO, cm_off(c0 + j, t, 16), lo);
+      for (uint32_t j = 0; j < 16; ++j) {
+         const float a = z[j] + b1f[u0 + j];
+         if (a > 0.0f) mask1 |= 1u << j;
+         z[j] = fmaxf(a, 0.0f);
+      }
+#pragma unroll
+      for (uint32_t c = 0; c < 16; c += 8) {
+         const Split8 p = split8(z + c);
+         put8(sm + SO_A_HI, cm_off(r, u0 + c, 8), p.hi);
+         put8(sm + SO_A_LO, cm_off(r, u0 + c, 8), p.lo);
+#pragma unroll
+         for (uint32_t i = 0; i < 8; ++i) {
+            put_bf16(sm + SO_H1B_HI, cm_off(u0 + c + i, r, 16), p.hi[i]);
+            put_bf16(sm + SO_H1B_LO, cm_off(u0 + c + i, r, 16), p.lo[i]);
          }
       }
-      for (uint32_t i = MLP_H; i < 80; ++i) {
-         put_bf16(sm + SO_H1B_HI, cm_off(i, t, 16), __float2bfloat16_rn(i == MLP_H ? 1.0f : 0.0f));
-         put_bf16(sm + SO_H1B_LO, cm_off(i, t, 16), __float2bfloat16_rn(0.0f));
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) {
+         const uint32_t u = MLP_H + 4 * q + i;
+         put_bf16(sm + SO_H1B_HI, cm_off(u, r, 16), u == MLP_H ? one : zero);
+         put_bf16(sm + SO_H1B_LO, cm_off(u, r, 16), zero);
       }
    }
    operands_ready();
@@ -314,54 +378,67 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
       ++committed;
       ok = mma_wait(bar, 1);
    }
+   float h[16];
+   if (ok) {  // the quarter's part of the output layer
+      tmem_ld16(lane_addr + TM_Z2 + u0, h);
+      float y0 = 0.0f, y1 = 0.0f;
+#pragma unroll
+      for (uint32_t j = 0; j < 16; ++j) {
+         const float a = h[j] + b2f[u0 + j];
+         if (a > 0.0f) mask2 |= 1u << j;
+         h[j] = fmaxf(a, 0.0f);
+         y0 = fmaf(W3f[u0 + j], h[j], y0);
+         y1 = fmaf(W3f[MLP_H + u0 + j], h[j], y1);
+      }
+      ypart[q * TC_S + r] = make_float2(y0, y1);
+   }
+   __syncthreads();
    if (ok) {
-      // output layer and its error
       float y0 = b3f[0], y1 = b3f[1];
-      for (uint32_t c0 = 0; c0 < MLP_H; c0 += 16) {
-         float z[16];
-         tmem_ld16(lane_addr + TM_Z2 + c0, z);
 #pragma unroll
-         for (uint32_t j = 0; j < 16; ++j) {
-            const float a = z[j] + b2f[c0 + j];
-            const float h = fmaxf(a, 0.0f);
-            if (a > 0.0f) mask2[(c0 + j) >> 5] |= 1u << ((c0 + j) & 31);
-            y0 = fmaf(W3f[c0 + j], h, y0);
-            y1 = fmaf(W3f[MLP_H + c0 + j], h, y1);
-         }
+      for (uint32_t k = 0; k < 4; ++k) {
+         const float2 y = ypart[k * TC_S + r];
+         y0 += y.x;
+         y1 += y.y;
       }
-      const float r0 = live ? y0 - T[static_cast<size_t>(s) * MLP_OUT] : 0.0f;
-      const float r1 = live ? y1 - T[static_cast<size_t>(s) * MLP_OUT + 1] : 0.0f;
+      const float r0 = live ? y0 - t0 : 0.0f, r1 = live ? y1 - t1 : 0.0f;
       const float d30 = 2.0f * r0 * inv_total, d31 = 2.0f * r1 * inv_total;
-      const float e2 = warp_sum(fmaf(r0, r0, r1 * r1));
-      const float g30 = warp_sum(d30), g31 = warp_sum(d31);
-      if (lane == 0) {
-         atomicAdd(loss, e2 * inv_total);
-         atomicAdd(grad + MLP_B3, g30);
-         atomicAdd(grad + MLP_B3 + 1, g31);
-      }
-      // delta2 = (W3^T d3) * relu'(z2): row t of D2 (hi, lo), column t of [D2_hi^T; D2_lo^T];
-      // dW3 = sum over the samples of d3 h2^T (warp sums, then one atomic per warp)
-      for (uint32_t c0 = 0; c0 < MLP_H; c0 += 16) {
-         float z[16];
-         tmem_ld16(lane_addr + TM_Z2 + c0, z);
-#pragma unroll
-         for (uint32_t j = 0; j < 16; ++j) {
-            const uint32_t u = c0 + j;
-            const float h = fmaxf(z[j] + b2f[u], 0.0f);
-            const bool on = (mask2[u >> 5] >> (u & 31)) & 1u;
-            const float d2 = on ? fmaf(W3f[u], d30, W3f[MLP_H + u] * d31) : 0.0f;
-            const __nv_bfloat16 hi = __float2bfloat16_rn(d2), lo = __float2bfloat16_rn(d2 - __bfloat162float(hi));
-            put_bf16(sm + SO_A_HI, cm_off(t, u, 8), hi);
-            put_bf16(sm + SO_A_LO, cm_off(t, u, 8), lo);
-            put_bf16(sm + SO_D2T, cm_off(u, t, 16), hi);
-            put_bf16(sm + SO_D2T, cm_off(MLP_H + u, t, 16), lo);
-            const float g0 = warp_sum(d30 * h), g1 = warp_sum(d31 * h);
-            if (lane == 0) {
-               atomicAdd(grad + MLP_W3 + u, g0);
-               atomicAdd(grad + MLP_W3 + MLP_H + u, g1);
-            }
+      if (q == 0) {
+         const float e2 = warp_sum(fmaf(r0, r0, r1 * r1));
+         const float g30 = warp_sum(d30), g31 = warp_sum(d31);
+         if (lane == 0) {
+            atomicAdd(loss, e2 * inv_total);
+            atomicAdd(grad + MLP_B3, g30);
+            atomicAdd(grad + MLP_B3 + 1, g31);
          }
       }
+      // delta2 = (W3^T d3) * relu'(z2): row r of D2 (hi, lo), column r of [D2_hi^T; D2_lo^T]
+#pragma unroll
+      for (uint32_t c = 0; c < 16; c += 8) {
+         float d2[8];
+#pragma unroll
+         for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t u = u0 + c + i;
+            d2[i] = (mask2 >> (c + i)) & 1u ? fmaf(W3f[u], d30, W3f[MLP_H + u] * d31) : 0.0f;
+         }
+         const Split8 p = split8(d2);
+         put8(sm + SO_A_HI, cm_off(r, u0 + c, 8), p.hi);
+         put8(sm + SO_A_LO, cm_off(r, u0 + c, 8), p.lo);
+#pragma unroll
+         for (uint32_t i = 0; i < 8; ++i) {
+            put_bf16(sm + SO_D2T, cm_off(u0 + c + i, r, 16), p.hi[i]);
+            put_bf16(sm + SO_D2T, cm_off(MLP_H + u0 + c + i, r, 16), p.lo[i]);
+         }
+      }
+      // dW3 = sum over the samples of d3 h2^T: the warp's sums, output lane >> 4, unit u0 + (lane & 15)
+      float v[32];
+#pragma unroll
+      for (uint32_t j = 0; j < 16; ++j) {
+         v[j] = d30 * h[j];
+         v[16 + j] = d31 * h[j];
+      }
+      const float g = warp_sums32(v, lane);
+      atomicAdd(grad + MLP_W3 + (lane >> 4) * MLP_H + u0 + (lane & 15), g);
    }
    operands_ready();
    // ---- phase 2: G1 = D2 W2; [D2_hi^T; D2_lo^T] [H1^T; 1]^T
@@ -376,31 +453,31 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
       ++committed;
       ok = mma_wait(bar, 0);
    }
+   float* g2 = reinterpret_cast<float*>(sm + SO_H1B_HI);
    if (ok) {
-      // delta1 = G1 * relu'(z1) into column t of [D1_hi^T; D1_lo^T] (over D2, which phase 2 has read)
-      for (uint32_t c0 = 0; c0 < MLP_H; c0 += 16) {
-         float g[16];
-         tmem_ld16(lane_addr + TM_G1 + c0, g);
+      // delta1 = G1 * relu'(z1) into column r of [D1_hi^T; D1_lo^T] (over D2, which phase 2 has read)
+      float g[16];
+      tmem_ld16(lane_addr + TM_G1 + u0, g);
 #pragma unroll
-         for (uint32_t j = 0; j < 16; ++j) {
-            const uint32_t u = c0 + j;
-            const float d1 = ((mask1[u >> 5] >> (u & 31)) & 1u) ? g[j] : 0.0f;
-            const __nv_bfloat16 hi = __float2bfloat16_rn(d1), lo = __float2bfloat16_rn(d1 - __bfloat162float(hi));
-            put_bf16(sm + SO_A_HI, cm_off(u, t, 16), hi);
-            put_bf16(sm + SO_A_HI, cm_off(MLP_H + u, t, 16), lo);
+      for (uint32_t j = 0; j < 16; ++j) g[j] = (mask1 >> j) & 1u ? g[j] : 0.0f;
+#pragma unroll
+      for (uint32_t c = 0; c < 16; c += 8) {
+         const Split8 p = split8(g + c);
+#pragma unroll
+         for (uint32_t i = 0; i < 8; ++i) {
+            put_bf16(sm + SO_A_HI, cm_off(u0 + c + i, r, 16), p.hi[i]);
+            put_bf16(sm + SO_A_HI, cm_off(MLP_H + u0 + c + i, r, 16), p.lo[i]);
          }
       }
-      // dW2 and db2: accumulator row t holds unit t & 63 (hi part for t < 64, lo part above)
-      const uint32_t j = t & (MLP_H - 1);
-      for (uint32_t c0 = 0; c0 < 80; c0 += 16) {
-         float v[16];
-         tmem_ld16(lane_addr + TM_DW2 + c0, v);
+      // dW2 and db2: accumulator row r holds unit r & 63 (hi part for r < 64, lo part above)
+      float v[16];
+      tmem_ld16(lane_addr + TM_DW2 + u0, v);
 #pragma unroll
-         for (uint32_t q = 0; q < 16; ++q) {
-            const uint32_t i = c0 + q;
-            if (i < MLP_H) atomicAdd(grad + MLP_W2 + j * MLP_H + i, v[q]);
-            else if (i == MLP_H) atomicAdd(grad + MLP_B2 + j, v[q]);
-         }
+      for (uint32_t j = 0; j < 16; j += 4)
+         *reinterpret_cast<float4*>(g2 + r * GR2 + u0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      if (q == 0) {
+         tmem_ld16(lane_addr + TM_DW2 + MLP_H, v);
+         g2[r * GR2 + MLP_H] = v[0];
       }
    }
    operands_ready();
@@ -410,22 +487,33 @@ __global__ void __launch_bounds__(TC_S, 1) mlp_grad_kernel(const __nv_bfloat16* 
       mma_k(tmem + TM_DW1, base + SO_A_HI, base + SO_XB_LO, 16, 8, mma_idesc(32), true);
       mma_commit(bar);
    }
+   // row j of the weights' gradient from accumulator rows j (hi) and 64 + j (lo), four elements a thread
+   auto add_rows = [&](const float* rows, uint32_t stride, uint32_t width, float* to, float* bias) {
+      for (uint32_t i = t; i < MLP_H * (width / 4); i += TC_T) {
+         const uint32_t j = i / (width / 4), k = 4 * (i % (width / 4));
+         const float4 a = *reinterpret_cast<const float4*>(rows + j * stride + k);
+         const float4 b = *reinterpret_cast<const float4*>(rows + (MLP_H + j) * stride + k);
+         atomicAdd(reinterpret_cast<float4*>(to + j * width + k), make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w));
+      }
+      if (t < MLP_H) atomicAdd(bias + t, rows[t * stride + width] + rows[(MLP_H + t) * stride + width]);
+   };
    if (ok) {
+      add_rows(g2, GR2, MLP_H, grad + MLP_W2, grad + MLP_B2);
       ++committed;
       ok = mma_wait(bar, 1);
    }
    if (ok) {
-      const uint32_t j = t & (MLP_H - 1);
-      for (uint32_t c0 = 0; c0 < 32; c0 += 16) {
+      float* g1 = reinterpret_cast<float*>(sm);
+      if (q < 2) {
          float v[16];
-         tmem_ld16(lane_addr + TM_DW1 + c0, v);
+         tmem_ld16(lane_addr + TM_DW1 + u0, v);
 #pragma unroll
-         for (uint32_t q = 0; q < 16; ++q) {
-            const uint32_t i = c0 + q;
-            if (i < MLP_IN) atomicAdd(grad + MLP_W1 + j * MLP_IN + i, v[q]);
-            else if (i == MLP_IN) atomicAdd(grad + MLP_B1 + j, v[q]);
-         }
+         for (uint32_t j = 0; j < 16; j += 4)
+            if (u0 + j < GR1)
+               *reinterpret_cast<float4*>(g1 + r * GR1 + u0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
       }
+      __syncthreads();  // ok is the CTA's
+      add_rows(g1, GR1, MLP_IN, grad + MLP_W1, grad + MLP_B1);
    } else if (t == 0) {
       atomicExch(&g_mlp_err, 1);
    }
@@ -488,7 +576,7 @@ cudaError_t mlp_gradient(const __nv_bfloat16* d_w, const float* d_X, const float
    if (n == 0) return cudaSuccess;
    cudaError_t e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SO_END));
    if (e != cudaSuccess) return e;
-   mlp_grad_kernel<<<(n + TC_S - 1) / TC_S, TC_S, SO_END, s>>>(d_w, d_X, d_T, n, 1.0f / static_cast<float>(n), d_grad, d_loss);
+   mlp_grad_kernel<<<(n + TC_S - 1) / TC_S, TC_T, SO_END, s>>>(d_w, d_X, d_T, n, 1.0f / static_cast<float>(n), d_grad, d_loss);
    return cudaGetLastError();
 }
 
