@@ -343,7 +343,10 @@ void launch_rows_write(const DevTable* d_table, const DevSeqCol& col_host, uint3
 void launch_first_k(const uint32_t* d_tiles, uint32_t nq, uint32_t nchunks, const uint32_t* d_k,
                     const uint32_t* d_out_off, uint32_t* d_ids, uint32_t* d_n, void* stream);
 
-// Events per CTA of the coverage pass.
-constexpr uint32_t EV_PER_CTA = 8192;
+// Events per CTA of the batched coverage pass: at most EV_PER_CTA, and down to a quarter of it while that
+// leaves fewer than EV_CTAS CTAs (six on each of 152 SMs). The covered regions' boundaries, of which hardly
+// two share a position, cost a flush of the counters each: a 32nd (with 8192 of them in a CTA it ran for
+// 250 us, longer than all others together at 500,000 rows).
+constexpr uint32_t EV_PER_CTA = 8192, EV_CTAS = 912;
 
 }  // namespace rhygpu

@@ -456,17 +456,19 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          d.n_cend = static_cast<uint32_t>(s.cend.size());
          d.hrow_off = upload(s.hrow_off);
          d.hent = upload(s.hent, s.hent.size() + 8);  // 8 entries of tail: the profile pass reads whole uint4 pairs
-         // coverage-pass work items: event ranges of at most EV_PER_CTA, never spanning two blocks
+         // coverage-pass work items: event ranges of one list and block (see EV_PER_CTA)
          std::vector<EvItem> items;
-         auto split = [&](uint32_t list, uint32_t block, uint32_t b, uint32_t e) {
-            for (uint32_t x = b; x < e; x += EV_PER_CTA) items.push_back({list, block, x, std::min(e, x + EV_PER_CTA)});
+         auto split = [&](uint32_t list, uint32_t block, uint32_t b, uint32_t e, uint32_t per) {
+            for (uint32_t x = b; x < e; x += per) items.push_back({list, block, x, std::min(e, x + per)});
          };
+         const uint64_t share = (s.mstart.size() + s.mend.size()) / EV_CTAS;
+         const uint32_t per = static_cast<uint32_t>(std::min<uint64_t>(EV_PER_CTA, std::max<uint64_t>(share, EV_PER_CTA / 4)));
          for (uint32_t b = 0; b < s.nblocks; ++b) {
-            split(EV_MSTART, b, s.mstart_off[b], s.mstart_off[b + 1]);
-            split(EV_MEND, b, s.mend_off[b], s.mend_off[b + 1]);
+            split(EV_MSTART, b, s.mstart_off[b], s.mstart_off[b + 1], per);
+            split(EV_MEND, b, s.mend_off[b], s.mend_off[b + 1], per);
          }
-         split(EV_CSTART, 0, 0, static_cast<uint32_t>(s.cstart.size()));
-         split(EV_CEND, 0, 0, static_cast<uint32_t>(s.cend.size()));
+         split(EV_CSTART, 0, 0, static_cast<uint32_t>(s.cstart.size()), EV_PER_CTA / 32);
+         split(EV_CEND, 0, 0, static_cast<uint32_t>(s.cend.size()), EV_PER_CTA / 32);
          n_ev_.push_back(static_cast<uint32_t>(items.size()));
          d_ev_.push_back(upload(items));
          const std::vector<CtrUnit> units = container_units(s, nchunks);

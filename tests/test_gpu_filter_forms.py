@@ -150,3 +150,48 @@ def test_programs_around_the_launch_parameters(children):
         want, wn = orc.mutations(q, 0)
         assert filtered == wn == n and np.array_equal(counts, want)
     dev.close()
+
+
+@pytest.fixture(scope="module")
+def heavy_counts():
+    """70,000 rows over 64 sites: containers of most rows of a chunk, missing intervals that start and end
+    together, covered regions that end alone; and the oracle's Mutations by query."""
+    n, L = 70000, 64
+    rng = np.random.default_rng(8)
+    ref = "ACGT" * (L // 4)
+    rows = np.tile(np.frombuffer(ref.encode(), np.uint8), (n, 1))
+    rows[rng.random(n) < 0.95, 20] = ord("N")
+    rows[rng.random(n) < 0.4, 21:25] = ord("-")
+    rows[rng.random(n) < 0.002, 40] = ord("T")
+    rows[rng.random(n) < 0.45, 41] = ord("T")
+    starts, ends = rng.integers(0, 10, n), rng.integers(L - 8, L + 1, n)
+    at, some = np.arange(L), rng.random(n) < 0.03
+    rows[some[:, None] & ((at < starts[:, None]) | (at >= ends[:, None]))] = ord("N")
+    b = RawBuilder(n)
+    b.add_sequences("main", 0, ref, [r.tobytes().decode() for r in rows])
+    raw = b.raw()
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    known = {}
+
+    def mutations(q):
+        if q not in known:
+            known[q] = orc.mutations(q, 0)
+        return known[q]
+
+    yield dev, mutations
+    dev.close()
+
+
+@pytest.mark.parametrize("slots", [1, 12, 33, 65, 129, 257, 300])
+def test_batched_counters(heavy_counts, slots):
+    """The batched passes at one to eight mask words per row and at a second pass of one and two; the counters'
+    planes fill up and are taken in between."""
+    dev, mutations = heavy_counts
+    forms = ["True", "Not(HasMut(main,41))", "SymEq(main,21,N)", "Not(SymEq(main,22,-))", "HasMut(main,42)"]
+    qs = [f"And({forms[i % 5]},{forms[i // 5 % 5]})" for i in range(25)]
+    qs = [qs[i * 7 % 25] for i in range(slots)]
+    counts, muts = dev.batch(qs, [1] * slots, [0] * slots)
+    for i, q in enumerate(qs):
+        want, n = mutations(q)
+        assert counts[i] == n and np.array_equal(muts[i], want), q
