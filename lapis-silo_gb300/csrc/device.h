@@ -262,9 +262,13 @@ enum : uint32_t { BMUT_PART_TRANSPOSE = 1, BMUT_PART_CTR = 2, BMUT_PART_COV = 4,
 // Filters of at most sparse_max rows (0: none) take the row-index pass (part MUT_PART_SPARSE) instead
 // of the container and coverage passes: their rows read their row-index entries.
 enum : uint32_t { MUT_PART_SPARSE = 8 };
+// MUT_PART_CLEAR: the counts, the scratch and *d_err_clear (if not null) start from zero here, else the caller
+// has cleared them.
+enum : uint32_t { MUT_PART_CLEAR = 16 };
 void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
                       const uint32_t* d_filter, const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
-                      void* stream, uint32_t parts = MUT_PART_ALL | MUT_PART_SPARSE, uint64_t sparse_max = 0);
+                      void* stream, uint32_t parts = MUT_PART_ALL | MUT_PART_SPARSE, uint64_t sparse_max = 0,
+                      int* d_err_clear = nullptr);
 // Testing the failure path of the filter kernels' bounded waits on the current device: while on,
 // the leaf payload copies they announce are never issued, so their waits give up and the kernels
 // set error 6 (DEVERR_WAIT_FILTER) instead of evaluating. Nothing is left in flight.

@@ -520,8 +520,8 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
       d_count = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long)));
       counts_words = max_words;
       scratch_words = mut_scratch_words(max_L);
-      d_counts = static_cast<uint32_t*>(alloc((counts_words + scratch_words) * 4));
-      d_scratch = d_counts + counts_words;
+      d_counts = static_cast<uint32_t*>(alloc(counts_words * 4));
+      d_scratch = static_cast<uint32_t*>(alloc(scratch_words * 4));
       d_code = static_cast<Instr*>(alloc(MAX_PROGRAM * sizeof(Instr)));
       d_err = static_cast<int*>(alloc(sizeof(int)));
       cuda_check(cudaMemset(d_err, 0, sizeof(int)), "memset");
@@ -783,10 +783,8 @@ void Engine::mutations(const Program& p, int column, uint32_t* host_counts, uint
    if (!stream) stream = stream_;
    const DevSeqCol& c = view_.seq[column];
    const size_t words = static_cast<size_t>(c.nsym) * c.L;
-   uint32_t* scratch = d_counts + words;  // cleared together
-   cuda_check(cudaMemsetAsync(d_counts, 0, (words + mut_scratch_words(c.L)) * 4, stream), "memset");
    launch_call(p, d_filter, stream, literals);
-   launch_mutations(column, d_filter, d_count, d_counts, scratch, stream);
+   launch_mutations(column, d_filter, d_count, d_counts, d_scratch, stream, MUT_PART_ALL | MUT_PART_SPARSE | MUT_PART_CLEAR);
    cuda_check(cudaMemcpyAsync(host_counts, d_counts, words * 4, cudaMemcpyDeviceToHost, stream), "copy counts");
    cuda_check(cudaMemcpyAsync(h_err_, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "copy error flag");
    cuda_check(cudaStreamSynchronize(stream), "mutations");

@@ -323,7 +323,7 @@ class Engine {
    uint32_t* d_filter = nullptr;      // nchunks * CHUNK_WORDS
    unsigned long long* d_count = nullptr;
    uint32_t* d_counts = nullptr;      // max nsym * L
-   uint32_t* d_scratch = nullptr;     // after the counts: mut_scratch_words(max L)
+   uint32_t* d_scratch = nullptr;     // mut_scratch_words(max L)
    Instr* d_code = nullptr;           // MAX_PROGRAM
    int* d_err = nullptr;
    size_t counts_words = 0, scratch_words = 0;

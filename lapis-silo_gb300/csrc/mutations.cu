@@ -8,9 +8,9 @@
 //                    differences over positions (reference: mutations_node.cpp:51-136).
 //  mut_final_kernel  prefix sums and the local-reference count per position
 //                    (reference: mutations_node.cpp:192-203).
-//  mut_sparse_kernel filters of few rows: each row of F adds its row-index entries, the same counts
-//                    the two passes above add for it (the reference's mixed path walks the filtered
-//                    rows for coverage the same way, mutations_node.cpp:111-136).
+//                    Filters of few rows: each row of F adds its row-index entries, the same counts
+//                    this and the container pass add for it (the reference's mixed path walks the
+//                    filtered rows for coverage the same way, mutations_node.cpp:111-136).
 // The filter count decides on the device between the full path (|F| == rows: stored
 // cardinalities, reference: mutations_node.cpp:240-266), the empty path and the mixed path.
 #include <cuda_runtime.h>
@@ -29,6 +29,16 @@ namespace {
 
 constexpr uint32_t MT = 256;
 constexpr uint32_t NW = MT / 32;
+
+// The pass is a chain of short kernels (2M rows: clearing 2 us, coverage 18, containers 36, prefix sums 6),
+// launched as programmatic dependents: each starts while the one before still runs, as soon as every CTA of
+// that has called pdl_trigger, and waits with pdl_wait for its completion where it needs its results. The
+// order is clear, coverage (waits after staging its filter words), containers (needs only the cleared
+// counts, which the coverage pass waited for before its trigger; fills the SMs beside it and waits for its
+// end before its own), prefix sums (waits at once). Both calls do nothing in a kernel launched otherwise.
+// One pass over a resident filter at 2M rows: 74 us as seven operations in a row, 57 so.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Shared-memory ring of the container pass.
 constexpr uint32_t RING_SLOTS = 16;
@@ -174,8 +184,12 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
                                                           unsigned long long sparse_max, uint32_t* counts, int* err) {
    extern __shared__ __align__(128) uint8_t ring_raw[];
    Ring& R = *reinterpret_cast<Ring*>(ring_raw);
+   pdl_trigger();
    const unsigned long long fc = *fcount;
-   if (fc == 0 || fc <= sparse_max) return;  // empty, or counted by the row-index pass
+   if (fc == 0 || fc <= sparse_max) {  // empty, or counted by the row-index pass
+      pdl_wait();
+      return;
+   }
    const bool full = fc == tab->n_rows;
    const DevSeqCol* cs = &tab->seq[col];
    const StreamRange rg = cs->ranges[blockIdx.x];
@@ -412,6 +426,7 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
          if (two) ring_wait(&R.tile[1], 0, 256, limit);
       }
    }
+   pdl_wait();  // the coverage pass, so that what follows this kernel follows both
 }
 
 // Coverage of the filter per position, as differences over positions (reference:
@@ -423,16 +438,29 @@ __global__ void __launch_bounds__(RING_T, RING_CTAS_PER_SM) mut_ring_kernel(cons
 // Bound: 4 bytes and about 14 instructions per boundary (31 MB at 2M rows) and 8 KiB of filter per CTA and
 // chunk. Before, the same boundaries sorted by position over all chunks each tested a filter bit in L2:
 // 58.8 us at 2M rows and 400,000 filtered rows, one 32-byte sector per boundary.
+//
+// Filters of 1..sparse_max rows take the row-index pass here instead (one warp per 32 filter words at a
+// time, any grid), in the same shared memory: a kernel of its own cost every other filter a launch.
 constexpr uint32_t COV_BLOCKS = 4, COV_CHUNKS = 4;
 __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                      const uint32_t* __restrict__ filter,
                                                      const unsigned long long* __restrict__ fcount,
-                                                     unsigned long long sparse_max, uint32_t* scratch) {
+                                                     unsigned long long sparse_max, bool coverage, uint32_t* counts,
+                                                     uint32_t* scratch) {
    __shared__ __align__(16) uint32_t F[COV_CHUNKS][CHUNK_WORDS];
    __shared__ int hist[COV_BLOCKS][NBLOCK];
    const unsigned long long fc = *fcount;
-   if (fc == 0 || fc <= sparse_max) return;  // empty, or counted by the row-index pass
    const DevSeqCol* cs = &tab->seq[col];
+   if (fc <= sparse_max || !coverage) {
+      pdl_wait();
+      pdl_trigger();
+      if (fc == 0 || fc > sparse_max) return;
+      static_assert(sizeof(F) >= NW * 1024 * sizeof(uint32_t), "the rows of 32 words per warp");
+      const uint32_t words = tab->nchunks * CHUNK_WORDS, nwarps = gridDim.x * NW, w0 = threadIdx.x >> 5;
+      for (uint32_t w = (blockIdx.x * NW + w0) * 32; w < words; w += nwarps * 32)
+         row_index_pass32(cs, filter, w, words, counts, scratch, F[0] + 1024 * w0);
+      return;
+   }
    const uint32_t L = cs->L, nseg = mut_nseg(L), nchunks = tab->nchunks, nblocks = cs->nblocks_ev;
    uint32_t* start_hist = scratch;
    uint32_t* ndiff = scratch + 2 * (L + 1);  // (the ends' histogram lies between)
@@ -446,6 +474,8 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
       const uint4* src = reinterpret_cast<const uint4*>(filter + static_cast<size_t>(v0) * CHUNK_WORDS);
       for (uint32_t i = threadIdx.x; i < nv * (CHUNK_WORDS / 4); i += MT) reinterpret_cast<uint4*>(F[0])[i] = __ldg(src + i);
       for (uint32_t i = threadIdx.x; i < COV_BLOCKS * NBLOCK; i += MT) hist[0][i] = 0;
+      pdl_wait();
+      pdl_trigger();
       __syncthreads();
       for (uint32_t j = warp; j < nb * nv; j += NW) {
          const uint32_t bl = j / nv, v = j % nv;
@@ -486,6 +516,8 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
       const uint32_t ns = cs->n_cstart, n = ns + cs->n_cend;
       const uint32_t i = (blockIdx.x - gb * gv) * MT + threadIdx.x;  // one event per thread
       const bool start = i < ns;
+      pdl_wait();
+      pdl_trigger();
       const uint2 e = i < n ? __ldg(reinterpret_cast<const uint2*>(start ? cs->cstart + i : cs->cend + (i - ns))) : make_uint2(0, 0);
       const bool in = i < n && ((__ldg(filter + (e.x >> 5)) >> (e.x & 31)) & 1u);
       // events are sorted by position: the lanes of a position, and those of a segment, add once
@@ -499,25 +531,19 @@ __global__ void __launch_bounds__(MT) mut_cov_kernel(const DevTable* __restrict_
 }
 static_assert(MUT_SEG % (COV_BLOCKS * NBLOCK) == 0, "a CTA's positions lie in one segment");
 
-// Filters of 1..sparse_max rows: one warp per 32 filter words at a time.
-__global__ void __launch_bounds__(MT) mut_sparse_kernel(const DevTable* __restrict__ tab, uint32_t col,
-                                                        const uint32_t* __restrict__ filter,
-                                                        const unsigned long long* __restrict__ fcount,
-                                                        unsigned long long sparse_max, uint32_t* counts,
-                                                        uint32_t* scratch) {
-   __shared__ uint32_t list[NW][1024];
-   const unsigned long long fc = *fcount;
-   if (fc == 0 || fc > sparse_max) return;
-   const DevSeqCol* cs = &tab->seq[col];
-   const uint32_t words = tab->nchunks * CHUNK_WORDS;
-   const uint32_t warp = threadIdx.x >> 5, nwarps = gridDim.x * NW;
-   for (uint32_t w = (blockIdx.x * NW + warp) * 32; w < words; w += nwarps * 32)
-      row_index_pass32(cs, filter, w, words, counts, scratch, list[warp]);
+__global__ void __launch_bounds__(1024) mut_clear_kernel(uint32_t* counts, uint32_t n_counts, uint32_t* scratch,
+                                                         uint32_t n_scratch, int* status) {
+   pdl_trigger();
+   const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+   for (uint32_t i = i0; i < n_counts; i += step) counts[i] = 0;
+   for (uint32_t i = i0; i < n_scratch; i += step) scratch[i] = 0;
+   if (status && i0 == 0) *status = 0;
 }
 
 __global__ void __launch_bounds__(MUT_SEG, 2) mut_final_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                             const unsigned long long* __restrict__ fcount,
                                                             uint32_t* counts, const uint32_t* __restrict__ scratch) {
+   pdl_wait();
    final_position_counts(&tab->seq[col], static_cast<uint32_t>(*fcount), counts, scratch);
 }
 
@@ -539,27 +565,47 @@ void mutations_setup() {
 void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
                       const uint32_t* d_filter,
                       const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
-                      void* stream, uint32_t parts, uint64_t sparse_max) {
+                      void* stream, uint32_t parts, uint64_t sparse_max, int* d_err_clear) {
    cudaStream_t s = static_cast<cudaStream_t>(stream);
    if (!(parts & MUT_PART_SPARSE)) sparse_max = 0;  // the dense passes count every filter
-   if (sparse_max) {
-      const uint32_t groups = nchunks * CHUNK_WORDS / 32;  // 32-word groups, one per warp and step
-      mut_sparse_kernel<<<std::max(1u, std::min(groups / NW, 2048u)), MT, 0, s>>>(
-         d_table, col, d_filter, d_filter_count, static_cast<unsigned long long>(sparse_max), d_counts, d_scratch);
+   // a dependent only of a kernel of this pass launched just before it, in the order above
+   auto launch = [&](auto* kernel, uint32_t grid, uint32_t threads, size_t smem, bool dependent, auto... args) {
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = grid;
+      cfg.blockDim = threads;
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = s;
+      cfg.attrs = &attr;
+      cfg.numAttrs = dependent ? 1 : 0;
+      cudaLaunchKernelEx(&cfg, kernel, args...);  // errors are read by the caller
+   };
+   const unsigned long long limit = sparse_max;
+   const bool clear = parts & MUT_PART_CLEAR;
+   if (clear) {
+      const uint32_t words = col_host.nsym * col_host.L;
+      launch(mut_clear_kernel, std::min((words + 1023) / 1024, 152u), 1024, 0, false, d_counts, words, d_scratch,
+             static_cast<uint32_t>(mut_scratch_words(col_host.L)), d_err_clear);
    }
-   if ((parts & MUT_PART_CTR) && col_host.nranges > 0)
-      mut_ring_kernel<<<col_host.nranges, RING_T, RING_SMEM, s>>>(
-         d_table, col, d_filter, d_filter_count, static_cast<unsigned long long>(sparse_max), d_counts, d_err);
-   if (parts & MUT_PART_COV) {
+   const bool coverage = parts & MUT_PART_COV;
+   const bool first = coverage || sparse_max > 0;
+   if (first) {
       const uint32_t buckets =
          ((nchunks + COV_CHUNKS - 1) / COV_CHUNKS) * ((col_host.nblocks_ev + COV_BLOCKS - 1) / COV_BLOCKS);
       const uint32_t events = (col_host.n_cstart + col_host.n_cend + MT - 1) / MT;
-      mut_cov_kernel<<<buckets + events, MT, 0, s>>>(d_table, col, d_filter, d_filter_count,
-                                                     static_cast<unsigned long long>(sparse_max), d_scratch);
+      const uint32_t groups = nchunks * CHUNK_WORDS / 32;  // 32-word groups, one per warp and step
+      const uint32_t sparse_ctas = sparse_max ? std::max(1u, std::min(groups / NW, 2048u)) : 1u;
+      launch(mut_cov_kernel, std::max(coverage ? buckets + events : 1u, sparse_ctas), MT, 0, clear, d_table, col, d_filter,
+             d_filter_count, limit, coverage, d_counts, d_scratch);
    }
+   const bool ring = (parts & MUT_PART_CTR) && col_host.nranges > 0;
+   if (ring) launch(mut_ring_kernel, col_host.nranges, RING_T, RING_SMEM, first, d_table, col, d_filter, d_filter_count, limit,
+                    d_counts, d_err);
    if (parts & MUT_PART_FINAL)
-      mut_final_kernel<<<(col_host.L + MUT_SEG - 1) / MUT_SEG, MUT_SEG, 0, s>>>(d_table, col, d_filter_count, d_counts,
-                                                                               d_scratch);
+      launch(mut_final_kernel, (col_host.L + MUT_SEG - 1) / MUT_SEG, MUT_SEG, 0, ring, d_table, col, d_filter_count, d_counts,
+             static_cast<const uint32_t*>(d_scratch));
 }
 
 }  // namespace rhygpu

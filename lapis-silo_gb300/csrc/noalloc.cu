@@ -75,12 +75,9 @@ void mutations_noalloc(Engine& engine, uint32_t column, const uint32_t* d_filter
    uint32_t* scratch = scratch_address(engine.device());
    cudaStream_t s = engine.stream_for(stream);
    // the pass accumulates into both buffers, so they start from zero; the status starts clear
-   cuda_check(cudaMemsetAsync(scratch, 0, mut_scratch_words(col.L) * sizeof(uint32_t), s), "clear scratch");
-   cuda_check(cudaMemsetAsync(d_counts, 0, static_cast<size_t>(col.nsym) * col.L * sizeof(uint32_t), s), "clear counts");
-   cuda_check(cudaMemsetAsync(d_status, 0, sizeof(int), s), "clear status");
    cudaGetLastError();
    launch_mutations(engine.d_table(), col, column, engine.nchunks(), d_filter, d_filter_count, d_counts, scratch, d_status, s,
-                    MUT_PART_ALL | MUT_PART_SPARSE, engine.sparse_rows_plain);
+                    MUT_PART_ALL | MUT_PART_SPARSE | MUT_PART_CLEAR, engine.sparse_rows_plain, d_status);
    cuda_check(cudaGetLastError(), "mutations (no allocation) launch");
 }
 

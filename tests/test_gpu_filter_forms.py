@@ -195,3 +195,25 @@ def test_batched_counters(heavy_counts, slots):
     for i, q in enumerate(qs):
         want, n = mutations(q)
         assert counts[i] == n and np.array_equal(muts[i], want), q
+
+
+@pytest.mark.parametrize("differing", [True, False])
+def test_mutations_around_the_row_index_limit(differing):
+    """Filters of no rows, one, the most that take the row index, one more and all, one call after another, over
+    a column with containers and one that equals its reference everywhere."""
+    n = 70000
+    rng = np.random.default_rng(4)
+    pool = ["ACGTACGT", "ACGAACGT", "NCGTACG-", "ACNNNCGT"] if differing else ["ACGTACGT"]
+    b = RawBuilder(n).add_sequences("main", 0, "ACGTACGT", [pool[i] for i in rng.integers(0, len(pool), n)])
+    b.add_dates("date", list(range(n)))
+    raw = b.raw()
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    limit = dev.sparse_rows()[0]
+    assert 1 < limit < n - 1
+    for rows in (limit, limit + 1, 1, n, 0, limit + 1, limit):
+        q = f"DateBetween(date,*,{rows - 1})" if rows else "And(True,Not(True))"
+        counts, filtered = dev.mutations(q, 0)
+        want, k = orc.mutations(q, 0)
+        assert filtered == k == rows and np.array_equal(counts, want)
+    dev.close()
