@@ -133,18 +133,6 @@ __device__ __forceinline__ bool wait_slot_unit(const uint32_t* hdr, uint32_t k, 
 // set_ring_withholding.
 __device__ uint32_t g_withhold_ring_copies = 0;
 
-// 32 x 32 bit transpose across a warp: lane j returns the word whose bit l is bit j of lane l's x.
-// Five exchange steps, step s swapping bit s of the lane index with bit s of the bit index.
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, uint32_t lane) {
-#pragma unroll
-   for (uint32_t s = 16; s >= 1; s >>= 1) {
-      const uint32_t M0 = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
-      const uint32_t p = __shfl_xor_sync(0xFFFFFFFFu, x, s);
-      x = (lane & s) ? ((x & ~M0) | ((p >> s) & M0)) : ((x & M0) | ((p << s) & ~M0));
-   }
-   return x;
-}
-
 // Membership bits of a unit's row ids in the filter tile F: W[it] holds the two u16 row ids of
 // elements 64 it + 2 lane and 64 it + 2 lane + 1, whose bits land at 2 it and 2 it + 1. The bit of
 // row r is bit r & 31 of word r >> 5; rotating that word right by (r - k) & 31 brings it to bit k

@@ -59,6 +59,18 @@ __device__ __forceinline__ uint32_t count_range(const uint32_t* F, uint32_t a, u
    return s;
 }
 
+// 32 x 32 bit transpose across a warp: lane j returns the word whose bit l is bit j of lane l's x.
+// Five exchange steps, step s swapping bit s of the lane index with bit s of the bit index.
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, uint32_t lane) {
+#pragma unroll
+   for (uint32_t s = 16; s >= 1; s >>= 1) {
+      const uint32_t M0 = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+      const uint32_t p = __shfl_xor_sync(0xFFFFFFFFu, x, s);
+      x = (lane & s) ? ((x & ~M0) | ((p >> s) & M0)) : ((x & M0) | ((p << s) & ~M0));
+   }
+   return x;
+}
+
 // Final pass for positions [blockIdx.x * MUT_SEG, +MUT_SEG) of one query (blockDim.x == MUT_SEG):
 //   ref(p) = |F| - #(start > p) - #(end <= p) - missing(p) - sum_s counts[s][p]
 //   counts[local_ref[p]][p] += ref(p)
