@@ -8,6 +8,7 @@
 //   transpose_kernel       filter row sets -> masks, pass-major rows (32 B per row and pass)
 //   mut_ctr_batch_kernel   container pass, one warp per (position, chunk range) unit: |F_q ∩ c|
 //                          for every container c (reference: mutations_node.cpp:138-190)
+//   mut_ctr_narrow_kernel  the same for a pass of at most 32 queries, masks in shared memory
 //   mut_cov_batch_kernel   missing-interval and coverage boundary events (reference:
 //                          mutations_node.cpp:51-136)
 //   mut_final_batch_kernel prefix sums and reference counts per query
@@ -18,6 +19,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <stdexcept>
+#include <string>
 
 #include "device.h"
 #include "mutations_common.cuh"
@@ -175,8 +178,8 @@ __device__ __forceinline__ void count_window_bits(BitCounter& k, const LaneSplit
 // this lane ends up with: query q of the mask word l.w, i counting the lane's queries (at most 8, the same
 // ones each time). The counts leave the planes as pairs of 16 bits (32 lanes of COUNT_MAX fit), and each
 // exchange between row groups halves the pairs a lane holds. qn: the queries a mask word can have.
-template <uint32_t N>
-__device__ __forceinline__ void halve_words(uint32_t (&W)[16], uint32_t off) {
+template <uint32_t N, uint32_t M>
+__device__ __forceinline__ void halve_words(uint32_t (&W)[M], uint32_t off) {
    const bool up = threadIdx.x & off;
 #pragma unroll
    for (uint32_t i = 0; i < N; ++i) {
@@ -259,7 +262,7 @@ __device__ __forceinline__ void take_counts(BitCounter& k, const LaneSplit& l, u
 // expanded 1024 rows at a time into a per-warp row list in shared memory.
 // Bound: issue slots (60% of them taken) and the latency of the mask gathers; loading the next containers'
 // descriptors and rows ahead cost 10%, and three CTAs per SM in place of four 20%. 2M rows and 263 queries
-// (256 and 7): 1.11 ms, 1.26 with byte counters; 12 queries at 500,000 rows: 107 us.
+// (256 and 7): 1.11 ms, 1.26 with byte counters; 0.75 without the 7 (mut_ctr_narrow_kernel).
 __global__ void __launch_bounds__(BT, 4) mut_ctr_batch_kernel(const DevTable* __restrict__ tab, uint32_t col,
                                                            const CtrUnit* __restrict__ units, uint32_t n_units,
                                                            const uint16_t* __restrict__ R,
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(BT, 4) mut_ctr_batch_kernel(const DevTable* __
    const uint32_t u = blockIdx.x * (BT / 32) + warp;
    const uint32_t nq = lists[2 * nq_max];  // dense slots: lists[0 .. nq)
    if (u >= n_units || blockIdx.y * PASS_GROUPS * MUT_GROUP >= nq) return;  // the whole warp leaves
+   if (pass_width_u32((nq + 31) / 32, blockIdx.y) == 1) return;              // mut_ctr_narrow_kernel's
    const DevSeqCol* cs = &tab->seq[col];
    const uint32_t L = cs->L;
    const size_t per_query = static_cast<size_t>(cs->nsym) * L;
@@ -373,6 +377,174 @@ __global__ void __launch_bounds__(BT, 4) mut_ctr_batch_kernel(const DevTable* __
          }
       }
       if (k.rows) flush();
+   }
+}
+
+// Container pass of a pass of one mask word (blockIdx.y: its first or second 16 queries). A CTA stages the
+// 16-bit masks of a chunk's rows in shared memory and counts its share of the chunk's containers, 32 at a time
+// per warp: arrays of up to NARROW_LIGHT rows four at a time, eight lanes each; longer arrays and runs with
+// the whole warp; bitsets by population counts with the filters' own words. Two rows' masks make a word whose
+// bits are added to nibble counters (nibble k of nib[j]: query j + 4 (k % 4)); their bytes are summed over
+// the lanes. Bound by issue slots, then by the gathers (one of 32 banks each): a mask from L2 takes a sector,
+// and the wide pass, whose lanes then are all on different rows, took 350 us at 2M rows and 7 queries,
+// 137 us so; 107 and 46 us at 500,000 rows and 12 queries. A pass of two words stays with the wide pass: 400 us
+// at 2M rows against four times 130.
+constexpr uint32_t NARROW_T = 1024, NARROW_LIGHT = 240;  // 15 additions of 16 rows to a nibble
+constexpr uint32_t NARROW_SMEM = CHUNK_ROWS * 2;
+
+// the 16 queries' counts of a lane's nibbles: byte k of E[j] is query j + 8 (k & 1) + 4 (k >> 1)
+__device__ __forceinline__ void nibble_bytes(const uint32_t (&nib)[4], uint32_t (&E)[4]) {
+#pragma unroll
+   for (uint32_t j = 0; j < 4; ++j) {
+      const uint32_t a = nib[j] & 0x0F0F0F0Fu, b = (nib[j] >> 4) & 0x0F0F0F0Fu;
+      E[j] = __byte_perm(a + (a >> 16), b + (b >> 16), 0x5410);
+   }
+}
+// adds rows row_of(t) < CHUNK_ROWS for the t below n among t0 + stride * i, i < 2 U
+template <uint32_t U, typename RowOf>
+__device__ __forceinline__ void add_masks(uint32_t (&nib)[4], const uint16_t* masks, uint32_t t0, uint32_t stride, uint32_t n,
+                                          RowOf&& row_of) {
+   uint32_t row[2 * U];
+#pragma unroll
+   for (uint32_t i = 0; i < 2 * U; ++i) row[i] = t0 + stride * i < n ? row_of(t0 + stride * i) : 0xFFFFFFFFu;
+#pragma unroll
+   for (uint32_t i = 0; i < 2 * U; i += 2) {
+      const uint32_t m0 = row[i] < CHUNK_ROWS ? masks[row[i]] : 0u, m1 = row[i + 1] < CHUNK_ROWS ? masks[row[i + 1]] : 0u;
+      const uint32_t w = m0 | (m1 << 16);
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) nib[j] += (w >> j) & 0x11111111u;
+   }
+}
+
+__global__ void __launch_bounds__(NARROW_T, 1) mut_ctr_narrow_kernel(const DevTable* __restrict__ tab, uint32_t col,
+                                                                     const uint32_t* __restrict__ filters,
+                                                                     const uint16_t* __restrict__ R,
+                                                                     const uint32_t* __restrict__ lists, uint32_t nq_max,
+                                                                     uint32_t per_chunk, uint32_t* __restrict__ counts) {
+   extern __shared__ __align__(16) uint16_t masks[];
+   __shared__ uint32_t next;
+   const uint32_t nq = lists[2 * nq_max];  // dense slots: lists[0 .. nq)
+   const uint32_t nqc = (nq + 31) / 32, pass = (nqc + 7) / 8 - 1, q0 = 256 * pass + 16 * blockIdx.y;
+   if (nq == 0 || pass_width_u32(nqc, pass) != 1 || q0 >= nq) return;
+   const DevSeqCol* cs = &tab->seq[col];
+   const uint32_t L = cs->L, lane = threadIdx.x & 31;
+   const uint32_t v = blockIdx.x / per_chunk, part = blockIdx.x % per_chunk;
+   const size_t words = static_cast<size_t>(tab->nchunks) * CHUNK_WORDS, rows = 32 * words;
+   const size_t per_query = static_cast<size_t>(cs->nsym) * L;
+   {
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(R) + pass * rows * 8 +
+                                                        static_cast<size_t>(v) * CHUNK_ROWS);
+      const uint32_t half = blockIdx.y ? 0x7632u : 0x5410u;
+      uint2* dst = reinterpret_cast<uint2*>(masks);
+#pragma unroll 8
+      for (uint32_t i = threadIdx.x; i < CHUNK_ROWS / 4; i += NARROW_T) {
+         const uint4 x = __ldg(src + i);
+         dst[i] = make_uint2(__byte_perm(x.x, x.y, half), __byte_perm(x.z, x.w, half));
+      }
+   }
+   if (threadIdx.x == 0) next = 0;
+   const CtrDesc* __restrict__ ctrs = cs->ctrs;
+   const uint16_t* __restrict__ payload = cs->payload;
+   const uint32_t a = __ldg(cs->off + static_cast<size_t>(v) * L), n_all = __ldg(cs->off + static_cast<size_t>(v) * L + L) - a;
+   const uint32_t c0 = a + static_cast<uint32_t>(static_cast<uint64_t>(n_all) * part / per_chunk);
+   const uint32_t c1 = a + static_cast<uint32_t>(static_cast<uint64_t>(n_all) * (part + 1) / per_chunk);
+   // the count tables of the queries this lane adds to: two of a light array, one of the others
+   auto table_of = [&](uint32_t q) { return q0 + q < nq ? counts + lists[q0 + q] * per_query : nullptr; };
+   const uint32_t qa = ((lane >> 1) & 3u) + 4 * (lane & 1u);
+   const uint32_t qh = (lane >> 3) + 8 * ((lane >> 2) & 1u) + 4 * (lane & 1u);  // of the lanes with bit 1 clear
+   uint32_t* const ta = table_of(qa);
+   uint32_t* const tb = table_of(qa + 8);
+   uint32_t* const th = table_of(qh);
+   __syncthreads();
+   for (;;) {
+      uint32_t c = 0;
+      if (lane == 0) c = atomicAdd(&next, 32u);
+      c = c0 + __shfl_sync(0xFFFFFFFFu, c, 0);
+      if (c >= c1) break;
+      const bool have = c + lane < c1;
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (have) raw = __ldg(reinterpret_cast<const uint4*>(ctrs) + c + lane);
+      const CtrDesc mine = *reinterpret_cast<const CtrDesc*>(&raw);
+      const uint32_t card = have ? mine.card_m1 + 1u : 0u;
+      const bool light = have && mine.type == CT_ARRAY && card <= NARROW_LIGHT;
+      const uint32_t n_light = light ? card : 0u, cell = mine.sym * L + mine.key;  // below 2^32: nsym * L is
+#pragma unroll 1
+      for (uint32_t k = 0; k < 8; ++k) {
+         const uint32_t j = 4 * k + (lane >> 3);
+         const uint32_t n = __shfl_sync(0xFFFFFFFFu, n_light, j), at = __shfl_sync(0xFFFFFFFFu, cell, j);
+         const uint16_t* p = payload + __shfl_sync(0xFFFFFFFFu, mine.payload, j);
+         const uint32_t n_max = __reduce_max_sync(0xFFFFFFFFu, n);
+         if (n_max == 0) continue;
+         uint32_t nib[4] = {0, 0, 0, 0}, E[4];
+#pragma unroll 1
+         for (uint32_t t = 0; t < n_max; t += 64)
+            add_masks<4>(nib, masks, t + (lane & 7u), 8, n, [&](uint32_t i) { return static_cast<uint32_t>(__ldcs(p + i)); });
+         nibble_bytes(nib, E);
+         halve_words<2>(E, 4);
+         halve_words<1>(E, 2);
+         E[0] += __shfl_xor_sync(0xFFFFFFFFu, E[0], 1);
+         const uint32_t x = E[0] >> (lane & 1u ? 16 : 0);  // queries qa and qa + 8
+         if (ta && (x & 0xFFu)) atomicAdd(ta + at, x & 0xFFu);
+         if (tb && ((x >> 8) & 0xFFu)) atomicAdd(tb + at, (x >> 8) & 0xFFu);
+      }
+      uint32_t heavy = __ballot_sync(0xFFFFFFFFu, have && !light);
+      while (heavy) {
+         const uint32_t j = __ffs(heavy) - 1;
+         heavy &= heavy - 1;
+         const uint4 dr = make_uint4(__shfl_sync(0xFFFFFFFFu, raw.x, j), __shfl_sync(0xFFFFFFFFu, raw.y, j),
+                                     __shfl_sync(0xFFFFFFFFu, raw.z, j), __shfl_sync(0xFFFFFFFFu, raw.w, j));
+         const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&dr);
+         const uint16_t* p = payload + d.payload;
+         const uint32_t at = d.sym * L + d.key;
+         // counts rows row_of(t), t < n <= 61,440: the pairs' sums fit 16 bits
+         auto count_rows = [&](uint32_t n, auto&& row_of) {
+            uint32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+            for (uint32_t b = 0; b < n; b += 960) {  // 15 additions of 64 rows to a nibble
+               uint32_t nib[4] = {0, 0, 0, 0}, E[4];
+#pragma unroll 1
+               for (uint32_t t = b; t < min(b + 960, n); t += 320)
+                  add_masks<5>(nib, masks, t + lane, 32, n, row_of);
+               nibble_bytes(nib, E);
+#pragma unroll
+               for (uint32_t i = 0; i < 4; ++i) {
+                  acc[2 * i] += E[i] & 0x00FF00FFu;
+                  acc[2 * i + 1] += (E[i] >> 8) & 0x00FF00FFu;
+               }
+            }
+            halve_words<4>(acc, 16);
+            halve_words<2>(acc, 8);
+            halve_words<1>(acc, 4);
+            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], 2);
+            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1);
+            const uint32_t x = lane & 1u ? acc[0] >> 16 : acc[0] & 0xFFFFu;
+            if (!(lane & 2u) && th && x) atomicAdd(th + at, x);
+         };
+         if (d.type == CT_ARRAY) {
+            count_rows(d.card_m1 + 1u, [&](uint32_t i) { return static_cast<uint32_t>(__ldcs(p + i)); });
+         } else if (d.type == CT_RUN) {
+#pragma unroll 1
+            for (uint32_t i = 0; i < d.nruns; ++i) {
+               const uint32_t s0 = __ldg(p + 2 * i), n = __ldg(p + 2 * i + 1) + 1u;
+#pragma unroll 1
+               for (uint32_t b = 0; b < n; b += 32768) count_rows(min(n - b, 32768u), [&](uint32_t t) { return s0 + b + t; });
+            }
+         } else {
+            const uint4* bits = reinterpret_cast<const uint4*>(p);
+#pragma unroll 1
+            for (uint32_t q = 0; q < 16 && q0 + q < nq; ++q) {
+               const uint4* f = reinterpret_cast<const uint4*>(filters + lists[q0 + q] * words + static_cast<size_t>(v) * CHUNK_WORDS);
+               uint32_t k = 0;
+#pragma unroll 4
+               for (uint32_t i = lane; i < CHUNK_WORDS / 4; i += 32) {
+                  const uint4 x = __ldg(bits + i), y = __ldg(f + i);
+                  k += __popc(x.x & y.x) + __popc(x.y & y.y) + __popc(x.z & y.z) + __popc(x.w & y.w);
+               }
+               k = __reduce_add_sync(0xFFFFFFFFu, k);
+               if (lane == 0 && k) atomicAdd(counts + lists[q0 + q] * per_query + at, k);
+            }
+         }
+      }
    }
 }
 
@@ -590,6 +762,13 @@ static_assert(MUT_SEG / 32 == 32, "one lane per warp's total");
 
 }  // namespace
 
+void mutations_batch_setup() {
+   const cudaError_t e =
+      cudaFuncSetAttribute(mut_ctr_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(NARROW_SMEM));
+   if (e != cudaSuccess)
+      throw std::runtime_error(std::string("shared memory of the narrow container pass: ") + cudaGetErrorString(e));
+}
+
 size_t mutations_batch_mask_bytes(uint32_t nq, uint32_t nchunks) {
    const uint32_t nqc = (nq + 31) / 32;
    return static_cast<size_t>(nqc) * nchunks * CHUNK_ROWS * 4;
@@ -614,6 +793,9 @@ void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, 
    if ((parts & BMUT_PART_CTR) && n_units > 0) {
       const dim3 grid((n_units + BT / 32 - 1) / (BT / 32), (ngroups + PASS_GROUPS - 1) / PASS_GROUPS);
       mut_ctr_batch_kernel<<<grid, BT, 0, s>>>(d_table, col, d_units, n_units, d_masks, d_lists, nq, d_counts);
+      const uint32_t per_chunk = std::max(1u, 152u / nchunks);  // one CTA per SM
+      mut_ctr_narrow_kernel<<<dim3(nchunks * per_chunk, nq > 16 ? 2 : 1), NARROW_T, NARROW_SMEM, s>>>(
+         d_table, col, d_filters, d_masks, d_lists, nq, per_chunk, d_counts);
    }
    if ((parts & BMUT_PART_COV) && n_ev > 0)
       mut_cov_batch_kernel<<<dim3(n_ev, (ngroups + PASS_GROUPS - 1) / PASS_GROUPS), BT, 0, s>>>(d_table, col, d_ev, d_masks, d_lists, nq,

@@ -251,6 +251,7 @@ enum : int { DEVERR_WAIT_FILTER = 6, DEVERR_WAIT_MUTATIONS = 7 };
 // Sets the container pass's shared-memory size on the current device (once per device, before
 // its first launch).
 void mutations_setup();
+void mutations_batch_setup();
 
 // Kernel selection masks (all bits set = the whole pass); used to time the kernels one by one.
 enum : uint32_t { MUT_PART_CTR = 1, MUT_PART_COV = 2, MUT_PART_FINAL = 4, MUT_PART_ALL = 7 };

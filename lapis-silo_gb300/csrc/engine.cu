@@ -397,6 +397,7 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
    try {
       cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
       mutations_setup();
+      mutations_batch_setup();
       const uint32_t nchunks = t.nchunks();
       view_.nchunks = nchunks;
       view_.n_rows = t.n_rows;

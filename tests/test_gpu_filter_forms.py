@@ -217,3 +217,50 @@ def test_mutations_around_the_row_index_limit(differing):
         want, k = orc.mutations(q, 0)
         assert filtered == k == rows and np.array_equal(counts, want)
     dev.close()
+
+
+@pytest.fixture(scope="module")
+def container_forms():
+    """140,000 rows: arrays of 1 to 4,096 rows around the narrow pass's steps, bitsets, and runs up to a whole
+    chunk, a site each; and the oracle's Mutations by query."""
+    n = 140000
+    cards = [1, 15, 16, 17, 63, 64, 65, 239, 240, 241, 319, 320, 321, 959, 960, 961, 4095, 4096, 4097, 30000]
+    spans = [(0, 65536), (65536, 131072), (10, 40000), (65530, 65540), (70000, 70033), (131072, 140000)]
+    L = len(cards) + len(spans) + 1
+    rng = np.random.default_rng(21)
+    rows = np.full((n, L), ord("A"), np.uint8)
+    for i, k in enumerate(cards):
+        rows[rng.choice(65536, k, replace=False), i] = ord("C")
+        rows[65536 + rng.choice(65536, k, replace=False), i] = ord("G")
+    for i, (a, e) in enumerate(spans):
+        rows[a:e, len(cards) + i] = ord("T")
+    rows[rng.random(n) < 0.5, L - 1] = ord("C")
+    b = RawBuilder(n)
+    b.add_sequences("main", 0, "A" * L, [r.tobytes().decode() for r in rows])
+    raw = b.raw()
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    known = {}
+
+    def mutations(q):
+        if q not in known:
+            known[q] = orc.mutations(q, 0)
+        return known[q]
+
+    yield dev, mutations, L
+    dev.close()
+
+
+@pytest.mark.parametrize("slots", [1, 15, 16, 17, 32, 33, 257, 289])
+def test_narrow_container_pass(container_forms, slots):
+    """Passes of one mask word (up to 32 queries, alone and after 256 others) and of two."""
+    dev, mutations, L = container_forms
+    forms = ["True", f"HasMut(main,{L})", f"Not(HasMut(main,{L}))", "HasMut(main,20)", f"Not(HasMut(main,{L - 1}))",
+             "Not(HasMut(main,18))", "HasMut(main,21)", f"Or(HasMut(main,22),HasMut(main,{L}))"]
+    qs = [f"Or({a},{b})" for a in forms for b in forms]
+    qs = [qs[i * 11 % len(qs)] for i in range(slots)]
+    dev.sparse_rows(batch=0)  # every filter takes the container pass
+    counts, muts = dev.batch(qs, [1] * slots, [0] * slots)
+    for i, q in enumerate(qs):
+        want, n = mutations(q)
+        assert counts[i] == n and np.array_equal(muts[i], want), q
