@@ -28,11 +28,14 @@
 //                          position, 6 bytes) staged in shared memory, one CTA of 1,024 threads
 //                          per SM walking the row words;
 //   profile_kernel         longer genomes: 8-byte terms read through L1/L2.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "device.h"
 
 namespace rhygpu {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -175,65 +178,79 @@ __global__ void __launch_bounds__(ST, 1) profile_staged_kernel(const DevTable* _
       profile_word(tab, cs, pr, terms, w, lp, out + w);
 }
 
-// One CTA per 16,384 rows: their counts in shared memory, the positions shared out over the warps. The
-// rows of a position's containers and those not covered there get the profile's terms in place of the
-// local reference's. A warp looks up to 32 positions up at once, then their containers, numbered across
-// the warp, and reads the rows of four containers at a time. Bound: the home distances (4 bytes per
-// row) and latency, about ten dependent loads per 32 positions (a missing run of the profile is
-// hundreds of positions with a few containers each).
-constexpr uint32_t DT = 1024, DELTA_TILE = 16384, DELTA_BITSETS = 512;
+// A cluster of CTAs per chunk: each CTA takes a share of the positions and keeps what they add to every row
+// of the chunk in shared memory (16-bit halves of a word: at most PROFILE_DELTA_MAX positions of 2), and the
+// CTAs then add the shares of a part of the rows each, from one another's shared memory, to the stored
+// distances. The rows of a position's containers and those not covered there get the profile's terms in place
+// of the local reference's. A warp looks up to 32 positions up at once, then their containers, numbered across
+// the warp, and reads the rows of four containers at a time. Bound: latency, about ten dependent loads per 32
+// positions (a missing run of the profile is hundreds of positions with a few containers each), and the
+// home distances (4 bytes per row). 1,344 positions at 2M rows: 50 us; 72 with a CTA per 16,384 rows, which
+// read the rows of a chunk's containers for a quarter of them (of the 50: staging and the sums' exchange 14,
+// containers 14, bitsets 17, rows not covered 5; bitsets by whole warps alone made it 90).
+constexpr uint32_t DT = 1024, DELTA_BITSETS = 512, DELTA_SMEM = CHUNK_ROWS * 2;
+static_assert(2 * PROFILE_DELTA_MAX < 32768, "a row's sum fits 16 bits");
+// what two rows' sums in one word are: the lower half is signed, and its borrow is in the upper one
+__device__ __forceinline__ int32_t delta_half(uint32_t x, uint32_t upper) {
+   const int32_t lo = static_cast<int16_t>(x);
+   return upper ? static_cast<int16_t>((x - static_cast<uint32_t>(lo)) >> 16) : lo;
+}
 __global__ void __launch_bounds__(DT) profile_delta_kernel(const DevTable* __restrict__ tab,
                                                            const DevProfile* __restrict__ profiles,
                                                            uint32_t* __restrict__ aux) {
-   extern __shared__ __align__(16) int32_t cnt[];
-   __shared__ uint16_t listed[PROFILE_DELTA_MAX];  // positions whose uncovered rows count differently
+   extern __shared__ __align__(16) uint32_t cnt[];
+   __shared__ uint16_t runs[PROFILE_DELTA_MAX];    // first differences of this CTA's position blocks
+   __shared__ int16_t sums[DT / 32][NBLOCK + 4];   // per warp: the uncovered rows' terms of positions below q
    __shared__ uint2 bitsets[DELTA_BITSETS];        // bitset containers: payload, term
-   __shared__ uint32_t n_listed, n_bitsets;
+   __shared__ uint32_t n_runs, n_bitsets;
    const DevProfile pr = profiles[blockIdx.y];
    if (pr.terms != nullptr) return;  // counted from the row index
    const DevSeqCol* cs = &tab->seq[pr.col];
    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   constexpr uint32_t T = CHUNK_ROWS / DELTA_TILE;
-   const uint32_t v = blockIdx.x / T, row0 = blockIdx.x % T * DELTA_TILE;
-   const size_t g0 = static_cast<size_t>(v) * CHUNK_ROWS + row0;
-   const int4* home = reinterpret_cast<const int4*>(cs->home + g0);
-   const int32_t base = static_cast<int32_t>(pr.base);
-   for (uint32_t i = threadIdx.x; i < DELTA_TILE / 4; i += DT) {
-      const int4 h = __ldg(home + i);
-      reinterpret_cast<int4*>(cnt)[i] = make_int4(h.x + base, h.y + base, h.z + base, h.w + base);
-   }
-   if (threadIdx.x == 0) n_listed = n_bitsets = 0;
+   const cg::cluster_group cluster = cg::this_cluster();
+   const uint32_t parts = cluster.num_blocks(), part = cluster.block_rank(), v = blockIdx.x / parts;
+   const size_t g0 = static_cast<size_t>(v) * CHUNK_ROWS;
+   for (uint32_t i = threadIdx.x; i < CHUNK_ROWS / 8; i += DT) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
+   auto add = [&](uint32_t row, int32_t a) { atomicAdd(cnt + (row >> 1), static_cast<uint32_t>(a) << (16 * (row & 1u))); };
+   if (threadIdx.x == 0) n_runs = n_bitsets = 0;
    __syncthreads();
    const uint32_t missing = cs->nsym - 1;  // the missing symbol is the last one
    // what a row with symbol s at the position adds beyond d_ref
    auto term = [](uint32_t mask, uint32_t home, int32_t d_ref, uint32_t s) {
       return static_cast<int32_t>((mask >> s) & 1u) - static_cast<int32_t>((home >> s) & 1u) - d_ref;
    };
-   auto add_bitset = [&](uint32_t payload, int32_t a) {
-      const uint32_t* words = reinterpret_cast<const uint32_t*>(cs->payload + payload) + (row0 >> 5);
-      constexpr uint32_t U = 8;  // loads in flight
-      for (uint32_t w0 = lane; w0 < DELTA_TILE / 32; w0 += 32 * U) {
-         uint32_t y[U];
+   constexpr uint32_t PIECE = 256, PIECES = CHUNK_WORDS / PIECE;  // words of a bitset that a warp takes at a time
+   auto add_bitset = [&](uint32_t payload, uint32_t piece, int32_t a) {
+      const uint32_t* words = reinterpret_cast<const uint32_t*>(cs->payload + payload);
+      constexpr uint32_t U = PIECE / 32;  // loads in flight
+      const uint32_t w0 = PIECE * piece + lane;
+      uint32_t y[U];
 #pragma unroll
-         for (uint32_t u = 0; u < U; ++u) y[u] = __ldg(words + w0 + 32 * u);
+      for (uint32_t u = 0; u < U; ++u) y[u] = __ldg(words + w0 + 32 * u);
 #pragma unroll
-         for (uint32_t u = 0; u < U; ++u)
-            for (uint32_t z = y[u]; z; z &= z - 1) atomicAdd(cnt + 32 * (w0 + 32 * u) + (__ffs(z) - 1), a);
-      }
+      for (uint32_t u = 0; u < U; ++u)
+         for (uint32_t k = 0; k < 16; ++k) {  // two words at a time, a lane per pair of their rows
+            const uint32_t j = 2 * k + (lane >> 4), bits = (__shfl_sync(0xFFFFFFFFu, y[u], j) >> (2 * (lane & 15u))) & 3u;
+            if (bits) atomicAdd(cnt + 16 * (w0 - lane + 32 * u + j) + (lane & 15u), ((bits | (bits << 15)) & 0x10001u) * static_cast<uint32_t>(a));
+         }
    };
    // positions per warp and step: at most 32, the same for every warp and step
-   const uint32_t steps = (pr.n_delta + DT - 1) / DT, per = steps ? (pr.n_delta + steps * (DT / 32) - 1) / (steps * (DT / 32)) : 1u;
-   for (uint32_t i0 = warp * per; i0 < pr.n_delta; i0 += per * (DT / 32)) {
-      const uint32_t np = min(per, pr.n_delta - i0);
+   for (uint32_t i = threadIdx.x; i < pr.n_delta; i += DT) {
+      const uint32_t blk = __ldg(&pr.delta[i].x) / NBLOCK;
+      if (blk % parts == part && (i == 0 || __ldg(&pr.delta[i - 1].x) / NBLOCK != blk))
+         runs[atomicAdd(&n_runs, 1u)] = static_cast<uint16_t>(i);
+   }
+   const uint32_t nd = (pr.n_delta - part + parts - 1) / parts;  // this CTA's positions: part, part + parts, ...
+   const uint32_t steps = (nd + DT - 1) / DT, per = steps ? (nd + steps * (DT / 32) - 1) / (steps * (DT / 32)) : 1u;
+   for (uint32_t i0 = warp * per; i0 < nd; i0 += per * (DT / 32)) {
+      const uint32_t np = min(per, nd - i0);
       uint4 d = make_uint4(0, 0, 0, 0);  // lane l < np: position l and its containers
       uint32_t c0 = 0, nc = 0;
       if (lane < np) {
-         d = __ldg(pr.delta + i0 + lane);
+         d = __ldg(pr.delta + (i0 + lane) * parts + part);
          const size_t slot = static_cast<size_t>(v) * cs->L + d.x;
          c0 = __ldg(cs->off + slot);
          nc = __ldg(cs->off + slot + 1) - c0;
-         if (term(d.y, d.z, static_cast<int32_t>(d.w), missing) != 0)
-            listed[atomicAdd(&n_listed, 1u)] = static_cast<uint16_t>(i0 + lane);
       }
       uint32_t first = nc;  // containers before this position's, after the scan
 #pragma unroll
@@ -284,13 +301,13 @@ __global__ void __launch_bounds__(DT) profile_delta_kernel(const DevTable* __res
 #pragma unroll
                for (uint32_t h = 0; h < 2; ++h)
                   row[u][h] = small && lane + 32 * h <= x[u].card_m1
-                                 ? static_cast<uint32_t>(__ldg(cs->payload + x[u].payload + 32 * h + lane)) - row0
+                                 ? static_cast<uint32_t>(__ldg(cs->payload + x[u].payload + 32 * h + lane))
                                  : 0xFFFFFFFFu;
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
-               if (row[u][0] < DELTA_TILE) atomicAdd(cnt + row[u][0], ax[u]);
-               if (row[u][1] < DELTA_TILE) atomicAdd(cnt + row[u][1], ax[u]);
+               if (row[u][0] < CHUNK_ROWS) add(row[u][0], ax[u]);
+               if (row[u][1] < CHUNK_ROWS) add(row[u][1], ax[u]);
                if (ax[u] == 0 || (x[u].type == CT_ARRAY && x[u].card_m1 < 64)) continue;
                if (x[u].type == CT_ARRAY) {  // 8 rows per lane and load
                   const uint32_t lead = x[u].payload & 7u, end = lead + x[u].card_m1 + 1u;
@@ -300,17 +317,16 @@ __global__ void __launch_bounds__(DT) profile_delta_kernel(const DevTable* __res
                      const uint32_t w[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
                      for (uint32_t q = 0; q < 8; ++q) {
-                        const uint32_t e = ((w[q >> 1] >> (16 * (q & 1))) & 0xFFFFu) - row0;
-                        if (k + q >= lead && k + q < end && e < DELTA_TILE) atomicAdd(cnt + e, ax[u]);
+                        if (k + q >= lead && k + q < end) add((w[q >> 1] >> (16 * (q & 1))) & 0xFFFFu, ax[u]);
                      }
                   }
                } else if (x[u].type == CT_BITSET) {
-                  add_bitset(x[u].payload, ax[u]);
+                  for (uint32_t k = 0; k < PIECES; ++k) add_bitset(x[u].payload, k, ax[u]);
                } else {
                   const uint16_t* p = cs->payload + x[u].payload;
                   for (uint32_t k = lane; k < x[u].nruns; k += 32) {
                      const uint32_t s = __ldg(p + 2 * k), e = s + __ldg(p + 2 * k + 1) + 1u;
-                     for (uint32_t y = max(s, row0); y < min(e, row0 + DELTA_TILE); ++y) atomicAdd(cnt + (y - row0), ax[u]);
+                     for (uint32_t y = s; y < min(e, CHUNK_ROWS); ++y) add(y, ax[u]);
                   }
                }
             }
@@ -318,17 +334,48 @@ __global__ void __launch_bounds__(DT) profile_delta_kernel(const DevTable* __res
       }
    }
    __syncthreads();
-   for (uint32_t i = warp; i < min(n_bitsets, DELTA_BITSETS); i += DT / 32)
-      add_bitset(bitsets[i].x, static_cast<int32_t>(bitsets[i].y));
-   for (uint32_t i = warp; i < n_listed; i += DT / 32) {  // a warp per position again
-      const uint4 d = __ldg(pr.delta + listed[i]);
-      const uint32_t pos = d.x, q = pos % NBLOCK;
-      const int32_t a = term(d.y, d.z, static_cast<int32_t>(d.w), missing);
-      const size_t b = static_cast<size_t>(pos / NBLOCK) * tab->nchunks + v;
+   for (uint32_t i = warp; i < min(n_bitsets, DELTA_BITSETS) * PIECES; i += DT / 32)
+      add_bitset(bitsets[i / PIECES].x, i % PIECES, static_cast<int32_t>(bitsets[i / PIECES].y));
+   // The rows not covered, a warp per block of positions: the terms of the block's differences (sorted by
+   // position) are summed below each position, so that an interval, read once, adds the sum over its
+   // positions (a missing run of the profile is hundreds of differences in a few blocks).
+   for (uint32_t i = warp; i < n_runs; i += DT / 32) {
+      const uint32_t first = runs[i], blk = __ldg(&pr.delta[first].x) / NBLOCK;
+      int16_t* P = sums[warp];
+      for (uint32_t q = lane; q < NBLOCK; q += 32) P[q] = 0;
+      __syncwarp();
+      for (uint32_t k = first + lane;; k += 32) {
+         uint4 d = make_uint4(0, 0, 0, 0);
+         const bool in = k < pr.n_delta && (d = __ldg(pr.delta + k)).x / NBLOCK == blk;
+         if (in) P[d.x % NBLOCK] = static_cast<int16_t>(term(d.y, d.z, static_cast<int32_t>(d.w), missing));
+         if (!__all_sync(0xFFFFFFFFu, in)) break;
+      }
+      __syncwarp();
+      int32_t t[4], sum = 0;  // exclusive sums: lane l has the positions 4 l .. 4 l + 3
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+         t[j] = sum;
+         sum += P[4 * lane + j];
+      }
+      int32_t incl = sum;
+#pragma unroll
+      for (uint32_t o = 1; o < 32; o <<= 1) {
+         const int32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+         if (lane >= o) incl += y;
+      }
+      const int32_t all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+      __syncwarp();
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) P[4 * lane + j] = static_cast<int16_t>(incl - sum + t[j]);
+      if (lane == 0) P[NBLOCK] = static_cast<int16_t>(all);
+      const bool any = __any_sync(0xFFFFFFFFu, sum != 0 || t[1] != 0 || t[2] != 0 || t[3] != 0);
+      __syncwarp();
+      if (!any) continue;  // the missing symbol counts as the local reference does at all of them
+      const size_t b = static_cast<size_t>(blk) * tab->nchunks + v;
       const uint32_t* toff = cs->nblk_toff + b * TOFF_N;
-      const uint32_t m0 = __ldg(toff + row0 / TOFF_ROWS), m1 = __ldg(toff + (row0 + DELTA_TILE) / TOFF_ROWS);
+      const uint32_t m0 = __ldg(toff), m1 = __ldg(toff + TOFF_N - 1);
       const uint4 g = __ldg(cs->cov_rng + b);
-      constexpr uint32_t U = 4;  // loads in flight; four intervals each, rows outside the tile drop out
+      constexpr uint32_t U = 4;  // loads in flight; four intervals each (0: none)
       for (uint32_t k0 = m0 / 4 + lane; k0 < (m1 + 3) / 4; k0 += 32 * U) {
          uint4 x[U];
 #pragma unroll
@@ -339,28 +386,49 @@ __global__ void __launch_bounds__(DT) profile_delta_kernel(const DevTable* __res
             const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) {
-               const uint32_t r = (w[j] & 0xFFFFu) - row0;
-               if (r < DELTA_TILE && ((w[j] >> 16) & 0xFFu) <= q && q < (w[j] >> 24)) atomicAdd(cnt + r, a);
+               const int32_t a = P[min(w[j] >> 24, NBLOCK)] - P[min((w[j] >> 16) & 0xFFu, NBLOCK)];
+               if (a != 0) add(w[j] & 0xFFFFu, a);
             }
          }
       }
-      for (uint32_t k = lane; k < g.y + g.w; k += 32) {
+      const uint32_t p0 = blk * NBLOCK;
+      for (uint32_t k = lane; k < g.y + g.w; k += 32) {  // positions before a late start, or from an early end on
          const bool late = k < g.y;
          const CovBound e = late ? cs->cov_late[g.x + k] : cs->cov_early[g.z + (k - g.y)];
-         const uint32_t r = e.row - row0;
-         if (r < DELTA_TILE && (e.bound > pos) == late) atomicAdd(cnt + r, a);
+         const int32_t below = P[e.bound <= p0 ? 0u : min(e.bound - p0, NBLOCK)], a = late ? below : all - below;
+         if (a != 0) add(e.row, a);
       }
+      __syncwarp();  // P is read until here
    }
-   __syncthreads();
+   cluster.sync();
    const uint32_t csize = __ldg(tab->chunk_sizes + v);
    const int32_t limit = static_cast<int32_t>(min(pr.distance, 0x7FFFFFFFu));
    uint32_t* out = aux + static_cast<size_t>(blockIdx.y) * tab->nchunks * CHUNK_WORDS + g0 / 32;
-   for (uint32_t w = warp; w < DELTA_TILE / 32; w += DT / 32) {
-      const uint32_t r = 32 * w + lane;
-      const bool null_row = (__ldg(cs->null_tiles + g0 / 32 + w) >> lane) & 1u;
-      const uint32_t bits = __ballot_sync(0xFFFFFFFFu, row0 + r < csize && (null_row || cnt[r] <= limit));
-      if (lane == 0) out[w] = bits;
+   // four rows a lane, four words a warp and step
+   const uint32_t r1 = CHUNK_ROWS / parts * (part + 1), base = pr.base;
+#pragma unroll 2
+   for (uint32_t r = CHUNK_ROWS / parts * part + 4 * threadIdx.x; r < r1; r += 4 * DT) {
+      const uint32_t null4 = __ldg(cs->null_tiles + (g0 + r) / 32) >> (r & 31u);
+      const int4 h = __ldg(reinterpret_cast<const int4*>(cs->home + g0 + r));
+      int32_t n[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll 4
+      for (uint32_t k = 0; k < parts; ++k) {
+         const uint2 x = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(cnt, k) + r / 2);
+         n[0] += delta_half(x.x, 0);
+         n[1] += delta_half(x.x, 1);
+         n[2] += delta_half(x.y, 0);
+         n[3] += delta_half(x.y, 1);
+      }
+      uint32_t bits = 0;
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j)
+         if (r + j < csize && (((null4 >> j) & 1u) || n[j] + static_cast<int32_t>(base) <= limit)) bits |= 1u << j;
+      bits <<= r & 31u;
+#pragma unroll
+      for (uint32_t o = 1; o < 8; o <<= 1) bits |= __shfl_xor_sync(0xFFFFFFFFu, bits, o);
+      if ((lane & 7u) == 0) out[r / 32] = bits;
    }
+   cluster.sync();  // the others read this CTA's sums until then
 }
 
 __global__ void __launch_bounds__(PT) profile_home_kernel(const DevTable* __restrict__ tab, uint32_t col, uint32_t rows,
@@ -389,10 +457,24 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
    const uint32_t words = nchunks * CHUNK_WORDS;
    const cudaStream_t s = static_cast<cudaStream_t>(stream);
    if (any_delta) {
-      cudaFuncSetAttribute(profile_delta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DELTA_TILE * 4);
-      for (uint32_t k = 0; k < n; k += 65535)  // grid.y is at most 65535
-         profile_delta_kernel<<<dim3(nchunks * (CHUNK_ROWS / DELTA_TILE), n - k < 65535 ? n - k : 65535), DT, DELTA_TILE * 4, s>>>(
-            d_table, d_profiles + k, d_aux + static_cast<size_t>(k) * words);
+      cudaFuncSetAttribute(profile_delta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DELTA_SMEM);
+      for (uint32_t k = 0; k < n; k += 65535) {  // grid.y is at most 65535
+         const uint32_t m = n - k < 65535 ? n - k : 65535;
+         // CTAs per chunk: eight (the most that every device takes) while they find an SM each, else four
+         const uint32_t parts = static_cast<uint64_t>(nchunks) * m * 8 <= 152 ? 8 : 4;
+         cudaLaunchAttribute attr{};
+         attr.id = cudaLaunchAttributeClusterDimension;
+         attr.val.clusterDim.x = parts;
+         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+         cudaLaunchConfig_t cfg{};
+         cfg.gridDim = dim3(nchunks * parts, m);
+         cfg.blockDim = DT;
+         cfg.dynamicSmemBytes = DELTA_SMEM;
+         cfg.stream = s;
+         cfg.attrs = &attr;
+         cfg.numAttrs = 1;
+         cudaLaunchKernelEx(&cfg, profile_delta_kernel, d_table, d_profiles + k, d_aux + static_cast<size_t>(k) * words);
+      }
    }
    if (max_L == 0) return;
    const size_t smem = (ST / 32) * PW * 4 + static_cast<size_t>(max_L) * 4 + (static_cast<size_t>(max_L) + 1) * 2;

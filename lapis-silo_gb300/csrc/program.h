@@ -79,8 +79,8 @@ enum RowOp : int { A_OR = 0, A_ANDNOT = 1, A_ADD = 2 };
 constexpr uint16_t GROUP_PUSH = 4;
 
 // A MutationProfile that differs from the local reference at up to this many positions is counted from
-// the differences (profile_delta_kernel), any other from the whole row index (see profile.cu): 72 us for
-// 1,344 positions at 2M rows and about 50 us per further thousand, against 133 us for the row index.
+// the differences (profile_delta_kernel), any other from the whole row index (see profile.cu): 50 us for
+// 1,344 positions at 2M rows, against 133 us for the row index; a row's sum in the kernel has 16 bits.
 constexpr uint32_t PROFILE_DELTA_MAX = 2048;
 
 constexpr uint32_t MAX_PROGRAM = 4096;   // instructions per program
