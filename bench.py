@@ -506,8 +506,8 @@ def main():
     total_s = max_over_ranks(sum(step_ms) / 1000.0, ws)
     value = n * args.steps * ws / total_s
     # one persistent filter launch for all classes of programs, then per column with Mutations
-    # queries: the slot split, transpose, container, coverage, row-index (when on) and final kernels
-    per_col = 5 + (1 if dev.sparse_rows()[1] > 0 else 0)
+    # queries: the slot split, transpose, wide and narrow container, coverage, row-index (when on) and final kernels
+    per_col = 6 + (1 if dev.sparse_rows()[1] > 0 else 0)
     launches_per_step = info.n_filter_launches + per_col * len({int(c) for c, a in zip(columns, actions) if a == 1})
 
     # results of the batched path for the parity self-check against the plain path

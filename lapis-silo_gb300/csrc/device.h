@@ -6,7 +6,7 @@
 //   offset table, per-chunk coverage exceptions, missing-interval buckets per 128-position block,
 //   a dense null-row bitmap (8 KiB per chunk) and the local reference;
 //   dictionary column: the inverted index in the same container format, keyed by value id;
-//   date column: bit-sliced index (one dense bitmap per bit of date - min date) and a null bitmap.
+//   date column: range-encoded index (dense bitmaps per digit value of date - min date) and a null bitmap.
 // Row sets are dense bitmaps of 2^16 bits (8 KiB) per chunk.
 #pragma once
 

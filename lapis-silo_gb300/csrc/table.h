@@ -16,7 +16,8 @@
 // The coverage layout is redesigned for the GPU: rows whose covered region is not the whole genome
 // are kept as a short per-chunk exception list, and the missing positions inside coverage are kept
 // as intervals bucketed by 128-position blocks, so a coverage tile at one position reads only the
-// exceptions and the intervals of one block instead of every row.
+// exceptions that concern its block (ordered by bound at upload) and the intervals of one block instead
+// of every row.
 #pragma once
 
 #include <cstdint>
