@@ -264,3 +264,46 @@ def test_narrow_container_pass(container_forms, slots):
     for i, q in enumerate(qs):
         want, n = mutations(q)
         assert counts[i] == n and np.array_equal(muts[i], want), q
+
+
+@pytest.mark.parametrize("density", [0.0005, 0.3])
+def test_resident_pass_under_capture(density):
+    """The chain of dependent launches recorded into a CUDA graph, and replayed on another filter: the row index
+    (few rows) and the dense passes."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+    t = R.Table.generate(100000, seed=17, genome_len=3000, pool_sites=500, null_fraction=0.01)
+    dev = R.Device(t, 0)
+    col = t.columns[0]
+    rng = np.random.default_rng(3)
+    rows = [np.concatenate([rng.random(t.n_rows) < density, np.zeros(t.n_chunks * R.CHUNK_ROWS - t.n_rows, bool)])
+            for _ in range(2)]
+    bits = [torch.from_numpy(np.packbits(r, bitorder="little").view(np.int32).copy()).cuda() for r in rows]
+    f, n = torch.zeros_like(bits[0]), torch.zeros(1, dtype=torch.int64, device="cuda")
+    counts = torch.empty(col.n_symbols, col.L, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(stream):
+        dev.mutations_noalloc(0, f.data_ptr(), n.data_ptr(), counts.data_ptr(), status.data_ptr(),
+                              ctypes.c_void_p(stream.cuda_stream))
+
+    def load(i):
+        f.copy_(bits[i])
+        n.fill_(int(rows[i].sum()))
+        torch.cuda.synchronize()  # the call below may run on the handle's own stream
+
+    want = []
+    for i in (0, 1):
+        load(i)
+        run(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        want.append(counts.clone())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(torch.cuda.current_stream())
+    for i in (1, 0, 0, 1):
+        load(i)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(status) == 0 and torch.equal(counts, want[i])
+    dev.close()
