@@ -11,8 +11,9 @@
 // What bounds them: issue slots and latency, not bytes (a container holds 36 rows on average, a tile is
 // 8 KiB). Hence a leaf followed by the operator that consumes it is one instruction (fuse_leaves),
 // whose rows go straight into the top tile or the counter planes; leaves whose order does not
-// matter are applied together, a warp each (group_leaves); arrays of DENSE_MIN rows and more are
-// stored a second time as bitsets, combined word by word by the threads that own the words.
+// matter are applied together, a warp each (group_leaves); arrays and run containers of DENSE_MIN rows and
+// more are stored a second time as bitsets (or read as the few runs they are), combined word by word by
+// the threads that own the words.
 // Measured (2M rows, 4,096 trees of 1-64 leaves, one launch): 34.5 ms with a tile per leaf, 20.9 ms
 // this way; the benchmark's 2,048 queries 3.28 -> 3.05 ms. 128 threads per CTA instead of 256: 25.6
 // and 2.9 ms (the trees wait on latency, and more warps hide it).
@@ -66,19 +67,23 @@ constexpr uint32_t LC_PAY = 3072;      // u16 of array payloads copied into shar
 constexpr uint32_t LC_BIG = 0x80000000u;
 constexpr uint32_t LC_OWNER_MAX = 64;  // leaves of at most this many copied rows are set by their words' owners
 
-// A container of a staged leaf: y = kind << 28 | rows (runs for E_RUN), x = where its payload is.
-enum : uint32_t { E_COPIED = 0, E_ARRAY = 1, E_BITSET = 2, E_RUN = 3 };  // E_COPIED: x = byte offset in shared memory, else u16 offset in the arena
+// A container of a staged leaf: y = kind << 28 | rows (runs for E_RUN), x = where its payload is. Bitsets and the
+// containers of few long runs (E_SPANS) have no rows to go through one by one.
+// E_COPIED: x = byte offset in shared memory, else u16 offset in the arena. E_SPANS: runs << 24 in place of rows; x = the
+// run (first row | rows - 1 << 16) of a container of one.
+enum : uint32_t { E_COPIED = 0, E_ARRAY = 1, E_BITSET = 2, E_RUN = 3, E_SPANS = 4 };
+constexpr uint32_t E_COUNT = 0x00FFFFFFu;
 
 struct LeafCache {
    uint4 code[LC_CODE];
    uint4 pay4[LC_PAY / 8];        // array payloads (TMA bulk copies, 16-byte aligned runs)
    uint4 cov[LC_COV];             // a coverage leaf's late and early rows
    uint2 covm[LC_COV];            // and its missing intervals
-   uint2 ent[LC_ENTS];            // leaf k's entries: arrays and runs from beg[k] up, bitsets from beg[k] + n[k] down
+   uint2 ent[LC_ENTS];            // leaf k's entries: arrays and runs from beg[k] up, bitsets and spans from beg[k] + n[k] down
    const uint4* src[LC_LEAVES];   // the leaf's descriptors
    const uint16_t* pay[LC_LEAVES];
    uint32_t symmask[LC_LEAVES];   // symbols the leaf ORs (every container for dictionary leaves)
-   uint32_t cnt[LC_LEAVES];       // its array and run entries, bitset entries << 16
+   uint32_t cnt[LC_LEAVES];       // its array and run entries, bitset and span entries << 16
    uint32_t tot[LC_LEAVES];       // rows of the leaf's copied arrays; LC_BIG: it has other arrays or runs
    uint16_t n[LC_LEAVES];         // descriptors of the leaf's slot
    uint16_t beg[LC_LEAVES];       // LC_NONE: not staged (the leaf reads its descriptors from global memory)
@@ -249,8 +254,9 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
       const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
       if (!((lc.symmask[k] >> d.sym) & 1u)) continue;  // a symbol the leaf does not OR
       const uint32_t card = d.card_m1 + 1u;
+      const bool spans = d.type == CT_RUN && card >= DENSE_MIN && d.nruns <= SPAN_RUNS;
       uint32_t at_ent;
-      if (d.type == CT_BITSET) at_ent = lc.beg[k] + lc.n[k] - 1 - (atomicAdd(&lc.cnt[k], 0x10000u) >> 16);
+      if (d.type == CT_BITSET || spans) at_ent = lc.beg[k] + lc.n[k] - 1 - (atomicAdd(&lc.cnt[k], 0x10000u) >> 16);
       else at_ent = lc.beg[k] + (atomicAdd(&lc.cnt[k], 1u) & 0xFFFFu);
       // the arena ends with 16 spare bytes, so rounding the end up stays inside it
       const uint16_t* p = lc.pay[k] + d.payload;
@@ -284,6 +290,10 @@ __device__ bool stage_leaves(LeafCache& lc, const TileCtx& c, const Instr* __res
       } else if (d.type == CT_BITSET) {
          lc.ent[at_ent] = make_uint2(d.payload, static_cast<uint32_t>(E_BITSET) << 28);
          prefetch_l2(p + (c.row0 >> 4), p + ((c.row0 + c.W) >> 4));
+      } else if (spans) {
+         const uint32_t x = d.nruns == 1 ? __ldg(p) | static_cast<uint32_t>(__ldg(p + 1)) << 16 : d.payload;
+         lc.ent[at_ent] = make_uint2(x, (E_SPANS << 28) | static_cast<uint32_t>(d.nruns) << 24);
+         if (d.nruns > 1) prefetch_l2(p, p + 2u * d.nruns);
       } else {
          lc.ent[at_ent] = make_uint2(d.payload, (E_RUN << 28) | d.nruns);
          atomicOr(&lc.tot[k], LC_BIG);
@@ -335,15 +345,13 @@ __device__ __forceinline__ bool ne4(uint4 a, uint4 b) {
 // container on average), so this takes a fraction of the instructions of building the leaf's tile
 // and combining it word by word.
 
-// Rows r0 and, with `two`, r1 of the tile at T (A_ADD: of the P counter planes at T, WW words apart), their
-// atomics in flight together. Additions commute, also when threads add to one row at a time: each
-// plane's exchange returns the old bit as the carry, so a plane receives half as many carries as the
-// one below it received bits, in any order; the top plane only ever gets set.
-__device__ __forceinline__ void apply_rows(uint32_t* T, uint32_t WW, uint32_t P, uint32_t A, uint32_t r0, bool one,
-                                           uint32_t r1, bool two) {
-   uint32_t b0 = one ? 1u << (r0 & 31) : 0u, b1 = two ? 1u << (r1 & 31) : 0u;
-   uint32_t* q0 = T + (r0 >> 5);
-   uint32_t* q1 = T + (r1 >> 5);
+// The rows of the masks b0 at word q0 and b1 at word q1 of a tile (A_ADD: of the P counter planes there,
+// WW words apart), their atomics in flight together; an empty mask touches nothing. Additions commute, also when
+// threads add to one row at a time: each plane's exchange returns the old bits as the carries, so a plane
+// receives half as many carries at a row as the one below it received bits, in any order; the top plane
+// only ever gets set.
+__device__ __forceinline__ void apply_masks(uint32_t* q0, uint32_t b0, uint32_t* q1, uint32_t b1, uint32_t WW, uint32_t P,
+                                            uint32_t A) {
    if (A == A_ADD) {
 #pragma unroll 1
       for (uint32_t i = 0; i + 1 < P && (b0 | b1); ++i, q0 += WW, q1 += WW) {
@@ -361,6 +369,11 @@ __device__ __forceinline__ void apply_rows(uint32_t* T, uint32_t WW, uint32_t P,
       if (b0) atomicOr(q0, b0);
       if (b1) atomicOr(q1, b1);
    }
+}
+// Rows r0 (with `one`) and r1 (with `two`) of the tile at T.
+__device__ __forceinline__ void apply_rows(uint32_t* T, uint32_t WW, uint32_t P, uint32_t A, uint32_t r0, bool one,
+                                           uint32_t r1, bool two) {
+   apply_masks(T + (r0 >> 5), one ? 1u << (r0 & 31) : 0u, T + (r1 >> 5), two ? 1u << (r1 & 31) : 0u, WW, P, A);
 }
 __device__ __forceinline__ void apply_row(uint32_t* T, uint32_t WW, uint32_t P, uint32_t A, uint32_t r) {
    apply_rows(T, WW, P, A, r, true, 0, false);
@@ -404,15 +417,80 @@ __device__ __forceinline__ void apply_array(uint32_t* T, uint32_t P, uint32_t A,
       }
    }
 }
+// Runs that are not in one of the other forms (fewer than DENSE_MIN rows, or a leaf that was not staged). Whole
+// warps (thread t of nt): 32 runs at a time, each lane the first and the last word of its own run and, where they
+// are few, the words between them; the words inside a longer run go to the whole warp. Applied row by row by one
+// thread a run, a count over a column that the rows are sorted by (runs of up to a whole chunk) took 780 us
+// at 400,000 rows, and 18 us so; NOf of 30 such sites 27.4 ms, and 0.11.
+constexpr uint32_t RUN_OWN = 4;  // words inside a run that its own lane takes
 __device__ __forceinline__ void apply_runs(uint32_t* T, uint32_t P, uint32_t A, const TileCtx& c,
                                            const uint16_t* __restrict__ p, uint32_t n, uint32_t t, uint32_t nt) {
+   const uint32_t lane = t & 31, WW = c.W >> 5;
+   constexpr uint32_t NO_RUN = 0xFFFFFFFFu;  // first row | rows - 1 << 16
+   auto load = [&](uint32_t i) { return i < n ? __ldg(p + 2 * i) | static_cast<uint32_t>(__ldg(p + 2 * i + 1)) << 16 : NO_RUN; };
+   uint32_t next = load(t);
 #pragma unroll 1
-   for (uint32_t i = t; i < n; i += nt) {
-      const uint32_t s = __ldg(p + 2 * i);
-      const uint32_t e = s + __ldg(p + 2 * i + 1) + 1u;  // run covers [s, e)
-      const uint32_t a = max(s, c.row0), b = min(e, c.row0 + c.W);
+   for (uint32_t i = t; i - lane < n; i += nt) {
+      const uint32_t run = next;
+      next = load(i + nt);
+      uint32_t a = 0, b = 0;  // this lane's run in the tile: [a, b)
+      if (run != NO_RUN) {
+         const uint32_t s = run & 0xFFFFu, e = s + (run >> 16) + 1u;
+         a = max(s, c.row0) - c.row0;
+         b = max(min(e, c.row0 + c.W), c.row0) - c.row0;
+      }
+      uint32_t w = 0, last = 0;
+      if (a < b) {
+         w = a >> 5;
+         last = (b - 1) >> 5;
+         const uint32_t head = 0xFFFFFFFFu << (a & 31), tail = 0xFFFFFFFFu >> (31 - ((b - 1) & 31));
+         apply_masks(T + w, w == last ? head & tail : head, T + last, w == last ? 0u : tail, WW, P, A);
+      }
+      const bool wide = last - w > RUN_OWN + 1;
+      uint32_t todo = __ballot_sync(0xFFFFFFFFu, wide);
+      if (!wide)
 #pragma unroll 1
-      for (uint32_t r = a; r < b; ++r) apply_row(T, c.W >> 5, P, A, r - c.row0);
+         for (++w; w < last; w += 2) apply_masks(T + w, 0xFFFFFFFFu, T + w + 1, w + 1 < last ? 0xFFFFFFFFu : 0u, WW, P, A);
+      __syncwarp();
+#pragma unroll 1
+      for (; todo; todo &= todo - 1) {
+         const uint32_t l = __ffs(todo) - 1, e = __shfl_sync(0xFFFFFFFFu, last, l);
+#pragma unroll 1
+         for (uint32_t x = __shfl_sync(0xFFFFFFFFu, w, l) + 1 + lane; x < e; x += 64)
+            apply_masks(T + x, 0xFFFFFFFFu, T + x + 32, x + 32 < e ? 0xFFFFFFFFu : 0u, WW, P, A);
+      }
+   }
+}
+
+// Bits below n (0 .. 32) of a word.
+__device__ __forceinline__ uint32_t low_bits(int32_t n) { return ~__funnelshift_lc(0u, 0xFFFFFFFFu, static_cast<uint32_t>(min(max(n, 0), 32))); }
+
+// The n <= SPAN_RUNS runs of a container (x: the run itself if it is one, else where they are in the arena) meet
+// the target as a bitset's words do, each combined by the thread that owns it: no atomics, no barrier. A warp
+// passes over the runs that miss its 4,096 rows.
+__device__ __forceinline__ void put_spans(uint4* T4, uint32_t P, uint32_t f, const TileCtx& c,
+                                          const uint16_t* __restrict__ payload, uint32_t x, uint32_t n) {
+   const uint32_t lane = threadIdx.x & 31, W4 = c.W >> 7;
+   uint32_t mine = x;  // lane j: run j
+   if (n > 1 && lane < n) {
+      const uint16_t* p = payload + x + 2 * lane;
+      mine = __ldg(p) | static_cast<uint32_t>(__ldg(p + 1)) << 16;
+   }
+#pragma unroll 1
+   for (uint32_t b4 = threadIdx.x - lane; b4 < W4; b4 += blockDim.x) {  // the warp's 32 words
+      const int32_t r0 = static_cast<int32_t>(c.row0 + 128 * b4), r = r0 + 128 * static_cast<int32_t>(lane);
+      uint4 v = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+      for (uint32_t j = 0; j < n; ++j) {
+         const uint32_t run = __shfl_sync(0xFFFFFFFFu, mine, j);
+         const int32_t s = static_cast<int32_t>(run & 0xFFFFu), e = s + static_cast<int32_t>(run >> 16) + 1;
+         if (e <= r0 || s >= r0 + 4096) continue;  // the same in every lane
+         v.x |= low_bits(e - r) & ~low_bits(s - r);
+         v.y |= low_bits(e - r - 32) & ~low_bits(s - r - 32);
+         v.z |= low_bits(e - r - 64) & ~low_bits(s - r - 64);
+         v.w |= low_bits(e - r - 96) & ~low_bits(s - r - 96);
+      }
+      if (b4 + lane < W4 && any4(v)) put_word(T4, W4, P, f, b4 + lane, v);
    }
 }
 
@@ -521,8 +599,13 @@ __device__ __forceinline__ void apply_leaves(uint32_t* T, uint32_t P, uint32_t A
                   nb = lc.cnt[l] >> 16;
                   continue;
                }
-               const uint4* p = reinterpret_cast<const uint4*>(lc.pay[l] + lc.ent[lc.beg[l] + lc.n[l] - nb].x) + (c.row0 >> 7);
+               const uint2 en = lc.ent[lc.beg[l] + lc.n[l] - nb];
                --nb;
+               if (en.y >> 28 == E_SPANS) {
+                  put_spans(reinterpret_cast<uint4*>(T), P, f, c, lc.pay[l], en.x, (en.y >> 24) & 15u);
+                  continue;
+               }
+               const uint4* p = reinterpret_cast<const uint4*>(lc.pay[l] + en.x) + (c.row0 >> 7);
                if (have == 0) p0 = p;
                else if (have == 1) p1 = p;
                else p2 = p;
@@ -561,7 +644,7 @@ __device__ __forceinline__ void apply_leaves(uint32_t* T, uint32_t P, uint32_t A
 #pragma unroll 1
          for (uint32_t i0 = lc.beg[k0]; i0 < e; i0 += 32) {
             const uint2 mine = i0 + lane < e ? lc.ent[i0 + lane] : make_uint2(0, 0);
-            uint32_t todo = __ballot_sync(0xFFFFFFFFu, (mine.y & 0x0FFFFFFFu) != 0u);  // bitsets have no count
+            uint32_t todo = __ballot_sync(0xFFFFFFFFu, (mine.y & E_COUNT) != 0u);  // bitsets and spans have no count
 #pragma unroll 1
             for (; todo; todo &= todo - 1) {
                if (turn) {
@@ -571,7 +654,7 @@ __device__ __forceinline__ void apply_leaves(uint32_t* T, uint32_t P, uint32_t A
                turn = lone ? 0u : (blockDim.x >> 5) - 1u;
                const uint32_t l = __ffs(todo) - 1;
                const uint32_t x = __shfl_sync(0xFFFFFFFFu, mine.x, l), y = __shfl_sync(0xFFFFFFFFu, mine.y, l);
-               const uint32_t kind = y >> 28, n = y & 0x0FFFFFFFu;
+               const uint32_t kind = y >> 28, n = y & E_COUNT;
                if (kind == E_COPIED) {
                   const uint16_t* sp = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(&lc) + x);
 #pragma unroll 1
@@ -1057,7 +1140,8 @@ __global__ void __launch_bounds__(256) date_index_kernel(const int32_t* __restri
    if (lane == 0) nulls[w] = b;
 }
 
-// Dense forms of the filter path: one CTA per array of at least DENSE_MIN rows writes its bitset.
+// Dense forms of the filter path: one CTA per array of at least DENSE_MIN rows, or run container of as many in
+// more than SPAN_RUNS runs, writes its bitset.
 __global__ void __launch_bounds__(256) dense_forms_kernel(uint16_t* arena, const DenseJob* __restrict__ jobs) {
    __shared__ uint4 tile[CHUNK_WORDS / 4];
    const DenseJob j = jobs[blockIdx.x];
@@ -1066,9 +1150,14 @@ __global__ void __launch_bounds__(256) dense_forms_kernel(uint16_t* arena, const
    __syncthreads();
    uint32_t* t = reinterpret_cast<uint32_t*>(tile);
 #pragma unroll 1
-   for (uint32_t i = threadIdx.x; i < j.card; i += blockDim.x) {
+   for (uint32_t i = threadIdx.x; i < j.rows; i += blockDim.x) {
       const uint32_t r = arena[j.src + i];
       atomicOr(&t[r >> 5], 1u << (r & 31));
+   }
+   for (uint32_t i = threadIdx.x; i < j.runs; i += blockDim.x) {
+      const uint32_t s = arena[j.src + 2 * i], e = s + arena[j.src + 2 * i + 1];  // [s, e]
+      for (uint32_t w = s >> 5; w <= e >> 5; ++w)
+         atomicOr(&t[w], (w == s >> 5 ? 0xFFFFFFFFu << (s & 31) : 0xFFFFFFFFu) & (w == e >> 5 ? 0xFFFFFFFFu >> (31 - (e & 31)) : 0xFFFFFFFFu));
    }
    __syncthreads();
    uint4* dst = reinterpret_cast<uint4*>(arena + j.dst);

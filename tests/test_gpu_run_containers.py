@@ -1,0 +1,116 @@
+"""Run containers, as the columns hold that a table is sorted by: row sets, counts, profiles, grouped counts and
+batched Mutations against the oracle (equal bit for bit), over runs of one row to a whole chunk at every tile
+width, and their cost beside the same work over bitsets of as many rows."""
+import time
+
+import numpy as np
+import pytest
+
+import rhydb_gpu as R
+from rawtable import RawBuilder, oracle_for
+
+pytestmark = pytest.mark.gpu
+
+N = 140000
+# (first row, rows, gap to the next run, runs): one run around the dense limit of 1,024 rows, whole chunks and runs
+# over a chunk's end, few runs on both sides of eight, many runs below and above 1,024 rows
+RUNS = [(5, 1, 0, 1), (100, 1023, 0, 1), (100, 1024, 0, 1), (4095, 1026, 0, 1), (0, 65536, 0, 1), (65536, 65536, 0, 1),
+        (10, N - 20, 0, 1), (65500, 80, 0, 1), (131072, N - 131072, 0, 1), (3, 4000, 100, 8), (3, 4000, 100, 9),
+        (7, 700, 1300, 40), (64, 32, 32, 31), (64, 32, 32, 33), (1, 3, 5, 300), (2, 17, 30, 2500), (31, 34, 4000, 17),
+        (2000, 130, 2, 7), (0, 200, 16, 5), (70000, 5, 3, 120)]
+DENSE = 24  # bitset sites, then as many sites of whole-chunk and half-chunk runs
+RUN0, WIDE0 = len(RUNS), len(RUNS) + DENSE
+L = len(RUNS) + 2 * DENSE + 1
+
+
+def site(p):
+    return f"HasMut(main,{p + 1})"
+
+
+@pytest.fixture(scope="module")
+def sorted_table():
+    rng = np.random.default_rng(2)
+    rows = np.full((N, L), ord("A"), np.uint8)
+    r = np.arange(N)
+    for i, (a, n, gap, k) in enumerate(RUNS):
+        rows[(r >= a) & ((r - a) % (n + gap if gap else N) < n) & (r - a < k * (n + gap if gap else N)), i] = ord("C")
+    for i in range(DENSE):
+        rows[rng.random(N) < 0.45, RUN0 + i] = ord("G")
+        a = int(rng.integers(0, 20000))
+        rows[a:a + 33000 + 1000 * i, WIDE0 + i] = ord("T")  # one run per chunk
+    rows[rng.random(N) < 0.3, L - 1] = ord("-")
+    seqs = [x.tobytes().decode() for x in rows]
+    for i in range(131100, N, 97):  # null rows; in the last chunk they split runs
+        seqs[i] = None
+    lineage = [f"L{i:02d}" for i in np.sort(rng.integers(0, 12, N))]
+    b = RawBuilder(N).add_sequences("main", 0, "A" * L, seqs).add_dict("lineage", lineage)
+    raw = b.raw()
+    t = R.Table.from_raw(raw)
+    assert (t.containers(0)[4] == 2).sum() > 40
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+    yield t, dev, orc
+    dev.close()
+
+
+def queries():
+    s = [site(p) for p in range(len(RUNS))] + [f"StrEq(lineage,L{i:02d})" for i in (0, 3, 11)]
+    wide = [site(WIDE0 + i) for i in range(4)]
+    dense = site(RUN0)
+    qs = s + [f"Not({x})" for x in s] + [f"And({dense},{x})" for x in s] + [f"And({dense},Not({x}))" for x in s]
+    qs += [f"Or({','.join(s[i:i + 5])})" for i in range(0, len(s), 4)]
+    qs += [f"NOf({n},{k},{','.join(s)},{dense},{','.join(wide)},Not({s[6]}))" for n in (1, 2, 5, 9) for k in ("atleast", "exactly")]
+    qs += [f"NOf(3,exactly,{','.join(s[i:i + 6])})" for i in range(0, len(s), 5)]
+    qs += [f"And({','.join(wide)})", f"And({dense},Not({s[4]}),Not({s[5]}),Not({s[15]}),Not({s[10]}))"]
+    return qs
+
+
+@pytest.mark.parametrize("width", [4096, 16384, 65536])
+def test_filters_over_runs(sorted_table, width):
+    t, _, orc = sorted_table
+    dev = R.Device(t, 0)
+    dev.set_tile_bits(width)
+    qs = queries()
+    want = []
+    for q in qs:
+        bits, n = dev.compute_filter(q)
+        obits, on = orc.compute_filter(q)
+        assert n == on and np.array_equal(bits, obits), q
+        want.append(on)
+    assert dev.batch(qs, tile_bits=width)[0].tolist() == want
+    dev.close()
+
+
+def test_leaves_past_the_staged_ones_over_runs(sorted_table):
+    """More container leaves than an item stages: the last ones are read from their descriptors."""
+    t, dev, orc = sorted_table
+    s = [site(p) for p in range(len(RUNS))] + [site(WIDE0 + i) for i in range(DENSE)]
+    many = [s[(5 * i) % len(s)] for i in range(160)]
+    qs = [f"NOf({n},{k},{','.join(f'And({a},{b})' for a, b in zip(many, many[1:]))})" for n in (2, 20) for k in ("atleast", "exactly")]
+    qs += [f"And({site(RUN0)},Or({','.join(many)}))"]
+    want = [orc.count(q) for q in qs]
+    assert [dev.count(q) for q in qs] == want and dev.batch(qs)[0].tolist() == want
+
+
+def best_of(fn, reps=15):
+    fn()
+    times = []
+    for _ in range(reps):
+        t0 = time.perf_counter()
+        fn()
+        times.append(time.perf_counter() - t0)
+    return min(times)
+
+
+def cost(dev, kind, sites):
+    if kind == "filter":
+        q = f"NOf(5,atleast,{','.join(site(p) for p in sites)})"
+        return best_of(lambda: dev.count(q))
+
+
+@pytest.mark.parametrize("kind", ["filter"])
+def test_runs_cost_no_more_than_bitsets(sorted_table, kind):
+    """One run per chunk at 24 sites against a bitset of about as many rows. Applied row by row the runs took 20
+    to 100 times as long."""
+    _, dev, _ = sorted_table
+    bitsets, runs = (cost(dev, kind, list(range(a, a + DENSE))) for a in (RUN0, WIDE0))
+    assert runs < 1.5 * bitsets, (runs, bitsets)
