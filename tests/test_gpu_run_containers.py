@@ -91,6 +91,17 @@ def test_leaves_past_the_staged_ones_over_runs(sorted_table):
     assert [dev.count(q) for q in qs] == want and dev.batch(qs)[0].tolist() == want
 
 
+def test_profiles_over_runs(sorted_table):
+    t, dev, orc = sorted_table
+    differ = [[f"{p + 1}:C" for p in range(len(RUNS))], [f"{WIDE0 + i + 1}:T" for i in range(DENSE)], [f"{RUN0 + i + 1}:G" for i in range(4)]]
+    for muts in (*differ, sum(differ, []), [f"{p + 1}:N" for p in range(0, L, 2)]):
+        for d in (0, 1, 5, 12, 30):
+            q = f"MutProfileMutations(main,{d},{','.join(muts)})"
+            bits, n = dev.compute_filter(q)
+            obits, on = orc.compute_filter(q)
+            assert n == on and np.array_equal(bits, obits), q
+
+
 def best_of(fn, reps=15):
     fn()
     times = []
@@ -105,9 +116,12 @@ def cost(dev, kind, sites):
     if kind == "filter":
         q = f"NOf(5,atleast,{','.join(site(p) for p in sites)})"
         return best_of(lambda: dev.count(q))
+    char = "T" if sites[0] >= WIDE0 else "G"
+    q = f"MutProfileMutations(main,3,{','.join(f'{p + 1}:{char}' for p in sites)})"
+    return best_of(lambda: dev.count(q))
 
 
-@pytest.mark.parametrize("kind", ["filter"])
+@pytest.mark.parametrize("kind", ["filter", "profile"])
 def test_runs_cost_no_more_than_bitsets(sorted_table, kind):
     """One run per chunk at 24 sites against a bitset of about as many rows. Applied row by row the runs took 20
     to 100 times as long."""
