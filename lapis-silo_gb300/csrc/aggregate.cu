@@ -24,6 +24,7 @@ namespace {
 constexpr uint32_t AT = 256;
 
 constexpr uint32_t AGG_TILE = 8192;  // rows per CTA
+constexpr uint32_t RUN_OWN = 16;     // a run of at most so many rows is its own lane's
 
 // The symbol of every row of the tile at a position, one byte per row: the local reference, then the
 // missing symbol where the row is not covered, then the symbols of the position's containers (no row is
@@ -64,9 +65,28 @@ __device__ __forceinline__ void tile_symbols(uint8_t* sym, const DevTable* __res
             if (r < AGG_TILE) sym[r] = d.sym;
          }
       } else {
-         for (uint32_t i = lane; i < d.nruns; i += 32) {
-            const uint32_t s = __ldg(p + 2 * i), e = s + __ldg(p + 2 * i + 1) + 1u;
-            for (uint32_t r = max(s, row0); r < min(e, row0 + AGG_TILE); ++r) sym[r - row0] = d.sym;
+         // 32 runs at a time: a short one by its own lane, the others by the warp, four rows a store (two
+         // positions of 400,000 rows in long runs: a call 252 us with a lane per run, 79 us so)
+         for (uint32_t i0 = 0; i0 < d.nruns; i0 += 32) {
+            uint32_t a = 0, b = 0;  // this lane's run in the tile: [a, b)
+            if (i0 + lane < d.nruns) {
+               const uint32_t s = __ldg(p + 2 * (i0 + lane)), e = s + __ldg(p + 2 * (i0 + lane) + 1) + 1u;
+               a = max(s, row0) - row0;
+               b = max(min(e, row0 + AGG_TILE), row0) - row0;
+            }
+            uint32_t wide = __ballot_sync(0xFFFFFFFFu, a < b && b - a > RUN_OWN);
+            if (a < b && b - a <= RUN_OWN)
+               for (uint32_t r = a; r < b; ++r) sym[r] = d.sym;
+            for (; wide; wide &= wide - 1) {
+               const uint32_t j = __ffs(wide) - 1, x = __shfl_sync(0xFFFFFFFFu, a, j), y = __shfl_sync(0xFFFFFFFFu, b, j);
+               for (uint32_t w = x / 4 + lane; w <= (y - 1) / 4; w += 32) {
+                  if (4 * w >= x && 4 * w + 4 <= y) {
+                     reinterpret_cast<uint32_t*>(sym)[w] = d.sym * 0x01010101u;
+                  } else {
+                     for (uint32_t r = max(4 * w, x); r < min(4 * w + 4, y); ++r) sym[r] = d.sym;
+                  }
+               }
+            }
          }
       }
    }

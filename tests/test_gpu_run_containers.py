@@ -102,6 +102,23 @@ def test_profiles_over_runs(sorted_table):
             assert n == on and np.array_equal(bits, obits), q
 
 
+def test_grouped_counts_over_runs(sorted_table):
+    t, dev, orc = sorted_table
+    for p in [*range(len(RUNS)), WIDE0, RUN0]:
+        for q in ("True", f"Not({site(RUN0 + 1)})"):
+            got, n = dev.aggregate(q, [("seq", 0, p + 1), ("seq", 0, WIDE0 + 2)])
+            assert n == orc.count(q) and sum(c for _, c in got) == n
+            for (a, b), c in got:
+                want = orc.count(f"And({q},{symbol(p, a)},{symbol(WIDE0 + 1, b)})")
+                assert c == want, (p, q, a, b)
+
+
+def symbol(p, s):
+    if s is None:  # null rows match no symbol
+        return "And(" + ",".join(f"Not(SymEq(main,{p + 1},{x}))" for x in "ACGTN-") + ")"
+    return f"SymEq(main,{p + 1},{s})"
+
+
 def best_of(fn, reps=15):
     fn()
     times = []
@@ -116,12 +133,14 @@ def cost(dev, kind, sites):
     if kind == "filter":
         q = f"NOf(5,atleast,{','.join(site(p) for p in sites)})"
         return best_of(lambda: dev.count(q))
-    char = "T" if sites[0] >= WIDE0 else "G"
-    q = f"MutProfileMutations(main,3,{','.join(f'{p + 1}:{char}' for p in sites)})"
-    return best_of(lambda: dev.count(q))
+    if kind == "profile":
+        char = "T" if sites[0] >= WIDE0 else "G"
+        q = f"MutProfileMutations(main,3,{','.join(f'{p + 1}:{char}' for p in sites)})"
+        return best_of(lambda: dev.count(q))
+    return best_of(lambda: dev.aggregate("True", [("seq", 0, p + 1) for p in sites[:4]]))
 
 
-@pytest.mark.parametrize("kind", ["filter", "profile"])
+@pytest.mark.parametrize("kind", ["filter", "profile", "aggregate"])
 def test_runs_cost_no_more_than_bitsets(sorted_table, kind):
     """One run per chunk at 24 sites against a bitset of about as many rows. Applied row by row the runs took 20
     to 100 times as long."""
