@@ -8,7 +8,8 @@
 //   transpose_kernel       filter row sets -> masks, pass-major rows (32 B per row and pass)
 //   mut_ctr_batch_kernel   container pass, one warp per (position, chunk range) unit: |F_q ∩ c|
 //                          for every container c (reference: mutations_node.cpp:138-190)
-//   mut_ctr_narrow_kernel  the same for a pass of at most 32 queries, masks in shared memory
+//   mut_ctr_narrow_kernel  the same for a pass of at most 32 queries, masks in shared memory; its run
+//   mut_runs_narrow_kernel containers apart, the filters' words in shared memory
 //   mut_cov_batch_kernel   missing-interval and coverage boundary events (reference:
 //                          mutations_node.cpp:51-136)
 //   mut_final_batch_kernel prefix sums and reference counts per query
@@ -382,8 +383,8 @@ __global__ void __launch_bounds__(BT, 4) mut_ctr_batch_kernel(const DevTable* __
 
 // Container pass of a pass of one mask word (blockIdx.y: its first or second 16 queries). A CTA stages the
 // 16-bit masks of a chunk's rows in shared memory and counts its share of the chunk's containers, 32 at a time
-// per warp: arrays of up to NARROW_LIGHT rows four at a time, eight lanes each; longer arrays and runs with
-// the whole warp; bitsets by population counts with the filters' own words. Two rows' masks make a word whose
+// per warp: arrays of up to NARROW_LIGHT rows four at a time, eight lanes each; longer arrays with the whole
+// warp; bitsets by population counts with the filters' own words; run containers: mut_runs_narrow_kernel. Two rows' masks make a word whose
 // bits are added to nibble counters (nibble k of nib[j]: query j + 4 (k % 4)); their bytes are summed over
 // the lanes. Bound by issue slots, then by the gathers (one of 32 banks each): a mask from L2 takes a sector,
 // and the wide pass, whose lanes then are all on different rows, took 350 us at 2M rows and 7 queries,
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(NARROW_T, 1) mut_ctr_narrow_kernel(const DevTa
          if (ta && (x & 0xFFu)) atomicAdd(ta + at, x & 0xFFu);
          if (tb && ((x >> 8) & 0xFFu)) atomicAdd(tb + at, (x >> 8) & 0xFFu);
       }
-      uint32_t heavy = __ballot_sync(0xFFFFFFFFu, have && !light);
+      uint32_t heavy = __ballot_sync(0xFFFFFFFFu, have && !light && mine.type != CT_RUN);
       while (heavy) {
          const uint32_t j = __ffs(heavy) - 1;
          heavy &= heavy - 1;
@@ -522,13 +523,6 @@ __global__ void __launch_bounds__(NARROW_T, 1) mut_ctr_narrow_kernel(const DevTa
          };
          if (d.type == CT_ARRAY) {
             count_rows(d.card_m1 + 1u, [&](uint32_t i) { return static_cast<uint32_t>(__ldcs(p + i)); });
-         } else if (d.type == CT_RUN) {
-#pragma unroll 1
-            for (uint32_t i = 0; i < d.nruns; ++i) {
-               const uint32_t s0 = __ldg(p + 2 * i), n = __ldg(p + 2 * i + 1) + 1u;
-#pragma unroll 1
-               for (uint32_t b = 0; b < n; b += 32768) count_rows(min(n - b, 32768u), [&](uint32_t t) { return s0 + b + t; });
-            }
          } else {
             const uint4* bits = reinterpret_cast<const uint4*>(p);
 #pragma unroll 1
@@ -545,6 +539,100 @@ __global__ void __launch_bounds__(NARROW_T, 1) mut_ctr_narrow_kernel(const DevTa
             }
          }
       }
+   }
+}
+
+// The run containers of such a pass, by population counts with the filters' words of the chunk, which a CTA stages in
+// shared memory, 16 filters at a time; a warp takes a container, 32 runs of it at once: each lane the words of its
+// own run, and the words of a run of more than NARROW_RUN rows the whole warp. One of many long runs is read as
+// the bitset that filters have of it. Bound by the shared-memory reads, one per word and filter. 16 queries over 64
+// sites of 1,800 runs each at 70,000 rows: 51 us; 760 us as a part of the kernel above, which took their rows
+// from the masks and reduced the counts once per run.
+constexpr uint32_t NARROW_RUN = 96;
+__global__ void __launch_bounds__(NARROW_T, 1) mut_runs_narrow_kernel(const DevTable* __restrict__ tab, uint32_t col,
+                                                                      const uint32_t* __restrict__ filters,
+                                                                      const uint32_t* __restrict__ lists, uint32_t nq_max,
+                                                                      uint32_t per_chunk, uint32_t* __restrict__ counts) {
+   extern __shared__ __align__(16) uint32_t words_of[];  // 16 filters x CHUNK_WORDS
+   static_assert(NARROW_SMEM == 16 * CHUNK_WORDS * 4, "16 filters of a chunk");
+   __shared__ uint32_t next;
+   const uint32_t nq = lists[2 * nq_max];  // dense slots: lists[0 .. nq)
+   const uint32_t nqc = (nq + 31) / 32, pass = (nqc + 7) / 8 - 1, q0 = 256 * pass + 16 * blockIdx.y;
+   if (nq == 0 || pass_width_u32(nqc, pass) != 1 || q0 >= nq) return;
+   const DevSeqCol* cs = &tab->seq[col];
+   const uint32_t v = blockIdx.x / per_chunk, part = blockIdx.x % per_chunk, lane = threadIdx.x & 31;
+   const uint32_t a = __ldg(cs->run_off + v), n = __ldg(cs->run_off + v + 1) - a;
+   const uint32_t r0 = a + static_cast<uint32_t>(static_cast<uint64_t>(n) * part / per_chunk);
+   const uint32_t r1 = a + static_cast<uint32_t>(static_cast<uint64_t>(n) * (part + 1) / per_chunk);
+   if (r0 == r1) return;
+   const size_t words = static_cast<size_t>(tab->nchunks) * CHUNK_WORDS, per_query = static_cast<size_t>(cs->nsym) * cs->L;
+   for (uint32_t i = threadIdx.x; i < 16 * CHUNK_WORDS / 4; i += NARROW_T) {
+      const uint32_t q = i / (CHUNK_WORDS / 4), w = i % (CHUNK_WORDS / 4);
+      uint4 x = make_uint4(0, 0, 0, 0);
+      if (q0 + q < nq) x = __ldg(reinterpret_cast<const uint4*>(filters + lists[q0 + q] * words + static_cast<size_t>(v) * CHUNK_WORDS) + w);
+      reinterpret_cast<uint4*>(words_of)[i] = x;
+   }
+   if (threadIdx.x == 0) next = r0;
+   __syncthreads();
+   for (;;) {
+      uint32_t r = 0;
+      if (lane == 0) r = atomicAdd(&next, 1u);
+      r = __shfl_sync(0xFFFFFFFFu, r, 0);
+      if (r >= r1) break;
+      const uint32_t c = __ldg(cs->run_ctrs + r);
+      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(cs->fctrs) + c);
+      const CtrDesc d = *reinterpret_cast<const CtrDesc*>(&raw);
+      uint32_t sum[16];
+#pragma unroll
+      for (uint32_t q = 0; q < 16; ++q) sum[q] = 0;
+      auto add_word = [&](uint32_t w, uint32_t m) {  // the rows of mask m in word w
+#pragma unroll
+         for (uint32_t q = 0; q < 16; ++q) sum[q] += __popc(words_of[q * CHUNK_WORDS + w] & m);
+      };
+      auto mask = [](uint32_t w, uint32_t s, uint32_t e) {  // the rows [s, e) in word w, which holds one of them
+         const uint32_t b = 32 * w;
+         return (s > b ? 0xFFFFFFFFu << (s - b) : 0xFFFFFFFFu) & (e < b + 32 ? 0xFFFFFFFFu >> (b + 32 - e) : 0xFFFFFFFFu);
+      };
+      if (d.type == CT_BITSET) {
+         const uint32_t* bits = reinterpret_cast<const uint32_t*>(cs->payload + d.payload) + lane;
+         constexpr uint32_t U = 8;  // loads in flight
+#pragma unroll 1
+         for (uint32_t w = 0; w < CHUNK_WORDS; w += 32 * U) {
+            uint32_t x[U];
+#pragma unroll
+            for (uint32_t k = 0; k < U; ++k) x[k] = __ldg(bits + w + 32 * k);
+#pragma unroll
+            for (uint32_t k = 0; k < U; ++k) add_word(w + 32 * k + lane, x[k]);
+         }
+      } else {
+         const uint16_t* p = cs->payload + d.payload;
+#pragma unroll 1
+         for (uint32_t i0 = 0; i0 < d.nruns; i0 += 32) {
+            uint32_t s = 0, e = 0;
+            if (i0 + lane < d.nruns) {
+               s = __ldg(p + 2 * (i0 + lane));
+               e = s + __ldg(p + 2 * (i0 + lane) + 1) + 1u;
+            }
+            uint32_t wide = __ballot_sync(0xFFFFFFFFu, e - s > NARROW_RUN);
+            if (s < e && e - s <= NARROW_RUN)
+#pragma unroll 1
+               for (uint32_t w = s >> 5; w <= (e - 1) >> 5; ++w) add_word(w, mask(w, s, e));
+            __syncwarp();
+#pragma unroll 1
+            for (; wide; wide &= wide - 1) {
+               const uint32_t j = __ffs(wide) - 1, x = __shfl_sync(0xFFFFFFFFu, s, j), z = __shfl_sync(0xFFFFFFFFu, e, j);
+#pragma unroll 1
+               for (uint32_t w = (x >> 5) + lane; w <= (z - 1) >> 5; w += 32) add_word(w, mask(w, x, z));
+            }
+         }
+      }
+      uint32_t mine = 0;  // lane q: query q
+#pragma unroll
+      for (uint32_t q = 0; q < 16; ++q) {
+         const uint32_t k = __reduce_add_sync(0xFFFFFFFFu, sum[q]);
+         if (lane == q) mine = k;
+      }
+      if (mine) atomicAdd(counts + lists[q0 + lane] * per_query + static_cast<size_t>(d.sym) * cs->L + d.key, mine);
    }
 }
 
@@ -763,8 +851,10 @@ static_assert(MUT_SEG / 32 == 32, "one lane per warp's total");
 }  // namespace
 
 void mutations_batch_setup() {
-   const cudaError_t e =
+   cudaError_t e =
       cudaFuncSetAttribute(mut_ctr_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(NARROW_SMEM));
+   if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(mut_runs_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(NARROW_SMEM));
    if (e != cudaSuccess)
       throw std::runtime_error(std::string("shared memory of the narrow container pass: ") + cudaGetErrorString(e));
 }
@@ -796,6 +886,11 @@ void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, 
       const uint32_t per_chunk = std::max(1u, 152u / nchunks);  // one CTA per SM
       mut_ctr_narrow_kernel<<<dim3(nchunks * per_chunk, nq > 16 ? 2 : 1), NARROW_T, NARROW_SMEM, s>>>(
          d_table, col, d_filters, d_masks, d_lists, nq, per_chunk, d_counts);
+      if (col_host.n_run_ctrs > 0) {  // a container per warp at least
+         const uint32_t ctas = std::clamp(col_host.n_run_ctrs / nchunks / (NARROW_T / 32), 1u, per_chunk);
+         mut_runs_narrow_kernel<<<dim3(nchunks * ctas, nq > 16 ? 2 : 1), NARROW_T, NARROW_SMEM, s>>>(
+            d_table, col, d_filters, d_lists, nq, ctas, d_counts);
+      }
    }
    if ((parts & BMUT_PART_COV) && n_ev > 0)
       mut_cov_batch_kernel<<<dim3(n_ev, (ngroups + PASS_GROUPS - 1) / PASS_GROUPS), BT, 0, s>>>(d_table, col, d_ev, d_masks, d_lists, nq,

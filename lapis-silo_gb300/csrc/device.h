@@ -93,6 +93,9 @@ struct DevSeqCol {
    const ArrUnit* au;          // array units of the Mutations container pass, chunk-major
    const OtherUnit* ou;        // its bitset and run units, chunk-major
    const StreamRange* ranges;  // its CTAs
+   const uint32_t* run_ctrs;   // the run containers, chunk-major (indices into ctrs)
+   const uint32_t* run_off;    // nchunks + 1
+   uint32_t n_run_ctrs;
    const uint32_t* nblk_toff;  // nblocks * nchunks * TOFF_N: tile row-range offsets into each nblk bucket
    const uint32_t* null_tiles; // nchunks * CHUNK_WORDS
    const uint8_t* local_ref;   // L

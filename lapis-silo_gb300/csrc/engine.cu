@@ -414,6 +414,18 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          d.payload = payload;
          d.fctrs = fctrs;
          d.off = upload(s.vertical.off);
+         {
+            std::vector<uint32_t> runs, at(nchunks + 1, 0);
+            for (uint32_t i = 0; i < s.vertical.ctrs.size(); ++i)
+               if (s.vertical.ctrs[i].type == CT_RUN) {
+                  runs.push_back(i);
+                  ++at[s.vertical.ctrs[i].v + 1];
+               }
+            for (uint32_t v = 0; v < nchunks; ++v) at[v + 1] += at[v];
+            d.n_run_ctrs = static_cast<uint32_t>(runs.size());
+            d.run_ctrs = upload(runs);
+            d.run_off = upload(at);
+         }
          upload_coverage(s, nchunks, d);
          upload_missing(s, nchunks, d);
          {

@@ -119,6 +119,21 @@ def symbol(p, s):
     return f"SymEq(main,{p + 1},{s})"
 
 
+@pytest.mark.parametrize("slots", [1, 16, 17, 32, 40])
+def test_batched_mutations_over_runs(sorted_table, slots):
+    t, dev, orc = sorted_table
+    forms = ["True", site(RUN0), f"Not({site(RUN0 + 1)})", site(6), site(WIDE0 + 3), f"Not({site(14)})"]
+    qs = [f"Or({forms[i % 6]},{forms[(i // 6) % 6]})" for i in range(slots)]
+    keep = dev.sparse_rows()
+    dev.sparse_rows(batch=0)  # every filter takes the container pass
+    counts, muts = dev.batch(qs, [1] * slots, [0] * slots)
+    dev.sparse_rows(*keep)
+    known = {q: orc.mutations(q, 0) for q in set(qs)}
+    for i, q in enumerate(qs):
+        want, n = known[q]
+        assert counts[i] == n and np.array_equal(muts[i], want), q
+
+
 def best_of(fn, reps=15):
     fn()
     times = []
@@ -147,3 +162,39 @@ def test_runs_cost_no_more_than_bitsets(sorted_table, kind):
     _, dev, _ = sorted_table
     bitsets, runs = (cost(dev, kind, list(range(a, a + DENSE))) for a in (RUN0, WIDE0))
     assert runs < 1.5 * bitsets, (runs, bitsets)
+
+
+def test_narrow_pass_over_many_runs():
+    """The container pass of 16 queries (one mask word) over containers of 1,800 runs of eight rows beside that of
+    64 queries, which reads the same containers once. Reduced run by run, the narrow pass
+    took a third longer than the wide one."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+    n, sites = 70000, 64
+    rows = np.full((n, sites), ord("A"), np.uint8)
+    r = np.arange(n)
+    for i in range(sites):
+        rows[(r + 5 * i) % 36 < 8, i] = ord("C")
+    b = RawBuilder(n).add_sequences("main", 0, "A" * sites, [x.tobytes().decode() for x in rows])
+    raw = b.raw()
+    dev = R.Device(R.Table.from_raw(raw), 0)
+    dev.sparse_rows(batch=0)  # every filter takes the container pass
+    stream = torch.cuda.Stream()
+    ptr = ctypes.c_void_p(stream.cuda_stream)
+
+    def container_pass(slots):
+        dev.batch_prepare([f"Not({site(i % sites)})" for i in range(slots)], [1] * slots, [0] * slots)
+        dev.batch_launch(ptr, True, False)
+        times = []
+        for _ in range(9):
+            a, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            dev.batch_launch_parts(4, ptr)
+            e.record(stream)
+            e.synchronize()
+            times.append(a.elapsed_time(e))
+        return min(times)
+
+    narrow, wide = container_pass(16), container_pass(64)
+    assert narrow < wide, (narrow, wide)
+    dev.close()
