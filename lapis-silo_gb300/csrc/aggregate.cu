@@ -15,6 +15,9 @@
 // dictionary dimension's groups are its values in string order and then the null group (:237-259).
 #include <cuda_runtime.h>
 
+#include <stdexcept>
+#include <string>
+
 #include "aggregate.h"
 
 namespace rhygpu {
@@ -199,13 +202,16 @@ __global__ void __launch_bounds__(AT) agg_write_kernel(const uint32_t* __restric
 
 }  // namespace
 
+void aggregate_setup() {
+   const cudaError_t e = cudaFuncSetAttribute(agg_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              static_cast<int>(AGG_TILE * 5 + AGG_DENSE * 4));
+   if (e != cudaSuccess) throw std::runtime_error(std::string("shared memory of the aggregation: ") + cudaGetErrorString(e));
+}
+
 cudaError_t launch_agg_keys(const DevTable* d_table, uint32_t nchunks, const uint32_t* d_filter, const AggDim* d_dims,
                             uint32_t nd, uint64_t keys, uint32_t* d_counters, void* stream) {
    const bool hist = keys <= AGG_DENSE;  // a tile's counters in shared memory: up to 32 KiB beside its 40 KiB
    const size_t smem = AGG_TILE * 5 + (hist ? keys * 4 : 0);
-   const cudaError_t e =
-      cudaFuncSetAttribute(agg_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-   if (e != cudaSuccess) return e;
    agg_keys_kernel<<<nchunks * (CHUNK_ROWS / AGG_TILE), AT, smem, static_cast<cudaStream_t>(stream)>>>(
       d_table, d_filter, d_dims, nd, static_cast<uint32_t>(keys), hist, d_counters);
    return cudaGetLastError();

@@ -255,10 +255,16 @@ cudaError_t launch_dense_forms(uint16_t* d_arena, const DenseJob* d_jobs, uint32
 // in a filter kernel (6) or in the Mutations container pass (7).
 enum : int { DEVERR_WAIT_FILTER = 6, DEVERR_WAIT_MUTATIONS = 7 };
 
-// Sets the container pass's shared-memory size on the current device (once per device, before
-// its first launch).
+// The shared memory that the kernels may take, set on the current device before their first launch: each to the
+// most that its launches ask for. The limit belongs to the kernel on the device, not to a launch, so a
+// handle that set it to the size of its own call would take it from under another handle's.
+void filter_setup();
+void profile_setup();
+void aggregate_setup();
 void mutations_setup();
 void mutations_batch_setup();
+// The filter kernels' tiles of one program (Program::tiles) take at most so much of it.
+constexpr size_t TILES_BYTES = 200 * 1024;
 
 // Kernel selection masks (all bits set = the whole pass); used to time the kernels one by one.
 enum : uint32_t { MUT_PART_CTR = 1, MUT_PART_COV = 2, MUT_PART_FINAL = 4, MUT_PART_ALL = 7 };

@@ -397,6 +397,9 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
    cuda_check(cudaSetDevice(device), "cudaSetDevice");
    try {
       cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+      filter_setup();
+      profile_setup();
+      aggregate_setup();
       mutations_setup();
       mutations_batch_setup();
       const uint32_t nchunks = t.nchunks();
@@ -815,10 +818,10 @@ namespace rhygpu {
 
 uint32_t Engine::fit_tile_bits(uint32_t requested, const Program& p, bool batch) const {
    uint32_t W = requested ? requested : batch ? batch_tile_bits : tile_bits;
-   // shared memory: the program's tiles under 200 KiB; the depth limit of the narrowest tile is that
+   // shared memory: the program's tiles under TILES_BYTES; the depth limit of the narrowest tile is that
    // of the whole stack
-   if (static_cast<size_t>(p.max_depth) * (4096 / 8) > 200 * 1024) throw IllegalQuery("filter expression nests too deeply");
-   while (W > 2048 && static_cast<size_t>(p.tiles) * (W / 8) > 200 * 1024) W >>= 1;
+   if (static_cast<size_t>(p.max_depth) * (4096 / 8) > TILES_BYTES) throw IllegalQuery("filter expression nests too deeply");
+   while (W > 2048 && static_cast<size_t>(p.tiles) * (W / 8) > TILES_BYTES) W >>= 1;
    return W;
 }
 

@@ -1169,6 +1169,17 @@ __global__ void __launch_bounds__(256) dense_forms_kernel(uint16_t* arena, const
 // ------------------------------------------------------------------------------------------------
 // launchers
 
+static_assert(LC_BYTES + CHUNK_ROWS / 8 + TILES_BYTES <= 227 * 1024, "shared memory of a CTA");
+void filter_setup() {
+   const auto allow = [](const void* kernel, size_t bytes) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+      if (e != cudaSuccess) throw std::runtime_error(std::string("shared memory of the filter kernels: ") + cudaGetErrorString(e));
+   };
+   allow(reinterpret_cast<const void*>(filter_kernel<false>), LC_BYTES + TILES_BYTES);
+   allow(reinterpret_cast<const void*>(filter_kernel<true>), LC_BYTES + TILES_BYTES);
+   allow(reinterpret_cast<const void*>(filter_batch_kernel), LC_BYTES + CHUNK_ROWS / 8 + TILES_BYTES);
+}
+
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
                           uint32_t n_leaves, uint32_t tile_bits, uint32_t stack_tiles, uint32_t* d_out_tiles, unsigned long long* d_count,
                           int* d_err, void* stream, uint32_t* d_trace, const uint32_t* d_aux, const CallEnd& end,
@@ -1182,8 +1193,6 @@ cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr
    const uint32_t threads = std::max(32u, std::min(FT, tile_bits / 128));
    const size_t smem = LC_BYTES + static_cast<size_t>(std::max(stack_tiles, 1u)) * (tile_bits / 8);
    const auto kernel = d_trace ? filter_kernel<true> : filter_kernel<false>;
-   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-   if (e != cudaSuccess) return e;
    kernel<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(d_table, inline_code ? nullptr : d_code, ncode, n_leaves, tile_bits,
                                                                       stack_tiles - 1, d_out_tiles, d_count, d_err, d_trace,
                                                                       d_aux, end, ic);
@@ -1192,11 +1201,6 @@ cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr
 
 int filter_batch_blocks_per_sm(size_t scratch_bytes, size_t stack_bytes) {
    const size_t smem = LC_BYTES + scratch_bytes + stack_bytes;
-   if (cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-       cudaSuccess) {
-      cudaGetLastError();
-      return 1;
-   }
    int n = 0;
    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, filter_batch_kernel, FT, smem) != cudaSuccess) {
       cudaGetLastError();
@@ -1210,9 +1214,6 @@ cudaError_t launch_filter_batch(const DevTable* d_table, const Instr* d_code, co
                          uint32_t* d_out_tiles, unsigned long long* d_counts, uint32_t* d_next, uint32_t grid, int* d_err,
                          void* stream, const uint32_t* d_aux) {
    const size_t smem = LC_BYTES + scratch_bytes + stack_bytes;
-   cudaError_t e =
-      cudaFuncSetAttribute(filter_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-   if (e != cudaSuccess) return e;
    filter_batch_kernel<<<grid, FT, smem, static_cast<cudaStream_t>(stream)>>>(
       d_table, d_code, d_queries, d_items, n_items, scratch_bytes, stack_bytes, d_out_tiles, d_counts, d_next, d_err, d_aux);
    return cudaGetLastError();

@@ -31,6 +31,9 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <stdexcept>
+#include <string>
+
 #include "device.h"
 
 namespace rhygpu {
@@ -487,12 +490,23 @@ cudaError_t launch_profile_home(const DevTable* d_table, uint32_t col, uint32_t 
    return cudaGetLastError();
 }
 
+// prefix windows, mask, diff (see profile_staged_kernel)
+static size_t staged_smem(uint32_t L) { return (ST / 32) * PW * 4 + static_cast<size_t>(L) * 4 + (static_cast<size_t>(L) + 1) * 2; }
+
+void profile_setup() {
+   const auto allow = [](const void* kernel, size_t bytes) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+      if (e != cudaSuccess) throw std::runtime_error(std::string("shared memory of the profile kernels: ") + cudaGetErrorString(e));
+   };
+   allow(reinterpret_cast<const void*>(profile_delta_kernel), DELTA_SMEM);
+   allow(reinterpret_cast<const void*>(profile_staged_kernel), staged_smem(STAGE_MAX_L));
+}
+
 void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile* d_profiles, uint32_t n,
                      bool any_delta, uint32_t max_L, uint32_t* d_aux, void* stream) {
    const uint32_t words = nchunks * CHUNK_WORDS;
    const cudaStream_t s = static_cast<cudaStream_t>(stream);
    if (any_delta) {
-      cudaFuncSetAttribute(profile_delta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DELTA_SMEM);
       for (uint32_t k = 0; k < n; k += 65535) {  // grid.y is at most 65535
          const uint32_t m = n - k < 65535 ? n - k : 65535;
          // CTAs per chunk: eight (the most that every device takes) while they find an SM each, else four
@@ -512,14 +526,10 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
       }
    }
    if (max_L == 0) return;
-   const size_t smem = (ST / 32) * PW * 4 + static_cast<size_t>(max_L) * 4 + (static_cast<size_t>(max_L) + 1) * 2;
-   int dev = 0, sms = 0, optin = 0;
-   bool staged = max_L <= STAGE_MAX_L && cudaGetDevice(&dev) == cudaSuccess &&
-                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-                 cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
-                 smem <= static_cast<size_t>(optin) &&
-                 cudaFuncSetAttribute(profile_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)) == cudaSuccess;
+   const size_t smem = staged_smem(max_L);
+   int dev = 0, sms = 0;
+   const bool staged = max_L <= STAGE_MAX_L && cudaGetDevice(&dev) == cudaSuccess &&
+                       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
    for (uint32_t k = 0; k < n; k += 65535) {  // grid.y is at most 65535
       const uint32_t m = n - k < 65535 ? n - k : 65535;
       if (staged)
