@@ -400,8 +400,10 @@ int rhy_mutations_noalloc(RhyDevice* d, uint32_t column, const uint32_t* d_filte
  * issue them, so a wait gives up after 1 ms and the call reports RHY_CUDA ("a bounded device wait
  * for bulk copies gave up", device error 6); bit 1 does the same for the Mutations container pass's
  * ring copies (device error 7; rhy_mutations_noalloc reports it in its status word). The withheld
- * copies never start, so no copy is left in flight and the device stays usable. Synchronises the
- * device; off (0) by default. Not for production use. */
+ * copies never start, so no copy is left in flight and the device stays usable. Bit 2 withholds the tensor-core
+ * products of this handle's rhy_mlp_gradient calls, which then report RHY_INTERNAL ("a bounded wait of the
+ * gradient kernel gave up"); bits 0 and 1 are the device's. Synchronises the device; off (0) by default.
+ * Not for production use. */
 int rhy_test_withhold_copies(RhyDevice* d, int on);
 
 /* Formats counts like the reference's Mutations action; returns the number of rows in *n_rows. */

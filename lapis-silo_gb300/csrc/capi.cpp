@@ -983,6 +983,7 @@ int rhy_test_withhold_copies(RhyDevice* d, int on) {
       rhygpu::cuda_check(cudaDeviceSynchronize(), "synchronise before switching copy withholding");
       rhygpu::set_copy_withholding((on & 1) != 0);
       rhygpu::set_ring_withholding((on & 2) != 0);
+      d->engine->withhold_products = (on & 4) != 0;
    });
 }
 

@@ -1573,7 +1573,9 @@ size_t Engine::collect_traces(const std::vector<std::string>& exprs, std::vector
 
 std::unique_ptr<PlannerNet> Engine::take_net() {
    std::lock_guard<std::mutex> lock(net_mu_);
-   return net_ ? std::move(net_) : std::make_unique<PlannerNet>(device_);
+   std::unique_ptr<PlannerNet> net = net_ ? std::move(net_) : std::make_unique<PlannerNet>(device_);
+   net->withhold = withhold_products;
+   return net;
 }
 
 void Engine::give_net(std::unique_ptr<PlannerNet> net) {

@@ -1,6 +1,7 @@
 // Device-resident partition and the execution of filter / count / mutations queries on it.
 #pragma once
 
+#include <atomic>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -289,6 +290,7 @@ class Engine {
    // other thread has it, else a new one. A call gives it back when it has succeeded; one is kept, if its
    // buffers hold at most NET_KEPT samples (15 MB). Making and freeing one took 200 us of such a call.
    std::unique_ptr<PlannerNet> take_net();
+   std::atomic<bool> withhold_products{false};  // testing: of the networks taken here (see mlp_gradient)
    void give_net(std::unique_ptr<PlannerNet> net);
    static constexpr uint32_t NET_KEPT = 1u << 17;
    // Plans a batch: rule-based, or with the learned planner's estimates (one GPU inference over

@@ -146,10 +146,6 @@ static_assert(MLP_W1 % 8 == 0 && MLP_W2 % 8 == 0 && MLP_IN % 8 == 0, "weight row
 // TMEM columns of the accumulators
 constexpr uint32_t TM_Z1 = 0, TM_Z2 = 64, TM_G1 = 128, TM_DW2 = 192, TM_DW1 = 272, TM_COLS = 512;
 
-// a device error of the gradient kernel (a bounded wait for its MMAs that gave up); read and cleared
-// by mlp_read_error and mlp_clear_error
-__device__ int g_mlp_err = 0;
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // shared-memory matrix descriptor: no swizzle, start address, leading byte offset (next 16-byte
@@ -183,9 +179,9 @@ __device__ __forceinline__ void operands_ready() {
    __syncthreads();
    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// waits (bounded: 2 s on the global timer) for the MMAs committed as phase `parity`; the whole CTA
+// waits (bounded by limit_ns on the global timer) for the MMAs committed as phase `parity`; the whole CTA
 // agrees on the outcome
-__device__ __forceinline__ bool mma_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mma_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
    const uint32_t b = smem_u32(bar);
    uint64_t t0 = 0;
    bool done = false;
@@ -200,7 +196,7 @@ __device__ __forceinline__ bool mma_wait(uint64_t* bar, uint32_t parity) {
          uint64_t now;
          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
          if (t0 == 0) t0 = now;
-         else if (now - t0 > 2000000000ull) break;
+         else if (now - t0 > limit_ns) break;
       }
    }
    done = __syncthreads_and(done) != 0;
@@ -259,7 +255,7 @@ __device__ __forceinline__ void put8(uint8_t* base, uint32_t off, const __nv_bfl
 __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* __restrict__ w,
                                                            const float* __restrict__ X, const float* __restrict__ T,
                                                            uint32_t n, float inv_total, float* __restrict__ grad,
-                                                           float* __restrict__ loss) {
+                                                           float* __restrict__ loss, int* err, bool withhold) {
    extern __shared__ __align__(1024) uint8_t sm[];
    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
    const uint32_t r = t & (TC_S - 1), q = t / TC_S, u0 = 16 * q;  // sample row, quarter, its first unit
@@ -330,14 +326,15 @@ __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* 
    const uint32_t lane_addr = tmem + ((32u * (warp & 3)) << 16);
    bool ok = true;
    uint32_t committed = 0;  // MMA phases committed to the barrier (the same in every thread)
+   const uint64_t limit = withhold ? 1000000ull : 2000000000ull;
    // ---- phase 0: Z1 = X W1^T
-   if (t == 0) {
+   if (t == 0 && !withhold) {
       mma_k(tmem + TM_Z1, base + SO_XA_HI, base + SO_W1, 4, 2, mma_idesc(64), false);
       mma_k(tmem + TM_Z1, base + SO_XA_LO, base + SO_W1, 4, 2, mma_idesc(64), true);
       mma_commit(bar);
    }
    ++committed;
-   ok = mma_wait(bar, 0);
+   ok = mma_wait(bar, 0, limit);
    uint32_t mask1 = 0, mask2 = 0;  // the quarter's units with a positive input
    if (ok) {
       // h1 = relu(z1 + b1): row r of H1 (hi, lo) and column r of [H1^T; 1; 0]
@@ -376,7 +373,7 @@ __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* 
    }
    if (ok) {
       ++committed;
-      ok = mma_wait(bar, 1);
+      ok = mma_wait(bar, 1, limit);
    }
    float h[16];
    if (ok) {  // the quarter's part of the output layer
@@ -451,7 +448,7 @@ __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* 
    }
    if (ok) {
       ++committed;
-      ok = mma_wait(bar, 0);
+      ok = mma_wait(bar, 0, limit);
    }
    float* g2 = reinterpret_cast<float*>(sm + SO_H1B_HI);
    if (ok) {
@@ -500,7 +497,7 @@ __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* 
    if (ok) {
       add_rows(g2, GR2, MLP_H, grad + MLP_W2, grad + MLP_B2);
       ++committed;
-      ok = mma_wait(bar, 1);
+      ok = mma_wait(bar, 1, limit);
    }
    if (ok) {
       float* g1 = reinterpret_cast<float*>(sm);
@@ -515,11 +512,11 @@ __global__ void __launch_bounds__(TC_T, 1) mlp_grad_kernel(const __nv_bfloat16* 
       __syncthreads();  // ok is the CTA's
       add_rows(g1, GR1, MLP_IN, grad + MLP_W1, grad + MLP_B1);
    } else if (t == 0) {
-      atomicExch(&g_mlp_err, 1);
+      atomicExch(err, 1);
    }
    // a wait that gave up leaves MMAs possibly in flight: wait for the phase it gave up on (bounded)
    // before the tensor memory is freed
-   if (!ok) mma_wait(bar, (committed - 1) & 1u);
+   if (!ok) mma_wait(bar, (committed - 1) & 1u, limit);
    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
    __syncthreads();
    if (warp == 0) {
@@ -572,21 +569,13 @@ cudaError_t mlp_predict(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, 
 }
 
 cudaError_t mlp_gradient(const __nv_bfloat16* d_w, const float* d_X, const float* d_T, uint32_t n, float* d_grad,
-                         float* d_loss, cudaStream_t s) {
+                         float* d_loss, int* d_err, bool withhold, cudaStream_t s) {
    if (n == 0) return cudaSuccess;
    cudaError_t e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SO_END));
    if (e != cudaSuccess) return e;
-   mlp_grad_kernel<<<(n + TC_S - 1) / TC_S, TC_T, SO_END, s>>>(d_w, d_X, d_T, n, 1.0f / static_cast<float>(n), d_grad, d_loss);
+   mlp_grad_kernel<<<(n + TC_S - 1) / TC_S, TC_T, SO_END, s>>>(d_w, d_X, d_T, n, 1.0f / static_cast<float>(n), d_grad, d_loss,
+                                                                   d_err, withhold);
    return cudaGetLastError();
-}
-
-cudaError_t mlp_read_error(int* v, cudaStream_t s) {
-   return cudaMemcpyFromSymbolAsync(v, g_mlp_err, sizeof(int), 0, cudaMemcpyDeviceToHost, s);
-}
-
-cudaError_t mlp_clear_error() {
-   const int zero = 0;
-   return cudaMemcpyToSymbol(g_mlp_err, &zero, sizeof(int));
 }
 
 cudaError_t mlp_adam(float* d_master, __nv_bfloat16* d_w, float* d_grad, float* d_m, float* d_v, float lr, uint32_t step,

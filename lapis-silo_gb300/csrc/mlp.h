@@ -34,13 +34,11 @@ struct MlpScale {
 cudaError_t mlp_predict(const __nv_bfloat16* d_w, const float* d_X, uint32_t n, const MlpScale& scale, double* d_sel,
                         double* d_cost, cudaStream_t s);
 // Adds the gradient of mean_n sum_k (net(X)_k - T_k)^2 with respect to the BF16 weights to d_grad
-// and the loss to *d_loss.
+// and the loss to *d_loss; *d_err is set to 1 if a bounded wait for the tensor-core products gave up (each network
+// has its own word, so that one caller's error is not another's). withhold: testing the failure path, the
+// products are never issued and the wait gives up after 1 ms.
 cudaError_t mlp_gradient(const __nv_bfloat16* d_w, const float* d_X, const float* d_T, uint32_t n, float* d_grad,
-                         float* d_loss, cudaStream_t s);
-// A device error of the gradient kernel since it was cleared last (1: a bounded wait for its tensor-core
-// products gave up): read on the stream into *v, which is valid once the stream has passed it.
-cudaError_t mlp_read_error(int* v, cudaStream_t s);
-cudaError_t mlp_clear_error();
+                         float* d_loss, int* d_err, bool withhold, cudaStream_t s);
 // One Adam step (beta 0.9 / 0.999, eps 1e-8, bias-corrected at `step` >= 1) on the master weights;
 // refreshes the BF16 copy and clears the gradient.
 cudaError_t mlp_adam(float* d_master, __nv_bfloat16* d_w, float* d_grad, float* d_m, float* d_v, float lr, uint32_t step,

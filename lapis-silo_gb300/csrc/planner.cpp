@@ -218,7 +218,8 @@ void PlannerNet::reserve(uint32_t n) {
    if (!d_master_) {
       for (float** p : {&d_master_, &d_m_, &d_v_, &d_grad_})
          cuda_check(cudaMalloc(p, MLP_NPARAM * sizeof(float)), "cudaMalloc (planner)");
-      cuda_check(cudaMalloc(&d_loss_, sizeof(float)), "cudaMalloc (planner)");
+      cuda_check(cudaMalloc(&d_loss_, sizeof(float) + sizeof(int)), "cudaMalloc (planner)");
+      d_err_ = reinterpret_cast<int*>(d_loss_ + 1);
       cuda_check(cudaMalloc(&d_w_, MLP_NPARAM * sizeof(__nv_bfloat16)), "cudaMalloc (planner)");
    }
    if (n > cap_) {
@@ -259,8 +260,8 @@ void PlannerNet::gradient(const float* X, const float* T, uint32_t n, float* gra
    cuda_check(cudaMemcpyAsync(d_X_, X, static_cast<size_t>(n) * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
    cuda_check(cudaMemcpyAsync(d_T_, T, static_cast<size_t>(n) * MLP_OUT * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
    cuda_check(cudaMemsetAsync(d_grad_, 0, MLP_NPARAM * sizeof(float), s), "memset");
-   cuda_check(cudaMemsetAsync(d_loss_, 0, sizeof(float), s), "memset");
-   cuda_check(mlp_gradient(d_w_, d_X_, d_T_, n, d_grad_, d_loss_, s), "mlp gradient");
+   cuda_check(cudaMemsetAsync(d_loss_, 0, sizeof(float) + sizeof(int), s), "memset");
+   cuda_check(mlp_gradient(d_w_, d_X_, d_T_, n, d_grad_, d_loss_, d_err_, withhold, s), "mlp gradient");
    if (Y) cuda_check(mlp_forward(d_w_, d_X_, n, d_Y_, s), "mlp forward");
    if (grad) cuda_check(cudaMemcpyAsync(grad, d_grad_, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
    if (loss) cuda_check(cudaMemcpyAsync(loss, d_loss_, sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
@@ -279,11 +280,9 @@ void PlannerNet::gradient_at(const float* w, const float* X, const float* T, uin
 
 void PlannerNet::finish(cudaStream_t s, const char* what) {
    int e = 0;
-   cuda_check(mlp_read_error(&e, s), "planner error flag");
+   cuda_check(cudaMemcpyAsync(&e, d_err_, sizeof(int), cudaMemcpyDeviceToHost, s), "planner error flag");
    cuda_check(cudaStreamSynchronize(s), what);
-   if (e == 0) return;
-   mlp_clear_error();
-   throw std::runtime_error("planner network: a bounded wait of the gradient kernel gave up");
+   if (e != 0) throw std::runtime_error("planner network: a bounded wait of the gradient kernel gave up");
 }
 
 float PlannerNet::train(const std::vector<float>& X, const std::vector<float>& T, uint32_t n, uint32_t epochs,
@@ -307,12 +306,12 @@ float PlannerNet::train(const std::vector<float>& X, const std::vector<float>& T
       }
       cuda_check(cudaMemcpyAsync(d_X_, Xs.data(), Xs.size() * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
       cuda_check(cudaMemcpyAsync(d_T_, Ts.data(), Ts.size() * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-      cuda_check(cudaMemsetAsync(d_loss_, 0, sizeof(float), s), "memset");
+      cuda_check(cudaMemsetAsync(d_loss_, 0, sizeof(float) + sizeof(int), s), "memset");
       uint32_t nb = 0;
       for (uint32_t b = 0; b + batch <= n || (b < n && nb == 0); b += batch, ++nb) {
          const uint32_t m = std::min(batch, n - b);
          cuda_check(mlp_gradient(d_w_, d_X_ + static_cast<size_t>(b) * MLP_IN, d_T_ + static_cast<size_t>(b) * MLP_OUT, m,
-                                 d_grad_, d_loss_, s),
+                                 d_grad_, d_loss_, d_err_, false, s),
                     "mlp gradient");
          cuda_check(mlp_adam(d_master_, d_w_, d_grad_, d_m_, d_v_, lr, ++step_, s), "adam");
       }

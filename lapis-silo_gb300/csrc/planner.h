@@ -89,6 +89,7 @@ class PlannerNet {
    // Selectivity and cost (either may be null) of n raw feature rows.
    void predict_rows(const float* X, uint32_t n, const MlpScale& scale, double* sel, double* cost);
    uint32_t capacity() const { return cap_; }  // samples its buffers hold
+   bool withhold = false;   // testing: see mlp_gradient
    // Pinned host rows (n x MLP_IN) to fill before predict_staged, which runs the network on them
    // and returns its outputs (n x MLP_OUT, pinned, valid until the next call).
    float* staged_input(uint32_t n);
@@ -106,6 +107,7 @@ class PlannerNet {
    float* d_v_ = nullptr;
    float* d_grad_ = nullptr;
    float* d_loss_ = nullptr;
+   int* d_err_ = nullptr;   // the gradient kernel's error word, behind *d_loss_ and cleared with it
    __nv_bfloat16* d_w_ = nullptr;
    float* d_X_ = nullptr;
    float* d_T_ = nullptr;

@@ -69,3 +69,36 @@ def test_two_handles_in_two_threads(kind, rounds):
         d.close()
     assert not errors, errors
     assert got == [w * rounds for w in want]
+
+
+def test_gradient_failure_stays_with_its_call():
+    """One handle's bounded wait for the network's products gives up on every call (they are withheld, nothing is in
+    flight); calls of another handle at the same time succeed, and every failed call reports it."""
+    devs = [partition(s)[1] for s in (3, 4)]
+    rng = np.random.default_rng(5)
+    w = rng.normal(0, 0.1, R.MLP_NPARAM).astype(np.float32)
+    x, t = rng.normal(size=(300, 24)).astype(np.float32), rng.normal(size=(300, 2)).astype(np.float32)
+    want = devs[1].mlp_gradient(w, x, t)
+    devs[0].test_withhold_copies(False, gradient=True)
+    outcome = [[], []]
+
+    def run(i):
+        for _ in range(200):
+            try:
+                g, loss, y = devs[i].mlp_gradient(w, x, t)
+                outcome[i].append(np.allclose(g, want[0], rtol=1e-4, atol=1e-6) and abs(loss - want[1]) <= 1e-5 * want[1])
+            except R.RhyError as e:
+                outcome[i].append("gave up" in str(e) and "failed")
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in (0, 1)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    devs[0].test_withhold_copies(False)
+    after = devs[0].mlp_gradient(w, x, t)
+    for d in devs:
+        d.close()
+    assert outcome[0] == ["failed"] * 200
+    assert outcome[1] == [True] * 200
+    assert np.allclose(after[0], want[0], rtol=1e-4, atol=1e-6)
