@@ -62,7 +62,7 @@ constexpr uint16_t fuse_flags(FuseOp op, uint32_t planes) { return static_cast<u
 // Comparators of the date predicate (reference: src/rhydb/query_engine/filter/operators/selection.h:40-72).
 enum CmpCode : uint32_t { CMP_EQ = 0, CMP_NE = 1, CMP_LT = 2, CMP_LE = 3, CMP_GT = 4, CMP_GE = 5 };
 
-struct Instr {
+struct alignas(16) Instr {  // the kernels read it as one 16-byte load
    uint8_t op;
    uint8_t col;
    uint16_t flags;
@@ -70,7 +70,7 @@ struct Instr {
    uint32_t b;
    uint32_t c;
 };
-static_assert(sizeof(Instr) == 16, "instruction layout");
+static_assert(sizeof(Instr) == 16 && alignof(Instr) == 16, "instruction layout");
 
 // How a leaf's rows reach their target: set in the top tile, removed from it, or counted in the planes.
 enum RowOp : int { A_OR = 0, A_ANDNOT = 1, A_ADD = 2 };
