@@ -74,7 +74,8 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, uint32_t lane) 
 // Final pass for positions [blockIdx.x * MUT_SEG, +MUT_SEG) of one query (blockDim.x == MUT_SEG):
 //   ref(p) = |F| - #(start > p) - #(end <= p) - missing(p) - sum_s counts[s][p]
 //   counts[local_ref[p]][p] += ref(p)
-// All arithmetic is modulo 2^32 like the reference's uint32 vectors; the result is exact. Returns the
+// The scratch may have been written by a kernel that this one's launch overlaps (mutations.cu), so it is read
+// from L2. All arithmetic is modulo 2^32 like the reference's uint32 vectors; the result is exact. Returns the
 // position's local reference and its final count (0, 0 past the genome). Bound by latency: a load of the
 // symbols' mask, the counts of the symbols in it (a position has a few of the column's 16 or 28, and reading
 // the others' zeros took most of the pass's bytes) and a block scan of three prefix sums; 32 registers let
@@ -84,7 +85,7 @@ struct FinalCount {
    uint32_t count;
 };
 __device__ __forceinline__ FinalCount final_position_counts(const DevSeqCol* cs, uint32_t total, uint32_t* counts,
-                                                            const uint32_t* __restrict__ scratch) {
+                                                            const uint32_t* scratch) {
    __shared__ uint32_t wtot[3][MUT_SEG / 32], pre[4];
    const uint32_t L = cs->L, nseg = mut_nseg(L);
    const uint32_t* seg_s = scratch + 3 * (L + 1);
@@ -96,21 +97,21 @@ __device__ __forceinline__ FinalCount final_position_counts(const DevSeqCol* cs,
    uint32_t s = 0, e = 0, n = 0, rest = 0;
    FinalCount f{0, 0};
    if (in) {
-      s = scratch[p];
-      e = scratch[L + 1 + p];
-      n = scratch[2 * (L + 1) + p];
+      s = __ldcg(scratch + p);
+      e = __ldcg(scratch + L + 1 + p);
+      n = __ldcg(scratch + 2 * (L + 1) + p);
       f.local = cs->local_ref[p];
       rest = sum_counts(cs->syms[p], [&](uint32_t k) { return counts[static_cast<size_t>(k) * L + p]; });
    }
    if (warp == MUT_SEG / 32 - 1) {  // the segments before this one, and every start
       uint32_t ps = 0, pe = 0, pn = 0, ts = 0;
       for (uint32_t k = lane; k < nseg; k += 32) {
-         const uint32_t x = seg_s[k];
+         const uint32_t x = __ldcg(seg_s + k);
          ts += x;
          if (k < blockIdx.x) {
             ps += x;
-            pe += seg_e[k];
-            pn += seg_n[k];
+            pe += __ldcg(seg_e + k);
+            pn += __ldcg(seg_n + k);
          }
       }
       ps = __reduce_add_sync(0xFFFFFFFFu, ps);
