@@ -712,6 +712,11 @@ void Engine::launch_program(const Instr* code, const Instr* inline_code, const P
    const uint32_t* aux = nullptr;
    if (p.n_literals > 0 && literals == nullptr) throw std::invalid_argument("the program reads caller row sets");
    const size_t set_words = static_cast<size_t>(nchunks()) * CHUNK_WORDS;
+   if (!p.aux.empty()) {  // a graph would copy from the staging below on every replay, whatever a later call put there
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      cuda_check(cudaStreamIsCapturing(stream, &capture), "profile upload");
+      if (capture != cudaStreamCaptureStatusNone) throw CudaError("profile upload: not permitted while the stream is capturing");
+   }
    if (!p.aux.empty() || p.n_literals > 0)
       grow_device(d_aux_, aux_cap_, (p.aux.size() + p.n_literals) * set_words);
    if (!p.aux.empty()) {  // MutationProfile row sets, before the program that reads them

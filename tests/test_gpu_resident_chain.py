@@ -47,3 +47,28 @@ def test_passes_in_a_row_equal_passes_alone(column):
     for i, k in enumerate(order):
         assert torch.equal(tables[i], alone[k]), (i, int(k))
     dev.close()
+
+
+@pytest.mark.parametrize("mode", ["global", "relaxed"])
+def test_prepared_profile_is_not_recorded(mode):
+    """A single call's profile is copied from host memory that the next call reuses: recording it is refused in every
+    capture mode. Programs without one are recorded and replayed."""
+    torch = pytest.importorskip("torch")
+    t = R.Table.generate(70000, seed=3, genome_len=3000, pool_sites=300)
+    dev = R.Device(t, 0)
+    stream = torch.cuda.Stream()
+    ptr = ctypes.c_void_p(stream.cuda_stream)
+    profile = "MutProfileMutations(main,4,241:T,1059:T,2100:G,2500:A)"
+    assert dev.count(profile) > 0  # the buffers exist
+    dev.plain_prepare([profile, "HasMut(main,9)"], [1, 1], [0, 0])
+    with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=stream, capture_error_mode=mode):
+        with pytest.raises(R.RhyError):
+            dev.plain_launch(0, ptr)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        dev.plain_launch(1, ptr)
+    graph.replay()
+    torch.cuda.synchronize()
+    dev.plain_launch(0, ptr)  # and outside a capture
+    torch.cuda.synchronize()
+    dev.close()
