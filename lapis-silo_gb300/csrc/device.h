@@ -228,7 +228,7 @@ struct CallEnd {
 
 // ---- launchers (kernels.cu) ----
 // With inline_code (host memory, at most INLINE_CODE instructions) the program travels with the launch.
-// tile_bits: 4096, 8192, 16384, 32768 or 65536. stack_tiles: Program::tiles. n_leaves: container
+// tile_bits: 2048 (programs of more than 400 tiles), 4096, 8192, 16384, 32768 or 65536. stack_tiles: Program::tiles. n_leaves: container
 // leaves | coverage leaves << 16. d_trace (trace mode, optional): nchunks * (CHUNK_ROWS / tile_bits)
 // tiles x ncode x 2 u32 (cycles, result popcount per executed instruction), zeroed by the caller.
 cudaError_t launch_filter(const DevTable* d_table, uint32_t nchunks, const Instr* d_code, uint32_t ncode,
