@@ -726,11 +726,14 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
    auto spec = std::make_shared<ProfileSpec>();
    spec->col = ci;
    spec->distance = static_cast<uint32_t>(e.n);
+   uint32_t differs[32];  // the symbols that differ from each symbol as the profile's
+   for (uint32_t x = 0; x < A.count; ++x) differs[x] = profile_mask(A, static_cast<uint8_t>(x));
+   const uint8_t *own = profile.data(), *local = col.local_ref.data();
    for (uint32_t p = 0; p < L && spec->delta.size() <= PROFILE_DELTA_MAX; ++p) {
-      if (profile[p] == col.local_ref[p]) continue;
-      const uint32_t m = profile_mask(A, profile[p]), h = profile_mask(A, col.local_ref[p]);
+      if (own[p] == local[p]) continue;
+      const uint32_t m = differs[own[p]], h = differs[local[p]];
       if (m == h) continue;
-      const int32_t d = static_cast<int32_t>((m >> col.local_ref[p]) & 1u) - static_cast<int32_t>((h >> col.local_ref[p]) & 1u);
+      const int32_t d = static_cast<int32_t>((m >> local[p]) & 1u) - static_cast<int32_t>((h >> local[p]) & 1u);
       spec->delta.push_back({p, m, h, d});
       spec->base_delta += d;
    }
@@ -738,15 +741,17 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
    if (!spec->use_delta) {
       spec->delta.clear();
       spec->mask.resize(L);
-      spec->diff.assign(L + 1, 0);
-      uint32_t loc = 0;
+      spec->diff.resize(L + 1);
+      uint32_t *mask = spec->mask.data(), *diff = spec->diff.data(), d = 0, loc = 0;
+      const uint32_t missing = A.missing;
       for (uint32_t p = 0; p < L; ++p) {
-         const uint32_t m = profile_mask(A, profile[p]);
-         const uint32_t lbit = (m >> col.local_ref[p]) & 1u;
-         spec->mask[p] = m | lbit << 31;
-         spec->diff[p + 1] = spec->diff[p] + ((m >> A.missing) & 1u) - lbit;
+         const uint32_t m = differs[own[p]], lbit = (m >> local[p]) & 1u;
+         mask[p] = m | lbit << 31;
+         diff[p] = d;
+         d += ((m >> missing) & 1u) - lbit;
          loc += lbit;
       }
+      diff[L] = d;
       spec->base = loc;
    }
    auto o = mk(OpT::PROFILE);
