@@ -648,7 +648,7 @@ uint64_t Engine::instr_bytes(const Instr& in) const {
          uint64_t bounds = 0;  // rows whose covered region misses the position
          for (const CovExc& x : c.cov_exc) bounds += x.start > in.a || x.end <= in.a;
          return bounds * sizeof(CovBound) +
-                static_cast<uint64_t>(c.nblk_off[(blk + 1) * nv] - c.nblk_off[blk * nv]) * sizeof(NRunEntry);
+                static_cast<uint64_t>(c.nblk_off[(blk + 1) * nv] - c.nblk_off[blk * nv]) * sizeof(uint32_t);  // DevSeqCol::nblk
       }
       case OP_PUSH_DATE: {  // the planes of its two comparisons (see DevDateCol), and the null dates where they match
          const DevDateCol& c = view_.date[in.col];
