@@ -864,7 +864,7 @@ size_t mutations_batch_mask_bytes(uint32_t nq, uint32_t nchunks) {
    return static_cast<size_t>(nqc) * nchunks * CHUNK_ROWS * 4;
 }
 
-void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
+void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks, uint32_t sms,
                             const uint32_t* d_filters, uint32_t nq, const unsigned long long* d_fcounts,
                             const uint32_t* d_slot_query, const EvItem* d_ev, uint32_t n_ev, const CtrUnit* d_units,
                             uint32_t n_units, uint16_t* d_masks, uint32_t* d_counts, uint32_t* d_scratch,
@@ -883,7 +883,7 @@ void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, 
    if ((parts & BMUT_PART_CTR) && n_units > 0) {
       const dim3 grid((n_units + BT / 32 - 1) / (BT / 32), (ngroups + PASS_GROUPS - 1) / PASS_GROUPS);
       mut_ctr_batch_kernel<<<grid, BT, 0, s>>>(d_table, col, d_units, n_units, d_masks, d_lists, nq, d_counts);
-      const uint32_t per_chunk = std::max(1u, 152u / nchunks);  // one CTA per SM
+      const uint32_t per_chunk = std::max(1u, sms / nchunks);  // one CTA per SM
       mut_ctr_narrow_kernel<<<dim3(nchunks * per_chunk, nq > 16 ? 2 : 1), NARROW_T, NARROW_SMEM, s>>>(
          d_table, col, d_filters, d_masks, d_lists, nq, per_chunk, d_counts);
       if (col_host.n_run_ctrs > 0) {  // a container per warp at least

@@ -202,8 +202,8 @@ struct DevProfile {
 };
 // aux[k] (nchunks * CHUNK_WORDS words each) = the rows of profiles[k] within its distance. any_delta:
 // some profile is counted from its differences; max_L: the longest genome among the columns of the
-// others (0: none).
-void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile* d_profiles, uint32_t n,
+// others (0: none); sms: the device's SMs.
+void launch_profiles(const DevTable* d_table, uint32_t nchunks, uint32_t sms, const DevProfile* d_profiles, uint32_t n,
                      bool any_delta, uint32_t max_L, uint32_t* d_aux, void* stream);
 // home[row] = the row's number of differences from the local reference (null rows: unused): base plus
 // its row-index entries' terms (as DevProfile's; Engine's upload).
@@ -279,7 +279,7 @@ enum : uint32_t { MUT_PART_SPARSE = 8 };
 // MUT_PART_CLEAR: the counts, the scratch and *d_err_clear (if not null) start from zero here, else the caller
 // has cleared them.
 enum : uint32_t { MUT_PART_CLEAR = 16 };
-void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
+void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks, uint32_t sms,
                       const uint32_t* d_filter, const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
                       void* stream, uint32_t parts = MUT_PART_ALL | MUT_PART_SPARSE, uint64_t sparse_max = 0,
                       int* d_err_clear = nullptr);
@@ -338,7 +338,7 @@ constexpr uint32_t CTR_UNIT_ELEMENTS = 4096;
 // also makes every slot's Mutations output rows (RowsOut).
 enum : uint32_t { BMUT_PART_SPARSE = 16 };
 size_t mutations_batch_mask_bytes(uint32_t nq, uint32_t nchunks);
-void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
+void launch_mutations_batch(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks, uint32_t sms,
                             const uint32_t* d_filters, uint32_t nq, const unsigned long long* d_fcounts,
                             const uint32_t* d_slot_query, const EvItem* d_ev, uint32_t n_ev, const CtrUnit* d_units,
                             uint32_t n_units, uint16_t* d_masks, uint32_t* d_counts, uint32_t* d_scratch,
@@ -362,9 +362,9 @@ void launch_first_k(const uint32_t* d_tiles, uint32_t nq, uint32_t nchunks, cons
                     const uint32_t* d_out_off, uint32_t* d_ids, uint32_t* d_n, void* stream);
 
 // Events per CTA of the batched coverage pass: at most EV_PER_CTA, and down to a quarter of it while that
-// leaves fewer than EV_CTAS CTAs (six on each of 152 SMs). The covered regions' boundaries, of which hardly
+// leaves fewer than EV_CTAS_PER_SM CTAs for each SM. The covered regions' boundaries, of which hardly
 // two share a position, cost a flush of the counters each: a 32nd (with 8192 of them in a CTA it ran for
 // 250 us, longer than all others together at 500,000 rows).
-constexpr uint32_t EV_PER_CTA = 8192, EV_CTAS = 912;
+constexpr uint32_t EV_PER_CTA = 8192, EV_CTAS_PER_SM = 6;
 
 }  // namespace rhygpu

@@ -397,6 +397,9 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
    cuda_check(cudaSetDevice(device), "cudaSetDevice");
    try {
       cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+      int sms = 0;
+      cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "SM count");
+      sms_ = static_cast<uint32_t>(std::max(sms, 1));
       filter_setup();
       profile_setup();
       aggregate_setup();
@@ -437,10 +440,7 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
             d.ou = upload(P.ou);
             d.nau = static_cast<uint32_t>(P.au.size());
             // one wave of the container pass's CTAs
-            int sms = 0;
-            cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "SM count");
-            const std::vector<StreamRange> ranges =
-               pass_ranges(s, P, nchunks, static_cast<uint32_t>(std::max(sms, 1)) * RING_CTAS_PER_SM);
+            const std::vector<StreamRange> ranges = pass_ranges(s, P, nchunks, sms_ * RING_CTAS_PER_SM);
             d.ranges = upload(ranges);
             d.nranges = static_cast<uint32_t>(ranges.size());
          }
@@ -478,7 +478,7 @@ Engine::Engine(const TableImage& t, int device) : table_(t), device_(device), pl
          auto split = [&](uint32_t list, uint32_t block, uint32_t b, uint32_t e, uint32_t per) {
             for (uint32_t x = b; x < e; x += per) items.push_back({list, block, x, std::min(e, x + per)});
          };
-         const uint64_t share = (s.mstart.size() + s.mend.size()) / EV_CTAS;
+         const uint64_t share = (s.mstart.size() + s.mend.size()) / (EV_CTAS_PER_SM * sms_);
          const uint32_t per = static_cast<uint32_t>(std::min<uint64_t>(EV_PER_CTA, std::max<uint64_t>(share, EV_PER_CTA / 4)));
          for (uint32_t b = 0; b < s.nblocks; ++b) {
             split(EV_MSTART, b, s.mstart_off[b], s.mstart_off[b + 1], per);
@@ -733,7 +733,7 @@ void Engine::launch_program(const Instr* code, const Instr* inline_code, const P
       cuda_check(cudaMemcpyAsync(d_prof_, h_prof_, n * sizeof(DevProfile), cudaMemcpyHostToDevice, stream), "H2D");
       if (nw) cuda_check(cudaMemcpyAsync(d_prof_data_, h_prof_data_, nw * 4, cudaMemcpyHostToDevice, stream), "H2D");
       cuda_check(cudaEventRecord(prof_ev_, stream), "event");
-      launch_profiles(d_table_, nchunks(), d_prof_, n, profile_any_delta(p.aux), profile_max_L(p.aux), d_aux_, stream);
+      launch_profiles(d_table_, nchunks(), sms_, d_prof_, n, profile_any_delta(p.aux), profile_max_L(p.aux), d_aux_, stream);
       cuda_check(cudaGetLastError(), "profile launch");
    }
    for (uint32_t k = 0; k < p.n_literals; ++k)  // the caller's row sets after the profiles' (the caller owns them)
@@ -753,7 +753,7 @@ void Engine::launch_program(const Instr* code, const Instr* inline_code, const P
 void Engine::launch_mutations(int column, const uint32_t* filter, const unsigned long long* count, uint32_t* counts,
                               uint32_t* scratch, cudaStream_t stream, uint32_t parts) {
    const DevSeqCol& c = view_.seq[column];
-   rhygpu::launch_mutations(d_table_, c, static_cast<uint32_t>(column), nchunks(), filter, count, counts, scratch, d_err, stream, parts, sparse_rows_plain);
+   rhygpu::launch_mutations(d_table_, c, static_cast<uint32_t>(column), nchunks(), sms_, filter, count, counts, scratch, d_err, stream, parts, sparse_rows_plain);
    cuda_check(cudaGetLastError(), "mutations kernel launch");
 }
 
@@ -1041,9 +1041,7 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    // not end their class alone. A launch of few items (nine for each of three CTAs per SM) ends with the items that
    // begin last, so there every tile of the longest programs comes first: 40 queries over 2M rows, 112 -> 81 us;
    // 40 trees of up to 64 leaves, 804 -> 549 us. At 256 queries (7,936 items) either order takes 0.41 ms.
-   int props = 0;
-   cuda_check(cudaDeviceGetAttribute(&props, cudaDevAttrMultiProcessorCount, device_), "attribute");
-   const bool few_items = nitems < 27 * static_cast<size_t>(props);
+   const bool few_items = nitems < 27 * static_cast<size_t>(sms_);
    b.fgroups.clear();
    size_t k = 0;
    for (auto& [w, qv] : by_w) {
@@ -1077,7 +1075,7 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    if (sch.ctas_per_sm) per_sm = std::min(per_sm, sch.ctas_per_sm);
    b.stack_bytes = static_cast<uint32_t>(stack);
    b.scratch_bytes = static_cast<uint32_t>(scratch);
-   b.grid = static_cast<uint32_t>(props) * per_sm;
+   b.grid = sms_ * per_sm;
    std::memcpy(b.h_slot_query, slot_query.data(), slot_query.size() * sizeof(uint32_t));
    b.n_queries = n;
    b.n_slots = nslots;
@@ -1118,7 +1116,7 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
       cuda_check(cudaMemsetAsync(b.d_err, 0, sizeof(int), s), "memset");
    }
    if ((parts & 1) && b.n_aux) {
-      launch_profiles(d_table_, nchunks(), b.d_prof, b.n_aux, b.profile_any_delta, b.profile_max_L, b.d_aux, s);
+      launch_profiles(d_table_, nchunks(), sms_, b.d_prof, b.n_aux, b.profile_any_delta, b.profile_max_L, b.d_aux, s);
       cuda_check(cudaGetLastError(), "profile launch");
    }
    if (parts & 1) {
@@ -1133,7 +1131,7 @@ void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool cop
    }
    const size_t words = static_cast<size_t>(nchunks()) * CHUNK_WORDS;
    for (const auto& g : b.groups) {
-      launch_mutations_batch(d_table_, view_.seq[g.column], static_cast<uint32_t>(g.column), nchunks(),
+      launch_mutations_batch(d_table_, view_.seq[g.column], static_cast<uint32_t>(g.column), nchunks(), sms_,
                              b.d_tiles + static_cast<size_t>(g.slot_begin) * words, g.n, b.d_counts,
                              b.d_slot_query + g.slot_begin, d_ev_[g.column], n_ev_[g.column], d_cu_[g.column],
                              n_cu_[g.column], b.d_masks, b.d_mcounts + g.counts_off, b.d_mscratch + g.scratch_off,

@@ -146,6 +146,7 @@ class Engine {
    Engine& operator=(const Engine&) = delete;
 
    const TableImage& table() const { return table_; }
+   uint32_t sms() const { return sms_; }
    int device() const { return device_; }
    uint32_t nchunks() const { return table_.nchunks(); }
    const DevTable* d_table() const { return d_table_; }
@@ -308,12 +309,10 @@ class Engine {
    void learned_compile(const std::vector<std::string>& exprs, uint32_t threads, LearnedPlans& lp);
    std::vector<BatchQuery> learned_lower(LearnedPlans& lp, const std::vector<uint32_t>& idx, uint32_t threads);
 
-   const EvItem* d_ev(int column) const { return d_ev_[column]; }
-   uint32_t n_ev(int column) const { return n_ev_[column]; }
    uint64_t mutation_payload_bytes(int column) const;
    // Algorithmic bytes of one filter program over the whole table: the payloads and descriptors of
    // the containers its index-scan leaves read, the coverage exceptions and the missing intervals of
-   // the position's block its coverage leaves read, the bit planes its date leaves read, the dense
+   // the position's block its coverage leaves read, the planes its date leaves read, the dense
    // row sets of null and aux leaves, and the output (a dense row set, or one count). Intermediates
    // between operators are not counted.
    uint64_t program_bytes(const Program& p, bool writes_rows) const;
@@ -342,6 +341,7 @@ class Engine {
    void upload_dates(const DateColumnImage& dc, uint32_t nchunks, DevDateCol& out);
 
    const TableImage& table_;
+   uint32_t sms_ = 1;         // the device's SMs
    int device_;
    cudaStream_t stream_ = nullptr;
    DevTable view_{};

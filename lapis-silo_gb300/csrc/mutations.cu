@@ -552,7 +552,7 @@ void mutations_setup() {
       throw std::runtime_error(std::string("shared memory of the Mutations container pass: ") + cudaGetErrorString(e));
 }
 
-void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks,
+void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32_t col, uint32_t nchunks, uint32_t sms,
                       const uint32_t* d_filter,
                       const unsigned long long* d_filter_count, uint32_t* d_counts, uint32_t* d_scratch, int* d_err,
                       void* stream, uint32_t parts, uint64_t sparse_max, int* d_err_clear) {
@@ -576,7 +576,7 @@ void launch_mutations(const DevTable* d_table, const DevSeqCol& col_host, uint32
    const bool clear = parts & MUT_PART_CLEAR;
    if (clear) {
       const uint32_t words = col_host.nsym * col_host.L;
-      launch(mut_clear_kernel, std::min((words + 1023) / 1024, 152u), 1024, 0, false, d_counts, words, d_scratch,
+      launch(mut_clear_kernel, std::min((words + 1023) / 1024, sms), 1024, 0, false, d_counts, words, d_scratch,
              static_cast<uint32_t>(mut_scratch_words(col_host.L)), d_err_clear);
    }
    const bool coverage = parts & MUT_PART_COV;

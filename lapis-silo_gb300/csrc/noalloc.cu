@@ -76,7 +76,7 @@ void mutations_noalloc(Engine& engine, uint32_t column, const uint32_t* d_filter
    cudaStream_t s = engine.stream_for(stream);
    // the pass accumulates into both buffers, so they start from zero; the status starts clear
    cudaGetLastError();
-   launch_mutations(engine.d_table(), col, column, engine.nchunks(), d_filter, d_filter_count, d_counts, scratch, d_status, s,
+   launch_mutations(engine.d_table(), col, column, engine.nchunks(), engine.sms(), d_filter, d_filter_count, d_counts, scratch, d_status, s,
                     MUT_PART_ALL | MUT_PART_SPARSE | MUT_PART_CLEAR, engine.sparse_rows_plain, d_status);
    cuda_check(cudaGetLastError(), "mutations (no allocation) launch");
 }

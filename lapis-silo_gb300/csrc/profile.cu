@@ -502,7 +502,7 @@ void profile_setup() {
    allow(reinterpret_cast<const void*>(profile_staged_kernel), staged_smem(STAGE_MAX_L));
 }
 
-void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile* d_profiles, uint32_t n,
+void launch_profiles(const DevTable* d_table, uint32_t nchunks, uint32_t sms, const DevProfile* d_profiles, uint32_t n,
                      bool any_delta, uint32_t max_L, uint32_t* d_aux, void* stream) {
    const uint32_t words = nchunks * CHUNK_WORDS;
    const cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -510,7 +510,7 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
       for (uint32_t k = 0; k < n; k += 65535) {  // grid.y is at most 65535
          const uint32_t m = n - k < 65535 ? n - k : 65535;
          // CTAs per chunk: eight (the most that every device takes) while they find an SM each, else four
-         const uint32_t parts = static_cast<uint64_t>(nchunks) * m * 8 <= 152 ? 8 : 4;
+         const uint32_t parts = static_cast<uint64_t>(nchunks) * m * 8 <= sms ? 8 : 4;
          cudaLaunchAttribute attr{};
          attr.id = cudaLaunchAttributeClusterDimension;
          attr.val.clusterDim.x = parts;
@@ -527,9 +527,7 @@ void launch_profiles(const DevTable* d_table, uint32_t nchunks, const DevProfile
    }
    if (max_L == 0) return;
    const size_t smem = staged_smem(max_L);
-   int dev = 0, sms = 0;
-   const bool staged = max_L <= STAGE_MAX_L && cudaGetDevice(&dev) == cudaSuccess &&
-                       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+   const bool staged = max_L <= STAGE_MAX_L;
    for (uint32_t k = 0; k < n; k += 65535) {  // grid.y is at most 65535
       const uint32_t m = n - k < 65535 ? n - k : 65535;
       if (staged)
