@@ -279,7 +279,6 @@ int rhy_seq_column_checksum(const RhyTable* t, uint32_t column, uint64_t* out) {
       vec(c.nrow_end);
       vec(c.nblk);
       vec(c.nblk_off);
-      vec(c.exc_toff);
       vec(c.nblk_toff);
       vec(c.mstart);
       vec(c.mend);

@@ -105,10 +105,8 @@ struct SeqColumnImage {
    std::vector<uint32_t> nrow_start, nrow_end;
    std::vector<NRunEntry> nblk;        // bucketed by (block, chunk), sorted by row
    std::vector<uint32_t> nblk_off;     // nblocks * nchunks + 1
-   // Row-range offsets for tiles: exc_toff[v * TOFF_N + k] is the index of the first coverage
-   // exception of chunk v with row >= k * TOFF_ROWS, nblk_toff[(b * nchunks + v) * TOFF_N + k] the
-   // same inside bucket (b, v) of nblk.
-   std::vector<uint32_t> exc_toff;
+   // Row-range offsets for tiles: nblk_toff[(b * nchunks + v) * TOFF_N + k] is the index of the first
+   // interval of bucket (b, v) of nblk with row >= k * TOFF_ROWS.
    std::vector<uint32_t> nblk_toff;
    uint32_t nblocks = 0;
    // Mutations pass: the same missing intervals as start and end events, packed as
