@@ -63,6 +63,7 @@ constexpr uint32_t RING_CTAS_PER_SM = 3;
 // with sixteen in a bitset. The Mutations passes read the arrays.
 constexpr uint32_t DENSE_MIN = 1024;
 constexpr uint32_t SPAN_RUNS = 8;
+constexpr uint8_t CT_SPANS = 3;  // in fctrs: a run container of at least DENSE_MIN rows in at most SPAN_RUNS runs
 struct DenseJob {
    uint32_t src, dst;    // u16 offsets of the container and of its bitset in the arena
    uint32_t rows, runs;  // an array's rows or a run container's runs, the other 0

@@ -247,9 +247,14 @@ void Engine::upload_containers(const ContainerSet& cs, uint16_t*& payload, CtrDe
    constexpr uint64_t BITSET = CHUNK_ROWS / 16;  // u16 per bitset
    uint64_t end = (cs.payload.size() + 8 + 7) & ~7ull;
    for (CtrDesc& d : f) {
-      const bool array = d.type == CT_ARRAY, runs = d.type == CT_RUN && d.nruns > SPAN_RUNS;
-      if (!(array || runs) || d.card_m1 + 1u < DENSE_MIN || end + BITSET > 0xFFFFFFFFull) continue;
-      jobs.push_back({d.payload, static_cast<uint32_t>(end), array ? d.card_m1 + 1u : 0u, runs ? d.nruns : 0u});
+      if (d.type == CT_BITSET || d.card_m1 + 1u < DENSE_MIN) continue;
+      if (d.type == CT_RUN && d.nruns <= SPAN_RUNS) {
+         d.type = CT_SPANS;
+         continue;
+      }
+      if (end + BITSET > 0xFFFFFFFFull) continue;
+      const bool array = d.type == CT_ARRAY;
+      jobs.push_back({d.payload, static_cast<uint32_t>(end), array ? d.card_m1 + 1u : 0u, array ? 0u : d.nruns});
       d.type = CT_BITSET;
       d.payload = static_cast<uint32_t>(end);
       end += BITSET;
