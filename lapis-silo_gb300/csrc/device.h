@@ -61,8 +61,6 @@ constexpr uint32_t RING_CTAS_PER_SM = 3;
 // chunk of the nucleotide column (32 MB). Up to SPAN_RUNS runs stay as they are, each combined as masks: NOf of
 // 12 sites at 400,000 rows, 128 of them in one launch, 0.39 ms with eight runs a container and 0.33 ms
 // with sixteen in a bitset. The Mutations passes read the arrays.
-constexpr uint32_t DENSE_MIN = 1024;
-constexpr uint32_t SPAN_RUNS = 8;
 constexpr uint8_t CT_SPANS = 3;  // in fctrs: a run container of at least DENSE_MIN rows in at most SPAN_RUNS runs
 struct DenseJob {
    uint32_t src, dst;    // u16 offsets of the container and of its bitset in the arena

@@ -91,8 +91,8 @@ struct ProfileSpec {
    int col = 0;
    uint32_t distance = 0;
    uint32_t base = 0;
-   // Where the profile differs from the local reference at no more than PROFILE_DELTA_MAX positions, the
-   // differences only: the device starts from every row's distance to the local reference (a stored
+   // Where the profile differs from the local reference at no more than PROFILE_DELTA_MAX positions (and their
+   // containers hold few enough rows), the differences only: the device starts from every row's distance to the local reference (a stored
    // index), adds base_delta and corrects the rows listed at these positions. Else (delta unused):
    bool use_delta = false;
    int32_t base_delta = 0;  // sum of d_ref over the positions

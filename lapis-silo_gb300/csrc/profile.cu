@@ -12,11 +12,12 @@
 // reference's. Null rows match no SymbolInSet, so they count no difference. A row is in the set
 // when its count is at most the distance.
 //
-// A profile that differs from the local reference at few positions (a sequence of the data set, a list of
-// mutations) needs none of that: profile_delta_kernel starts from every row's stored distance to the
+// A profile that differs from the local reference at few positions (a list of mutations, a sequence of which
+// little is missing) needs none of that: profile_delta_kernel starts from every row's stored distance to the
 // local reference and corrects the rows in the lists of those positions. A row's sequence with 20
-// substitutions differs at 300 to 1,350 positions, most of them in its missing runs: 72 us for 1,344
-// positions at 2M rows, 133 us for the whole row index.
+// substitutions differs at 300 to 1,350 positions, most of them in its missing runs (every missing position
+// is a difference: 7% of the genome are too many): 50 us for 1,344 positions at 2M rows, 133 us for the
+// whole row index.
 //
 // The row index otherwise. One warp per 32 consecutive rows. Their entries are one contiguous range of
 // the row index, read in windows of 256: each lane loads 8 consecutive entries as two 16-byte loads

@@ -78,8 +78,9 @@ enum RowOp : int { A_OR = 0, A_ANDNOT = 1, A_ADD = 2 };
 // A_ANDNOT), bits 11..15 the planes of A_ADD (as in a leaf's flags).
 constexpr uint16_t GROUP_PUSH = 4;
 
-// A MutationProfile that differs from the local reference at up to this many positions is counted from
-// the differences (profile_delta_kernel), any other from the whole row index (see profile.cu): 50 us for
+// A MutationProfile that differs from the local reference at up to this many positions, held by few enough rows
+// (profile_by_differences), is counted from the differences (profile_delta_kernel), any other from the whole
+// row index (see profile.cu): 50 us for
 // 1,344 positions at 2M rows, against 133 us for the row index; a row's sum in the kernel has 16 bits.
 constexpr uint32_t PROFILE_DELTA_MAX = 2048;
 

@@ -571,6 +571,12 @@ void finish_seq_column(SeqColumnImage& col, const std::vector<ChunkRows>& chunks
          col.nblk_toff[bv * TOFF_N + k] = i;
       }
    }
+   col.delta_rows.assign(L, 0);
+   for (const CtrDesc& d : col.vertical.ctrs) {
+      const uint32_t card = d.card_m1 + 1u;
+      const bool bitset = d.type == CT_BITSET || (card >= DENSE_MIN && (d.type == CT_ARRAY || d.nruns > SPAN_RUNS));
+      col.delta_rows[d.key] += bitset ? CHUNK_ROWS / 2 : d.type == CT_RUN ? std::min(card, 64u * d.nruns) : card;
+   }
    build_mutation_events(col, chunks, chunk_sizes);
    build_row_index(col, chunk_sizes, threads);
 }

@@ -48,6 +48,11 @@ struct CtrDesc {
 };
 static_assert(sizeof(CtrDesc) == 16, "descriptor layout");
 
+// Containers of at least DENSE_MIN rows have a form of their own for filters, run containers of more than SPAN_RUNS
+// runs another than those of fewer (see DevSeqCol::fctrs).
+constexpr uint32_t DENSE_MIN = 1024;
+constexpr uint32_t SPAN_RUNS = 8;
+
 struct CovExc {  // a row whose covered region is not [0, L)
    uint32_t row;   // row within chunk
    uint32_t start;
@@ -125,6 +130,9 @@ struct SeqColumnImage {
    std::vector<uint32_t> hrow_off;     // nchunks * CHUNK_ROWS + 1
    std::vector<uint32_t> hent;
    uint32_t flipped_positions = 0;
+   // What a position costs the MutationProfile pass over differences, in rows of its containers (L): a bitset, also
+   // one made for filters, counts as half a chunk, a run as 64 rows at most.
+   std::vector<uint32_t> delta_rows;
 };
 constexpr uint32_t ROW_COV_START = 28, ROW_COV_END = 29, ROW_MISS_START = 30, ROW_MISS_END = 31;
 

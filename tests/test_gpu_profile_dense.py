@@ -1,0 +1,47 @@
+"""A MutationProfile off the local reference at many positions that large parts of the rows differ at: the pass is chosen
+by what the positions' containers hold, not by their number alone."""
+import ctypes as C
+import time
+
+import numpy as np
+import pytest
+
+import rhydb_gpu as R
+from rawtable import oracle_for
+
+pytestmark = pytest.mark.gpu
+
+
+def test_many_dense_differences_take_the_row_index():
+    n, L, sites = 65536, 3000, 1000
+    rng = np.random.default_rng(5)
+    share = np.array([0.3, 0.1, 0.03, 0.45])
+    key = np.sort(np.concatenate([np.flatnonzero(rng.random(n) < share[p % 4]).astype(np.int64) * L + p for p in range(sites)]))
+    pos, length = (key % L).astype(np.uint32), np.ones(len(key), np.uint32)
+    char, off, null = np.full(len(key), ord("C"), np.uint8), np.zeros(n + 1, np.uint64), np.zeros(n, np.uint8)
+    np.cumsum(np.bincount(key // L, minlength=n), out=off[1:])
+    ptr = lambda a, t: a.ctypes.data_as(C.POINTER(t))
+    col = (R.RawSeqColumn * 1)()
+    col[0].name, col[0].kind, col[0].reference, col[0].L = b"main", 0, b"A" * L, L
+    col[0].is_null, col[0].row_off, col[0].run_pos = ptr(null, C.c_uint8), ptr(off, C.c_uint64), ptr(pos, C.c_uint32)
+    col[0].run_len, col[0].run_char = ptr(length, C.c_uint32), ptr(char, C.c_char)
+    raw = R.RawTable()
+    raw.n_rows, raw.n_seq, raw.seq = n, 1, C.cast(col, C.POINTER(R.RawSeqColumn))
+    t = R.Table.from_raw(raw)
+    dev, orc = R.Device(t, 0), oracle_for(t, raw)
+
+    def call(differences, distance):
+        q = f"MutProfileMutations(main,{distance},{','.join(f'{p + 1}:C' for p in range(differences))})"
+        got, best = dev.count(q), 1.0
+        for _ in range(15):
+            t0 = time.perf_counter()
+            dev.count(q)
+            best = min(best, time.perf_counter() - t0)
+        return q, got, best
+
+    few, dense, index = call(1, 0), call(sites, 780), call(2100, 1880)  # the last is past the limit of the differences
+    for q, got, _ in (few, dense):
+        assert got == orc.count(q)
+    assert 0 < dense[1] < n
+    assert dense[2] < 1.3 * index[2], (few[2], dense[2], index[2])
+    dev.close()
