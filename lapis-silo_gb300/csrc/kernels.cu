@@ -14,8 +14,8 @@
 // matter are applied together, a warp each (group_leaves); arrays and run containers of DENSE_MIN rows and
 // more are stored a second time as bitsets (or read as the few runs they are), combined word by word by
 // the threads that own the words.
-// Measured (2M rows, 4,096 trees of 1-64 leaves, one launch): 34.5 ms with a tile per leaf, 20.9 ms
-// this way; the benchmark's 2,048 queries 3.28 -> 3.05 ms. 128 threads per CTA instead of 256: 25.6
+// Measured (2M rows, 4,096 trees of 1-64 leaves, one launch): 34.5 ms with a tile per leaf, 20.8 ms
+// this way; the benchmark's 2,048 queries 3.28 -> 2.83 ms. 128 threads per CTA instead of 256: 25.6
 // and 2.9 ms (the trees wait on latency, and more warps hide it).
 // All arithmetic is integer; results are bit-exact with the CPU operators.
 #include <cuda_runtime.h>

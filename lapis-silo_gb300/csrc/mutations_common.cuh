@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, uint32_t lane) 
 // position's local reference and its final count (0, 0 past the genome). Bound by latency: a load of the
 // symbols' mask, the counts of the symbols in it (a position has a few of the column's 16 or 28, and reading
 // the others' zeros took most of the pass's bytes) and a block scan of three prefix sums; 32 registers let
-// two CTAs share an SM.
+// two CTAs share an SM (the batched form, which makes rows too, spills 18 bytes a thread for it).
 struct FinalCount {
    uint32_t local;
    uint32_t count;

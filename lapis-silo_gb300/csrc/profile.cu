@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(ST, 1) profile_staged_kernel(const DevTable* _
 // positions (a missing run of the profile is hundreds of positions with a few containers each), and the
 // home distances (4 bytes per row). 1,344 positions at 2M rows: 50 us; 72 with a CTA per 16,384 rows, which
 // read the rows of a chunk's containers for a quarter of them (of the 50: staging and the sums' exchange 14,
-// containers 14, bitsets 17, rows not covered 5; bitsets by whole warps alone made it 90).
+// containers 14, bitsets 17, rows not covered 5; bitsets by whole warps alone made it 90). 1,024 threads leave 64
+// registers each, and 60 bytes of a thread are spilled.
 // Runs of up to a whole chunk (a table sorted by lineage holds them at the lineages' positions) add once per
 // SPAN rows they cover, and the spans are added to their rows at the end: a count of the rows within 30 of the
 // reference over 400,000 rows sorted by lineage takes 0.11 ms, and took 0.65 with an atomic per row of one lane.
