@@ -333,7 +333,8 @@ typedef struct {
 /* Split form of rhy_batch for callers that reuse one batch shape: prepare plans and stages the
  * batch (allocates on first use or growth), launch enqueues it without synchronising,
  * capture/replay record it once into a CUDA graph and replay it, results copies the outputs of the
- * last completed launch (the caller synchronises the stream first). */
+ * last completed launch (the caller synchronises the stream first). The first launch after a prepare copies the
+ * batch in (copy_in, or a captured graph); one without it is refused (RHY_INVALID_ARGUMENT). */
 int rhy_batch_prepare(RhyDevice* d, const char* const* exprs, const int* actions, const uint32_t* columns, uint32_t n,
                       uint32_t tile_bits, uint32_t plan_threads);
 int rhy_batch_launch(RhyDevice* d, void* stream, int copy_in, int copy_out);
@@ -344,14 +345,15 @@ int rhy_batch_info(RhyDevice* d, RhyBatchInfo* out);
 
 /* Schedule of the batched filter launches (results never depend on it): the widest tile of a class
  * (bits), the stack budget that narrows a class's tile (KiB), persistent CTAs per SM (0 = as many
- * as fit) and the work-item order (0 = tile-major, 1 = every tile of one query in turn). */
+ * as fit) and the work-item order (0 = tile-major, 1 = every tile of one query in turn, as small batches take
+ * in any case, their longest programs first). */
 typedef struct {
    uint32_t max_tile_bits, stack_kb, ctas_per_sm, query_major;
 } RhyBatchSchedule;
 /* Sets the schedule when `set` is not NULL, then reports the one in force when `get` is not NULL. */
 int rhy_batch_schedule(RhyDevice* d, const RhyBatchSchedule* set, RhyBatchSchedule* get);
 /* Autotuner: plans the batch, times its filter launches under every candidate schedule (tile widths
- * 16 / 32 / 64 Kbit x stack budgets 24 / 40 / 64 KiB x all or two CTAs per SM x both item orders;
+ * 16 / 32 / 64 Kbit x stack budgets 24 / 48 / 80 KiB x all or two CTAs per SM x both item orders;
  * `reps` timed runs each, median, CUDA events on `stream`), keeps the fastest in force and returns
  * the candidates fastest first in tried[0 .. min(cap, *n_tried)) with their milliseconds. */
 int rhy_batch_autotune(RhyDevice* d, const char* const* exprs, const int* actions, const uint32_t* columns, uint32_t n,

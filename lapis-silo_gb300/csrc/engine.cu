@@ -1094,12 +1094,16 @@ void Engine::batch_prepare(BatchState& b, const std::vector<BatchQuery>& qs, uin
    b.counts_words = counts_words;
    b.scratch_words = scratch_words;
    b.mask_bytes = mask_bytes;
+   b.uploaded = false;
 }
 
 void Engine::batch_enqueue(BatchState& b, cudaStream_t s, bool copy_in, bool copy_out, uint32_t parts) {
    s = stream_for(s);
    if (b.n_queries == 0) return;
+   // the device still holds the batch before this one, whose items do not fit these buffers
+   if (!copy_in && !b.uploaded) throw std::invalid_argument("the prepared batch has not been copied to the device");
    if (copy_in) {
+      b.uploaded = true;
       cuda_check(cudaMemcpyAsync(b.d_code, b.h_code, b.n_code * sizeof(Instr), cudaMemcpyHostToDevice, s), "H2D");
       cuda_check(cudaMemcpyAsync(b.d_q, b.h_q, b.n_queries * sizeof(QueryDesc), cudaMemcpyHostToDevice, s), "H2D");
       cuda_check(cudaMemcpyAsync(b.d_items, b.h_items, static_cast<size_t>(b.n_items) * sizeof(WorkItem),

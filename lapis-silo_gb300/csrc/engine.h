@@ -68,6 +68,7 @@ struct BatchState {
       uint32_t item_off, n_items, tile_bits, tiles;
    };
    std::vector<FilterGroup> fgroups;
+   bool uploaded = false;  // the prepared programs have been copied to the device (or a graph that does it recorded)
    uint32_t stack_bytes = 0, scratch_bytes = 0;
    struct ColGroup {
       int column;

@@ -38,3 +38,20 @@ def test_small_batch_starts_its_longest_programs_first():
     own = filter_time(qs[::-1])
     dev.close()
     assert own < 1.08 * ordered, (own, ordered)
+
+
+def test_a_prepared_batch_is_copied_in_before_it_is_launched():
+    torch = pytest.importorskip("torch")
+    t = R.Table.generate(3000, seed=5, genome_len=1500, pool_sites=400)
+    dev = R.Device(t, 0)
+    for queries in (t.queries(3, seed=1), t.queries(60, seed=2)):
+        want = [dev.count(q) for q in queries]
+        dev.batch_prepare(queries)
+        for call in (lambda: dev.batch_launch(None, False, True), lambda: dev.batch_launch_parts(1)):
+            with pytest.raises(R.RhyError):
+                call()
+        dev.batch_launch(None, True, True)
+        dev.batch_launch_parts(1)
+        torch.cuda.synchronize()
+        assert dev.batch_results(False)[0].tolist() == want
+    dev.close()
