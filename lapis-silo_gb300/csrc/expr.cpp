@@ -2,8 +2,10 @@
 #include "expr.h"
 
 #include <algorithm>
+#include <array>
 #include <cctype>
 #include <cmath>
+#include <cstring>
 #include <cstdio>
 #include <map>
 #include <string_view>
@@ -719,11 +721,17 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
          throw IllegalQuery("querySequence length " + std::to_string(e.value.size()) +
                             " does not match the reference sequence length " + std::to_string(L));
       profile.resize(L);
+      const char* text = e.value.data();
+      int8_t any = 0;  // negative if a character is no symbol
       for (uint32_t p = 0; p < L; ++p) {
-         const int sy = A.sym(e.value[p]);
-         if (sy < 0) throw IllegalQuery(std::string("Invalid symbol '") + e.value[p] + "' in querySequence for MutationProfile");
+         const int8_t sy = A.char_to_sym[static_cast<uint8_t>(text[p])];
          profile[p] = static_cast<uint8_t>(sy);
+         any = static_cast<int8_t>(any | sy);
       }
+      if (any < 0)
+         for (uint32_t p = 0; p < L; ++p)
+            if (A.sym(text[p]) < 0)
+               throw IllegalQuery(std::string("Invalid symbol '") + text[p] + "' in querySequence for MutationProfile");
    } else {
       profile = col.global_ref;
       for (uint32_t m : e.muts) {
@@ -741,7 +749,10 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
    const uint8_t *own = profile.data(), *local = col.local_ref.data();
    uint64_t rows = 0;  // that the differences pass goes through
    for (uint32_t p = 0; p < L && spec->delta.size() <= PROFILE_DELTA_MAX; ++p) {
-      if (own[p] == local[p]) continue;
+      if (own[p] == local[p]) {
+         while (p + 9 <= L && std::memcmp(own + p + 1, local + p + 1, 8) == 0) p += 8;  // most are equal
+         continue;
+      }
       const uint32_t m = differs[own[p]], h = differs[local[p]];
       if (m == h) continue;
       const int32_t d = static_cast<int32_t>((m >> local[p]) & 1u) - static_cast<int32_t>((h >> local[p]) & 1u);
@@ -754,14 +765,22 @@ OpPtr compile_profile(const TableImage& t, const Expr& e) {
       spec->delta.clear();
       spec->mask.resize(L);
       spec->diff.resize(L + 1);
+      struct Term {
+         uint32_t mask, step;  // of a position with this symbol in the profile and that one in the local reference
+      };
+      std::array<Term, 32 * 32> term;
+      for (uint32_t x = 0; x < A.count; ++x)
+         for (uint32_t y = 0; y < A.count; ++y) {
+            const uint32_t m = differs[x], lbit = (m >> y) & 1u;
+            term[32 * x + y] = {m | lbit << 31, ((m >> A.missing) & 1u) - lbit};
+         }
       uint32_t *mask = spec->mask.data(), *diff = spec->diff.data(), d = 0, loc = 0;
-      const uint32_t missing = A.missing;
       for (uint32_t p = 0; p < L; ++p) {
-         const uint32_t m = differs[own[p]], lbit = (m >> local[p]) & 1u;
-         mask[p] = m | lbit << 31;
+         const Term x = term[32u * own[p] + local[p]];
+         mask[p] = x.mask;
          diff[p] = d;
-         d += ((m >> missing) & 1u) - lbit;
-         loc += lbit;
+         d += x.step;
+         loc += x.mask >> 31;
       }
       diff[L] = d;
       spec->base = loc;
